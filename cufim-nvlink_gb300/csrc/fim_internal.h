@@ -137,10 +137,6 @@ void set_last_error(const char *msg);
 cudaError_t launch_metric(const int32_t *tslots, const int64_t *cidx, const double *xyz, const double *evec,
                           int64_t nT, const double *fib, const double *cf, const double *ct, int64_t e0, int64_t e1,
                           double *cgeo, float *cgf, uint4 *crec, unsigned long long *bad, cudaStream_t stream);
-// Stages the six edge vectors of every tet (18 doubles, SoA) for the
-// metric kernel.
-cudaError_t launch_edge_vectors(const int32_t *tslots, const double *xyz, int64_t nT, double *evec,
-                                cudaStream_t stream);
 // The persistent cooperative solve is compiled once per batch shape
 // (fim_solve_s*.cu: vertices x corners a block stages per batch); the
 // autotuner picks the shape, the grid and the tet-prefix warps per problem.
@@ -167,6 +163,47 @@ cudaError_t launch_mark_seeds(const FimDev &d, uint8_t *is_seed, cudaStream_t st
 // Resets every vertex with a time >= tmin to INF / far, lists every other
 // reached vertex as narrow, then re-seeds the stimuli (two launches).
 cudaError_t launch_warm_reset(const FimDev &d, double tmin, cudaStream_t stream);
+
+// ---- mesh staging (fim_stage.cu) ----
+// Results of the staging kernels that the host reads: first offenders
+// (all bits set: none), largest squared edge length (bit pattern), vertex
+// copies too large for lists_kernel.
+struct StageCtl {
+  unsigned long long bad_id;    // flat index of the first tet id outside [0, nV)
+  unsigned long long bad_tet;   // first tet with a repeated vertex (all ids in range)
+  unsigned long long bad_xyz;   // first non-finite coordinate
+  unsigned long long max_edge2;
+  int32_t n_big;
+  int32_t pad;
+};
+// Buffers of launch_stage_lists: cptr, crec, cidx, nptr are results; cnt,
+// big_list, mark [nL], keys [4 nT], scratch [16 nT] and tile_sum [nL] are
+// overwritten (scratch and nptr feed launch_stage_compact).
+struct StageLists {
+  const int32_t *cslots;  // [4 nT] vertex copies of every tet in slot order
+  int64_t *cptr, *nptr;   // [nL + 1]
+  uint4 *crec;
+  int64_t *cidx;          // [4 nT]
+  int32_t *cnt, *big_list, *mark, *scratch;
+  uint32_t *keys;
+  long long *tile_sum;
+};
+// Checks tets (device, 4 nT ids) and xyz (device) into ctl; first (or
+// nullptr) receives every vertex's first appearance.
+cudaError_t launch_stage_check(int64_t nV, int64_t nT, const int64_t *tets, const double *xyz, uint32_t *first,
+                               StageCtl *ctl, cudaStream_t st);
+// Slots of a mesh with one submesh, from checked tets.
+cudaError_t launch_stage_slots(int64_t nT, const int64_t *tets, const uint32_t *first, int32_t *slots,
+                               cudaStream_t st);
+// Corners of every vertex copy (increasing tet index) and the lengths of the
+// neighbourhoods; launch_stage_compact then writes the neighbourhoods.
+cudaError_t launch_stage_lists(int64_t nL, int64_t nT, const StageLists &x, StageCtl *ctl, cudaStream_t st);
+cudaError_t launch_stage_compact(int64_t nL, const StageLists &x, int32_t *nbr, cudaStream_t st);
+cudaError_t launch_stage_in_tet(int64_t nV, const int64_t *cptr, uint8_t *in_tet, cudaStream_t st);
+// Edge vectors of every tet (18 doubles, SoA; evec nullptr: not stored) and
+// the largest squared edge length.
+cudaError_t launch_edge_vectors(const int32_t *tslots, const double *xyz, int64_t nT, double *evec, StageCtl *ctl,
+                                cudaStream_t stream);
 
 // ---- learned warm start (fim_mlp.cu) ----
 // Network 7 (padded to kMlpIn) -> kMlpH -> kMlpH -> kMlpH -> 1.  Parameter

@@ -14,8 +14,6 @@
 //    types.cpp:227-257), written straight into the four corner records of
 //    the tet in the relabelled order the local solver reads
 //    (gray-code tables, cuda_fim.h:41-48), plus the three edge lengths.
-//  * edge_vector_kernel -- the six edge vectors of every tet, staged once
-//    per mesh for the metric kernel;
 //  * the support check and warm-start reset of a warm-started solve.
 // The solve itself, fim_solve_kernel (fim_solve.cuh, compiled once per
 // batch shape by fim_solve_s*.cu), is one persistent cooperative launch for
@@ -85,7 +83,7 @@ __global__ void fim_metric_kernel(const int32_t *__restrict__ tslots, const int6
     const double M5 = vf*ff + vs*(1. - ff);
     double g[6];
     if (evec) {
-      // the edge vectors of the mesh, staged once (edge_vector_kernel)
+      // the edge vectors of the mesh, staged once (edge_vector_kernel, fim_stage.cu)
 #pragma unroll
       for (int k = 0; k < 6; ++k) {
         const double ex = evec[(3 * k + 0) * nT + e], ey = evec[(3 * k + 1) * nT + e], ez = evec[(3 * k + 2) * nT + e];
@@ -154,36 +152,8 @@ __global__ void fim_metric_kernel(const int32_t *__restrict__ tslots, const int6
   }
 }
 
-// Edge vectors of every tet in the metric kernel's edge order, x_a - x_b
-// for (a, b) = (0,1) (0,2) (1,2) (0,3) (1,3) (2,3) of its slots
-// (load_edge, types.h:210-216): they depend on the mesh only, so
-// fim_set_mesh stages them once and every conduction upload saves their 18
-// FP64 subtractions per tet.  Layout: evec[(3 k + axis) nT + e].
-__global__ void edge_vector_kernel(const int32_t *__restrict__ tslots, const double *__restrict__ xyz, int64_t nT,
-                                   double *__restrict__ evec)
-{
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nT; e += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t v0 = tslots[4 * e + 0], v1 = tslots[4 * e + 1];
-    const int32_t v2 = tslots[4 * e + 2], v3 = tslots[4 * e + 3];
-    const int32_t va[6] = {v0, v0, v1, v0, v1, v2};
-    const int32_t vb[6] = {v1, v2, v2, v3, v3, v3};
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-#pragma unroll
-      for (int a = 0; a < 3; ++a) evec[(3 * k + a) * nT + e] = xyz[3 * (int64_t)va[k] + a] - xyz[3 * (int64_t)vb[k] + a];
-  }
-}
-
 // ---------------------------------------------------------------------------
 // launch wrappers
-
-cudaError_t launch_edge_vectors(const int32_t *tslots, const double *xyz, int64_t nT, double *evec,
-                                cudaStream_t stream)
-{
-  if (nT <= 0) return cudaSuccess;
-  edge_vector_kernel<<<152 * 8, 256, 0, stream>>>(tslots, xyz, nT, evec);
-  return cudaGetLastError();
-}
 
 cudaError_t launch_metric(const int32_t *tslots, const int64_t *cidx, const double *xyz, const double *evec,
                           int64_t nT, const double *fib, const double *cf, const double *ct, int64_t e0, int64_t e1,

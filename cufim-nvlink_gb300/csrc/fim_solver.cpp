@@ -3,7 +3,8 @@
 //
 // Host staging replaces the reference's CudaSolverFIM constructor
 // (src/eikonal/cuda_fim.cu:1218-1501): instead of per-submesh blobs with
-// in-blob pointers it builds flat device arrays --
+// in-blob pointers it builds flat device arrays (on the device, fim_stage.cu;
+// only the vertex copies of a mesh with submesh tags are numbered here) --
 //   * the reference's vertex order inside every tet (extract_submeshes2,
 //     src/core/types.cpp:306-570: first appearance inside the tet's submesh,
 //     then ascending local id), which the local solver's result depends on;
@@ -25,10 +26,6 @@
 #include <unordered_map>
 #include <vector>
 
-#ifdef _OPENMP
-#include <omp.h>
-#endif
-
 using namespace fimgb;
 
 namespace {
@@ -41,6 +38,7 @@ template <class T>
 struct DevBuf {
   T *p = nullptr;
   size_t n = 0;
+  bool own = true;  // false: part of another allocation (view)
   cudaError_t alloc(size_t count)
   {
     release();
@@ -56,14 +54,31 @@ struct DevBuf {
     if (p && n >= (count ? count : 1)) return cudaSuccess;
     return alloc(count);
   }
+  void view(void *q, size_t count)
+  {
+    release();
+    p = static_cast<T *>(q);
+    n = count;
+    own = false;
+  }
   void release()
   {
-    if (p) cudaFree(p);
+    if (p && own) cudaFree(p);
     p = nullptr;
     n = 0;
+    own = true;
   }
   ~DevBuf() { release(); }
 };
+
+// A kept buffer serves a new mesh of up to its size, but not one that would
+// leave more than half of it (and more than 64 MB) unused.
+template <class T>
+cudaError_t reserve_near(DevBuf<T> &b, size_t count)
+{
+  if (b.p && b.n >= count && (b.n <= 2 * count || b.n * sizeof(T) <= (size_t(64) << 20))) return cudaSuccess;
+  return b.alloc(count);
+}
 
 }  // namespace
 
@@ -106,7 +121,7 @@ struct fim_solver {
   int64_t nV = 0, nT = 0, nC = 0, nL = 0;
   int32_t n_submeshes = 1;
   std::vector<int64_t> h_sub_ptr;   // first vertex copy of every submesh (+ end)
-  std::vector<int64_t> h_cptr;      // corner offsets of the vertex copies (host copy)
+  std::vector<int64_t> h_cptr;      // corner offsets of the vertex copies (submesh sweeps: read back on first use)
   DevBuf<int32_t> blk_ptr;          // submesh sweeps: copies owned by each block
   int blk_grid = -1;                // grid blk_ptr was computed for
   std::vector<uint8_t> in_tet;
@@ -118,6 +133,12 @@ struct fim_solver {
   DevBuf<uint8_t> st_out;
   bool have_mesh = false, have_cond = false, have_stim = false, solved = false;
   double front_width = 0.0;
+  // one allocation holds every per-mesh array below except nbr, evec and the
+  // seeds (their DevBufs are views into it): 35 allocations of a 135k-vertex
+  // slab cost 1.6 ms, one of the same size 0.08 ms, and 1.2 against 0.2 ms
+  // to free
+  DevBuf<unsigned char> arena;
+  DevBuf<unsigned char> stage;      // the caller's mesh while it is checked and staged
   DevBuf<double> xyz;
   DevBuf<int32_t> tslots;
   DevBuf<double> evec;  // edge vectors of every tet (metric kernel); empty when they did not fit
@@ -285,15 +306,15 @@ extern "C" int fim_set_stream(fim_solver *s, void *stream)
 
 namespace {
 
-// The reference's slot order of every tet: aggregates numbered by first
-// appearance of their tag, local vertex ids by first appearance while
-// walking the aggregate's tets in increasing tet index with each tet's
-// global ids ascending, then each tet's local ids ascending
-// (types.cpp:63-67, 331-345, 383-398, 473).
+// The reference's slot order of every tet of a mesh with submesh tags:
+// aggregates numbered by first appearance of their tag, local vertex ids by
+// first appearance while walking the aggregate's tets in increasing tet
+// index with each tet's global ids ascending, then each tet's local ids
+// ascending (types.cpp:63-67, 331-345, 383-398, 473).  (One submesh:
+// launch_stage_slots.)
 //   slots  -- 4*nT mesh vertex ids in slot order (for the metric)
 //   cslots -- 4*nT vertex-copy ids in slot order (for the corners)
-//   gptr/gcopy -- copies of every mesh vertex (left empty with one submesh,
-//                 where copy == vertex)
+//   gptr/gcopy -- copies of every mesh vertex
 struct Staging {
   std::vector<int32_t> slots, cslots;
   int64_t n_copies = 0;
@@ -303,21 +324,26 @@ struct Staging {
   std::vector<int32_t> gcopy;
 };
 
-void reference_slots(int64_t nV, int64_t nT, const int64_t *tets, const int32_t *atags, Staging &S)
+// Aggregate of every tet; returns the number of aggregates.
+int32_t aggregates(int64_t nT, const int32_t *atags, std::vector<int32_t> &agg)
+{
+  std::unordered_map<int32_t, int32_t> t2a;
+  int32_t nagg = 0;
+  agg.resize(nT);
+  for (int64_t e = 0; e < nT; ++e) {
+    if (e && atags[e] == atags[e - 1]) { agg[e] = agg[e - 1]; continue; }
+    auto it = t2a.find(atags[e]);
+    if (it == t2a.end()) it = t2a.emplace(atags[e], nagg++).first;
+    agg[e] = it->second;
+  }
+  return nagg;
+}
+
+void reference_slots(int64_t nV, int64_t nT, const int64_t *tets, const std::vector<int32_t> &agg, int32_t nagg,
+                     Staging &S)
 {
   S.slots.resize(4 * nT);
   S.cslots.resize(4 * nT);
-  std::vector<int32_t> agg(nT, 0);
-  int32_t nagg = 1;
-  if (atags) {
-    std::unordered_map<int32_t, int32_t> t2a;
-    nagg = 0;
-    for (int64_t e = 0; e < nT; ++e) {
-      auto it = t2a.find(atags[e]);
-      if (it == t2a.end()) it = t2a.emplace(atags[e], nagg++).first;
-      agg[e] = it->second;
-    }
-  }
   S.n_submeshes = nagg;
   // tets grouped by aggregate, increasing index inside each group
   std::vector<int64_t> aptr(nagg + 1, 0), order(nT);
@@ -329,7 +355,7 @@ void reference_slots(int64_t nV, int64_t nT, const int64_t *tets, const int32_t 
   }
   std::vector<int64_t> rank(nV, -1);  // first-appearance rank inside the current aggregate
   std::vector<int32_t> touched;
-  std::vector<int32_t> copy_owner;    // copy -> mesh vertex (several submeshes)
+  std::vector<int32_t> copy_owner;    // copy -> mesh vertex
   int64_t base = 0;
   for (int32_t a = 0; a < nagg; ++a) {
     int64_t next = 0;
@@ -341,12 +367,12 @@ void reference_slots(int64_t nV, int64_t nT, const int64_t *tets, const int32_t 
         if (rank[g[j]] < 0) {
           rank[g[j]] = next++;
           touched.push_back((int32_t)g[j]);
-          if (nagg > 1) copy_owner.push_back((int32_t)g[j]);
+          copy_owner.push_back((int32_t)g[j]);
         }
       std::sort(g, g + 4, [&](int64_t x, int64_t y) { return rank[x] < rank[y]; });
       for (int j = 0; j < 4; ++j) {
         S.slots[4 * e + j] = (int32_t)g[j];
-        S.cslots[4 * e + j] = nagg > 1 ? (int32_t)(base + rank[g[j]]) : (int32_t)g[j];
+        S.cslots[4 * e + j] = (int32_t)(base + rank[g[j]]);
       }
     }
     S.sub_ptr.push_back(base);
@@ -354,18 +380,27 @@ void reference_slots(int64_t nV, int64_t nT, const int64_t *tets, const int32_t 
     for (int32_t v : touched) rank[v] = -1;
     touched.clear();
   }
-  if (nagg > 1) {
-    S.n_copies = base;
-    S.gptr.assign(nV + 1, 0);
-    for (int32_t g : copy_owner) S.gptr[g + 1]++;
-    for (int64_t v = 0; v < nV; ++v) S.gptr[v + 1] += S.gptr[v];
-    S.gcopy.resize(base);
-    std::vector<int64_t> fill(S.gptr.begin(), S.gptr.end() - 1);
-    for (int64_t c = 0; c < base; ++c) S.gcopy[fill[copy_owner[c]]++] = (int32_t)c;
-  } else {
-    S.n_copies = nV;
-  }
+  S.n_copies = base;
+  S.gptr.assign(nV + 1, 0);
+  for (int32_t g : copy_owner) S.gptr[g + 1]++;
+  for (int64_t v = 0; v < nV; ++v) S.gptr[v + 1] += S.gptr[v];
+  S.gcopy.resize(base);
+  std::vector<int64_t> fill(S.gptr.begin(), S.gptr.end() - 1);
+  for (int64_t c = 0; c < base; ++c) S.gcopy[fill[copy_owner[c]]++] = (int32_t)c;
 }
+
+// Sub-allocator of an arena: 256-byte aligned parts; a first pass without a
+// base adds up the size.
+struct Parts {
+  unsigned char *base = nullptr;
+  size_t off = 0;
+  template <class T>
+  void add(DevBuf<T> &b, size_t count)
+  {
+    if (base) b.view(base + off, count);
+    off += (count * sizeof(T) + 255) & ~size_t(255);
+  }
+};
 
 }  // namespace
 
@@ -378,95 +413,53 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
   if (nV >= (int64_t)INT32_MAX || 4 * nT >= (int64_t)INT32_MAX)
     return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: mesh too large (%lld vertices, %lld tets)",
                    (long long)nV, (long long)nT);
-  for (int64_t i = 0; i < 4 * nT; ++i)
-    if (tets[i] < 0 || tets[i] >= nV)
-      return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: tet %lld has vertex %lld outside [0,%lld)",
-                     (long long)(i / 4), (long long)tets[i], (long long)nV);
-  for (int64_t e = 0; e < nT; ++e) {
-    const int64_t *t = tets + 4 * e;
-    if (t[0] == t[1] || t[0] == t[2] || t[0] == t[3] || t[1] == t[2] || t[1] == t[3] || t[2] == t[3])
-      return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: tet %lld repeats a vertex", (long long)e);
-  }
-  for (int64_t i = 0; i < 3 * nV; ++i)
-    if (!std::isfinite(xyz[i]))
-      return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: coordinate %lld is not finite", (long long)i);
-
-  Staging S;
-  reference_slots(nV, nT, tets, atags, S);
-  const std::vector<int32_t> &slots = S.slots;
-  const int64_t nL = S.n_copies;
-
-  // corners of every vertex copy, in increasing tet index
-  const int64_t nC = 4 * nT;
-  std::vector<int64_t> cptr(nL + 1, 0), cidx(nC);
-  for (int64_t i = 0; i < nC; ++i) cptr[S.cslots[i] + 1]++;
-  for (int64_t v = 0; v < nL; ++v) cptr[v + 1] += cptr[v];
-  std::vector<int4> cids(nC);
-  {
-    std::vector<int64_t> fill(cptr.begin(), cptr.end() - 1);
-    for (int64_t e = 0; e < nT; ++e)
-      for (int t = 0; t < 4; ++t) {
-        const int32_t v = S.cslots[4 * e + t];
-        const int64_t c = fill[v]++;
-        cidx[4 * e + t] = c;
-        cids[c] = make_int4(S.cslots[4 * e + ((t + 1) & 3)], S.cslots[4 * e + ((t + 2) & 3)],
-                            S.cslots[4 * e + ((t + 3) & 3)], (int)e);
-      }
-  }
-  // neighbourhood of every copy incl. itself (sorted), two passes
-  std::vector<int64_t> nptr(nL + 1, 0);
-  std::vector<int32_t> nbr;
-  {
-    std::vector<int32_t> cnt(nL);
-#pragma omp parallel
-    {
-      std::vector<int32_t> buf;
-#pragma omp for schedule(static)
-      for (int64_t v = 0; v < nL; ++v) {
-        buf.clear();
-        buf.push_back((int32_t)v);
-        for (int64_t c = cptr[v]; c < cptr[v + 1]; ++c) {
-          buf.push_back(cids[c].x); buf.push_back(cids[c].y); buf.push_back(cids[c].z);
-        }
-        std::sort(buf.begin(), buf.end());
-        cnt[v] = (int32_t)(std::unique(buf.begin(), buf.end()) - buf.begin());
-      }
-    }
-    for (int64_t v = 0; v < nL; ++v) nptr[v + 1] = nptr[v] + cnt[v];
-    nbr.resize(nptr[nL]);
-#pragma omp parallel
-    {
-      std::vector<int32_t> buf;
-#pragma omp for schedule(static)
-      for (int64_t v = 0; v < nL; ++v) {
-        buf.clear();
-        buf.push_back((int32_t)v);
-        for (int64_t c = cptr[v]; c < cptr[v + 1]; ++c) {
-          buf.push_back(cids[c].x); buf.push_back(cids[c].y); buf.push_back(cids[c].z);
-        }
-        std::sort(buf.begin(), buf.end());
-        const int64_t m = std::unique(buf.begin(), buf.end()) - buf.begin();
-        std::copy(buf.begin(), buf.begin() + m, nbr.begin() + nptr[v]);
-      }
-    }
-  }
-  // vertices in at least one tet (seeds elsewhere are dropped, as the
-  // reference seeds through submeshes only)
-  std::vector<uint8_t> in_tet(nV, 0);
-  for (int64_t i = 0; i < nC; ++i) in_tet[slots[i]] = 1;
-  // reference front width: 1.01 * longest edge / 0.6 (compute_dwf, cuda_fim.h:1536-1576)
-  double maxe2 = 0.0;
-  for (int64_t e = 0; e < nT; ++e)
-    for (int i = 0; i < 4; ++i)
-      for (int j = i + 1; j < 4; ++j) {
-        const int64_t a = tets[4 * e + i], b = tets[4 * e + j];
-        const double dx = xyz[3 * b] - xyz[3 * a], dy = xyz[3 * b + 1] - xyz[3 * a + 1], dz = xyz[3 * b + 2] - xyz[3 * a + 2];
-        const double l = dx * dx + dy * dy + dz * dz;
-        if (l > maxe2) maxe2 = l;
-      }
-  s->front_width = 1.01 * std::sqrt(maxe2) / 0.6;
 
   CUDA_TRY(s, cudaSetDevice(s->device));
+  cudaStream_t st = s->stream;
+  // The caller's arrays go to the device and are checked there, while the
+  // previous mesh is still in place (a rejected mesh leaves it usable).
+  // Staging buffer: control words, tets, coordinates, first appearances.
+  const auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
+  const size_t o_tets = up(sizeof(StageCtl)), o_xyz = o_tets + up(sizeof(int64_t) * 4 * nT);
+  const size_t o_first = o_xyz + up(sizeof(double) * 3 * nV);
+  CUDA_TRY(s, s->stage.reserve(o_first + up(sizeof(uint32_t) * nV)));
+  struct StageGuard {  // a large staging buffer is given back when the call ends
+    DevBuf<unsigned char> &b;
+    ~StageGuard() { if (b.n > (size_t(64) << 20)) b.release(); }
+  } guard{s->stage};
+  StageCtl *d_ctl = reinterpret_cast<StageCtl *>(s->stage.p);
+  int64_t *d_tets = reinterpret_cast<int64_t *>(s->stage.p + o_tets);
+  double *d_xyz = reinterpret_cast<double *>(s->stage.p + o_xyz);
+  uint32_t *d_first = reinterpret_cast<uint32_t *>(s->stage.p + o_first);
+  CUDA_TRY(s, cudaMemcpyAsync(d_tets, tets, sizeof(int64_t) * 4 * nT, cudaMemcpyHostToDevice, st));
+  CUDA_TRY(s, cudaMemcpyAsync(d_xyz, xyz, sizeof(double) * 3 * nV, cudaMemcpyHostToDevice, st));
+  CUDA_TRY(s, launch_stage_check(nV, nT, d_tets, d_xyz, d_first, d_ctl, st));
+  StageCtl h{};
+  CUDA_TRY(s, cudaMemcpyAsync(&h, d_ctl, sizeof h, cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(s, cudaStreamSynchronize(st));
+  if (h.bad_id != ~0ull)
+    return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: tet %lld has vertex %lld outside [0,%lld)",
+                   (long long)(h.bad_id / 4), (long long)tets[h.bad_id], (long long)nV);
+  if (h.bad_tet != ~0ull)
+    return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: tet %lld repeats a vertex", (long long)h.bad_tet);
+  if (h.bad_xyz != ~0ull)
+    return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: coordinate %lld is not finite", (long long)h.bad_xyz);
+
+  // slots: on the device with one submesh, on the host with several
+  Staging S;
+  {
+    std::vector<int32_t> agg;
+    const int32_t nagg = atags ? aggregates(nT, atags, agg) : 1;
+    if (nagg > 1) reference_slots(nV, nT, tets, agg, nagg, S);
+    else {
+      S.n_copies = nV;
+      S.sub_ptr.push_back(0);
+    }
+  }
+  const int64_t nL = S.n_copies;
+  const int64_t nC = 4 * nT;
+  const bool multi = S.n_submeshes > 1;
+
   s->warm = nullptr;  // a warm start belongs to the previous mesh
   if (s->tuned) {      // so does a tuned launch configuration
     s->tuned = false;
@@ -477,75 +470,75 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
   s->n_submeshes = S.n_submeshes;
   S.sub_ptr.push_back(nL);
   s->h_sub_ptr.swap(S.sub_ptr);
+  s->h_cptr.clear();
   s->blk_grid = -1;
-  s->in_tet.swap(in_tet);
   s->h_gptr.swap(S.gptr);
   s->h_gcopy.swap(S.gcopy);
-  const bool multi = S.n_submeshes > 1;
-  CUDA_TRY(s, s->xyz.alloc(3 * nV));
-  CUDA_TRY(s, s->tslots.alloc(4 * nT));
-  CUDA_TRY(s, s->cidx.alloc(nC));
-  CUDA_TRY(s, s->cptr.alloc(nL + 1));
-  CUDA_TRY(s, s->crec.alloc((size_t)kCrecWords * nC));
-  CUDA_TRY(s, s->cgeo.alloc((size_t)kCgeoStride * nC));
-  CUDA_TRY(s, s->cgf.alloc((size_t)kCgfStride * nC));
-  CUDA_TRY(s, s->nptr.alloc(nL + 1));
-  CUDA_TRY(s, s->nbr.alloc(nbr.size()));
-  CUDA_TRY(s, s->fib.alloc(3 * nT));
-  CUDA_TRY(s, s->cf.alloc(nT));
-  CUDA_TRY(s, s->ct.alloc(nT));
-  CUDA_TRY(s, s->phi.alloc(nL));
-  CUDA_TRY(s, s->phi_f.alloc(nL));
-  CUDA_TRY(s, s->phi2.alloc(nL));
-  CUDA_TRY(s, s->phi2_f.alloc(nL));
-  CUDA_TRY(s, s->st.alloc(nL));
-  CUDA_TRY(s, s->tst.alloc(nL));
-  CUDA_TRY(s, s->dec.alloc(nL));
-  CUDA_TRY(s, s->sw.alloc(nL));
-  CUDA_TRY(s, s->list0.alloc(nL));
-  CUDA_TRY(s, s->list1.alloc(nL));
-  CUDA_TRY(s, s->list2.alloc(nL));
-  CUDA_TRY(s, s->lfrozen.alloc(nL));
-  CUDA_TRY(s, s->lmarked.alloc(nL));
+  const auto parts = [&](unsigned char *base) {
+    Parts a;
+    a.base = base;
+    a.add(s->xyz, 3 * nV); a.add(s->tslots, 4 * nT); a.add(s->cidx, nC);
+    a.add(s->cptr, nL + 1); a.add(s->nptr, nL + 1);
+    a.add(s->crec, (size_t)kCrecWords * nC); a.add(s->cgeo, (size_t)kCgeoStride * nC);
+    a.add(s->cgf, (size_t)kCgfStride * nC);
+    a.add(s->fib, 3 * nT); a.add(s->cf, nT); a.add(s->ct, nT);
+    a.add(s->phi, nL); a.add(s->phi_f, nL); a.add(s->phi2, nL); a.add(s->phi2_f, nL);
+    a.add(s->st, nL); a.add(s->tst, nL); a.add(s->dec, nL); a.add(s->sw, nL);
+    a.add(s->list0, nL); a.add(s->list1, nL); a.add(s->list2, nL); a.add(s->lfrozen, nL); a.add(s->lmarked, nL);
+    if (multi) { a.add(s->gptr, nV + 1); a.add(s->gcopy, nL); a.add(s->phi_out, nV); a.add(s->st_out, nV); }
+    return a.off;
+  };
+  s->gptr.release(); s->gcopy.release(); s->phi_out.release(); s->st_out.release();
+  CUDA_TRY(s, reserve_near(s->arena, parts(nullptr)));
+  parts(s->arena.p);
+
+  CUDA_TRY(s, cudaMemcpyAsync(s->xyz.p, d_xyz, sizeof(double) * 3 * nV, cudaMemcpyDeviceToDevice, st));
+  StageLists ls{};
   if (multi) {
-    CUDA_TRY(s, s->gptr.alloc(nV + 1));
-    CUDA_TRY(s, s->gcopy.alloc(nL));
-    CUDA_TRY(s, s->phi_out.alloc(nV));
-    CUDA_TRY(s, s->st_out.alloc(nV));
+    // (the tets on the device have served their purpose: the copies' slots
+    // take their place)
+    CUDA_TRY(s, cudaMemcpyAsync(s->tslots.p, S.slots.data(), sizeof(int32_t) * nC, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(s, cudaMemcpyAsync(d_tets, S.cslots.data(), sizeof(int32_t) * nC, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(s, cudaMemcpyAsync(s->gptr.p, s->h_gptr.data(), sizeof(int64_t) * (nV + 1), cudaMemcpyHostToDevice, st));
+    CUDA_TRY(s, cudaMemcpyAsync(s->gcopy.p, s->h_gcopy.data(), sizeof(int32_t) * nL, cudaMemcpyHostToDevice, st));
+    ls.cslots = reinterpret_cast<const int32_t *>(d_tets);
   } else {
-    s->gptr.release(); s->gcopy.release(); s->phi_out.release(); s->st_out.release();
+    CUDA_TRY(s, launch_stage_slots(nT, d_tets, d_first, s->tslots.p, st));
+    ls.cslots = s->tslots.p;
   }
-  cudaStream_t st = s->stream;
-  CUDA_TRY(s, cudaMemcpyAsync(s->xyz.p, xyz, sizeof(double) * 3 * nV, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(s, cudaMemcpyAsync(s->tslots.p, slots.data(), sizeof(int32_t) * 4 * nT, cudaMemcpyHostToDevice, st));
   // the edge vectors for the metric kernel (144 B per tet); without room
   // for them the kernel forms them from xyz
-  if (s->evec.alloc((size_t)18 * nT) == cudaSuccess) {
-    CUDA_TRY(s, launch_edge_vectors(s->tslots.p, s->xyz.p, nT, s->evec.p, st));
-  } else {
+  if (reserve_near(s->evec, (size_t)18 * nT) != cudaSuccess) {
     cudaGetLastError();
     s->evec.release();
   }
-  CUDA_TRY(s, cudaMemcpyAsync(s->cidx.p, cidx.data(), sizeof(int64_t) * nC, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(s, cudaMemcpyAsync(s->cptr.p, cptr.data(), sizeof(int64_t) * (nL + 1), cudaMemcpyHostToDevice, st));
+  CUDA_TRY(s, launch_edge_vectors(s->tslots.p, s->xyz.p, nT, s->evec.p, d_ctl, st));
+  // corners and neighbourhoods; arrays that are not in use before the first
+  // conduction upload or solve serve as scratch
+  ls.cptr = s->cptr.p; ls.nptr = s->nptr.p; ls.crec = s->crec.p; ls.cidx = s->cidx.p;
+  ls.cnt = s->list0.p; ls.big_list = s->list1.p; ls.mark = s->list2.p;
+  ls.keys = reinterpret_cast<uint32_t *>(s->cgf.p);
+  ls.scratch = reinterpret_cast<int32_t *>(s->cgeo.p);
+  ls.tile_sum = reinterpret_cast<long long *>(s->phi2.p);
+  CUDA_TRY(s, launch_stage_lists(nL, nT, ls, d_ctl, st));
+  int64_t n_nbr = 0;
+  CUDA_TRY(s, cudaMemcpyAsync(&n_nbr, s->nptr.p + nL, sizeof n_nbr, cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(s, cudaMemcpyAsync(&h, d_ctl, sizeof h, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(s, cudaStreamSynchronize(st));
-  s->h_cptr.swap(cptr);
-  {
-    // the ids part of the first-read records (the metric kernel fills the rest)
-    std::vector<uint4> crec((size_t)kCrecWords * nC);
-#pragma omp parallel for schedule(static)
-    for (int64_t c = 0; c < nC; ++c) {
-      crec[kCrecWords * c] = make_uint4((unsigned)cids[c].x, (unsigned)cids[c].y, (unsigned)cids[c].z, 0u);
-      crec[kCrecWords * c + 1] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    CUDA_TRY(s, cudaMemcpyAsync(s->crec.p, crec.data(), sizeof(uint4) * crec.size(), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(s, cudaStreamSynchronize(st));
-  }
-  CUDA_TRY(s, cudaMemcpyAsync(s->nptr.p, nptr.data(), sizeof(int64_t) * (nL + 1), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(s, cudaMemcpyAsync(s->nbr.p, nbr.data(), sizeof(int32_t) * nbr.size(), cudaMemcpyHostToDevice, st));
+  CUDA_TRY(s, reserve_near(s->nbr, (size_t)n_nbr));
+  CUDA_TRY(s, launch_stage_compact(nL, ls, s->nbr.p, st));
+  // reference front width: 1.01 * longest edge / 0.6 (compute_dwf, cuda_fim.h:1536-1576)
+  double maxe2;
+  std::memcpy(&maxe2, &h.max_edge2, sizeof maxe2);
+  s->front_width = 1.01 * std::sqrt(maxe2) / 0.6;
+  // vertices in at least one tet (seeds elsewhere are dropped, as the
+  // reference seeds through submeshes only)
+  s->in_tet.resize(nV);
   if (multi) {
-    CUDA_TRY(s, cudaMemcpyAsync(s->gptr.p, s->h_gptr.data(), sizeof(int64_t) * (nV + 1), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(s, cudaMemcpyAsync(s->gcopy.p, s->h_gcopy.data(), sizeof(int32_t) * nL, cudaMemcpyHostToDevice, st));
+    for (int64_t v = 0; v < nV; ++v) s->in_tet[v] = s->h_gptr[v + 1] > s->h_gptr[v] ? 1 : 0;
+  } else {
+    CUDA_TRY(s, launch_stage_in_tet(nV, s->cptr.p, s->dec.p, st));
+    CUDA_TRY(s, cudaMemcpyAsync(s->in_tet.data(), s->dec.p, nV, cudaMemcpyDeviceToHost, st));
   }
   CUDA_TRY(s, cudaStreamSynchronize(st));
   s->stats.n_corners = nC;
@@ -731,8 +724,13 @@ static int warm_check(fim_solver *s, cudaStream_t st);
 
 // Submesh sweeps: whole submeshes to blocks, contiguous in copy order, with
 // about the same number of corners each (the corners are the work).
-static void block_ranges(const fim_solver *s, int grid, std::vector<int32_t> &out)
+static cudaError_t block_ranges(fim_solver *s, int grid, std::vector<int32_t> &out)
 {
+  if (s->h_cptr.empty()) {
+    s->h_cptr.resize(s->nL + 1);
+    const cudaError_t e = cudaMemcpy(s->h_cptr.data(), s->cptr.p, sizeof(int64_t) * (s->nL + 1), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) { s->h_cptr.clear(); return e; }
+  }
   const std::vector<int64_t> &sp = s->h_sub_ptr;
   const int nsub = (int)sp.size() - 1;
   const int64_t total = s->h_cptr[s->nL];
@@ -744,6 +742,7 @@ static void block_ranges(const fim_solver *s, int grid, std::vector<int32_t> &ou
     const int64_t done = s->h_cptr[sp[a + 1]];
     while (b < grid && done * grid >= total * b) out[b++] = (int32_t)sp[a + 1];
   }
+  return cudaSuccess;
 }
 
 // Launch parameters and device view of the solver's staged problem.
@@ -830,7 +829,7 @@ static int run_solve(fim_solver *s, cudaStream_t st, int shape, int grid, int da
     p.two_phase = 0;
     if (s->blk_grid != grid) {
       std::vector<int32_t> ranges;
-      block_ranges(s, grid, ranges);
+      CUDA_TRY(s, block_ranges(s, grid, ranges));
       CUDA_TRY(s, s->blk_ptr.reserve(ranges.size()));
       CUDA_TRY(s, cudaMemcpyAsync(s->blk_ptr.p, ranges.data(), sizeof(int32_t) * ranges.size(),
                                   cudaMemcpyHostToDevice, st));
@@ -1212,6 +1211,10 @@ extern "C" int fim_solve_noalloc(fim_solver *s, int64_t n, const int64_t *vertic
   d.seed_v = sc.seed_v; d.seed_t = sc.seed_t; d.nseed = (int32_t)entries;
   d.phi_init = s->warm;  // the caller's own device array (fim_set_warm_start): nothing to allocate
   d.ctl = sc.ctl;
+#ifdef FIM_PROBE
+  CUDA_TRY(s, s->probe.reserve((size_t)s->grid * kProbeSlots));  // (instrumented builds do allocate)
+  d.probe = s->probe.p;
+#endif
   FimParams p{};
   p.dt = s->opts.dt;
   p.n_steps = s->opts.n_steps;

@@ -1,18 +1,18 @@
 // fim_mlp.cu -- the learned warm start: per-vertex features and a small
 // MLP (7 -> 128 -> 128 -> 128 -> 1, ReLU) trained and evaluated on the GPU.
 //
-// Every product of the three hidden layers, forward and backward, is one
-// tcgen05 GEMM (C[M x 128] = A[M x K] B[128 x K]^T, BF16 operands staged by
-// TMA with the 128-byte swizzle, FP32 accumulator in tensor memory) with the
-// epilogue fused: bias + ReLU + BF16 store (forward), ReLU mask + BF16 store
-// (backward data), FP32 store (weight gradients).  The forward GEMMs read
-// transposed BF16 copies of the weights, the backward-data GEMMs the copies
-// as stored, and the weight gradients transposed activations, so that every
-// operand has K contiguous.
-// The output layer (128 -> 1), the loss, the bias gradients and Adam are
-// element-wise FP32 kernels.  Master weights are FP32; the GEMMs read BF16
-// copies refreshed after every update.  The input width is padded from 7
-// features to kMlpIn = 64 columns (zeros), one 128-byte K slice.
+// One persistent kernel, mlp_kernel, runs the whole network over 128-row
+// tiles: the three hidden layers forward and, when training, back again,
+// every product a tcgen05 MMA with BF16 operands in shared memory and an
+// FP32 accumulator in tensor memory.  A tile's activations never leave the
+// SM: each layer's epilogue (bias + ReLU, or the ReLU mask) writes BF16 rows
+// back to shared memory in the layout the next MMA reads.  The weight
+// gradients accumulate in tensor memory over all tiles of a CTA, and
+// mlp_reduce_kernel adds the CTAs' sums in a fixed order and, in a training
+// step, applies Adam.  Master weights, biases, output layer, loss and bias
+// gradients are FP32; the MMAs read a BF16 copy of the weights refreshed
+// after every update.  The input width is padded from 7 features to
+// kMlpIn = 64 columns (zeros), one 128-byte K slice.
 //
 // No counterpart in the reference.
 #include "fim_internal.h"
@@ -33,33 +33,19 @@ namespace fimgb {
 namespace {
 
 // ---------------------------------------------------------------------------
-// tcgen05 GEMMs: C[M x 128] = A[M x K] B[128 x K]^T, A and B BF16 and
-// K-major (rows of K contiguous), the FP32 accumulator in tensor memory.
-// Operands are staged by TMA as 64-wide K slices (128 bytes, the swizzle
-// span) with the 128-byte swizzle, and every mbarrier wait is bounded
-// (%globaltimer): a wait that runs out sets the error word, the CTA skips
-// its stores, waits (bounded) for the copies and MMAs it issued and frees
-// its tensor memory.
-//
-// umma_gemm_kernel (the weight gradients: M <= 128, long K): one CTA of four
-// warps per 128-row tile and split of K (a long K is split over up to 32
-// CTAs, whose partial sums split_sum_kernel adds in a fixed order).  Warp 0
-// (one lane) streams the K slices of A and B through a ring of kGemmStages
-// stages (full/empty mbarriers); warp 1 (one
-// lane) issues four tcgen05.mma (M = N = 128, K = 16) per slice and commits
-// each slice's MMAs to the stage's empty barrier, the last one to the done
-// barrier; warp 2 owns the 128 tensor-memory columns of the accumulator; all
-// four warps then read it back (warp w: lanes 32w..32w+31, the tile rows)
-// with tcgen05.ld and store FP32.
-enum { kEpiBiasRelu = 0, kEpiMask = 1 };
-constexpr int kGemmM = 128, kGemmN = 128, kGemmK = 64;  // tile rows, columns, K per stage (128 B of BF16)
-constexpr int kGemmStages = 3;
-constexpr uint32_t kGemmTileBytes = kGemmM * kGemmK * 2;  // one operand's slice: 16 KB (N == M)
-constexpr int kGemmSmem = kGemmStages * 2 * kGemmTileBytes + 1024;  // + slack to align the ring to 1024 B
-constexpr uint64_t kGemmWaitNs = 2000000000ull;  // bound of every mbarrier wait
-constexpr int kGemmSplitSlices = 4;   // K slices per CTA of a split weight-gradient GEMM (at least)
-constexpr int kGemmMaxSplits = 32;    // CTAs per 128-row tile at most
-static_assert(kGemmN == kGemmM, "the ring holds equal A and B slices");
+// tcgen05 building blocks.  Operands lie in shared memory as blocks of 64
+// columns (128 bytes, the span of the 128-byte swizzle) by 128 rows, 16 KB
+// each, as a TMA load with that swizzle puts them.  Such a block is a
+// K-major operand when its columns are the contraction (activations times
+// weights), and an MN-major one when its rows are (weight gradients:
+// contraction over the tile's rows; data gradients: over the weights' output
+// rows), so no operand is ever transposed in memory.  Every mbarrier wait is
+// bounded (%globaltimer): a wait that runs out sets the error word, the
+// group leaves at its next barrier, and the CTA waits (bounded) for the
+// copies and MMAs it issued and frees its tensor memory.
+constexpr int kTileM = 128, kBlkCols = 64;
+constexpr uint32_t kBlkBytes = kTileM * kBlkCols * 2;  // 16 KB
+constexpr uint64_t kMlpWaitNs = 2000000000ull;         // bound of every mbarrier wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
@@ -90,7 +76,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
   return ok != 0;
 }
 // waits until the phase with the given parity has completed; false after limit_ns
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns = kGemmWaitNs)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns = kMlpWaitNs)
 {
   if (mbar_try(bar, parity)) return true;
   const uint64_t t0 = gtimer();
@@ -106,34 +92,34 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int x, int y)
+// Shared-memory matrix descriptors (128-byte swizzle: layout type 2,
+// descriptor version 1).  K-major: 8-row groups 1024 B apart (stride byte
+// offset), leading byte offset unused.  MN-major: 64-column blocks kBlkBytes
+// apart (leading byte offset), 8-row groups (of the contraction) 1024 B
+// apart (stride byte offset).
+constexpr uint64_t kDescBase = ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+__device__ __forceinline__ uint64_t desc_k(uint32_t addr)
 {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y)
-               : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | kDescBase;
 }
-
-// Shared-memory matrix descriptor of a K-major operand slice with the
-// 128-byte swizzle: rows of 128 B, 8-row groups 1024 B apart (stride byte
-// offset), descriptor version 1, layout type 2 (128-byte swizzle).  The
-// leading byte offset is unused for this layout (set to 16 B).
-__device__ __forceinline__ uint64_t sdesc_k128(uint32_t addr)
+__device__ __forceinline__ uint64_t desc_mn(uint32_t addr)
 {
-  return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+  return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)(kBlkBytes >> 4) << 16) | kDescBase;
 }
 // Instruction descriptor of tcgen05.mma kind::f16: FP32 accumulator (bits
-// 4-5 = 1), BF16 A and B (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 =
-// 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-constexpr uint32_t kGemmIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kGemmN >> 3) << 17) |
-                                ((uint32_t)(kGemmM >> 4) << 24);
-__device__ __forceinline__ void umma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accumulate)
+// 4-5 = 1), BF16 A and B (bits 7-9, 10-12 = 1), A / B MN-major (bits 15,
+// 16), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
+__host__ __device__ constexpr uint32_t idesc(int n, bool a_mn, bool b_mn)
+{
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
+         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+}
+__device__ __forceinline__ void umma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate)
 {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(tmem), "l"(a), "l"(b), "r"(kGemmIdesc), "r"(accumulate)
+      ::"r"(tmem), "l"(a), "l"(b), "r"(id), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar)
@@ -142,396 +128,554 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// 32 consecutive FP32 columns of this thread's tensor-memory lane (issued;
-// tmem_wait_ld makes them readable)
-__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t *v)
+// 32 consecutive FP32 columns of this thread's tensor-memory lane; the load
+// and its wait are one statement, so that no use of v can move between them
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *v)
 {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+      "tcgen05.wait::ld.sync.aligned;"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
         "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
         "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
         "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
+      : "r"(taddr)
+      : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *v)
+// 64 consecutive FP32 columns of this thread's tensor-memory lane; the load
+// and its wait are one statement, so that no use of v can move between them
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t *v)
 {
-  tmem_ld32_issue(taddr, v);
-  tmem_wait_ld();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
+      "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%65];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]),
+        "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]),
+        "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]),
+        "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]),
+        "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
+      : "r"(taddr), "r"(taddr + 32u)
+      : "memory");
+}
+// Index of weight i (W1 [kMlpIn x kMlpH], W2, W3 [kMlpH x kMlpH], each
+// [in x out] row-major) in the transposed copies [out x in] that the MMAs
+// read.
+__device__ __forceinline__ int transposed_index(int i)
+{
+  if (i < kMlpOW2) return kMlpOW1 + (i % kMlpH) * kMlpIn + i / kMlpH;
+  const int off = i < kMlpOW3 ? kMlpOW2 : kMlpOW3, k = i - off;
+  return off + (k % kMlpH) * kMlpH + k / kMlpH;
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
+// acc (tile rows x 128) = A (K-major, kblk blocks of 64 columns) times the
+// K-major 128 x 64 kblk operand B, transposed
+__device__ __forceinline__ void mma_rows(uint32_t acc, uint32_t a, uint32_t b, int kblk)
 {
-  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(lo)) |
-         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16(hi)) << 16);
-}
-
-__global__ void __launch_bounds__(128, 1) umma_gemm_kernel(const __grid_constant__ CUtensorMap ta,
-                                                           const __grid_constant__ CUtensorMap tb, int M, int K,
-                                                           int kps, float *out32, int ldc, size_t split_stride,
-                                                           unsigned int *err)
-{
-  extern __shared__ __align__(1024) unsigned char gemm_smem[];
-  __shared__ __align__(8) uint64_t full_bar[kGemmStages], empty_bar[kGemmStages], done_bar;
-  __shared__ uint32_t tmem_base;
-  __shared__ volatile int s_fail, s_consumed;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t ring = (smem_u32(gemm_smem) + 1023u) & ~1023u;
-  const int m0 = blockIdx.x * kGemmM;
-  // split blockIdx.y of K: slices [k0, k0 + nk), its partial sums at out32 + blockIdx.y * split_stride
-  const int k0 = blockIdx.y * kps;
-  const int nk = min(kps, K / kGemmK - k0);
-  out32 += blockIdx.y * split_stride;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kGemmStages; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), 1);
-      mbar_init(smem_u32(&empty_bar[s]), 1);
-    }
-    mbar_init(smem_u32(&done_bar), 1);
-    s_fail = 0;
-    s_consumed = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta)) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tb)) : "memory");
-  }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "r"(kGemmN)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_base;
-
-  int issued = 0;
-  if (warp == 0 && lane == 0) {
-    // producer: K slice i into stage i % kGemmStages once the MMAs of slice
-    // i - kGemmStages have released it
-    for (int i = 0; i < nk; ++i) {
-      const int s = i % kGemmStages;
-      const uint32_t ph = (uint32_t)(i / kGemmStages) & 1u;
-      if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1u)) { s_fail = 1; break; }
-      const uint32_t fb = smem_u32(&full_bar[s]);
-      mbar_expect_tx(fb, 2 * kGemmTileBytes);
-      tma_load_2d(ring + s * kGemmTileBytes, &ta, (k0 + i) * kGemmK, m0, fb);
-      tma_load_2d(ring + (kGemmStages + s) * kGemmTileBytes, &tb, (k0 + i) * kGemmK, 0, fb);
-      issued = i + 1;
-    }
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer: four K = 16 steps per slice (32 bytes apart within the
-    // swizzled 128-byte rows)
-    int i = 0;
-    for (; i < nk; ++i) {
-      const int s = i % kGemmStages;
-      const uint32_t ph = (uint32_t)(i / kGemmStages) & 1u;
-      if (!mbar_wait(smem_u32(&full_bar[s]), ph)) { s_fail = 1; break; }
-      tc_fence_after();
-      const uint32_t a = ring + s * kGemmTileBytes, b = ring + (kGemmStages + s) * kGemmTileBytes;
+  for (int s = 0; s < kblk; ++s)
 #pragma unroll
-      for (int k = 0; k < kGemmK / 16; ++k)
-        umma_bf16(tmem, sdesc_k128(a + 32 * k), sdesc_k128(b + 32 * k), (uint32_t)(i | k));
-      umma_commit(smem_u32(&empty_bar[s]));
-    }
-    s_consumed = i;
-    umma_commit(smem_u32(&done_bar));  // arrives once every MMA issued above has completed
-  }
-  __syncwarp();
-  // the whole K loop runs before this completes: the bound grows with it
-  if (!mbar_wait(smem_u32(&done_bar), 0, kGemmWaitNs + 20000ull * (uint64_t)nk)) s_fail = 1;
-  tc_fence_after();
-  const bool ok = s_fail == 0;
-
-  // epilogue: this thread's row, 32 columns per tensor-memory load
-  const int row = m0 + warp * 32 + lane;
-  const bool store = ok && row < M;
-#pragma unroll 1
-  for (int c0 = 0; c0 < kGemmN; c0 += 32) {
-    uint32_t v[32];
-    tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-    if (!store) continue;
-    float4 *o = reinterpret_cast<float4 *>(out32 + (size_t)row * ldc + c0);
+    for (int k = 0; k < kBlkCols / 16; ++k)
+      umma_bf16(acc, desc_k(a + s * kBlkBytes + 32 * k), desc_k(b + s * kBlkBytes + 32 * k), idesc(128, false, false),
+                (uint32_t)(s | k));
+}
+// acc (tile rows x 128) = A (K-major, 128 columns) times W (128 rows x 128
+// columns, contraction over its rows)
+__device__ __forceinline__ void mma_data(uint32_t acc, uint32_t a, uint32_t w)
+{
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      o[q] = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]),
-                         __uint_as_float(v[4 * q + 3]));
-  }
-  if (!ok) {
-    if (threadIdx.x == 0) atomicOr(err, 1u);
-    // copies issued but not consumed by an MMA still land in the ring: wait for them
-    if (warp == 0 && lane == 0)
-      for (int i = s_consumed; i < issued; ++i)
-        (void)mbar_wait(smem_u32(&full_bar[i % kGemmStages]), (uint32_t)(i / kGemmStages) & 1u);
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 2)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGemmN) : "memory");
+  for (int k = 0; k < 128 / 16; ++k)
+    umma_bf16(acc, desc_k(a + (uint32_t)(k / 4) * kBlkBytes + 32 * (k % 4)), desc_mn(w + 2048 * k),
+              idesc(128, false, true), (uint32_t)k);
+}
+// acc (128 x n) (+)= D^T H over the tile's rows: D 128 columns, H n columns
+__device__ __forceinline__ void mma_weight(uint32_t acc, uint32_t d, uint32_t h, int n, bool first)
+{
+  const uint32_t id = n == 128 ? idesc(128, true, true) : idesc(64, true, true);
+#pragma unroll
+  for (int k = 0; k < kTileM / 16; ++k)
+    umma_bf16(acc, desc_mn(d + 2048 * k), desc_mn(h + 2048 * k), id, (first && k == 0) ? 0u : 1u);
 }
 
+__device__ __forceinline__ uint64_t f2_pack(float x, float y)
+{
+  return (uint64_t)__float_as_uint(x) | ((uint64_t)__float_as_uint(y) << 32);
+}
+__device__ __forceinline__ float f2_lo(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float f2_hi(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b)
+{
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c)
+{
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// two floats as BF16 (round to nearest), first in the low half
+__device__ __forceinline__ uint32_t bf2(float lo, float hi)
+{
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
+// relu of two BF16 values (a NaN becomes 0, as fmaxf(x, 0) makes it)
+__device__ __forceinline__ uint32_t bf2_relu(uint32_t x)
+{
+  uint32_t d;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(0u));
+  return d;
+}
+__device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 // ---------------------------------------------------------------------------
-// Persistent row-tile GEMM for the tall products (M = rows, K = 64 or 128):
-// C[M x 128] = A[M x K] W[128 x K]^T, one CTA per SM looping over 128-row
-// tiles.  The weights (B) are loaded once per CTA; warp 0 streams A tiles
-// through a ring of kRowStages stages; warp 1 issues the MMAs of tile j into
-// tensor-memory accumulator j % 2; warps 2-9 drain accumulator j % 2 (warp w
-// reads lanes 32 (w % 4) .. +31, the tile rows, and columns 64 h .. 64 h + 63
-// with h = (w - 2) / 4) while the MMAs of tile j + 1 run, release it (tempty)
-// and then apply the epilogue:
-//   kEpiBiasRelu:    out_bf16 = relu(C + bias)
-//   kEpiMask:        out_bf16 = C * (mask_bf16 > 0)
-//   kEpiBiasReluOut: h = bf16(relu(C + bias)) (stored when out_bf16 is set),
-//                    y = h . w4 + b4 (the output layer), and with targets
-//                    dy = 2 (y - t) / M and the summed squared error; the
-//                    warps of columns 64..127 hand their partial dot
-//                    products to those of columns 0..63 through shared
-//                    memory (mbarrier ypart), which add them in a fixed
-//                    order and release the accumulator after reading them.
-enum { kEpiBiasReluOut = 3 };
-constexpr int kRowStages = 3;
-constexpr int kRowKMax = 128, kRowSlices = kRowKMax / kGemmK;
-constexpr uint32_t kRowStageBytes = kRowSlices * kGemmTileBytes;     // one A tile (32 KB)
-constexpr uint32_t kRowStgBytes = 32 * kGemmK * 2;  // one epilogue warp's 32 x 64 output box (4 KB)
-constexpr int kRowEpiWarps = 8;
-// B + the A ring + two output boxes per epilogue warp + alignment slack
-constexpr int kRowSmem = (1 + kRowStages) * kRowStageBytes + 2 * kRowEpiWarps * kRowStgBytes + 1024;
-constexpr int kRowThreads = 320;  // producer, MMA issuer, 8 epilogue warps
+// The network over 128-row tiles.  A group of warps owns a tile: warp w reads
+// tensor-memory lanes 32 (w % 4) .. + 31 (the tile's rows); the group's
+// thread 0 issues the TMA loads and the MMAs.
+//
+// Forward: four groups of four warps per CTA on tiles of their own, so that
+// one tile's MMAs (20 steps) and waits run beside the epilogues of the
+// others.  A group needs 32 KB: its activations, overwritten layer by layer;
+// the next tile's features are loaded into them while the last layer's
+// epilogue runs, which no longer touches them.
+// Training: one group of eight warps (two column halves), since a tile's
+// features and three activations (112 KB) leave no room for a second tile
+// beside the 80 KB of weights; the next tile's features are loaded a tile
+// ahead.
+//
+// Measured over 1.03M rows (features 132 MB), predict call: three GEMM
+// kernels with H1 and H2 in memory 252 us, this kernel 106 us (98 us on the
+// device: tensor pipe 39 % busy; with both operands in shared memory a
+// 128 x 128 x 16 step reads 8 KB in the 64 cycles it takes, so the MMAs alone
+// use the shared-memory bandwidth that the epilogues need too).  Two groups
+// of eight warps 125 us, four of eight 115 us.  Training step of 4,096 rows
+// (22 launches before, 2 now) 191 -> 46 us; gradients of 131,136 rows, whose
+// activations and their transposes went through memory, 500 -> 97 us.
+constexpr uint32_t kW1Bytes = kBlkBytes, kW2Bytes = 2 * kBlkBytes;
+constexpr uint32_t kWBytes = kW1Bytes + 2 * kW2Bytes;  // the weights, [out][in]
+constexpr uint32_t kActBytes = 2 * kBlkBytes;          // 128 x 128 activations
+template <bool kTrain>
+struct MlpShape {
+  static constexpr int kGroups = kTrain ? 1 : 4;
+  static constexpr int kGroupThreads = kTrain ? 256 : 128;
+  static constexpr int kThreads = kGroups * kGroupThreads;
+  static constexpr uint32_t kGroupBytes = kTrain ? 2 * kBlkBytes + 3 * kActBytes : kActBytes;
+  static constexpr int kSmem = (int)(kWBytes + kGroups * kGroupBytes) + 1024;  // + slack to align to 1024 B
+};
+constexpr int kTmemCols = 512;
+// tensor-memory columns in training: the layer's accumulator, then the
+// transposed weight gradients [out][in] of layers 3, 2, 1
+constexpr uint32_t kTmW3 = 128, kTmW2 = 256, kTmW1 = 384;
+// partial results of a training CTA: gradients in parameter order, then the
+// summed squared error
+constexpr int kPartStride = (kMlpParams + 1 + 63) & ~63;
 
-template <int EPI>
-__global__ void __launch_bounds__(kRowThreads, 1) umma_rows_kernel(
-    const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
-    const __grid_constant__ CUtensorMap to, int M, int K, const float *__restrict__ bias,
-    const __nv_bfloat16 *__restrict__ mask, int store, int ldc,
-    const float *__restrict__ w4, const float *__restrict__ b4, float *y, const float *__restrict__ tgt, float *dy,
-    float *loss, unsigned int *err)
+template <int kThreads>
+__device__ __forceinline__ void group_sync(int g)
 {
-  extern __shared__ __align__(1024) unsigned char gemm_smem[];
-  __shared__ __align__(8) uint64_t bfull, afull[kRowStages], aempty[kRowStages], tfull[2], tempty[2], ypart[2];
-  __shared__ float s_part[2][kGemmM];
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kThreads) : "memory");
+}
+
+template <bool kTrain>
+__global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
+    const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw1,
+    const __grid_constant__ CUtensorMap tw2, const __grid_constant__ CUtensorMap tw3, int M,
+    const float *__restrict__ P, float *y, const float *__restrict__ tgt, float *part, volatile unsigned int *err)
+{
+  using S = MlpShape<kTrain>;
+  extern __shared__ unsigned char mlp_smem[];
+  __shared__ __align__(8) uint64_t wfull, xfull[S::kGroups][2], mdone[S::kGroups];
   __shared__ uint32_t tmem_base;
-  __shared__ float s_bias[kGemmN], s_w4[kGemmN];
-  __shared__ volatile int s_fail;
-  __shared__ int s_issued, s_consumed, s_mma_issued, s_drained;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t bsm = (smem_u32(gemm_smem) + 1023u) & ~1023u, aring = bsm + kRowStageBytes;
-  const uint32_t stg0 = aring + kRowStages * kRowStageBytes;  // output boxes: [warp - 2][tile parity]
-  const int nks = K / kGemmK;
-  const uint32_t tile_bytes = (uint32_t)nks * kGemmTileBytes;
-  const int ntiles = (M + kGemmM - 1) / kGemmM;
+  __shared__ __align__(16) float s_bias[3][kMlpH], s_w4[kMlpH];
+  __shared__ float s_part[kTileM], s_dy[kTileM];  // training
+  __shared__ volatile int s_fail[S::kGroups][2];
+  const int g = threadIdx.x / S::kGroupThreads, t = threadIdx.x % S::kGroupThreads;
+  const int lane = t & 31, q = (t >> 5) & 3, h = t >> 7;  // h: column half (training; 0 forward, both halves in turn)
+  const uint32_t w1 = (smem_u32(mlp_smem) + 1023u) & ~1023u, w2 = w1 + kW1Bytes, w3 = w2 + kW2Bytes;
+  unsigned char *const sm = mlp_smem + (w1 - smem_u32(mlp_smem));  // generic address of w1
+  const uint32_t xs = w1 + kWBytes + (uint32_t)g * S::kGroupBytes;
+  const uint32_t h1 = kTrain ? xs + 2 * kBlkBytes : xs;  // forward: one buffer for features and activations
+  const uint32_t h2 = kTrain ? h1 + kActBytes : h1, h3 = kTrain ? h2 + kActBytes : h1;
+  const int ntiles = (M + kTileM - 1) / kTileM;
+  const int tstep = gridDim.x * S::kGroups;
+  const int tile0 = g * gridDim.x + blockIdx.x;  // few tiles: one per CTA
+
   if (threadIdx.x == 0) {
-    mbar_init(smem_u32(&bfull), 1);
-    for (int s = 0; s < kRowStages; ++s) {
-      mbar_init(smem_u32(&afull[s]), 1);
-      mbar_init(smem_u32(&aempty[s]), 1);
+    mbar_init(smem_u32(&wfull), 1);
+    for (int i = 0; i < S::kGroups; ++i) {
+      mbar_init(smem_u32(&xfull[i][0]), 1);
+      mbar_init(smem_u32(&xfull[i][1]), 1);
+      mbar_init(smem_u32(&mdone[i]), 1);
+      s_fail[i][0] = s_fail[i][1] = 0;
     }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(smem_u32(&tfull[a]), 1);
-      mbar_init(smem_u32(&tempty[a]), 8);  // one arrival per epilogue warp
-      mbar_init(smem_u32(&ypart[a]), 4);   // the warps of columns 64..127
-    }
-    s_fail = 0;
-    s_issued = s_consumed = s_mma_issued = s_drained = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta)) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tb)) : "memory");
-    if (store) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&to)) : "memory");
   }
-  if (threadIdx.x < kGemmN) {
-    s_bias[threadIdx.x] = (EPI == kEpiMask) ? 0.f : bias[threadIdx.x];
-    s_w4[threadIdx.x] = (EPI == kEpiBiasReluOut) ? w4[threadIdx.x] : 0.f;
-  }
-  if (warp == 2) {
+  if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "r"(2 * kGemmN)
+                 "r"(kTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      // producer: the weights once, then A tile j into stage j % kRowStages
-      mbar_expect_tx(smem_u32(&bfull), tile_bytes);
-      for (int ks = 0; ks < nks; ++ks)
-        tma_load_2d(bsm + ks * kGemmTileBytes, &tb, ks * kGemmK, 0, smem_u32(&bfull));
-      int j = 0;
-      for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++j) {
-        const int s = j % kRowStages;
-        if (s_fail || !mbar_wait(smem_u32(&aempty[s]), ((uint32_t)(j / kRowStages) & 1u) ^ 1u)) { s_fail = 1; break; }
-        const uint32_t fb = smem_u32(&afull[s]);
-        mbar_expect_tx(fb, tile_bytes);
-        for (int ks = 0; ks < nks; ++ks)
-          tma_load_2d(aring + s * kRowStageBytes + ks * kGemmTileBytes, &ta, ks * kGemmK, tile * kGemmM, fb);
-        s_issued = j + 1;
-      }
+  const uint32_t tmem = tmem_base + (kTrain ? 0u : (uint32_t)(g * 128));
+  const uint32_t bar_m = smem_u32(&mdone[g]);
+  const uint32_t bar_x0 = smem_u32(&xfull[g][0]), bar_x1 = smem_u32(&xfull[g][1]);
+  int issued = 0, consumed = 0;  // thread 0 of the group: feature tiles
+  // feature tile i of the group: its buffer, barrier and parity
+  const auto x_buf = [&](int i) { return xs + (kTrain ? (uint32_t)(i & 1) * kBlkBytes : 0u); };
+  const auto x_bar = [&](int i) { return kTrain && (i & 1) ? bar_x1 : bar_x0; };
+  const auto x_par = [&](int i) { return (uint32_t)(kTrain ? i >> 1 : i) & 1u; };
+  const auto load_x = [&](int tile) {
+    mbar_expect_tx(x_bar(issued), kBlkBytes);
+    tma_load_2d(x_buf(issued), &tx, 0, tile * kTileM, x_bar(issued));
+    ++issued;
+  };
+  if (t == 0 && tile0 < ntiles) load_x(tile0);
+  if (threadIdx.x == 0) {
+    mbar_expect_tx(smem_u32(&wfull), kWBytes);
+    tma_load_2d(w1, &tw1, 0, 0, smem_u32(&wfull));
+    for (int s = 0; s < 2; ++s) {
+      tma_load_2d(w2 + s * kBlkBytes, &tw2, s * kBlkCols, 0, smem_u32(&wfull));
+      tma_load_2d(w3 + s * kBlkBytes, &tw3, s * kBlkCols, 0, smem_u32(&wfull));
     }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      // MMA issuer: tile j into accumulator j % 2 once the epilogue has drained it
-      if (!mbar_wait(smem_u32(&bfull), 0)) s_fail = 1;
-      int j = 0;
-      for (int tile = blockIdx.x; tile < ntiles && !s_fail; tile += gridDim.x, ++j) {
-        const int s = j % kRowStages, acc = j & 1;
-        if (!mbar_wait(smem_u32(&tempty[acc]), ((uint32_t)(j >> 1) & 1u) ^ 1u) ||
-            !mbar_wait(smem_u32(&afull[s]), (uint32_t)(j / kRowStages) & 1u)) { s_fail = 1; break; }
-        tc_fence_after();
-        const uint32_t a = aring + s * kRowStageBytes, d = tmem + (uint32_t)(acc * kGemmN);
-        for (int ks = 0; ks < nks; ++ks)
-#pragma unroll
-          for (int k = 0; k < kGemmK / 16; ++k)
-            umma_bf16(d, sdesc_k128(a + ks * kGemmTileBytes + 32 * k), sdesc_k128(bsm + ks * kGemmTileBytes + 32 * k),
-                      (uint32_t)(ks | k));
-        umma_commit(smem_u32(&aempty[s]));
-        umma_commit(smem_u32(&tfull[acc]));
-        s_consumed = j + 1;
-        s_mma_issued = j + 1;
-      }
-    }
-  } else {
-    // epilogue warps 2..9: tensor-memory lanes 32 q .. 32 q + 31 (tile rows),
-    // columns cb .. cb + 63
-    const int q = warp & 3, h = (warp - 2) >> 2, cb = 64 * h;
-    auto release = [&](int acc, int j) {
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[acc])) : "memory");
-      if (warp == 2 && lane == 0) s_drained = j + 1;
-    };
-    int j = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++j) {
-      const int acc = j & 1;
-      const uint32_t par = (uint32_t)(j >> 1) & 1u;
-      if (s_fail || !mbar_wait(smem_u32(&tfull[acc]), par)) { s_fail = 1; break; }
-      tc_fence_after();
-      const int row = tile * kGemmM + q * 32 + lane;
-      const bool in = row < M;
-      uint32_t v[64];
-      const uint32_t tv = tmem + (uint32_t)(acc * kGemmN) + ((uint32_t)(q * 32) << 16) + (uint32_t)cb;
-      tmem_ld32_issue(tv, v);
-      tmem_ld32_issue(tv + 32, v + 32);
-      tmem_wait_ld();
-      const bool combine = EPI == kEpiBiasReluOut && h == 0;  // releases after reading the partials
-      if (!combine) release(acc, j);
-      // this warp's 32 x 64 output box goes through shared memory (128-byte
-      // swizzle: 16-byte chunk c of row r at chunk c ^ (r % 8)) and one TMA
-      // store, which clips the rows past M; first the store issued from the
-      // same buffer two tiles ago must have read it
-      const uint32_t stg = stg0 + (uint32_t)(((warp - 2) * 2 + (j & 1)) * kRowStgBytes);
-      if (store) {
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        __syncwarp();
-      }
-      float ysum = 0.f;
-#pragma unroll
-      for (int c = 0; c < 64; c += 32) {
-        const int col = cb + c;
-        uint32_t w[16];
-        if (EPI == kEpiMask) {
-          const uint4 *mk = reinterpret_cast<const uint4 *>(mask + (size_t)row * ldc + col);
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            const uint4 mm = in ? mk[q4] : make_uint4(0u, 0u, 0u, 0u);
-            const uint32_t mw[4] = {mm.x, mm.y, mm.z, mm.w};
-#pragma unroll
-            for (int hh = 0; hh < 4; ++hh) {
-              const int e = 4 * q4 + hh;
-              const float lo = __bfloat162float(__ushort_as_bfloat16((unsigned short)(mw[hh] & 0xffffu)));
-              const float hi = __bfloat162float(__ushort_as_bfloat16((unsigned short)(mw[hh] >> 16)));
-              w[e] = pack_bf16(lo > 0.f ? __uint_as_float(v[c + 2 * e]) : 0.f,
-                               hi > 0.f ? __uint_as_float(v[c + 2 * e + 1]) : 0.f);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            w[e] = pack_bf16(fmaxf(__uint_as_float(v[c + 2 * e]) + s_bias[col + 2 * e], 0.f),
-                             fmaxf(__uint_as_float(v[c + 2 * e + 1]) + s_bias[col + 2 * e + 1], 0.f));
-            if (EPI == kEpiBiasReluOut) {  // the output layer on the stored (BF16) activations
-              ysum += __bfloat162float(__ushort_as_bfloat16((unsigned short)(w[e] & 0xffffu))) * s_w4[col + 2 * e];
-              ysum += __bfloat162float(__ushort_as_bfloat16((unsigned short)(w[e] >> 16))) * s_w4[col + 2 * e + 1];
-            }
-          }
-        }
-        if (store) {
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            const uint32_t chunk = (uint32_t)((c >> 3) + k4) ^ (uint32_t)(lane & 7);
-            const uint32_t a = stg + (uint32_t)lane * 128u + chunk * 16u;
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w[4 * k4]), "r"(w[4 * k4 + 1]),
-                         "r"(w[4 * k4 + 2]), "r"(w[4 * k4 + 3])
-                         : "memory");
-          }
-        }
-      }
-      if (store) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) tma_store_2d(&to, stg, cb, tile * kGemmM + q * 32);
-      }
-      if (EPI == kEpiBiasReluOut) {
-        if (h == 1) {  // hand the partial dot product over
-          s_part[acc][q * 32 + lane] = ysum;
-          __syncwarp();
-          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ypart[acc])) : "memory");
-        } else {
-          const bool okp = mbar_wait(smem_u32(&ypart[acc]), par);
-          if (!okp) s_fail = 1;
-          const float p1 = s_part[acc][q * 32 + lane];
-          release(acc, j);
-          float se = 0.f;
-          if (okp && in) {
-            const float yv = (ysum + p1) + b4[0];
-            y[row] = yv;
-            if (tgt) {
-              const float e = yv - tgt[row];
-              dy[row] = 2.f * e / (float)M;
-              se = e * e;
-            }
-          }
-          if (tgt) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
-            if (lane == 0) atomicAdd(loss, se);
-          }
-        }
-      }
-    }
-    if (store && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // the output is written
   }
+  for (int i = threadIdx.x; i < 4 * kMlpH; i += S::kThreads) {
+    if (i < 3 * kMlpH) s_bias[i / kMlpH][i % kMlpH] = P[kMlpOB1 + i];
+    else s_w4[i - 3 * kMlpH] = P[kMlpOW4 + i - 3 * kMlpH];
+  }
+  const float b4 = P[kMlpOB4];
   __syncthreads();
-  if (s_fail) {
-    if (threadIdx.x == 0) {
-      atomicOr(err, 1u);
-      // the weights, copies issued but not consumed, MMAs issued but not
-      // drained: let them land (bounded)
-      (void)mbar_wait(smem_u32(&bfull), 0);
-      for (int j = s_consumed; j < s_issued; ++j)
-        (void)mbar_wait(smem_u32(&afull[j % kRowStages]), (uint32_t)(j / kRowStages) & 1u);
-      for (int j = s_drained; j < s_mma_issued; ++j)
-        (void)mbar_wait(smem_u32(&tfull[j & 1]), (uint32_t)(j >> 1) & 1u);
+  bool wok = true;
+  if (t == 0) wok = mbar_wait(smem_u32(&wfull), 0);  // each group's issuer sees the weights
+
+  // A phase ends with the group's barrier; a wait that ran out in phase p
+  // is flagged in s_fail[g][p & 1] before that barrier and read after it, so
+  // the whole group leaves together (a later phase writes the other word).
+  int phase = 0;
+  uint32_t mpar = 0;       // parity of the next MMA completion
+  int commits = 0;         // thread 0: completions requested
+  int waited = 0;
+  const auto fail = [&]() { s_fail[g][phase & 1] = 1; };
+  const auto end_phase = [&]() {
+    group_sync<S::kGroupThreads>(g);
+    const bool bad = s_fail[g][phase & 1] != 0;
+    ++phase;
+    return !bad;
+  };
+  const auto wait_mma = [&]() {
+    if (!mbar_wait(bar_m, mpar)) fail();
+    else ++waited;
+    mpar ^= 1u;
+    __syncwarp();
+    tc_fence_after();
+  };
+  // publishes shared-memory rows written by this thread to the MMAs
+  const auto publish = [&]() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();
+    return end_phase();
+  };
+  const uint32_t tv = tmem + ((uint32_t)(q * 32) << 16);
+  const int r = q * 32 + lane;  // this thread's row of the tile
+  // 64 columns of the row: from the accumulator, and where they lie in an activation block
+  const auto load_acc = [&](int half, uint32_t *v) {
+    tmem_ld64(tv + 64 * half, v);
+  };
+  const auto chunk_ptr = [&](uint32_t base, int half, int c) {  // 16-byte chunk c, at chunk c ^ (row % 8)
+    return reinterpret_cast<uint4 *>(sm + (base - w1) + (uint32_t)half * kBlkBytes + (uint32_t)r * 128u +
+                                     ((uint32_t)(c ^ (r & 7)) << 4));
+  };
+  const int half0 = h, half1 = kTrain ? h + 1 : 2;  // the column halves of this thread
+
+  // training: sums over this thread's rows (columns 2 cp, 2 cp + 1, rows
+  // 32 rg .. + 31 of every tile) of the bias gradients and of gw4; over this
+  // thread's own row of dy and of the squared error
+  const int cp = t & 63, rg = t >> 6;
+  float gb1[2] = {0.f, 0.f}, gb2[2] = {0.f, 0.f}, gb3[2] = {0.f, 0.f}, gw4[2] = {0.f, 0.f};
+  float gb4 = 0.f, sse = 0.f;
+  const uint32_t coloff = (uint32_t)(cp >> 5) * kBlkBytes + (uint32_t)(cp & 3) * 4u;
+  const auto pair_ptr = [&](uint32_t base, int row) {
+    return reinterpret_cast<uint32_t *>(sm + (base - w1) + coloff + (uint32_t)row * 128u +
+                                        ((uint32_t)(((cp & 31) >> 2) ^ (row & 7)) << 4));
+  };
+  const auto colsum = [&](uint32_t base, float *s) {
+#pragma unroll 16
+    for (int i = 0; i < 32; ++i) {
+      const uint32_t w = *pair_ptr(base, 32 * rg + i);
+      s[0] += bf_lo(w);
+      s[1] += bf_hi(w);
     }
-    __syncthreads();
+  };
+
+  int j = 0;
+  bool ok = true;
+  for (int tile = tile0; tile < ntiles; tile += tstep, ++j) {
+    const bool in = tile * kTileM + r < M;
+    // layer 1
+    if (t == 0) {
+      if (kTrain && tile + tstep < ntiles) load_x(tile + tstep);  // its stage was read by MMAs that have completed
+      if (!wok || !mbar_wait(x_bar(j), x_par(j))) fail();
+      else {
+        ++consumed;
+        tc_fence_after();
+        mma_rows(tmem, x_buf(j), w1, 1);
+        umma_commit(bar_m);
+        ++commits;
+      }
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int layer = 0; layer < 2; ++layer) {
+      wait_mma();
+#pragma unroll 1
+      for (int half = half0; half < half1; ++half) {
+        uint32_t v[64];
+        load_acc(half, v);
+        const uint32_t dst = layer == 0 ? h1 : h2;
+        const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[layer][64 * half]);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint32_t w[4];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const ulonglong2 bb = bias[2 * c + k];
+            const uint64_t x0 = f2_add(f2_pack(__uint_as_float(v[8 * c + 4 * k]), __uint_as_float(v[8 * c + 4 * k + 1])), bb.x);
+            const uint64_t x1 = f2_add(f2_pack(__uint_as_float(v[8 * c + 4 * k + 2]), __uint_as_float(v[8 * c + 4 * k + 3])), bb.y);
+            w[2 * k] = bf2_relu(bf2(f2_lo(x0), f2_hi(x0)));
+            w[2 * k + 1] = bf2_relu(bf2(f2_lo(x1), f2_hi(x1)));
+            if (kTrain && !in) w[2 * k] = w[2 * k + 1] = 0u;  // rows past the matrix take no part in the gradients
+          }
+          *chunk_ptr(dst, half, c) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      if (!publish()) { ok = false; break; }
+      if (t == 0) {
+        tc_fence_after();
+        if (layer == 0) mma_rows(tmem, h1, w2, 2);
+        else mma_rows(tmem, h2, w3, 2);
+        umma_commit(bar_m);
+        ++commits;
+      }
+      __syncwarp();
+    }
+    if (!ok) break;
+    // layer 3 and the output layer: y = relu(.) . w4 + b4 on the BF16
+    // activations, the two column halves added in a fixed order
+    wait_mma();
+    if (!kTrain && t == 0 && tile + tstep < ntiles) load_x(tile + tstep);
+    float ysum = 0.f;
+#pragma unroll 1
+    for (int half = half0; half < half1; ++half) {
+      uint32_t v[64];
+      load_acc(half, v);
+      const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[2][64 * half]);
+      const ulonglong2 *wv = reinterpret_cast<const ulonglong2 *>(&s_w4[64 * half]);
+      uint64_t sum0 = 0ull, sum1 = 0ull;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const ulonglong2 bb = bias[2 * c + k], ww = wv[2 * c + k];
+          const uint64_t x0 = f2_add(f2_pack(__uint_as_float(v[8 * c + 4 * k]), __uint_as_float(v[8 * c + 4 * k + 1])), bb.x);
+          const uint64_t x1 = f2_add(f2_pack(__uint_as_float(v[8 * c + 4 * k + 2]), __uint_as_float(v[8 * c + 4 * k + 3])), bb.y);
+          w[2 * k] = bf2_relu(bf2(f2_lo(x0), f2_hi(x0)));
+          w[2 * k + 1] = bf2_relu(bf2(f2_lo(x1), f2_hi(x1)));
+          if (kTrain && !in) w[2 * k] = w[2 * k + 1] = 0u;
+          sum0 = f2_fma(f2_pack(bf_lo(w[2 * k]), bf_hi(w[2 * k])), ww.x, sum0);
+          sum1 = f2_fma(f2_pack(bf_lo(w[2 * k + 1]), bf_hi(w[2 * k + 1])), ww.y, sum1);
+        }
+        if (kTrain) *chunk_ptr(h3, half, c) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      ysum += (f2_lo(sum0) + f2_hi(sum0)) + (f2_lo(sum1) + f2_hi(sum1));
+    }
+    if (h == 1) s_part[r] = ysum;
+    tc_fence_before();  // (the accumulator is read: the next tile's first MMA may write it)
+    if (!end_phase()) { ok = false; break; }
+    if (!kTrain) {
+      if (in) y[tile * (int64_t)kTileM + r] = ysum + b4;
+      continue;
+    }
+    if (h == 0) {
+      float dy = 0.f;
+      if (in) {
+        const float e = ((ysum + s_part[r]) + b4) - tgt[tile * (int64_t)kTileM + r];
+        dy = 2.f * e / (float)M;
+        sse += e * e;
+        gb4 += dy;
+      }
+      s_dy[r] = dy;
+    }
+    if (!end_phase()) { ok = false; break; }
+    // dZ3 = bf16(dy w4) where H3 > 0, in place; sums of gw4 and gb3
+    {
+      const float wa = s_w4[2 * cp], wb = s_w4[2 * cp + 1];
+#pragma unroll 1
+      for (int i0 = 0; i0 < 32; i0 += 16) {
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) w[i] = *pair_ptr(h3, 32 * rg + i0 + i);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float dy = s_dy[32 * rg + i0 + i], x0 = bf_lo(w[i]), x1 = bf_hi(w[i]);
+          gw4[0] += x0 * dy;
+          gw4[1] += x1 * dy;
+          w[i] = bf2(x0 > 0.f ? dy * wa : 0.f, x1 > 0.f ? dy * wb : 0.f);
+          gb3[0] += bf_lo(w[i]);
+          gb3[1] += bf_hi(w[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) *pair_ptr(h3, 32 * rg + i0 + i) = w[i];
+      }
+    }
+    if (!publish()) { ok = false; break; }
+    // layers 3 and 2 back: dZ_(l-1) = (dZ_l W_l^T) where H_(l-1) > 0, in
+    // place of H_(l-1) once the weight gradient dW_l = H_(l-1)^T dZ_l is done
+#pragma unroll 1
+    for (int layer = 0; layer < 2; ++layer) {
+      const uint32_t dz = layer == 0 ? h3 : h2, hp = layer == 0 ? h2 : h1;
+      if (t == 0) {
+        tc_fence_after();
+        mma_data(tmem, dz, layer == 0 ? w3 : w2);
+        mma_weight(tmem + (layer == 0 ? kTmW3 : kTmW2), dz, hp, 128, j == 0);
+        umma_commit(bar_m);
+        ++commits;
+      }
+      __syncwarp();
+      if (layer == 1) colsum(h2, gb2);
+      wait_mma();
+      {
+        uint32_t v[64];
+        load_acc(h, v);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint4 *a = chunk_ptr(hp, h, c);
+          const uint4 mm = *a;
+          const uint32_t m[4] = {mm.x, mm.y, mm.z, mm.w};
+          uint32_t w[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            w[k] = bf2(bf_lo(m[k]) > 0.f ? __uint_as_float(v[8 * c + 2 * k]) : 0.f,
+                       bf_hi(m[k]) > 0.f ? __uint_as_float(v[8 * c + 2 * k + 1]) : 0.f);
+          *a = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      if (!publish()) { ok = false; break; }
+    }
+    if (!ok) break;
+    // dW1 = X^T dZ1
+    if (t == 0) {
+      tc_fence_after();
+      mma_weight(tmem + kTmW1, h1, x_buf(j), 64, j == 0);
+      umma_commit(bar_m);
+      ++commits;
+    }
+    __syncwarp();
+    colsum(h1, gb1);
+    wait_mma();
+    if (!end_phase()) { ok = false; break; }
+  }
+
+  if (kTrain && ok && tile0 < ntiles) {
+    // this CTA's sums, in parameter order ([in][out]): lane = output column
+    float *o = part + (size_t)blockIdx.x * kPartStride;
+#pragma unroll 1
+    for (int w = 0; w < 3; ++w) {
+      const int nin = w == 2 ? 32 : 64, in0 = nin * h;
+      float *dst = o + (w == 0 ? kMlpOW3 : (w == 1 ? kMlpOW2 : kMlpOW1)) + r;
+      const uint32_t src = tmem + (w == 0 ? kTmW3 : (w == 1 ? kTmW2 : kTmW1)) + ((uint32_t)(q * 32) << 16) + in0;
+      for (int c = 0; c < nin; c += 32) {
+        uint32_t v[32];
+        tmem_ld32(src + c, v);
+#pragma unroll
+        for (int k = 0; k < 32; ++k) dst[(in0 + c + k) * kMlpH] = __uint_as_float(v[k]);
+      }
+    }
+    // the four row groups' column sums, in order; the features' stages are free
+    float *sum = reinterpret_cast<float *>(mlp_smem + (xs - smem_u32(mlp_smem)));
+    float *mine = sum + rg * 4 * kMlpH + 2 * cp;
+    const float *src[4] = {gb1, gb2, gb3, gw4};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      mine[k * kMlpH] = src[k][0];
+      mine[k * kMlpH + 1] = src[k][1];
+    }
+    float *red = sum + 16 * kMlpH;
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) {
+      gb4 += __shfl_xor_sync(0xffffffffu, gb4, k);
+      sse += __shfl_xor_sync(0xffffffffu, sse, k);
+    }
+    if (lane == 0) { red[2 * (t >> 5)] = gb4; red[2 * (t >> 5) + 1] = sse; }
+    group_sync<S::kGroupThreads>(g);
+    for (int i = t; i < 4 * kMlpH; i += S::kGroupThreads)
+      o[kMlpOB1 + i] = ((sum[i] + sum[4 * kMlpH + i]) + sum[8 * kMlpH + i]) + sum[12 * kMlpH + i];
+    if (t < 2) o[kMlpOB4 + t] = ((red[t] + red[2 + t]) + red[4 + t]) + red[6 + t];
+  }
+  if (t == 0 && (!ok || !wok)) {
+    *err = 1u;
+    // copies and MMAs still in flight land before the CTA leaves (bounded)
+    (void)mbar_wait(smem_u32(&wfull), 0);
+    for (int i = consumed; i < issued; ++i) (void)mbar_wait(x_bar(i), x_par(i));
+    for (int i = waited; i < commits; ++i) (void)mbar_wait(bar_m, (uint32_t)i & 1u);
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 2)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kGemmN) : "memory");
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
-// out[c][r] = in[r][c] for an R x C BF16 matrix (R, C multiples of 32)
-__global__ void transpose_bf16_kernel(int R, int C, const __nv_bfloat16 *__restrict__ in, __nv_bfloat16 *out)
+// Sums of the CTAs' partial gradients, in a fixed order (four threads per
+// parameter take a quarter of the CTAs each), into G; the mean squared error
+// into *loss.  With lr > 0 also Adam (bias-corrected) on every parameter and
+// the BF16 copies of the weight matrices, transposed to [out][in].
+constexpr int kRedParams = 64;
+__global__ void __launch_bounds__(4 * kRedParams) mlp_reduce_kernel(int ctas, const float *__restrict__ part, int rows,
+                                                                    float *G, float *loss, float *P, float *m, float *v,
+                                                                    float lr, float b1, float b2, float eps, float c1,
+                                                                    float c2, __nv_bfloat16 *W16T)
 {
-  __shared__ __nv_bfloat16 t[32][33];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) t[k][threadIdx.x] = in[(size_t)(r0 + k) * C + c0 + threadIdx.x];
+  __shared__ float s[4][kRedParams];
+  const int k = threadIdx.x / kRedParams, l = threadIdx.x % kRedParams;
+  const int i = blockIdx.x * kRedParams + l;  // < kPartStride
+  const int lo = ctas * k / 4, hi = ctas * (k + 1) / 4;
+  float a = 0.f;
+  if (i <= kMlpParams) {
+#pragma unroll 8
+    for (int c = lo; c < hi; ++c) a += part[(size_t)c * kPartStride + i];
+  }
+  s[k][l] = a;
   __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) out[(size_t)(c0 + k) * R + r0 + threadIdx.x] = t[threadIdx.x][k];
+  if (k != 0 || i > kMlpParams) return;
+  const float g = ((s[0][l] + s[1][l]) + s[2][l]) + s[3][l];
+  if (i == kMlpParams) {
+    *loss = g / (float)rows;
+    return;
+  }
+  G[i] = g;
+  if (!(lr > 0.f)) return;
+  const float mi = b1 * m[i] + (1.f - b1) * g;
+  const float vi = b2 * v[i] + (1.f - b2) * g * g;
+  m[i] = mi;
+  v[i] = vi;
+  const float p = P[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  P[i] = p;
+  if (i < kMlpW16) W16T[transposed_index(i)] = __float2bfloat16(p);
+}
+
+__global__ void to_bf16_kernel(const float *__restrict__ src, __nv_bfloat16 *W16T)
+{
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpW16; i += gridDim.x * blockDim.x)
+    W16T[transposed_index(i)] = __float2bfloat16(src[i]);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
@@ -550,195 +694,17 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 // Tensor map of a rows x k BF16 matrix (row-major, k contiguous): boxes of
 // 64 columns (128 B, the swizzle span) by 128 rows; rows beyond the matrix
 // read as zeros.
-bool make_map(CUtensorMap *map, const void *base, uint64_t k, uint64_t rows, uint32_t box_rows = kGemmM)
+bool make_map(CUtensorMap *map, const void *base, uint64_t k, uint64_t rows)
 {
   const auto enc = tensor_map_encoder();
-  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15u) || k % kGemmK) return false;
+  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15u) || k % kBlkCols) return false;
   const cuuint64_t dims[2] = {k, rows};
   const cuuint64_t strides[1] = {k * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kGemmK, box_rows};
+  const cuuint32_t box[2] = {(cuuint32_t)kBlkCols, (cuuint32_t)kTileM};
   const cuuint32_t estr[2] = {1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-}  // namespace
-
-namespace {
-// out[r][c] = sum over the splits, in split order (deterministic), of the
-// partial sums ws[s][r][c] (row stride ldc, split stride M * ldc)
-__global__ void split_sum_kernel(int M, int ldc, int splits, const float *__restrict__ ws, float *out)
-{
-  const int n = M * kGemmN;
-  const size_t st = (size_t)M * ldc;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int r = i / kGemmN, c = i % kGemmN;
-    const float *p = ws + (size_t)r * ldc + c;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int s = 0; s < splits; ++s) acc += p[s * st];
-    out[(size_t)r * ldc + c] = acc;
-  }
-}
-}  // namespace
-
-// Weight gradients: C[M x 128] = A[M x K] B[128 x K]^T (FP32 out) for BF16
-// A (rows_a >= M rows) and B (128 rows), both with K contiguous, K a
-// multiple of 64 (the K loop of umma_gemm_kernel).  A long K is split over
-// up to kGemmMaxSplits CTAs per 128-row tile (kGemmSplitSlices K slices
-// each, partial sums in ws, which holds kGemmMaxSplits * M * ldc floats) and
-// summed in split order; without ws one CTA per tile runs the whole K.
-cudaError_t mlp_gemm_wgrad(int M, int K, const void *A, int rows_a, const void *B, float *out32, int ldc, float *ws,
-                           unsigned int *err, cudaStream_t st)
-{
-  if (M <= 0 || K <= 0 || K % kGemmK || rows_a < M) return cudaErrorInvalidValue;
-  CUtensorMap ta, tb;
-  if (!make_map(&ta, A, (uint64_t)K, (uint64_t)rows_a) || !make_map(&tb, B, (uint64_t)K, kGemmN))
-    return cudaErrorInvalidValue;
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem)) !=
-      cudaSuccess) return e;
-  const int nk = K / kGemmK;
-  int kps = nk, splits = 1;
-  if (ws && nk > kGemmSplitSlices) {
-    kps = std::max(kGemmSplitSlices, (nk + kGemmMaxSplits - 1) / kGemmMaxSplits);
-    splits = (nk + kps - 1) / kps;
-  }
-  const dim3 grid((M + kGemmM - 1) / kGemmM, splits);
-  if (splits == 1) {
-    umma_gemm_kernel<<<grid, 128, kGemmSmem, st>>>(ta, tb, M, K, kps, out32, ldc, 0, err);
-    return cudaGetLastError();
-  }
-  umma_gemm_kernel<<<grid, 128, kGemmSmem, st>>>(ta, tb, M, K, kps, ws, ldc, (size_t)M * ldc, err);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  split_sum_kernel<<<(M * kGemmN + 255) / 256, 256, 0, st>>>(M, ldc, splits, ws, out32);
-  return cudaGetLastError();
-}
-
-// The tall products: C[M x 128] = A[M x K] W[128 x K]^T with K = 64 or 128
-// (umma_rows_kernel, one CTA per SM); epilogue arguments as the kernel's.
-struct RowEpi {
-  const float *bias = nullptr;
-  const void *mask = nullptr;
-  void *out16 = nullptr;
-  const float *w4 = nullptr, *b4 = nullptr;
-  float *y = nullptr;
-  const float *tgt = nullptr;
-  float *dy = nullptr, *loss = nullptr;
-};
-
-cudaError_t mlp_gemm_rows(int epi, int M, int K, const void *A, const void *W, const RowEpi &x, unsigned int *err,
-                          cudaStream_t st)
-{
-  if (M <= 0 || (K != 64 && K != 128)) return cudaErrorInvalidValue;
-  CUtensorMap ta, tb;
-  CUtensorMap to;  // the output in 32 x 64 boxes (unused without a BF16 output)
-  const int store = x.out16 != nullptr;
-  if (!make_map(&ta, A, (uint64_t)K, (uint64_t)M) || !make_map(&tb, W, (uint64_t)K, kGemmN))
-    return cudaErrorInvalidValue;
-  if (!store) to = ta;
-  else if (!make_map(&to, x.out16, kGemmN, (uint64_t)M, 32)) return cudaErrorInvalidValue;
-  int dev = 0, nsm = 0;
-  cudaError_t e;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  const int ntiles = (M + kGemmM - 1) / kGemmM;
-  const dim3 grid(std::min(ntiles, nsm));
-  const auto *mk = static_cast<const __nv_bfloat16 *>(x.mask);
-#define FIM_ROWS_LAUNCH(E)                                                                                           \
-  do {                                                                                                              \
-    if ((e = cudaFuncSetAttribute(umma_rows_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmem)) !=   \
-        cudaSuccess)                                                                                                \
-      return e;                                                                                                     \
-    umma_rows_kernel<E><<<grid, kRowThreads, kRowSmem, st>>>(ta, tb, to, M, K, x.bias, mk, store, kGemmN, x.w4, x.b4, \
-                                                             x.y, x.tgt, x.dy, x.loss, err);                       \
-  } while (0)
-  if (epi == kEpiBiasRelu) FIM_ROWS_LAUNCH(kEpiBiasRelu);
-  else if (epi == kEpiMask) FIM_ROWS_LAUNCH(kEpiMask);
-  else if (epi == kEpiBiasReluOut) FIM_ROWS_LAUNCH(kEpiBiasReluOut);
-  else return cudaErrorInvalidValue;
-#undef FIM_ROWS_LAUNCH
-  return cudaGetLastError();
-}
-
-cudaError_t mlp_transpose(int R, int C, const void *in, void *out, cudaStream_t st)
-{
-  if (R % 32 || C % 32) return cudaErrorInvalidValue;
-  transpose_bf16_kernel<<<dim3(C / 32, R / 32), dim3(32, 8), 0, st>>>(R, C, static_cast<const __nv_bfloat16 *>(in),
-                                                                       static_cast<__nv_bfloat16 *>(out));
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// element-wise parts of the network
-
-namespace {
-
-// dZ3[r][c] = bf16(dy[r] w4[c]) where H3 > 0; gw4[c] += sum_r H3[r][c] dy[r];
-// gb4 += sum_r dy[r].  One block per 64 rows, one thread per column.
-__global__ void out_backward_kernel(int n, const __nv_bfloat16 *__restrict__ H3, const float *__restrict__ w4,
-                                    const float *__restrict__ dy, __nv_bfloat16 *dZ3, float *gw4, float *gb4)
-{
-  const int c = threadIdx.x;  // kMlpH threads
-  const int r0 = blockIdx.x * 64;
-  float sw = 0.f, sb = 0.f;
-  for (int r = r0; r < min(n, r0 + 64); ++r) {
-    const float h = __bfloat162float(H3[(size_t)r * kMlpH + c]);
-    sw += h * dy[r];
-    sb += dy[r];
-    dZ3[(size_t)r * kMlpH + c] = __float2bfloat16(h > 0.f ? dy[r] * w4[c] : 0.f);
-  }
-  atomicAdd(&gw4[c], sw);
-  if (c == 0) atomicAdd(gb4, sb);
-}
-
-// gb[c] += sum_r dZ[r][c] (bias gradients), one block per 64 rows.
-__global__ void colsum_kernel(int n, const __nv_bfloat16 *__restrict__ dZ, float *gb)
-{
-  const int c = threadIdx.x;
-  const int r0 = blockIdx.x * 64;
-  float s = 0.f;
-  for (int r = r0; r < min(n, r0 + 64); ++r) s += __bfloat162float(dZ[(size_t)r * kMlpH + c]);
-  atomicAdd(&gb[c], s);
-}
-
-// Index of weight i (W1 [kMlpIn x kMlpH], W2, W3 [kMlpH x kMlpH], each
-// [in x out] row-major) in the transposed copies [out x in] that the forward
-// GEMMs read as their K-major B operand.
-__device__ __forceinline__ int transposed_index(int i)
-{
-  if (i < kMlpOW2) return kMlpOW1 + (i % kMlpH) * kMlpIn + i / kMlpH;
-  const int off = i < kMlpOW3 ? kMlpOW2 : kMlpOW3, k = i - off;
-  return off + (k % kMlpH) * kMlpH + k / kMlpH;
-}
-
-// Adam (bias-corrected) on every parameter, then the BF16 copies of the
-// three GEMM weight matrices (as stored and transposed).
-__global__ void adam_kernel(int np, float *P, const float *__restrict__ G, float *m, float *v, float lr, float b1,
-                            float b2, float eps, float c1, float c2, __nv_bfloat16 *W16, __nv_bfloat16 *W16T)
-{
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const float g = G[i];
-    const float mi = b1 * m[i] + (1.f - b1) * g;
-    const float vi = b2 * v[i] + (1.f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    const float p = P[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    P[i] = p;
-    if (i < kMlpW16) {
-      W16[i] = __float2bfloat16(p);
-      W16T[transposed_index(i)] = __float2bfloat16(p);
-    }
-  }
-}
-
-__global__ void to_bf16_kernel(const float *__restrict__ src, __nv_bfloat16 *W16, __nv_bfloat16 *W16T)
-{
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpW16; i += gridDim.x * blockDim.x) {
-    W16[i] = __float2bfloat16(src[i]);
-    W16T[transposed_index(i)] = __float2bfloat16(src[i]);
-  }
 }
 
 }  // namespace
@@ -870,17 +836,19 @@ static_assert(FIM_MLP_PARAMS == kMlpParams, "parameter count of the C ABI");
 static_assert(FIM_MLP_INPUTS == kMlpIn, "feature width of the C ABI");
 
 struct fim_mlp {
-  int device = 0;
+  int device = 0, sms = 0;
   cudaStream_t st = nullptr;
-  float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr, *loss = nullptr;
-  __nv_bfloat16 *W16 = nullptr, *W16T = nullptr;  // GEMM weights as stored ([in x out]) and transposed
-  unsigned int *err = nullptr;                     // set by a GEMM whose bounded wait ran out
-  unsigned int h_err = 0;
-  int64_t cap = 0;
-  __nv_bfloat16 *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *dA = nullptr, *dB = nullptr;
-  __nv_bfloat16 *HT = nullptr, *DT = nullptr;     // [kMlpH x cap] transposes for the weight gradients
-  float *y = nullptr, *dy = nullptr;
-  float *ws = nullptr;                             // split-K partial sums of the weight gradients
+  float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;
+  __nv_bfloat16 *W16T = nullptr;     // BF16 weights, [out][in]
+  CUtensorMap tw1, tw2, tw3;
+  float *part = nullptr;             // partial gradients of up to sms CTAs
+  // mapped host memory: the loss of the last reduction, and a word set by a
+  // kernel whose bounded wait ran out (read after the stream has drained)
+  struct Result { float loss; unsigned int err; };
+  volatile Result *h_res = nullptr;
+  Result *d_res = nullptr;
+  float *y = nullptr;                // predictions on their way to an output that the kernel cannot write directly
+  int64_t y_cap = 0;
   int64_t steps = 0;
 };
 
@@ -899,45 +867,11 @@ int mlp_fail(const char *what, cudaError_t e)
     if (_e != cudaSuccess) return mlp_fail((what), _e);       \
   } while (0)
 
-void mlp_free_acts(fim_mlp *m)
+// Reports a bounded wait that ran out (after the stream has drained).
+int mlp_status(fim_mlp *m, const char *who)
 {
-  cudaFree(m->H1); cudaFree(m->H2); cudaFree(m->H3); cudaFree(m->dA); cudaFree(m->dB);
-  cudaFree(m->HT); cudaFree(m->DT);
-  cudaFree(m->y); cudaFree(m->dy);
-  m->H1 = m->H2 = m->H3 = m->dA = m->dB = m->HT = m->DT = nullptr;
-  m->y = m->dy = nullptr;
-  m->cap = 0;
-}
-
-int mlp_reserve(fim_mlp *m, int64_t n)
-{
-  if (n <= m->cap) return FIM_OK;
-  mlp_free_acts(m);
-  const size_t a = sizeof(__nv_bfloat16) * kMlpH * (size_t)n;
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->H1, a));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->H2, a));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->H3, a));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->dA, a));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->dB, a));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->HT, a));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->DT, a));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->y, sizeof(float) * n));
-  MLP_TRY("fim_mlp: activations", cudaMalloc(&m->dy, sizeof(float) * n));
-  m->cap = n;
-  return FIM_OK;
-}
-
-// Queues the read of the GEMMs' error word (before the caller's stream
-// synchronisation); mlp_gemm_status then reports it after the sync.
-cudaError_t mlp_read_err(fim_mlp *m)
-{
-  return cudaMemcpyAsync(&m->h_err, m->err, sizeof(unsigned int), cudaMemcpyDeviceToHost, m->st);
-}
-int mlp_gemm_status(fim_mlp *m, const char *who)
-{
-  if (m->h_err == 0) return FIM_OK;
-  m->h_err = 0;
-  cudaMemset(m->err, 0, sizeof(unsigned int));
+  if (m->h_res->err == 0) return FIM_OK;
+  m->h_res->err = 0;
   std::string msg = std::string(who) + ": a tensor-core GEMM wait ran out (results discarded)";
   set_last_error(msg.c_str());
   return FIM_ERR_TIMEOUT;
@@ -953,75 +887,43 @@ int mlp_check_n(int64_t n, const char *who)
   return FIM_OK;
 }
 
-// forward pass of n rows of X; with targets also the loss and dy
-cudaError_t mlp_forward(fim_mlp *m, int n, const void *X, const float *tgt)
+// Launches the network over n rows of X: predictions into y, or with targets
+// the partial gradients of *ctas CTAs into m->part.
+template <bool kTrain>
+cudaError_t mlp_launch(fim_mlp *m, int n, const void *X, float *y, const float *tgt, int *ctas)
 {
-  cudaError_t e;
-  const float *P = m->P;
-  // H_l = relu(H_{l-1} W_l + b_l): B operand = W_l^T [out x in]; the last
-  // layer's epilogue also evaluates the output layer (and, with targets,
-  // dy and the loss); H3 is stored only for the backward pass
-  RowEpi x1, x2, x3;
-  x1.bias = P + kMlpOB1; x1.out16 = m->H1;
-  x2.bias = P + kMlpOB2; x2.out16 = m->H2;
-  x3.bias = P + kMlpOB3; x3.out16 = tgt ? m->H3 : nullptr;
-  x3.w4 = P + kMlpOW4; x3.b4 = P + kMlpOB4; x3.y = m->y; x3.tgt = tgt; x3.dy = m->dy; x3.loss = m->loss;
-  if ((e = mlp_gemm_rows(kEpiBiasRelu, n, kMlpIn, X, m->W16T + kMlpOW1, x1, m->err, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_gemm_rows(kEpiBiasRelu, n, kMlpH, m->H1, m->W16T + kMlpOW2, x2, m->err, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_gemm_rows(kEpiBiasReluOut, n, kMlpH, m->H2, m->W16T + kMlpOW3, x3, m->err, m->st)) != cudaSuccess)
-    return e;
+  using S = MlpShape<kTrain>;
+  CUtensorMap tx;
+  if (!make_map(&tx, X, kMlpIn, (uint64_t)n)) return cudaErrorInvalidValue;
+  const int ntiles = (n + kTileM - 1) / kTileM;
+  const int grid = std::min(ntiles, m->sms);
+  if (ctas) *ctas = grid;
+  mlp_kernel<kTrain><<<grid, S::kThreads, S::kSmem, m->st>>>(tx, m->tw1, m->tw2, m->tw3, n, m->P, y, tgt, m->part,
+                                                             &m->d_res->err);
   return cudaGetLastError();
 }
 
-// backward pass after mlp_forward with targets: gradients into G (zeroed by the caller)
-cudaError_t mlp_backward(fim_mlp *m, int n, const void *X)
+// Loss and gradients of n rows; with lr > 0 also an Adam step.  Waits.
+int mlp_gradients(fim_mlp *m, int64_t n, const void *X, const float *tgt, float lr, float *grads, float *loss,
+                  const char *who)
 {
-  cudaError_t e;
-  float *G = m->G;
-  const int blocks = (n + 63) / 64;
-  out_backward_kernel<<<blocks, kMlpH, 0, m->st>>>(n, m->H3, m->P + kMlpOW4, m->dy, m->dA, G + kMlpOW4, G + kMlpOB4);
-  // layer l: dW_l = H_{l-1}^T dZ_l (both transposed so that K = rows is
-  // contiguous), db_l, dZ_{l-1} = (dZ_l W_l^T) o [H_{l-1} > 0] (B operand =
-  // W_l as stored, [in x out])
-  // layer 3
-  if ((e = mlp_transpose(n, kMlpH, m->H2, m->HT, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_transpose(n, kMlpH, m->dA, m->DT, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_gemm_wgrad(kMlpH, n, m->HT, kMlpH, m->DT, G + kMlpOW3, kMlpH, m->ws, m->err, m->st)) != cudaSuccess) return e;
-  colsum_kernel<<<blocks, kMlpH, 0, m->st>>>(n, m->dA, G + kMlpOB3);
-  RowEpi xm;
-  xm.mask = m->H2; xm.out16 = m->dB;
-  if ((e = mlp_gemm_rows(kEpiMask, n, kMlpH, m->dA, m->W16 + kMlpOW3, xm, m->err, m->st)) != cudaSuccess) return e;
-  // layer 2
-  if ((e = mlp_transpose(n, kMlpH, m->H1, m->HT, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_transpose(n, kMlpH, m->dB, m->DT, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_gemm_wgrad(kMlpH, n, m->HT, kMlpH, m->DT, G + kMlpOW2, kMlpH, m->ws, m->err, m->st)) != cudaSuccess) return e;
-  colsum_kernel<<<blocks, kMlpH, 0, m->st>>>(n, m->dB, G + kMlpOB2);
-  xm.mask = m->H1; xm.out16 = m->dA;
-  if ((e = mlp_gemm_rows(kEpiMask, n, kMlpH, m->dB, m->W16 + kMlpOW2, xm, m->err, m->st)) != cudaSuccess) return e;
-  // layer 1: X^T is kMlpIn rows; the tile's other rows (left over in HT)
-  // only reach output rows that are not stored
-  if ((e = mlp_transpose(n, kMlpIn, X, m->HT, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_transpose(n, kMlpH, m->dA, m->DT, m->st)) != cudaSuccess) return e;
-  if ((e = mlp_gemm_wgrad(kMlpIn, n, m->HT, kMlpH, m->DT, G + kMlpOW1, kMlpH, m->ws, m->err, m->st)) != cudaSuccess) return e;
-  colsum_kernel<<<blocks, kMlpH, 0, m->st>>>(n, m->dA, G + kMlpOB1);
-  return cudaGetLastError();
-}
-
-int mlp_loss_grads(fim_mlp *m, int64_t n, const void *X, const float *tgt, float *loss_out)
-{
-  int rc;
-  if ((rc = mlp_reserve(m, n)) != FIM_OK) return rc;
-  MLP_TRY("fim_mlp: clear", cudaMemsetAsync(m->G, 0, sizeof(float) * kMlpParams, m->st));
-  MLP_TRY("fim_mlp: clear", cudaMemsetAsync(m->loss, 0, sizeof(float), m->st));
-  MLP_TRY("fim_mlp: forward", mlp_forward(m, (int)n, X, tgt));
-  MLP_TRY("fim_mlp: backward", mlp_backward(m, (int)n, X));
-  if (loss_out) {
-    float l = 0.f;
-    MLP_TRY("fim_mlp: loss", cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
-    MLP_TRY("fim_mlp: sync", cudaStreamSynchronize(m->st));
-    *loss_out = l / (float)n;
+  const float b1 = 0.9f, b2 = 0.999f;
+  float c1 = 1.f, c2 = 1.f;
+  if (lr > 0.f) {
+    ++m->steps;
+    c1 = 1.f - std::pow(b1, (float)m->steps);
+    c2 = 1.f - std::pow(b2, (float)m->steps);
   }
-  return FIM_OK;
+  int ctas = 0;
+  MLP_TRY(who, mlp_launch<true>(m, (int)n, X, nullptr, tgt, &ctas));
+  mlp_reduce_kernel<<<kPartStride / kRedParams, 4 * kRedParams, 0, m->st>>>(
+      ctas, m->part, (int)n, m->G, &m->d_res->loss, m->P, m->M, m->V, lr, b1, b2, 1e-8f, c1, c2, m->W16T);
+  MLP_TRY(who, cudaGetLastError());
+  if (grads)
+    MLP_TRY(who, cudaMemcpyAsync(grads, m->G, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->st));
+  MLP_TRY(who, cudaStreamSynchronize(m->st));
+  if (loss) *loss = m->h_res->loss;
+  return mlp_status(m, who);
 }
 
 }  // namespace
@@ -1042,28 +944,41 @@ extern "C" int fim_mlp_create(int device, uint64_t seed, fim_mlp **out)
   int rc = FIM_OK;
   auto fail = [&](int code) { fim_mlp_destroy(m); return code; };
   cudaError_t e;
-  if ((e = cudaStreamCreateWithFlags(&m->st, cudaStreamDefault)) != cudaSuccess ||
+  void *h = nullptr;
+  if ((e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
+      (e = cudaStreamCreateWithFlags(&m->st, cudaStreamDefault)) != cudaSuccess ||
       (e = cudaMalloc(&m->P, sizeof(float) * kMlpParams)) != cudaSuccess ||
       (e = cudaMalloc(&m->G, sizeof(float) * kMlpParams)) != cudaSuccess ||
       (e = cudaMalloc(&m->M, sizeof(float) * kMlpParams)) != cudaSuccess ||
       (e = cudaMalloc(&m->V, sizeof(float) * kMlpParams)) != cudaSuccess ||
-      (e = cudaMalloc(&m->loss, sizeof(float))) != cudaSuccess ||
-      (e = cudaMalloc(&m->W16, sizeof(__nv_bfloat16) * kMlpW16)) != cudaSuccess ||
       (e = cudaMalloc(&m->W16T, sizeof(__nv_bfloat16) * kMlpW16)) != cudaSuccess ||
-      (e = cudaMalloc(&m->err, sizeof(unsigned int))) != cudaSuccess ||
-      (e = cudaMalloc(&m->ws, sizeof(float) * kGemmMaxSplits * kMlpH * kMlpH)) != cudaSuccess ||
-      (e = cudaMemset(m->err, 0, sizeof(unsigned int))) != cudaSuccess)
+      (e = cudaMalloc(&m->part, sizeof(float) * kPartStride * (size_t)m->sms)) != cudaSuccess ||
+      (e = cudaHostAlloc(&h, sizeof(fim_mlp::Result), cudaHostAllocMapped)) != cudaSuccess)
     return fail(mlp_fail("fim_mlp_create", e));
+  m->h_res = static_cast<volatile fim_mlp::Result *>(h);
+  m->h_res->loss = 0.f;
+  m->h_res->err = 0;
+  void *d = nullptr;
+  if ((e = cudaHostGetDevicePointer(&d, h, 0)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(mlp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                MlpShape<false>::kSmem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(mlp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                MlpShape<true>::kSmem)) != cudaSuccess)
+    return fail(mlp_fail("fim_mlp_create", e));
+  m->d_res = static_cast<fim_mlp::Result *>(d);
+  if (!make_map(&m->tw1, m->W16T + kMlpOW1, kMlpIn, kMlpH) || !make_map(&m->tw2, m->W16T + kMlpOW2, kMlpH, kMlpH) ||
+      !make_map(&m->tw3, m->W16T + kMlpOW3, kMlpH, kMlpH))
+    return fail(mlp_fail("fim_mlp_create", cudaErrorInvalidValue));
   // He initialisation (fixed seed); padded input rows and biases zero
-  std::vector<float> h(kMlpParams, 0.f);
+  std::vector<float> h0(kMlpParams, 0.f);
   std::mt19937_64 rng(seed);
   std::normal_distribution<float> nd(0.f, 1.f);
   for (int i = 0; i < kMlpFeatures; ++i)
-    for (int j = 0; j < kMlpH; ++j) h[kMlpOW1 + i * kMlpH + j] = nd(rng) * std::sqrt(2.f / kMlpFeatures);
-  for (int i = 0; i < kMlpH * kMlpH; ++i) h[kMlpOW2 + i] = nd(rng) * std::sqrt(2.f / kMlpH);
-  for (int i = 0; i < kMlpH * kMlpH; ++i) h[kMlpOW3 + i] = nd(rng) * std::sqrt(2.f / kMlpH);
-  for (int i = 0; i < kMlpH; ++i) h[kMlpOW4 + i] = nd(rng) * std::sqrt(1.f / kMlpH);
-  rc = fim_mlp_set_params(m, h.data());
+    for (int j = 0; j < kMlpH; ++j) h0[kMlpOW1 + i * kMlpH + j] = nd(rng) * std::sqrt(2.f / kMlpFeatures);
+  for (int i = 0; i < kMlpH * kMlpH; ++i) h0[kMlpOW2 + i] = nd(rng) * std::sqrt(2.f / kMlpH);
+  for (int i = 0; i < kMlpH * kMlpH; ++i) h0[kMlpOW3 + i] = nd(rng) * std::sqrt(2.f / kMlpH);
+  for (int i = 0; i < kMlpH; ++i) h0[kMlpOW4 + i] = nd(rng) * std::sqrt(1.f / kMlpH);
+  rc = fim_mlp_set_params(m, h0.data());
   if (rc != FIM_OK) return fail(rc);
   *out = m;
   return FIM_OK;
@@ -1074,9 +989,9 @@ extern "C" int fim_mlp_destroy(fim_mlp *m)
   if (!m) return FIM_OK;
   cudaSetDevice(m->device);
   if (m->st) cudaStreamSynchronize(m->st);
-  mlp_free_acts(m);
-  cudaFree(m->P); cudaFree(m->G); cudaFree(m->M); cudaFree(m->V); cudaFree(m->loss); cudaFree(m->W16);
-  cudaFree(m->W16T); cudaFree(m->err); cudaFree(m->ws);
+  cudaFree(m->P); cudaFree(m->G); cudaFree(m->M); cudaFree(m->V); cudaFree(m->W16T); cudaFree(m->part);
+  cudaFree(m->y);
+  if (m->h_res) cudaFreeHost(const_cast<fim_mlp::Result *>(m->h_res));
   if (m->st) cudaStreamDestroy(m->st);
   delete m;
   return FIM_OK;
@@ -1089,7 +1004,7 @@ extern "C" int fim_mlp_set_params(fim_mlp *m, const float *params)
   MLP_TRY("fim_mlp_set_params", cudaMemcpyAsync(m->P, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice, m->st));
   MLP_TRY("fim_mlp_set_params", cudaMemsetAsync(m->M, 0, sizeof(float) * kMlpParams, m->st));
   MLP_TRY("fim_mlp_set_params", cudaMemsetAsync(m->V, 0, sizeof(float) * kMlpParams, m->st));
-  to_bf16_kernel<<<64, 256, 0, m->st>>>(m->P, m->W16, m->W16T);
+  to_bf16_kernel<<<64, 256, 0, m->st>>>(m->P, m->W16T);
   MLP_TRY("fim_mlp_set_params", cudaGetLastError());
   MLP_TRY("fim_mlp_set_params", cudaStreamSynchronize(m->st));
   m->steps = 0;
@@ -1114,11 +1029,7 @@ extern "C" int fim_mlp_gradients(fim_mlp *m, int64_t n, const void *d_features, 
   int rc;
   if ((rc = mlp_check_n(n, "fim_mlp_gradients")) != FIM_OK) return rc;
   MLP_TRY("fim_mlp_gradients: set device", cudaSetDevice(m->device));
-  if ((rc = mlp_loss_grads(m, n, d_features, d_targets, loss)) != FIM_OK) return rc;
-  MLP_TRY("fim_mlp_gradients", cudaMemcpyAsync(grads, m->G, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->st));
-  MLP_TRY("fim_mlp_gradients", mlp_read_err(m));
-  MLP_TRY("fim_mlp_gradients", cudaStreamSynchronize(m->st));
-  return mlp_gemm_status(m, "fim_mlp_gradients");
+  return mlp_gradients(m, n, d_features, d_targets, 0.f, grads, loss, "fim_mlp_gradients");
 }
 
 extern "C" int fim_mlp_train_step(fim_mlp *m, int64_t n, const void *d_features, const float *d_targets, float lr,
@@ -1132,15 +1043,7 @@ extern "C" int fim_mlp_train_step(fim_mlp *m, int64_t n, const void *d_features,
   int rc;
   if ((rc = mlp_check_n(n, "fim_mlp_train_step")) != FIM_OK) return rc;
   MLP_TRY("fim_mlp_train_step: set device", cudaSetDevice(m->device));
-  if ((rc = mlp_loss_grads(m, n, d_features, d_targets, loss)) != FIM_OK) return rc;
-  const float b1 = 0.9f, b2 = 0.999f;
-  ++m->steps;
-  const float c1 = 1.f - std::pow(b1, (float)m->steps), c2 = 1.f - std::pow(b2, (float)m->steps);
-  adam_kernel<<<64, 256, 0, m->st>>>(kMlpParams, m->P, m->G, m->M, m->V, lr, b1, b2, 1e-8f, c1, c2, m->W16, m->W16T);
-  MLP_TRY("fim_mlp_train_step: adam", cudaGetLastError());
-  MLP_TRY("fim_mlp_train_step", mlp_read_err(m));
-  MLP_TRY("fim_mlp_train_step", cudaStreamSynchronize(m->st));
-  return mlp_gemm_status(m, "fim_mlp_train_step");
+  return mlp_gradients(m, n, d_features, d_targets, lr, nullptr, loss, "fim_mlp_train_step");
 }
 
 extern "C" int fim_mlp_predict(fim_mlp *m, int64_t n, const void *d_features, float *d_out)
@@ -1149,10 +1052,21 @@ extern "C" int fim_mlp_predict(fim_mlp *m, int64_t n, const void *d_features, fl
   int rc;
   if ((rc = mlp_check_n(n, "fim_mlp_predict")) != FIM_OK) return rc;
   MLP_TRY("fim_mlp_predict: set device", cudaSetDevice(m->device));
-  if ((rc = mlp_reserve(m, n)) != FIM_OK) return rc;
-  MLP_TRY("fim_mlp_predict: forward", mlp_forward(m, (int)n, d_features, nullptr));
-  MLP_TRY("fim_mlp_predict", cudaMemcpyAsync(d_out, m->y, sizeof(float) * n, cudaMemcpyDeviceToDevice, m->st));
-  MLP_TRY("fim_mlp_predict", mlp_read_err(m));
+  // The kernel writes the predictions in place unless d_out is not aligned
+  // to a float or overlaps the features it still reads.
+  const uintptr_t x = reinterpret_cast<uintptr_t>(d_features), o = reinterpret_cast<uintptr_t>(d_out);
+  const uintptr_t xn = sizeof(__nv_bfloat16) * kMlpIn * (uintptr_t)n, on = sizeof(float) * (uintptr_t)n;
+  const bool direct = o % sizeof(float) == 0 && (o + on <= x || x + xn <= o);
+  if (!direct && n > m->y_cap) {
+    cudaFree(m->y);
+    m->y = nullptr;
+    m->y_cap = 0;
+    MLP_TRY("fim_mlp: activations", cudaMalloc(&m->y, sizeof(float) * n));
+    m->y_cap = n;
+  }
+  MLP_TRY("fim_mlp_predict: forward", mlp_launch<false>(m, (int)n, d_features, direct ? d_out : m->y, nullptr, nullptr));
+  if (!direct)
+    MLP_TRY("fim_mlp_predict", cudaMemcpyAsync(d_out, m->y, sizeof(float) * n, cudaMemcpyDeviceToDevice, m->st));
   MLP_TRY("fim_mlp_predict", cudaStreamSynchronize(m->st));
-  return mlp_gemm_status(m, "fim_mlp_predict");
+  return mlp_status(m, "fim_mlp_predict");
 }

@@ -138,3 +138,51 @@ def test_training_beats_the_distance_feature_and_warm_solves(F, torch_cuda):
             s.set_warm_start(inf.data_ptr())
             s.solve()
             assert np.array_equal(s.times(with_state=False), m.phi)
+
+
+@pytest.mark.parametrize("n", [64, 128, 19456 + 64, 77888])
+def test_network_tile_counts(F, torch_cuda, n):
+    """One half tile, one tile, just over one tile per SM (152 x 128 rows) and
+    several tiles per CTA and group: predictions and gradients against the
+    restatement, the same bounds as above."""
+    from oracle import mlp_oracle as M
+    torch = torch_cuda
+    p, X, t = _random_problem(M, n, 5)
+    with F.Mlp(seed=3) as mlp:
+        mlp.set_params(p)
+        dX, dt = _to_device_bf16(torch, X), torch.from_numpy(t).cuda()
+        y = torch.full((n + 1,), 7.0, dtype=torch.float32, device="cuda")
+        mlp.predict(n, dX.data_ptr(), y.data_ptr())
+        g, loss = mlp.gradients(n, dX.data_ptr(), dt.data_ptr())
+        g2, loss2 = mlp.gradients(n, dX.data_ptr(), dt.data_ptr())
+    _, _, _, y_o = M.forward(p, X)
+    yg = y.cpu().numpy()
+    assert yg[n] == 7.0  # nothing past the rows is written
+    assert (~np.isclose(yg[:n], y_o, rtol=1e-3, atol=1e-3)).mean() < 0.01
+    assert np.array_equal(g, g2) and loss == loss2  # sums in a fixed order
+    loss_o, g_o = M.loss_and_gradients(p, X, t)
+    assert abs(loss - loss_o) <= 1e-3 * abs(loss_o)
+    for name, (a, b) in M.BLOCKS.items():
+        err = np.linalg.norm(g[a:b] - g_o[a:b]) / max(np.linalg.norm(g_o[a:b]), 1e-12)
+        assert err < 1e-2, (name, err)
+
+
+def test_prediction_into_its_own_features_or_an_odd_address(F, torch_cuda):
+    """Outputs that the kernel cannot write while it reads (over the feature
+    rows) or at all (not aligned to a float) take the copy."""
+    from oracle import mlp_oracle as M
+    torch = torch_cuda
+    n = 512
+    p, X, _ = _random_problem(M, n, 6)
+    with F.Mlp(seed=3) as mlp:
+        mlp.set_params(p)
+        dX = _to_device_bf16(torch, X)
+        y = torch.empty(n, dtype=torch.float32, device="cuda")
+        mlp.predict(n, dX.data_ptr(), y.data_ptr())
+        raw = torch.zeros(4 * n + 8, dtype=torch.uint8, device="cuda")
+        mlp.predict(n, dX.data_ptr(), raw.data_ptr() + 2)
+        odd = raw.cpu().numpy()[2:2 + 4 * n].copy().view(np.float32)
+        assert np.array_equal(odd, y.cpu().numpy())
+        mlp.predict(n, dX.data_ptr(), dX.data_ptr())
+        over = dX.cpu().numpy().reshape(-1)[:2 * n].copy().view(np.float32)
+        assert np.array_equal(over, y.cpu().numpy())

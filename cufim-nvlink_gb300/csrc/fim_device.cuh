@@ -126,6 +126,87 @@ __device__ __forceinline__ double tri_ref(double e12, double e13, double e23, do
   return FIM_INF;
 }
 
+// tri_ref again, its two roots separately and without FP64 divisions and
+// square roots.  Both only ever reach the result rounded to float -- l is a
+// float, and so is the sum that holds the square root -- and a float is
+// decided by an approximation good to 2^-40 unless that lies next to a
+// rounding boundary.  On GB300 the FP64 pipe takes 64 cycles per warp
+// instruction, and a division or square root is nine or ten of them: tri_ref
+// issues about 73 FP64 instructions for its two roots, this 38.
+//   l: q = N / D by the FP32 division (2^-21 relative), its residual
+//      N - q D exactly by one FP64 fma (D is a float), the correction by
+//      another FP32 division: q + dl is off by less than 2^-43 |l|.
+//   sum: s0 = sqrt(Q) by the FP32 reciprocal square root (2^-21), its
+//      residual Q - s0^2 exactly by one FP64 fma, the correction linear:
+//      s0 + d0 is off by less than 2^-42 s0; added to p2 - l p12 in FP64.
+// Where the float is not decided, or an operand is far from 1 (where the
+// bounds above could meet subnormals), tri_root_ref evaluates the root as
+// the reference does.
+struct TriPre {
+  double a, b, c, p2, p12, bpc, stp;
+  float dv;
+};
+
+__device__ __forceinline__ bool tri_prepare(double e12, double e13, double e23, double p1, double p2, TriPre &t)
+{
+  t.a = e23;
+  t.b = -0.5 * (e12 + e23 - e13);
+  t.c = e12;
+  t.p2 = p2;
+  t.p12 = p2 - p1;
+  const float dv = d2f(t.p12 * t.p12 - t.c);
+  const float sv = d2f(f2d(dv) * (t.b * t.b - t.a * t.c));
+  if (!(dv != 0.f && sv >= 0.f)) return false;
+  t.dv = d2f(t.c * f2d(dv));
+  t.bpc = t.b * t.p12 * t.p12 - t.b * t.c;
+  t.stp = f2d(sqrtf(sv)) * t.p12;
+  return true;
+}
+
+static __device__ __noinline__ double tri_root_ref(double a, double b, double c, double p2, double p12, double n, float dv)
+{
+  const float l = d2f(n / f2d(dv));
+  if (!((l >= 0.f) && (l <= 1.f))) return FIM_INF;
+  const double ld = f2d(l);
+  return f2d(d2f(p2 - ld * p12 + sqrt(a + 2.0 * ld * b + f2d(l * l) * c)));
+}
+
+__device__ __forceinline__ bool mid_range(float x) { return fabsf(x) >= 0x1p-60f && fabsf(x) <= 0x1p60f; }
+
+// Root 1 or 2 of the triangle solve: FIM_INF (or NaN) when it has no value.
+__device__ __forceinline__ double tri_root(const TriPre &t, bool second)
+{
+  const double n = -(t.bpc + (second ? t.stp : -t.stp));
+  const float nf = d2f(n);
+  const float q = __fdividef(nf, t.dv);
+  const float dl = __fdividef(d2f(fma(-f2d(q), f2d(t.dv), n)), t.dv);
+  const float l = q + dl, lr = dl - (l - q), lerr = fabsf(l) * 0x1p-42f;  // q + dl == l + lr
+  bool sure = mid_range(t.dv) && mid_range(nf) && fabsf(q) >= 0x1p-40f && fabsf(q) <= 0x1p40f &&
+              l + (lr + lerr) == l && l + (lr - lerr) == l;
+  if (sure) {
+    if (!((l >= 0.f) && (l <= 1.f))) return FIM_INF;
+    const double ld = f2d(l);
+    const double qd = t.a + f2d(2.f * l) * t.b + f2d(l * l) * t.c;
+    const float x = d2f(qd);
+    const float rs = rsqrtf(x), s0 = x * rs;
+    const double s0d = f2d(s0);
+    const float d0 = d2f(fma(-s0d, s0d, qd)) * 0.5f * rs;
+    const double w = t.p2 - ld * t.p12 + s0d + f2d(d0);
+    // (float)w with 2^14 of the FP64 units in the last place to spare on
+    // both sides of the rounding boundary: 2^-40 |w| and more while s0 is at
+    // most 4 |w|
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(w);
+    const uint32_t e = (uint32_t)(bits >> 52) & 0x7ffu, rest = (uint32_t)bits & 0x1fffffffu;
+    uint32_t r = ((e - 896u) << 23) | ((uint32_t)(bits >> 29) & 0x7fffffu);
+    r += rest > 0x10000000u ? 1u : 0u;
+    const float rf = __uint_as_float(r | ((uint32_t)(bits >> 32) & 0x80000000u));
+    sure = x >= 0x1p-60f && x <= 0x1p60f && e - 897u < 253u && rest - (0x10000000u - 0x4000u) > 0x8000u &&
+           s0 <= 4.f * fabsf(rf);
+    if (sure) return f2d(rf);
+  }
+  return tri_root_ref(t.a, t.b, t.c, t.p2, t.p12, n, t.dv);
+}
+
 // solve_tet_cu, cuda_fim.h:1302-1360 (the reference's closed form, term for term)
 __device__ __forceinline__ double tet_ref(double e13, double e23, double e34, double e12, double e14,
                                           double e24, double p1, double p2, double p3)

@@ -13,7 +13,9 @@
 // the largest in [0.5, 4)) as floats and the float copies of the times.
 // Both tet screens are checked (with branches, and the branch-free one the
 // solve uses).  Violations: a solve with a value that a screen calls impossible or puts
-// outside [lb, ub], or a certain upper bound where the solve has no value.
+// outside [lb, ub], or a certain upper bound where the solve has no value; for
+// triangles also any difference between tri_ref and the roots as the solve
+// evaluates them (tri_root).
 //
 // No counterpart in the reference.
 #include "fim_device.cuh"
@@ -129,6 +131,11 @@ __global__ void screen_selftest_kernel(int64_t n, uint64_t seed, unsigned long l
       } else {
         bad = cb.ub < INFINITY;
       }
+      // the solve's own evaluation, root by root
+      TriPre tp;
+      double w = FIM_INF;
+      if (tri_prepare(g[s12], g[s13], g[s23], p[ia], p[ib], tp)) w = fmin(fmin(w, tri_root(tp, false)), tri_root(tp, true));
+      bad = bad || (has ? __double_as_longlong(w) != __double_as_longlong(v) : w < FIM_INF);
       ++cnt[3];
       if (bad) ++cnt[4];
     }

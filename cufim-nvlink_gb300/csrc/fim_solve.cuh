@@ -66,6 +66,23 @@ constexpr int kCornerCap = FIM_CORNER_CAP;    // corners per batch
 constexpr int kTriCap = kCornerCap * 6 / 5;  // triangle screens per batch (more are screened on the spot)
 constexpr int kTetCap = kCornerCap; // tet screens per batch: never full
 constexpr int kQcap = 768;          // exact solves queued per kind and batch (more run on the spot)
+// Up to this many triangle solves of a batch run on two lanes each, one per
+// root: while they fill no more than four warps (one per sub-partition's
+// FP64 pipe) the shorter chain costs nothing (87k shell 2.26 ms with one lane
+// each, 2.19 with 64, 2.20 with 128; the other meshes within 1 %).
+#ifndef FIM_TRI_SPLIT
+#define FIM_TRI_SPLIT 64
+#endif
+constexpr int kTriSplit = FIM_TRI_SPLIT;
+// Batches whose listed solves take at most this many FP64 warp instructions
+// (fp64_cost) skip the screens.  Solve times in ms (9k cube, 17.7k slab, 87k
+// shell, 58k windowed slab, 1M slab) without the direct path 1.30, 1.76, 2.40,
+// 5.74, 12.46; up to 200: 1.13, 1.70, 2.29, 5.16, 12.28; up to 480: 0.98,
+// 1.46, 2.19, 4.77, 12.10; up to 900: 0.97, 1.43, 2.21, 4.73, 12.13.
+#ifndef FIM_DIRECT_COST
+#define FIM_DIRECT_COST 600
+#endif
+constexpr int kDirectCost = FIM_DIRECT_COST;
 // Phase D runs the queued tets on at most FimParams::dag_warps (<=
 // kDagWarpsMax) warps, one group of kDagLanes lanes per tet (scratch:
 // kDagGroups * kDagSlots doubles).
@@ -170,6 +187,19 @@ __device__ __forceinline__ int item_slot(uint32_t it) { return (int)(it & 255u);
 __device__ __forceinline__ int item_kind(uint32_t it) { return (int)((it >> 8) & 3u); }
 __device__ __forceinline__ int item_corner(uint32_t it) { return (int)(it >> 10); }
 
+// Queue item of batch corner j, kind k.
+__device__ __forceinline__ uint32_t list_item(const BatchSh &sh, int j, int k) { return make_item(sh.cs[j], k, j); }
+
+// FP64 warp instructions of phase D for that many tets, triangles and edges
+// (prefix levels and roots of the tets, triangle roots, square roots).
+__device__ __forceinline__ int fp64_cost(int ntet, int ntri, int nedge, int dag_warps)
+{
+  const int tw = (ntet * kDagLanes + 31) / 32;
+  return kDagLevels * tw + 50 * ((2 * ntet + 31) / 32) + (ntri <= kTriSplit ? 28 * ((2 * ntri + 31) / 32)
+                                                                             : 38 * ((ntri + 31) / 32)) +
+         12 * ((nedge + 31) / 32) + (tw > dag_warps ? 100000 : 0);
+}
+
 // Appends one item per lane with `need` to a list (warp-ballot compaction;
 // every lane of the warp takes part).  Returns the item's position, or -1.
 __device__ __forceinline__ int warp_append(int *counter, bool need, int lane)
@@ -217,10 +247,10 @@ __device__ __forceinline__ double exact_solve(const FimDev &d, const double *ph,
   return tri_ref(e12, e13, e23, pa, pb);
 }
 
-// FP64 triangle solve kind 0..2 of corner c (exact_solve without its tet
-// branch, for the warps that run only triangle solves).
+// Roots r0 .. r1 - 1 (of two) of the FP64 triangle solve kind 0..2 of corner
+// c (the fmin of both is tri_ref's value).
 __device__ __forceinline__ double exact_tri(const FimDev &d, const double *ph, int64_t c, int kind,
-                                            const int32_t *nb)
+                                            const int32_t *nb, int r0, int r1)
 {
   const double pa = __ldcg(ph + (kind == 1 ? nb[1] : nb[0])), pb = __ldcg(ph + (kind == 0 ? nb[1] : nb[2]));
   const double2 *gp = reinterpret_cast<const double2 *>(d.cgeo + kCgeoStride * c);
@@ -228,7 +258,13 @@ __device__ __forceinline__ double exact_tri(const FimDev &d, const double *ph, i
   const double e12 = kind == 0 ? t1.y : (kind == 1 ? t0.y : t0.x);
   const double e13 = kind == 1 ? t2.y : t2.x;
   const double e23 = kind == 0 ? t2.y : t1.x;
-  return tri_ref(e12, e13, e23, pa, pb);
+  TriPre t;
+  double val = FIM_INF;
+  if (tri_prepare(e12, e13, e23, pa, pb, t)) {
+#pragma unroll 1
+    for (int r = r0; r < r1; ++r) val = fmin(val, tri_root(t, r != 0));
+  }
+  return val;
 }
 
 // Position of e14, e24, e34 (the edges from neighbour 0, 1, 2 to the corner's
@@ -623,6 +659,12 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     __syncthreads();
     PROBE(kPrB);
 
+    // Few listed solves go to phase D as they are (direct): the screens' chain
+    // is as long for one solve as for 32, and so is that of the FP64 solves,
+    // so dropping the screens shortens the phase.
+    const bool direct = !exact_all && !fp32 && sh.ntri <= kTriCap &&
+                        fp64_cost(sh.ntet, sh.ntri, 3 * sh.nedge, dag_warps) <= kDirectCost;
+
     // S: screens over the compacted lists, handed out in chunks to whichever
     // warp is free -- tets first (32 per chunk, one per lane), then triangles
     // from the next chunk boundary (64 per chunk: each lane screens two with
@@ -631,7 +673,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     // chunk; a solve whose lower bound does not exceed the current bhi is
     // queued at once (bhi only decreases: phase D rechecks against the final
     // bound)
-    {
+    if (!direct) {
       const int ntet = min(sh.ntet, kTetCap), ntri = min(sh.ntri, kTriCap);
       const int tri0 = (ntet + 31) & ~31;
       const int edge_c0 = tri0 + ((ntri + 63) / 64) * 32;  // claim index of the first edge chunk
@@ -761,8 +803,8 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
         }
 #undef PROBE_CHUNK
       }
+      __syncthreads();
     }
-    __syncthreads();
     PROBE(kPrS);
 #ifdef FIM_PROBE
     __shared__ unsigned long long s_d_start, s_d_tri_end;
@@ -773,7 +815,10 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     // D: exact solves; tets (a lane group each) from thread 0, triangles and
     // edges each from the next warp boundary
     {
-      const int ntet = min(sh.nq[0], kQcap), ntri = min(sh.nq[1], kQcap), nedge = min(sh.nq[2], kQcap);
+      // (direct: the screen lists, with every edge of a listed corner; their
+      // lower bounds are at most bhi, which phase A left final)
+      const int ntet = direct ? sh.ntet : min(sh.nq[0], kQcap), ntri = direct ? sh.ntri : min(sh.nq[1], kQcap);
+      const int nedge = direct ? 3 * sh.nedge : min(sh.nq[2], kQcap);
       // tets: one group of kDagLanes lanes per tet runs the prefix
       // (tet_dag_prefix); then the roots, two per tet, on consecutive
       // threads from thread 0, so that they fill as few warps as possible
@@ -797,9 +842,9 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
           int slot = 0;
           bool run = false;
           if (pos < ntet) {
-            const uint32_t it = sh.q[0][pos];
+            const uint32_t it = direct ? list_item(sh, sh.tet[pos], 3) : sh.q[0][pos];
             slot = item_slot(it);
-            run = !(sh.qlb[0][pos] > funkey(sh.bhi[slot]));  // else overtaken by a later bound
+            run = direct || !(sh.qlb[0][pos] > funkey(sh.bhi[slot]));  // else overtaken by a later bound
             if (run) {
               const int jj = item_corner(it);
               const int64_t c = sh.c0[slot] + (jj - sh.cp[slot]);
@@ -816,9 +861,9 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
           asm volatile("bar.sync 1, %0;" ::"r"(tri0) : "memory");
           const int rpos = base + (tid >> 1);  // root (tid & 1) of tet rpos
           if (tid < 2 * ngrp && rpos < ntet) {
-            const uint32_t it = sh.q[0][rpos];
+            const uint32_t it = direct ? list_item(sh, sh.tet[rpos], 3) : sh.q[0][rpos];
             const int rslot = item_slot(it);
-            if (!(sh.qlb[0][rpos] > funkey(sh.bhi[rslot]))) {
+            if (direct || !(sh.qlb[0][rpos] > funkey(sh.bhi[rslot]))) {
               const double v = tet_root_tail(sh.dag[tid >> 1], (tid & 1) != 0);
               if ((tid & 1) == 0) ++n_exact;
               if (v < FIM_INF) atomicMin(&sh.res[rslot], dkey(v));
@@ -833,22 +878,36 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
         }
 #endif
       }
-      const int edge0 = tri0 + ((ntri + 31) & ~31);
+      // triangles: one lane each, or with few of them one lane per root
+      const bool split = ntri <= kTriSplit;
+      const int ntl = split ? 2 * ntri : ntri;
+      const int edge0 = tri0 + ((ntl + 31) & ~31);
       for (int j = tid; j < edge0 + nedge; j += kThreads) {  // threads past the tets' warps: concurrently
-        int qi, pos;
+        int qi, pos, r0 = 0, r1 = 2;
         if (j < tri0) continue;
-        else if (j < tri0 + ntri) { qi = 1; pos = j - tri0; }
+        else if (j < tri0 + ntl) {
+          qi = 1; pos = j - tri0;
+          if (split) { r0 = pos & 1; r1 = r0 + 1; pos >>= 1; }
+        }
         else if (j >= edge0) { qi = 2; pos = j - edge0; }
         else continue;
-        const uint32_t it = sh.q[qi][pos];
-        if (sh.qlb[qi][pos] > funkey(sh.bhi[item_slot(it)])) continue;  // overtaken by a later bound
+        uint32_t it;
+        if (direct) {
+          const int l = qi == 1 ? (int)sh.tri[pos] : (int)sh.edg[pos / 3];
+          it = list_item(sh, l & 0x3fff, qi == 1 ? l >> 14 : pos % 3);
+          if (qi == 2 && !((sh.vm[item_corner(it)] >> item_kind(it)) & 1u)) continue;  // no such edge
+        } else {
+          it = sh.q[qi][pos];
+          if (sh.qlb[qi][pos] > funkey(sh.bhi[item_slot(it)])) continue;  // overtaken by a later bound
+        }
         const int slot = item_slot(it), kind = item_kind(it), jj = item_corner(it);
         const int64_t c = sh.c0[slot] + (jj - sh.cp[slot]);
         int32_t nb[3];
         corner_nb(d, c, nb);
-        const double val = qi == 2 ? exact_edge(d, ph, c, kind, pick3(nb, kind)) : exact_tri(d, ph, c, kind, nb);
+        const double val = qi == 2 ? exact_edge(d, ph, c, kind, pick3(nb, kind))
+                                   : exact_tri(d, ph, c, kind, nb, r0, r1);
         if (val < FIM_INF) atomicMin(&sh.res[slot], dkey(val));
-        if (qi < 2) ++n_exact;
+        if (qi < 2 && r0 == 0) ++n_exact;
 #ifdef FIM_PROBE
         atomicMax(&s_d_tri_end, global_timer());
 #endif

@@ -257,23 +257,35 @@ __device__ __forceinline__ double tet_ref(double e13, double e23, double e34, do
 // expression tree).
 #include "tet_dag.inc"
 
+// x with its sign flipped where the word `flip` has its top bit set
 __device__ __forceinline__ double flip_sign(double x, uint32_t flip)
 {
-  return __longlong_as_double(__double_as_longlong(x) ^ ((unsigned long long)(flip != 0u) << 63));
+  return __hiloint2double(__double2hiint(x) ^ (int)flip, __double2loint(x));
 }
 
 // Runs the level program on scratch S (leaves already stored); gl is the
-// lane's index in its group.  All lanes of the warp take part.
+// lane's index in its group.  All lanes of the warp take part.  A lane's
+// program words are loaded four levels ahead: read level by level from
+// constant memory, with eight addresses per warp, they lengthened every level
+// of the chain.
 __device__ __forceinline__ void tet_dag_prefix(double *S, int gl)
 {
+  const uint4 *prog = kTetDagProg[gl];
+  uint4 next = __ldg(prog);
 #pragma unroll
-  for (int lv = 0; lv < kDagLevels; ++lv) {
-    const uint32_t w = kTetDagProg[lv][gl];
-    const double A = flip_sign(S[w & 255u], w & (1u << 24));
-    const double B = flip_sign(S[(w >> 8) & 255u], w & (1u << 25));
-    const double C = flip_sign(S[(w >> 16) & 255u], w & (1u << 26));
-    S[kDagLeaves + lv * kDagLanes + gl] = fma(A, B, C);
-    __syncwarp();
+  for (int l4 = 0; l4 < kDagLevels / 4; ++l4) {
+    const uint4 q = next;
+    if (l4 + 1 < kDagLevels / 4) next = __ldg(prog + l4 + 1);
+    const uint32_t ws[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t w = ws[k];
+      const double A = flip_sign(S[w & 255u], (w << 7) & 0x80000000u);
+      const double B = S[(w >> 8) & 255u];
+      const double C = flip_sign(S[(w >> 16) & 255u], (w << 5) & 0x80000000u);
+      S[kDagLeaves + (4 * l4 + k) * kDagLanes + gl] = fma(A, B, C);
+      __syncwarp();
+    }
   }
 }
 
@@ -362,10 +374,14 @@ __device__ __forceinline__ int ld_volatile_i32(const int32_t *p)
 // next flip needs its own arrival.  Every wait is bounded by timeout_ns of
 // %globaltimer and by a spin cap; on expiry the block records KERR_TIMEOUT
 // and the phase, and every block leaves the kernel at its next barrier.
-// Returns false when the caller must return.
-static __device__ bool grid_sync(FimCtl *ctl, uint32_t nblocks, uint64_t timeout_ns, int where)
+// Returns false when the caller must return.  *count (optional) receives the
+// list length at `counter`, which no block changes until the next barrier: it
+// is read together with the error word, one round trip to the L2 instead of
+// two.
+static __device__ bool grid_sync(FimCtl *ctl, uint32_t nblocks, uint64_t timeout_ns, int where,
+                                 const int32_t *counter = nullptr, int32_t *count = nullptr)
 {
-  __shared__ int s_ok;
+  __shared__ int s_ok, s_count;
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
@@ -385,10 +401,13 @@ static __device__ bool grid_sync(FimCtl *ctl, uint32_t nblocks, uint64_t timeout
         }
       }
     }
-    if (ok && ld_volatile_i32(&ctl->error) != KERR_NONE) ok = 0;
+    const int32_t err = ld_volatile_i32(&ctl->error);
+    if (counter) s_count = ld_volatile_i32(counter);
+    if (err != KERR_NONE) ok = 0;
     s_ok = ok;
   }
   __syncthreads();
+  if (counter) *count = s_count;
   return s_ok != 0;
 }
 

@@ -1138,10 +1138,11 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
 }
 
 // Grid barrier with its wait accounted in the phase probe.
-__device__ __forceinline__ bool grid_sync_probed(const FimDev &d, uint32_t nblocks, uint64_t timeout_ns, int where)
+__device__ __forceinline__ bool grid_sync_probed(const FimDev &d, uint32_t nblocks, uint64_t timeout_ns, int where,
+                                                 const int32_t *counter = nullptr, int32_t *count = nullptr)
 {
   PROBE(kPrLight);  // whatever ran since the last mark
-  const bool ok = grid_sync(d.ctl, nblocks, timeout_ns, where);
+  const bool ok = grid_sync(d.ctl, nblocks, timeout_ns, where, counter, count);
   PROBE(kPrBarrier);
   (void)d;
   return ok;
@@ -1243,13 +1244,13 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
       }
       if (stv == ST_NARROW) append_active(d.list[s], &ctl->n_narrow[s], (int32_t)v);
     }
-    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+    int32_t nn = 0, nm = 0;  // lengths of the narrow and the marked list
+    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_narrow[s], &nn)) return;
 
     int64_t it_window = 0;
     for (;;) {
       s = (int)(it % 3);
       const int s1 = (int)((it + 1) % 3), s2 = (int)((it + 2) % 3);
-      const int32_t nn = ld_volatile_i32(&ctl->n_narrow[s]);
       if (nn == 0) break;
       if ((p.max_iter > 0 && it_window >= p.max_iter) || it >= kMaxStampIterations) {
         if (gtid == 0 && atomicCAS(&ctl->error, KERR_NONE, KERR_MAX_ITER) == KERR_NONE) ctl->error_where = where;
@@ -1272,7 +1273,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         update_phase<kNarrow2>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
                                lo, my_evals, my_exact);
         my_updates += (gtid == 0) ? nn : 0;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_marked[s], &nm)) return;
 
         // Y -- apply the narrow list's times and states (the block's share
         // of the list, cuda_fim.cu:2291-2317), then re-solve the marked
@@ -1306,19 +1307,19 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
           }
         }
         PROBE(kPrLight);
-        const int32_t nm = ld_volatile_i32(&ctl->n_marked[s]);
         update_phase<kMarked2>(d, sh, d.lmarked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0,
                                stamp, dag, lo, my_evals, my_exact);
         my_updates += (gtid == 0) ? nm : 0;
         ++it;
         ++it_window;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_narrow[s1], &nn)) return;
       } else {
         // P1 -- solve on elements + reduce per vertex (cuda_fim.cu:2102-2163)
         update_phase<kNarrow4>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
                                lo, my_evals, my_exact);
         my_updates += (gtid == 0) ? nn : 0;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+        int32_t nf = 0;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_frozen[s], &nf)) return;
 
         // P2 -- apply the narrow times; mark downwind neighbours of the
         // vertices frozen now (cuda_fim.cu:2172-2205).  The two are
@@ -1329,7 +1330,6 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
           const int32_t v = lst[i];
           set_phi(d, v, __ldcg(d.phi2 + v));
         }
-        const int32_t nf = ld_volatile_i32(&ctl->n_frozen[s]);
         for (int64_t i = gtid / kMarkLanes; i < nf; i += nthreads / kMarkLanes) {
           const int32_t n = d.lfrozen[i];
           const double pn = __ldcg(d.phi2 + n);
@@ -1347,7 +1347,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
             }
           }
         }
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_marked[s], &nm)) return;
 
         // P3 -- the narrow vertices that are not re-solved now go to the next
         // list (or freeze), then the marked neighbours are re-solved
@@ -1365,13 +1365,12 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
             else append_active(lnext, &ctl->n_narrow[s1], v);
           }
         }
-        const int32_t nm = ld_volatile_i32(&ctl->n_marked[s]);
         update_phase<kMarked3>(d, sh, d.lmarked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0,
                                stamp, dag, lo, my_evals, my_exact);
         my_updates += (gtid == 0) ? nm : 0;
         ++it;
         ++it_window;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_narrow[s1], &nn)) return;
       }
     }
   }

@@ -14,9 +14,9 @@ reassociation: the tree is the one C++ builds, left to right, unary minus
 binding tightest).  Identical subexpressions are evaluated once.
 
 The nodes are list-scheduled onto kDagLanes lanes, most critical path first.
-Output: for every level and lane one word
+Output: for every lane and level one word
     bits 0-7 slot of A, 8-15 slot of B, 16-23 slot of C,
-    bits 24-26 sign flips of A, B, C
+    bits 24 and 26 sign flips of A and C (no node flips B)
 and the slots of the named results.  The node of level L and lane l writes
 slot kDagLeaves + L * kDagLanes + l.
 
@@ -188,6 +188,8 @@ def main():
             a, b, c = slot(x), ONE, slot(y)
             flips = (x[1], False, y[1] != (op == "sub"))
         word = a | (b << 8) | (c << 16)
+        if flips[1]:
+            raise ValueError("a negated second factor")
         for k, f in enumerate(flips):
             if f:
                 word |= 1 << (24 + k)
@@ -213,9 +215,12 @@ def main():
         "constexpr int kDagLeafE13 = 0, kDagLeafP1 = 6, kDagLeafConst = 9;",
     ]
     lines.append("constexpr int " + ", ".join("kDagOut_%s = %d" % (n, out[n]) for n in OUTPUTS) + ";")
-    lines.append("__constant__ uint32_t kTetDagProg[kDagLevels][kDagLanes] = {")
-    for lv in range(levels):
-        lines.append("  {" + ", ".join("0x%08xu" % w for w in prog[lv]) + "},")
+    if levels % 4:
+        raise ValueError("the levels of a lane are loaded four at a time")
+    lines.append("__device__ const uint4 kTetDagProg[kDagLanes][kDagLevels / 4] = {")
+    for ln in range(LANES):
+        lines.append("  {" + ",\n   ".join("{" + ", ".join("0x%08xu" % prog[lv + k][ln] for k in range(4)) + "}"
+                                           for lv in range(0, levels, 4)) + "},")
     lines.append("};")
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tet_dag.inc")
     with open(path, "w") as fh:

@@ -83,6 +83,9 @@ constexpr int kTriSplit = FIM_TRI_SPLIT;
 #define FIM_DIRECT_COST 600
 #endif
 constexpr int kDirectCost = FIM_DIRECT_COST;
+// Corners of a batch whose vertex ids stay in shared memory (over the queues)
+// for phase D: one L2 round trip less in its chain.
+constexpr int kIdsCap = 2 * kQcap;
 // Phase D runs the queued tets on at most FimParams::dag_warps (<=
 // kDagWarpsMax) warps, one group of kDagLanes lanes per tet (scratch:
 // kDagGroups * kDagSlots doubles).
@@ -160,8 +163,13 @@ struct BatchSh {
   uint16_t tri[kTriCap];
   uint16_t tet[kTetCap];
   uint16_t edg[kCornerCap];         // corners whose best edge can still be the minimum (phase B): never full
-  uint32_t q[3][kQcap];             // queued exact solves: [0] tets, [1] triangles, [2] edges
-  float qlb[3][kQcap];              // their lower bounds (rechecked against the final bhi)
+  union {
+    struct {
+      uint32_t q[3][kQcap];         // queued exact solves: [0] tets, [1] triangles, [2] edges
+      float qlb[3][kQcap];          // their lower bounds (rechecked against the final bhi)
+    };
+    int32_t ids[kIdsCap][3];        // batches of up to kIdsCap corners without queues (direct): the corners' other vertices
+  };
   int ntri, ntet, nedge, nq[3];
   int next_item;                    // next unclaimed screen item (phase S)
   int wsum[kSlots / 32];            // corner counts of each warp's 32 slots (setup)
@@ -402,6 +410,53 @@ __device__ __forceinline__ void set_phi_both(const FimDev &d, int64_t v, double 
   d.phi2[v] = x; d.phi2_f[v] = f;
 }
 
+// Work of another list that runs inside a phase: load() starts its loads
+// beside the first batch's, store() uses them once that batch is set up.
+struct NoSide {
+  __device__ __forceinline__ void load() {}
+  __device__ __forceinline__ void store() {}
+};
+// Phase Y's share of the narrow list: the new time of vertex lst[i] (one per
+// thread; none for i < 0) into the times, its state, the next list.
+struct ApplySide {
+  const FimDev &d;
+  const int32_t *lst;
+  int64_t i;
+  uint32_t stamp;
+  int32_t *next, *n_next;
+  bool pending;       // store() still to run (the same on every thread)
+  int32_t v = 0;
+  uint32_t w = 0;
+  uint8_t tv = 0;
+  double x = 0.0;
+  float xf = 0.f;
+  __device__ __forceinline__ void load()
+  {
+    if (!pending || i < 0) return;
+    v = lst[i];
+    w = __ldcg(d.sw + v);
+    tv = __ldcg(d.tst + v);
+    x = __ldcg(d.phi2 + v);
+    xf = __ldcg(d.phi2_f + v);
+  }
+  __device__ __forceinline__ void store()
+  {
+    if (!pending) return;
+    pending = false;
+    bool push = false;
+    if (i >= 0 && sw_stamp(w) != stamp) {  // (a narrow vertex is never marked here)
+      d.phi[v] = x;
+      d.phi_f[v] = xf;
+      if (sw_state(w) == ST_NARROW) {
+        if (tv == ST_FROZEN) d.sw[v] = ST_FROZEN;
+        else push = true;
+      }
+    }
+    const int p = warp_append(n_next, push, threadIdx.x & 31);
+    if (p >= 0) next[p] = v;
+  }
+};
+
 // Where an update phase appends the vertices of the next narrow list, and
 // the counters of this iteration's lists.
 struct ListOut {
@@ -451,11 +506,11 @@ struct ListOut {
 // list's new times live there until the phase applies them).  The minimum
 // over everything equals the reference's update_per_element minimum over
 // all corners (cuda_fim.h:1362-1411).
-template <int MODE>
+template <int MODE, class Side = NoSide>
 __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, int32_t n, double lower,
                              float lower_lo, float lower_hi, double phi_start, double dt, bool exact_all, bool fp32,
                              uint32_t stamp, int dag_warps, const ListOut &lo_, int64_t &n_filtered,
-                             int64_t &n_exact)
+                             int64_t &n_exact, Side &side)
 {
   constexpr bool kMarkedMode = is_marked_mode(MODE);
   const double *ph = MODE == kMarked2 ? d.phi2 : d.phi;      // times this phase reads
@@ -469,6 +524,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     PROBE_COUNT(kPrBatches);
     // batch: the longest run of vertices with <= kCornerCap corners (>= 1 vertex)
     const int cand = (int)min((int64_t)kSlots, lend - pos);
+    side.load();
     if (tid < cand) {
       const int32_t v = __ldcg(list + pos + tid);
       const double old = __ldcg(ph + v);
@@ -521,6 +577,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     const int total = sh.cp[nslot];     // may exceed kCornerCap for a single huge vertex
     const int kept = min(total, kCornerCap);
     __syncthreads();
+    side.store();
     PROBE(kPrSetup);
 
     // A: load, validity, float edge bounds.  Every thread walks its corners
@@ -575,6 +632,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
             elo = fminf(elo, re_lo(E));
           }
           sh.pf[j][i] = pf[i];
+          if (kept <= kIdsCap) sh.ids[j][i] = nbs[i];
         }
         // lower bounds of the triangle pairs and the tet: min(times) +
         // root-term bound (fp16, rounded down), for phase B's screen lists
@@ -819,6 +877,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
       // lower bounds are at most bhi, which phase A left final)
       const int ntet = direct ? sh.ntet : min(sh.nq[0], kQcap), ntri = direct ? sh.ntri : min(sh.nq[1], kQcap);
       const int nedge = direct ? 3 * sh.nedge : min(sh.nq[2], kQcap);
+      const bool shared_ids = direct && kept <= kIdsCap;
       // tets: one group of kDagLanes lanes per tet runs the prefix
       // (tet_dag_prefix); then the roots, two per tet, on consecutive
       // threads from thread 0, so that they fill as few warps as possible
@@ -850,7 +909,8 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
               const int64_t c = sh.c0[slot] + (jj - sh.cp[slot]);
               // leaves: e13 e23 e34 e12 e14 e24 p1 p2 (lanes 0..7), p3, 0.5 2.0 1.0 -0.0
               int32_t nb[3];
-              corner_nb(d, c, nb);
+              if (shared_ids) { nb[0] = sh.ids[jj][0]; nb[1] = sh.ids[jj][1]; nb[2] = sh.ids[jj][2]; }
+              else corner_nb(d, c, nb);
               S[gl] = gl < 6 ? __ldg(d.cgeo + kCgeoStride * c + gl) : __ldcg(ph + (gl == 6 ? nb[0] : nb[1]));
               if (gl == 0) S[kDagLeafP1 + 2] = __ldcg(ph + nb[2]);
               else if (gl <= 4) S[kDagLeafConst + gl - 1] = gl == 1 ? 0.5 : (gl == 2 ? 2.0 : (gl == 3 ? 1.0 : -0.0));
@@ -903,7 +963,8 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
         const int slot = item_slot(it), kind = item_kind(it), jj = item_corner(it);
         const int64_t c = sh.c0[slot] + (jj - sh.cp[slot]);
         int32_t nb[3];
-        corner_nb(d, c, nb);
+        if (shared_ids) { nb[0] = sh.ids[jj][0]; nb[1] = sh.ids[jj][1]; nb[2] = sh.ids[jj][2]; }
+        else corner_nb(d, c, nb);
         const double val = qi == 2 ? exact_edge(d, ph, c, kind, pick3(nb, kind))
                                    : exact_tri(d, ph, c, kind, nb, r0, r1);
         if (val < FIM_INF) atomicMin(&sh.res[slot], dkey(val));
@@ -1034,6 +1095,7 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
                              int64_t &my_evals, int64_t &my_exact, int64_t &my_updates, int where)
 {
   __shared__ int32_t b_narrow[3], b_frozen, b_marked;
+  NoSide none;
   const int tid = threadIdx.x;
   const int32_t c0 = d.blk_ptr[blockIdx.x], c1 = d.blk_ptr[blockIdx.x + 1];
   int s = (int)(it % 3);
@@ -1077,7 +1139,7 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
 
     // P1 -- update the narrow list
     update_phase<kNarrow4>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0,
-                           p.fp32 != 0, stamp, dag, lo, my_evals, my_exact);
+                           p.fp32 != 0, stamp, dag, lo, my_evals, my_exact, none);
     if (tid == 0) my_updates += nn;
     // P2 -- apply; mark the downwind neighbours of the vertices frozen now
     for (int32_t i = tid; i < nn; i += kThreads) {
@@ -1104,7 +1166,7 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
     // P3 -- re-solve the marked neighbours
     const int32_t nm = b_marked;
     update_phase<kMarked4>(d, sh, lo.marked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0,
-                           p.fp32 != 0, stamp, dag, lo, my_evals, my_exact);
+                           p.fp32 != 0, stamp, dag, lo, my_evals, my_exact, none);
     if (tid == 0) my_updates += nm;
     // P4 -- apply, decided states, next narrow list
     for (int32_t i = tid; i < nm + nn; i += kThreads) {
@@ -1166,6 +1228,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
   int where = 0;
   extern __shared__ __align__(16) unsigned char fim_smem[];
   BatchSh &sh = *reinterpret_cast<BatchSh *>(fim_smem);
+  NoSide none;
   const int dag = min(max(p.dag_warps, 1), kDagWarps);
   PROBE(-1);
 
@@ -1271,7 +1334,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         // X -- update the narrow list, mark the downwind neighbours of the
         // vertices frozen now (cuda_fim.cu:2102-2205)
         update_phase<kNarrow2>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
-                               lo, my_evals, my_exact);
+                               lo, my_evals, my_exact, none);
         my_updates += (gtid == 0) ? nn : 0;
         if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_marked[s], &nm)) return;
 
@@ -1279,36 +1342,24 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         // of the list, cuda_fim.cu:2291-2317), then re-solve the marked
         // neighbours (cuda_fim.cu:2215-2289), which read the new times from
         // phi2 and see every marked vertex as "neig"
-        {
-          const int64_t per_block = ((int64_t)nn + gridDim.x - 1) / gridDim.x;
-          const int64_t lbeg = min((int64_t)nn, (int64_t)blockIdx.x * per_block);
-          const int64_t lend = min((int64_t)nn, lbeg + per_block);
-          for (int64_t i0 = lbeg; i0 < lend; i0 += kThreads) {
-            const int64_t i = i0 + threadIdx.x;
-            bool push = false;
-            int32_t v = 0;
-            if (i < lend) {
-              v = lst[i];
-              const uint32_t w = __ldcg(d.sw + v);
-              const uint8_t tv = __ldcg(d.tst + v);
-              const double x = __ldcg(d.phi2 + v);
-              const float xf = __ldcg(d.phi2_f + v);
-              if (sw_stamp(w) != stamp) {  // (a narrow vertex is never marked here)
-                d.phi[v] = x;
-                d.phi_f[v] = xf;
-                if (sw_state(w) == ST_NARROW) {
-                  if (tv == ST_FROZEN) d.sw[v] = ST_FROZEN;
-                  else push = true;
-                }
-              }
-            }
-            const int pp = warp_append(lo.n_next, push, lane);
-            if (pp >= 0) lnext[pp] = v;
-          }
+        const int64_t per_block = ((int64_t)nn + gridDim.x - 1) / gridDim.x;
+        const int64_t lbeg = min((int64_t)nn, (int64_t)blockIdx.x * per_block);
+        const int64_t lend = min((int64_t)nn, lbeg + per_block);
+        ApplySide side{d, lst, -1, stamp, lnext, lo.n_next, true};
+        int64_t i0 = lbeg;
+        for (; i0 + kThreads < lend; i0 += kThreads) {  // all but the last round
+          side.i = i0 + threadIdx.x;
+          side.pending = true;
+          side.load();
+          side.store();
         }
+        side.i = i0 + threadIdx.x < lend ? i0 + threadIdx.x : -1;
+        side.pending = i0 < lend;
         PROBE(kPrLight);
         update_phase<kMarked2>(d, sh, d.lmarked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0,
-                               stamp, dag, lo, my_evals, my_exact);
+                               stamp, dag, lo, my_evals, my_exact, side);
+        side.load();  // (a block without marked vertices)
+        side.store();
         my_updates += (gtid == 0) ? nm : 0;
         ++it;
         ++it_window;
@@ -1316,7 +1367,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
       } else {
         // P1 -- solve on elements + reduce per vertex (cuda_fim.cu:2102-2163)
         update_phase<kNarrow4>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
-                               lo, my_evals, my_exact);
+                               lo, my_evals, my_exact, none);
         my_updates += (gtid == 0) ? nn : 0;
         int32_t nf = 0;
         if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_frozen[s], &nf)) return;
@@ -1366,7 +1417,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
           }
         }
         update_phase<kMarked3>(d, sh, d.lmarked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0,
-                               stamp, dag, lo, my_evals, my_exact);
+                               stamp, dag, lo, my_evals, my_exact, none);
         my_updates += (gtid == 0) ? nm : 0;
         ++it;
         ++it_window;

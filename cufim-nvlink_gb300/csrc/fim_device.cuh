@@ -355,59 +355,61 @@ __device__ __forceinline__ uint64_t global_timer()
   return t;
 }
 
-__device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p)
-{
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ int ld_volatile_i32(const int32_t *p)
 {
   return *(const volatile int32_t *)p;
 }
 
-// All blocks of the (co-resident) grid meet here.  One arrival word: block 0
-// adds 2^31 - (nblocks - 1), every other block adds 1, so the top bit flips
-// exactly when the last block arrives (and the low bits return to zero);
-// everyone waits for the flip.  A block cannot be two flips behind, since the
-// next flip needs its own arrival.  Every wait is bounded by timeout_ns of
-// %globaltimer and by a spin cap; on expiry the block records KERR_TIMEOUT
-// and the phase, and every block leaves the kernel at its next barrier.
-// Returns false when the caller must return.  *count (optional) receives the
-// list length at `counter`, which no block changes until the next barrier: it
-// is read together with the error word, one round trip to the L2 instead of
-// two.
-static __device__ bool grid_sync(FimCtl *ctl, uint32_t nblocks, uint64_t timeout_ns, int where,
-                                 const int32_t *counter = nullptr, int32_t *count = nullptr)
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p)
+{
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// All blocks of the (co-resident) grid meet here, for barrier k (1, 2, ...):
+// each adds 1 to the low half of the phase's word (FimCtl::phase) and waits
+// until all have.  *count receives the high half, the length of the list that
+// the phase appended to: one L2 round trip less per phase than reading it
+// after the barrier.  Every wait is bounded by timeout_ns of %globaltimer and
+// by a spin cap; on expiry the block records KERR_TIMEOUT and the phase and
+// sets the word's error bit, and every block leaves the kernel at its next
+// barrier.  Returns false when the caller must return.
+constexpr uint32_t kPhaseError = 0x80000000u;
+static __device__ bool grid_sync(FimCtl *ctl, uint32_t nblocks, uint64_t timeout_ns, int k, int32_t *count)
 {
   __shared__ int s_ok, s_count;
   __syncthreads();
   if (threadIdx.x == 0) {
-    int ok = 1;
-    const uint32_t inc = blockIdx.x == 0 ? 0x80000000u - (nblocks - 1u) : 1u;
+    unsigned long long *word = &ctl->phase[k & 3].v;
+    // the word of phase k + 2, last used by barrier k - 2, which every block has left
+    if (blockIdx.x == 0) ctl->phase[(k + 2) & 3].v = 0ull;
     __threadfence();
-    const uint32_t old = atomicAdd(&ctl->bar_count, inc);
+    atomicAdd(word, 1ull);
     const uint64_t t0 = global_timer();
     uint32_t spins = 0;
-    while (((ld_acquire_u32(&ctl->bar_count) ^ old) & 0x80000000u) == 0u) {
+    int ok = 1;
+    unsigned long long w;
+    for (;;) {
+      w = ld_acquire_u64(word);
+      if ((uint32_t)w >= nblocks) break;  // everyone is here (or the error bit is set)
       ++spins;
       if ((spins & 255u) == 0u) {
         if (ld_volatile_i32(&ctl->error) != KERR_NONE) { ok = 0; break; }
         if (global_timer() - t0 > timeout_ns || spins > (1u << 30)) {
-          if (atomicCAS(&ctl->error, KERR_NONE, KERR_TIMEOUT) == KERR_NONE) ctl->error_where = where;
+          if (atomicCAS(&ctl->error, KERR_NONE, KERR_TIMEOUT) == KERR_NONE) ctl->error_where = k;
+          atomicOr(word, (unsigned long long)kPhaseError);
           ok = 0;
           break;
         }
       }
     }
-    const int32_t err = ld_volatile_i32(&ctl->error);
-    if (counter) s_count = ld_volatile_i32(counter);
-    if (err != KERR_NONE) ok = 0;
+    if ((uint32_t)w & kPhaseError) ok = 0;
     s_ok = ok;
+    s_count = (int32_t)(w >> 32);
   }
   __syncthreads();
-  if (counter) *count = s_count;
+  *count = s_count;
   return s_ok != 0;
 }
 

@@ -34,15 +34,15 @@ constexpr int kSolveThreads = FIM_SOLVE_THREADS;
 // Kernel error codes written into FimCtl::error.
 enum : int { KERR_NONE = 0, KERR_TIMEOUT = 1, KERR_MAX_ITER = 2 };
 
-// Device control block: counters of the three rotating list slots, the grid
-// barrier, the error word and statistics.  Lives in device memory; the host
-// clears it before every launch.
+// Device control block: the words of the grid-synchronised phases, the error
+// word and statistics.  Lives in device memory; the host clears it before
+// every launch.
 struct FimCtl {
-  int32_t n_narrow[3];      // narrow list length of the iteration using this slot
-  int32_t n_frozen[3];      // vertices frozen in that iteration
-  int32_t n_marked[3];      // neighbours re-solved in that iteration
-  uint32_t bar_count;       // grid barrier arrival word (its top bit flips at every barrier)
-  uint32_t bar_pad;
+  // Phase k (the stretch before grid barrier k = 1, 2, ...) uses word k % 4:
+  // low half, blocks that have arrived at barrier k; high half, length of the
+  // one list the phase appends to.  So the load that sees the last arrival
+  // also brings the list length.  Block 0 clears word (k + 2) % 4 in phase k.
+  struct alignas(64) Word { unsigned long long v; } phase[4];
   int32_t error;            // KERR_*
   int32_t error_where;      // phase that failed
   int64_t iterations;

@@ -220,16 +220,28 @@ __device__ __forceinline__ int warp_append(int *counter, bool need, int lane)
   return need ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
 }
 
-// Appends v to a global list from inside a divergent branch: one atomic per
+// The same on the list of a grid-synchronised phase, whose length is the high
+// half of the phase's word.
+__device__ __forceinline__ int warp_append(unsigned long long *word, bool need, int lane)
+{
+  const unsigned mask = __ballot_sync(FULL_MASK, need);
+  if (mask == 0) return -1;
+  int base = 0;
+  if (lane == 0) base = (int)(atomicAdd(word, (unsigned long long)__popc(mask) << 32) >> 32);
+  base = __shfl_sync(FULL_MASK, base, 0);
+  return need ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
+}
+
+// Appends v to such a list from inside a divergent branch: one atomic per
 // group of lanes that reach it together (instead of one per lane on the
 // list's single counter).
-__device__ __forceinline__ void append_active(int32_t *list, int32_t *counter, int32_t v)
+__device__ __forceinline__ void append_active(int32_t *list, unsigned long long *word, int32_t v)
 {
   const unsigned act = __activemask();
   const int lane = threadIdx.x & 31;
   const int leader = __ffs(act) - 1;
   int base = 0;
-  if (lane == leader) base = atomicAdd(counter, __popc(act));
+  if (lane == leader) base = (int)(atomicAdd(word, (unsigned long long)__popc(act) << 32) >> 32);
   base = __shfl_sync(act, base, leader);
   list[base + __popc(act & ((1u << lane) - 1u))] = v;
 }
@@ -423,7 +435,8 @@ struct ApplySide {
   const int32_t *lst;
   int64_t i;
   uint32_t stamp;
-  int32_t *next, *n_next;
+  int32_t *next;
+  unsigned long long *word;  // of the phase
   bool pending;       // store() still to run (the same on every thread)
   int32_t v = 0;
   uint32_t w = 0;
@@ -452,20 +465,20 @@ struct ApplySide {
         else push = true;
       }
     }
-    const int p = warp_append(n_next, push, threadIdx.x & 31);
+    const int p = warp_append(word, push, threadIdx.x & 31);
     if (p >= 0) next[p] = v;
   }
 };
 
-// Where an update phase appends the vertices of the next narrow list, and
-// the counters of this iteration's lists.
+// Where an update phase appends.  Grid-synchronised phases append to one list
+// each, whose length is in the phase's word; submesh sweeps (local) have
+// their frozen list's length in shared memory.
 struct ListOut {
-  int32_t *next;      // next iteration's narrow list
-  int32_t *n_next;    // its length
+  unsigned long long *word;  // the phase's word
+  int32_t *next;      // kMarked2, kMarked3: next iteration's narrow list
   int32_t *frozen;    // kNarrow4: vertices frozen now
-  int32_t *n_frozen;
+  int32_t *n_frozen;  // (local)
   int32_t *marked;    // kNarrow2: neighbours marked now
-  int32_t *n_marked;
   uint8_t *dec;       // kMarked4: decided state per position of the marked list
   bool local;         // the list is this block's own (submesh sweeps): no split over the grid
 };
@@ -997,7 +1010,8 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
             d.sw[v] = ST_NEXT;
           } else if (fabs(old - nw) < (1e-6 * (1 + (old + nw) * .5))) {
             d.tst[v] = ST_FROZEN;
-            append_active(lo_.frozen, lo_.n_frozen, v);
+            if (lo_.local) lo_.frozen[atomicAdd(lo_.n_frozen, 1)] = v;
+            else append_active(lo_.frozen, lo_.word, v);
           }
         } else {
           lo_.dec[pos + slot] = (nw < old) ? (uint8_t)ST_NARROW : __ldcg(d.tst + v);
@@ -1047,7 +1061,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
             if (v[h] >= 0 && sw_state(w[h]) != ST_NARROW && sw_stamp(w[h]) != stamp && pn < pv[h]) {
               if (atomicCAS(d.sw + v[h], w[h], sw_make(sw_state(w[h]), stamp)) == w[h]) {
                 d.tst[v[h]] = (uint8_t)sw_state(w[h]);
-                append_active(lo_.marked, lo_.n_marked, v[h]);
+                append_active(lo_.marked, lo_.word, v[h]);
               }
             }
           }
@@ -1071,7 +1085,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
           d.sw[v] = sw_make(sv, stamp);  // still marked for the re-solves running now
           set_phi_both(d, v, nw);
         }
-        const int p = warp_append(lo_.n_next, push, lane);
+        const int p = warp_append(lo_.word, push, lane);
         if (p >= 0) lo_.next[p] = sh.vtx[slot];
       }
     }
@@ -1132,9 +1146,9 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
     if (tid == 0) { b_narrow[s2] = 0; b_frozen = 0; b_marked = 0; }
     __syncthreads();
     ListOut lo;
-    lo.next = lnext; lo.n_next = &b_narrow[s1];
+    lo.word = nullptr; lo.next = lnext;
     lo.frozen = d.lfrozen + c0; lo.n_frozen = &b_frozen;
-    lo.marked = d.lmarked + c0; lo.n_marked = &b_marked;
+    lo.marked = d.lmarked + c0;
     lo.dec = d.dec + c0; lo.local = true;
 
     // P1 -- update the narrow list
@@ -1199,14 +1213,13 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
   return true;
 }
 
-// Grid barrier with its wait accounted in the phase probe.
-__device__ __forceinline__ bool grid_sync_probed(const FimDev &d, uint32_t nblocks, uint64_t timeout_ns, int where,
-                                                 const int32_t *counter = nullptr, int32_t *count = nullptr)
+// Grid barrier k with its wait accounted in the phase probe.
+__device__ __forceinline__ bool grid_sync_probed(const FimDev &d, uint32_t nblocks, uint64_t timeout_ns, int k,
+                                                 int32_t *count)
 {
   PROBE(kPrLight);  // whatever ran since the last mark
-  const bool ok = grid_sync(d.ctl, nblocks, timeout_ns, where, counter, count);
+  const bool ok = grid_sync(d.ctl, nblocks, timeout_ns, k, count);
   PROBE(kPrBarrier);
-  (void)d;
   return ok;
 }
 
@@ -1223,9 +1236,10 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
   const uint32_t nblocks = gridDim.x;
   const int64_t gtid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  const int lane = threadIdx.x & 31;
   int64_t my_evals = 0, my_updates = 0, my_exact = 0;
-  int where = 0;
+  int where = 0;  // grid barriers passed: the phase running is where + 1
+  const auto word = [&]() { return &ctl->phase[(where + 1) & 3].v; };
+  int32_t nn = 0, nm = 0, nf = 0, unused = 0;  // lengths of the narrow, marked and frozen lists
   extern __shared__ __align__(16) unsigned char fim_smem[];
   BatchSh &sh = *reinterpret_cast<BatchSh *>(fim_smem);
   NoSide none;
@@ -1243,12 +1257,12 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
     // failure-detection test hook: this block never arrives at the barrier (a
     // flag that nothing sets), so the others' bounded waits must expire
     if (p.withhold_block > 0 && (int64_t)blockIdx.x == (int64_t)p.withhold_block - 1) return;
-    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &unused)) return;
     for (int64_t i = gtid; i < d.nseed; i += nthreads) {
       const int32_t v = d.seed_v[i];
       set_phi_both(d, v, d.seed_t[i]); d.sw[v] = ST_NARROW;
     }
-    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &unused)) return;
   }
 
   int64_t it = 0;  // global iteration counter (identical in every block)
@@ -1259,9 +1273,6 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
     const double lower = phi_start - p.front_width;
     const float lower_lo = __double2float_rd(lower), lower_hi = __double2float_ru(lower);
     int s = (int)(it % 3);
-    if (gtid == 0) {
-      for (int k = 0; k < 3; ++k) { ctl->n_narrow[k] = 0; ctl->n_frozen[k] = 0; ctl->n_marked[k] = 0; }
-    }
     // sync_step2 (cuda_fim.cu:1752-1787): every copy of a mesh vertex takes
     // the minimum over its copies; copies that were larger become narrow.
     // (The reference indexes its interface table with the thread id instead
@@ -1281,13 +1292,13 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         }
       }
     }
-    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &unused)) return;
     if (PATH == kPathLocal) {
       // submesh sweeps: each block runs its own submeshes through the window
       if (!local_window(d, sh, p, lower, lower_lo, lower_hi, phi_start, cur_time, it, dag, my_evals, my_exact,
                         my_updates, where))
         return;
-      if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where)) return;
+      if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &unused)) return;
       if (gtid == 0) {  // the window took as many iterations as its slowest block
         ctl->iters_total += ctl->win_iter_max;
         ctl->win_iter_max = 0;
@@ -1305,15 +1316,14 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
           set_phi_both(d, v, FIM_INF); d.sw[v] = ST_FAR;
         }
       }
-      if (stv == ST_NARROW) append_active(d.list[s], &ctl->n_narrow[s], (int32_t)v);
+      if (stv == ST_NARROW) append_active(d.list[s], word(), (int32_t)v);
     }
-    int32_t nn = 0, nm = 0;  // lengths of the narrow and the marked list
-    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_narrow[s], &nn)) return;
+    if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nn)) return;
 
     int64_t it_window = 0;
     for (;;) {
       s = (int)(it % 3);
-      const int s1 = (int)((it + 1) % 3), s2 = (int)((it + 2) % 3);
+      const int s1 = (int)((it + 1) % 3);
       if (nn == 0) break;
       if ((p.max_iter > 0 && it_window >= p.max_iter) || it >= kMaxStampIterations) {
         if (gtid == 0 && atomicCAS(&ctl->error, KERR_NONE, KERR_MAX_ITER) == KERR_NONE) ctl->error_where = where;
@@ -1322,11 +1332,11 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
       const uint32_t stamp = (uint32_t)(it + 1);
       const int32_t *lst = d.list[s];
       int32_t *lnext = d.list[s1];
-      if (gtid == 0) { ctl->n_narrow[s2] = 0; ctl->n_frozen[s2] = 0; ctl->n_marked[s2] = 0; }
       ListOut lo;
-      lo.next = lnext; lo.n_next = &ctl->n_narrow[s1];
-      lo.frozen = d.lfrozen; lo.n_frozen = &ctl->n_frozen[s];
-      lo.marked = d.lmarked; lo.n_marked = &ctl->n_marked[s];
+      lo.word = word();
+      lo.next = lnext;
+      lo.frozen = d.lfrozen; lo.n_frozen = nullptr;
+      lo.marked = d.lmarked;
       lo.dec = d.dec; lo.local = false;
       PROBE_COUNT(kPrPhases);
 
@@ -1336,7 +1346,8 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         update_phase<kNarrow2>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
                                lo, my_evals, my_exact, none);
         my_updates += (gtid == 0) ? nn : 0;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_marked[s], &nm)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nm)) return;
+        lo.word = word();
 
         // Y -- apply the narrow list's times and states (the block's share
         // of the list, cuda_fim.cu:2291-2317), then re-solve the marked
@@ -1345,7 +1356,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         const int64_t per_block = ((int64_t)nn + gridDim.x - 1) / gridDim.x;
         const int64_t lbeg = min((int64_t)nn, (int64_t)blockIdx.x * per_block);
         const int64_t lend = min((int64_t)nn, lbeg + per_block);
-        ApplySide side{d, lst, -1, stamp, lnext, lo.n_next, true};
+        ApplySide side{d, lst, -1, stamp, lnext, lo.word, true};
         int64_t i0 = lbeg;
         for (; i0 + kThreads < lend; i0 += kThreads) {  // all but the last round
           side.i = i0 + threadIdx.x;
@@ -1363,14 +1374,14 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         my_updates += (gtid == 0) ? nm : 0;
         ++it;
         ++it_window;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_narrow[s1], &nn)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nn)) return;
       } else {
         // P1 -- solve on elements + reduce per vertex (cuda_fim.cu:2102-2163)
         update_phase<kNarrow4>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
                                lo, my_evals, my_exact, none);
         my_updates += (gtid == 0) ? nn : 0;
-        int32_t nf = 0;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_frozen[s], &nf)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nf)) return;
+        lo.word = word();
 
         // P2 -- apply the narrow times; mark downwind neighbours of the
         // vertices frozen now (cuda_fim.cu:2172-2205).  The two are
@@ -1393,12 +1404,13 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
             if (sw_state(w) != ST_NARROW && sw_stamp(w) != stamp && pn < pv) {
               if (atomicCAS(d.sw + v, w, sw_make(ST_NEIG, stamp)) == w) {
                 d.tst[v] = (uint8_t)sw_state(w);
-                append_active(d.lmarked, &ctl->n_marked[s], v);
+                append_active(d.lmarked, lo.word, v);
               }
             }
           }
         }
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_marked[s], &nm)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nm)) return;
+        lo.word = word();
 
         // P3 -- the narrow vertices that are not re-solved now go to the next
         // list (or freeze), then the marked neighbours are re-solved
@@ -1413,7 +1425,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
           if (sw_stamp(w) == stamp) continue;  // re-solved below
           if (sw_state(w) == ST_NARROW) {
             if (tv == ST_FROZEN) d.sw[v] = ST_FROZEN;
-            else append_active(lnext, &ctl->n_narrow[s1], v);
+            else append_active(lnext, lo.word, v);
           }
         }
         update_phase<kMarked3>(d, sh, d.lmarked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0,
@@ -1421,7 +1433,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         my_updates += (gtid == 0) ? nm : 0;
         ++it;
         ++it_window;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &ctl->n_narrow[s1], &nn)) return;
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nn)) return;
       }
     }
   }

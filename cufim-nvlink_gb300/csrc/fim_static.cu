@@ -15,8 +15,8 @@
 // time), the stimulus entries expanded to vertex copies (i32, f64); the
 // control block FimCtl.
 //
-// What must start at zero: only the FimCtl block (barrier counter and
-// generation, list counters, error word).  fim_solve_noalloc clears it with
+// What must start at zero: only the FimCtl block (phase words, error
+// word).  fim_solve_noalloc clears it with
 // cudaMemsetAsync before every launch.  Everything else is written before it
 // is read within one call: the solve kernel resets phi/phi2/sw/tst of every
 // copy, the lists are filled behind their counters, and the stimulus

@@ -316,12 +316,6 @@ __device__ __forceinline__ double tet_root_tail(const double *S, bool second)
 // ---------------------------------------------------------------------------
 // corner relabelling and bound packing (metric kernel and solve)
 
-// Edge numbering of a tet with slots 0..3: (0,1) (0,2) (1,2) (0,3) (1,3) (2,3)
-// (types.cpp:240-245).
-__host__ __device__ constexpr int edge_index(int i, int j)
-{
-  return (i > j) ? edge_index(j, i) : (j == 1 ? 0 : (j == 2 ? (i == 0 ? 1 : 2) : 3 + i));
-}
 // For target slot t the other slots are relabelled "1","2","3" =
 // (t+1)%4, (t+2)%4, (t+3)%4 (the reference's gray-code mapping,
 // cuda_fim.h:41-48).  sel_of(t, k) is the edge index of the k-th relabelled

@@ -319,42 +319,42 @@ __device__ __forceinline__ CandBound tet_screen_bf(const float *gv, float p1f, f
 }
 
 // Per-corner lower bounds, in true units, of the square-root term of the
-// reference's local solves, from the scaled squared edge norms
-// g = e13, e23, e34, e12, e14, e24 (times 2^-k, k even):
+// reference's local solves, from the scaled squared edge norms (times 2^-k,
+// k even); the corner's vertex is "4", the others "1", "2", "3":
 //  * triangle pair (1,2), (2,3), (1,3): solve_tri_cu's root term is the
-//    metric distance from the target "4" to the point l x_a + (1-l) x_b of
-//    the pair's segment (its a + 2 l b + l^2 c is that squared distance), so
-//    the distance from "4" to the segment bounds it: foot
-//    lambda* = (Sb - (Sa + Sb - B)/2) / B; inside (0,1) the line distance
-//    h^2 = (Sa Sb - ((Sa + Sb - B)/2)^2) / B, else min(Sa, Sb);
+//    metric distance from "4" to the point l x_a + (1-l) x_b of the pair's
+//    segment (its a + 2 l b + l^2 c is that squared distance), so the distance
+//    from "4" to the segment bounds it: with the face's dot products at its
+//    corners (u_v = (x_w - x_v).(x_x - x_v), half of the two norms at v minus
+//    the opposite one), the foot lies beyond b where u_b <= 0 and beyond a
+//    where u_a <= 0 (the distance is then that to b or a), else the line
+//    distance h^2 = (S_a S_b - u_4^2) / e_ab bounds it (below the segment
+//    distance anywhere);
 //  * tet: solve_tet_cu's root term is sqrt(Q(l1, l2)) with the reference's
 //    Q = a + 2 l1 b + l1^2 c + 2 l1 l2 d + 2 l2 e + l2^2 f (cuda_fim.h:1302-1360;
 //    not a distance), at an accepted root (l1, l2, 1 - l1 - l2 > 0), so the
 //    minimum of Q over the closed triangle l1, l2 >= 0, l1 + l2 <= 1 bounds
 //    it: the minimum over the three edges (1D quadratics) and, when the
 //    Hessian is certainly positive definite, the unconstrained minimum.
+//    Its b, -c and -e are dot products at "3" of faces of the tet.
 // A solve's value is a convex combination of its times plus that term, so
 // min(times) + bound is below every value it returns (up to roundings the
 // caller adds).  Undecidable or degenerate cases give 0 (no bound).
+//
+// The metric kernel evaluates these for every corner, and its instruction
+// issue is as scarce as its FP64 pipe: the four faces' dot products and
+// determinants are formed once per tet, positions of minima are decided by
+// signs instead of quotients, and divisions and square roots are the hardware
+// approximations with their errors in the bounds.
 __device__ __forceinline__ float root_lo(Re q, float emax, float tk)
 {
   // the solves' own rounding of the squared term is absolute and below
   // 2^-23 emax (the triangle solve squares its float l: 2^-24 e12; FP64
   // roundings: below 2^-45 emax); then the rounding of the square root
   const float lo = re_lo(q) - 0x1p-22f * emax;
-  if (!(lo > 0.f)) return 0.f;
-  const float h = sqrtf(lo) * (1.f - 0x1p-22f);
-  const float r = h * tk;
+  if (!(lo >= 0x1p-120f)) return 0.f;
+  const float r = lo * rsqrtf(lo) * (1.f - 0x1p-20f) * tk;
   return isfinite(r) ? r : 0.f;
-}
-
-__device__ __forceinline__ float segment_lo(Re B, Re Sa, Re Sb, float emax, float tk)
-{
-  const Re uw = re_scale((Sa + Sb) - B, 0.5f);
-  const Re lam = re_div(Sb - uw, B);
-  if (re_hi(lam) <= 0.f) return root_lo(Sb, emax, tk);
-  if (re_lo(lam) >= 1.f) return root_lo(Sa, emax, tk);
-  return root_lo(re_div(Sa * Sb - uw * uw, B), emax, tk);  // line distance <= segment distance
 }
 
 // re_lo, with NaN (an overflowed bound) turned into -inf, so that a minimum
@@ -371,44 +371,73 @@ __device__ __forceinline__ float quad01_lo(Re al, Re be, Re ga)
   const float ends = fminf(safe_lo(al), safe_lo((al + re_scale(be, 2.f)) + ga));
   if (re_hi(ga) <= 0.f) return ends;         // concave or linear: the minimum is at an end
   if (!(re_lo(ga) > 0.f)) return -INFINITY;  // curvature sign undecided: no bound
-  const Re s = re_div(-be, ga);              // vertex of the parabola
-  if (re_hi(s) <= 0.f || re_lo(s) >= 1.f) return ends;
-  return fminf(ends, safe_lo(al - re_div(be * be, ga)));
+  // the parabola's vertex -be / ga outside (0, 1)
+  if (re_lo(be) >= 0.f || re_hi(be + ga) <= 0.f) return ends;
+  return fminf(ends, safe_lo(al - re_div_bf(be * be, ga)));
 }
 
-__device__ __forceinline__ void corner_bounds(const float *gs, int k, float *h)
+// Edge numbering of a tet with slots 0..3: (0,1) (0,2) (1,2) (0,3) (1,3) (2,3)
+// (types.cpp:240-245).
+// (Without recursion, so that it folds to a constant in unrolled loops: an
+// index that does not puts its array into local memory.)
+__host__ __device__ constexpr int edge_of(int lo, int hi) { return hi == 1 ? 0 : (hi == 2 ? 1 + lo : 3 + lo); }
+__host__ __device__ constexpr int edge_index(int i, int j) { return i < j ? edge_of(i, j) : edge_of(j, i); }
+// j-th vertex (ascending) of the face without vertex f
+__host__ __device__ constexpr int face_vertex(int f, int j) { return j < f ? j : j + 1; }
+
+// Dot products and determinants of a tet's faces (face f: without vertex f).
+struct FaceTerms {
+  Re u[4][4];  // u[f][v], v != f
+  Re det[4];
+};
+__device__ __forceinline__ void face_terms(const Re *S, FaceTerms &F)
 {
-  const Re e13 = re_in(gs[0]), e23 = re_in(gs[1]), e34 = re_in(gs[2]);
-  const Re e12 = re_in(gs[3]), e14 = re_in(gs[4]), e24 = re_in(gs[5]);
-  float emax = 0.f;
-  bool finite = true;
 #pragma unroll
-  for (int i = 0; i < 6; ++i) { emax = fmaxf(emax, gs[i]); finite = finite && isfinite(gs[i]); }
-  const float tk = re_pow2f(k / 2);
-  h[0] = h[1] = h[2] = h[3] = 0.f;
-  if (!finite || !(emax > 0.f) || !isfinite(tk)) return;
-  h[0] = segment_lo(e12, e14, e24, emax, tk);   // pair (1,2)
-  h[1] = segment_lo(e23, e24, e34, emax, tk);   // pair (2,3)
-  h[2] = segment_lo(e13, e14, e34, emax, tk);   // pair (1,3)
+  for (int f = 0; f < 4; ++f) {
+    const int p = face_vertex(f, 0), q = face_vertex(f, 1), r = face_vertex(f, 2);
+    const Re pq = S[edge_index(p, q)], pr = S[edge_index(p, r)], qr = S[edge_index(q, r)];
+    F.u[f][p] = re_scale((pq + pr) - qr, 0.5f);
+    F.u[f][q] = re_scale((pq + qr) - pr, 0.5f);
+    F.u[f][r] = re_scale((pr + qr) - pq, 0.5f);
+    F.det[f] = pq * pr - F.u[f][p] * F.u[f][p];
+  }
+}
+
+// Bound of the pair (a, b) of the corner t, in the face f of the three.
+__device__ __forceinline__ float segment_lo(const Re *S, const FaceTerms &F, int f, int t, int a, int b, float emax,
+                                            float tk)
+{
+  const Re B = S[edge_index(a, b)];
+  if (!(re_lo(B) > 0.f)) return 0.f;
+  Re q = re_div_bf(F.det[f], B);
+  if (re_hi(F.u[f][b]) <= 0.f) q = S[edge_index(b, t)];
+  else if (re_hi(F.u[f][a]) <= 0.f) q = S[edge_index(a, t)];
+  return root_lo(q, emax, tk);
+}
+
+// h[0..2]: pairs (1,2), (2,3), (1,3), h[3]: tet, of the corner at slot t ("1",
+// "2", "3" are the slots t+1, t+2, t+3 mod 4).
+__device__ __forceinline__ void corner_bounds(const Re *S, const FaceTerms &F, int t, float emax, float tk, float *h)
+{
+  const int v1 = (t + 1) & 3, v2 = (t + 2) & 3, v3 = (t + 3) & 3;
+  h[0] = segment_lo(S, F, v3, t, v1, v2, emax, tk);
+  h[1] = segment_lo(S, F, v1, t, v2, v3, emax, tk);
+  h[2] = segment_lo(S, F, v2, t, v1, v3, emax, tk);
   // the tet's Q with the reference's coefficients
-  const Re A = e13;
-  const Re B = re_scale((e23 + e13) - e12, 0.5f);
-  const Re C = re_scale((e34 + e13) - e14, -0.5f);
-  const Re D = e23;
-  const Re E = re_scale((e34 + e23) - e24, -0.5f);
-  const Re F = e34;
+  const Re A = S[edge_index(v1, v3)], D = S[edge_index(v2, v3)], E34 = S[edge_index(v3, t)];
+  const Re B = F.u[t][v3], C = -F.u[v2][v3], E = -F.u[v1][v3];
   float qmin = quad01_lo(A, B, C);                                   // l2 = 0
-  qmin = fminf(qmin, quad01_lo(A, E, F));                            // l1 = 0
+  qmin = fminf(qmin, quad01_lo(A, E, E34));                          // l1 = 0
   qmin = fminf(qmin, quad01_lo((A + re_scale(B, 2.f)) + C,           // l1 = 1 - s, l2 = s
-                               ((D + E) - B) - C, (C - re_scale(D, 2.f)) + F));
+                               ((D + E) - B) - C, (C - re_scale(D, 2.f)) + E34));
   // an interior minimum needs a positive definite Hessian (c > 0, cf - d^2 > 0);
   // unless that is excluded, the unconstrained minimum
   // a - (f b^2 - 2 d b e + c e^2) / (cf - d^2) joins the candidates (-inf when
   // the determinant's sign is undecided)
-  const Re det = C * F - D * D;
+  const Re det = C * E34 - D * D;
   if (!(re_hi(C) <= 0.f || re_hi(det) <= 0.f)) {
-    const Re num = ((F * B) * B - re_scale((D * B) * E, 2.f)) + (C * E) * E;
-    qmin = fminf(qmin, safe_lo(A - re_div(num, det)));
+    const Re num = ((E34 * B) * B - re_scale((D * B) * E, 2.f)) + (C * E) * E;
+    qmin = fminf(qmin, safe_lo(A - re_div_bf(num, det)));
   }
   h[3] = root_lo(re_make(qmin, 0.f), emax, tk);
 }

@@ -33,7 +33,52 @@ namespace fimgb {
 // ---------------------------------------------------------------------------
 // metric kernel
 
-__global__ void fim_metric_kernel(const int32_t *__restrict__ tslots, const int64_t *__restrict__ cidx,
+// Metric entries and squared edge norms of one tet in the reference's
+// expressions.  Z = 1: f2 is zero, Z = 2: f0 f1 is, too; the terms that
+// contain those products are then zero and are left out, which changes no
+// result: a sum only differs where it is itself zero (in its sign), and the
+// caller redoes a tet whose norms are not all positive and finite.  ev: the six
+// edge vectors.
+template <int Z>
+__device__ __forceinline__ void tet_norms(double vf, double vs, double f0, double f1, double f2, const double *ev,
+                                          double *g)
+{
+  // compute_velocity_tensor_f3 (types.h:173-188); aMb_sym (types.h:165-171)
+  const double fa = f0*f0, fd = f1*f1;
+  const double M0 = vf*fa + vs*(1. - fa);
+  const double M3 = vf*fd + vs*(1. - fd);
+  double M1 = 0.0, M2 = 0.0, M4 = 0.0, M5 = vs;
+  if (Z < 2) M1 = (vf - vs)*(f0*f1);
+  if (Z < 1) {
+    const double ff = f2*f2;
+    M2 = (vf - vs)*(f0*f2);
+    M4 = (vf - vs)*(f1*f2);
+    M5 = vf*ff + vs*(1. - ff);
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double ex = ev[3 * k], ey = ev[3 * k + 1], ez = ev[3 * k + 2];
+    if (Z == 0) g[k] = (M0*ex + M1*ey + M2*ez)*ex + (M1*ex + M3*ey + M4*ez)*ey + (M2*ex + M4*ey + M5*ez)*ez;
+    else if (Z == 1) g[k] = (M0*ex + M1*ey)*ex + (M1*ex + M3*ey)*ey + (M5*ez)*ez;
+    else g[k] = (M0*ex)*ex + (M3*ey)*ey + (M5*ez)*ez;
+  }
+}
+
+// x is +0 or -0
+__device__ __forceinline__ bool dzero(double x) { return ((unsigned long long)__double_as_longlong(x) << 1) == 0ull; }
+
+// The FP64 pipe bounds this kernel (72 % busy on a slab): a tet takes 142 FP64
+// operations, 85 where its fibre lies in the xy-plane and 58 where it is also
+// along an axis; a warp takes the shorter form when all its tets allow it.
+// Uploads from the device in ms (1M slab and 135k slab, fibres in the plane;
+// 87k shell, any fibres; 9k cube, along x): 2.25, 0.316, 0.172 and 0.043 with
+// 142 operations for all, 5,100 instructions per warp and the norms in local
+// memory; 1.47, 0.211, 0.165 and 0.023 now (3,200 instructions).  Blocks of 256
+// threads, two per SM: 1.43, 0.215, 0.169, 0.027; of 64 threads, ten per SM:
+// 1.64, 0.229, 0.175, 0.021.
+constexpr int kMetricBlock = 128, kMetricBlocks = 5;  // threads per block, blocks per SM
+__global__ void __launch_bounds__(kMetricBlock, kMetricBlocks) fim_metric_kernel(const int32_t *__restrict__ tslots,
+                                                         const int64_t *__restrict__ cidx,
                                   const double *__restrict__ xyz, const double *__restrict__ evec, int64_t nT,
                                   const double *__restrict__ fib,
                                   const double *__restrict__ cf, const double *__restrict__ ct,
@@ -45,12 +90,15 @@ __global__ void fim_metric_kernel(const int32_t *__restrict__ tslots, const int6
   // thread 0 of the block evaluates them for its own tet, and every warp
   // whose tets all have the same speeds (bit for bit) takes that result
   // instead of dividing: with piecewise-constant conduction most warps do.
+  // (One wave of blocks whose warps keep the terms of their last round needs
+  // no barrier, but measured 1.74 ms against 1.43.)
   __shared__ double s_sp[4];  // thread 0's cf, ct and their 1/cf/cf, 1/ct/ct
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t eb = e0 + blockIdx.x * (int64_t)blockDim.x; eb < e1; eb += stride) {  // block-uniform
     const int64_t e = eb + threadIdx.x;
     const bool in = e < e1;
     const double cfe = in ? cf[e] : 0.0, cte = in ? ct[e] : 0.0;
+    const double f0 = in ? fib[3 * e + 0] : 0.0, f1 = in ? fib[3 * e + 1] : 0.0, f2 = in ? fib[3 * e + 2] : 0.0;
     if (threadIdx.x == 0) {  // eb < e1: thread 0 is in range
       s_sp[0] = cfe; s_sp[1] = cte;
       s_sp[2] = 1. / cfe / cfe; s_sp[3] = 1. / cte / cte;
@@ -64,45 +112,38 @@ __global__ void fim_metric_kernel(const int32_t *__restrict__ tslots, const int6
     } else {
       vf = 1. / cfe / cfe; vs = 1. / cte / cte;
     }
+    const bool plane = __all_sync(0xffffffffu, dzero(f2));
+    const bool axis = plane && __all_sync(0xffffffffu, dzero(f0) || dzero(f1));
     __syncthreads();  // s_sp is rewritten by the next round
     if (!in) continue;
-    const double f0 = fib[3 * e + 0], f1 = fib[3 * e + 1], f2 = fib[3 * e + 2];
     // the input check of fim_set_conduction: positive finite speeds, finite
     // fibre; the first offending tet is reported
     // (sign and exponent tests on the integer pipes: the FP64 pipe is this
     // kernel's bound)
     if (!(dpos_finite(cfe) && dpos_finite(cte) && dfinite(f0) && dfinite(f1) && dfinite(f2)))
       atomicMin(bad, (unsigned long long)e);
-    // compute_velocity_tensor_f3 (types.h:173-188)
-    const double fa = f0*f0, fb = f0*f1, fc = f0*f2, fd = f1*f1, fe = f1*f2, ff = f2*f2;
-    const double M0 = vf*fa + vs*(1. - fa);
-    const double M1 = (vf - vs)*fb;
-    const double M2 = (vf - vs)*fc;
-    const double M3 = vf*fd + vs*(1. - fd);
-    const double M4 = (vf - vs)*fe;
-    const double M5 = vf*ff + vs*(1. - ff);
-    double g[6];
+    // the mesh's edge vectors, staged once (edge_vector_kernel, fim_stage.cu),
+    // or load_edge(a, b) = x_a - x_b (types.h:210-216)
+    double ev[18];
     if (evec) {
-      // the edge vectors of the mesh, staged once (edge_vector_kernel, fim_stage.cu)
 #pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const double ex = evec[(3 * k + 0) * nT + e], ey = evec[(3 * k + 1) * nT + e], ez = evec[(3 * k + 2) * nT + e];
-        g[k] = (M0*ex + M1*ey + M2*ez)*ex + (M1*ex + M3*ey + M4*ez)*ey + (M2*ex + M4*ey + M5*ez)*ez;
-      }
+      for (int i = 0; i < 18; ++i) ev[i] = __ldg(evec + i * nT + e);
     } else {
-      const int32_t v0 = tslots[4 * e + 0], v1 = tslots[4 * e + 1];
-      const int32_t v2 = tslots[4 * e + 2], v3 = tslots[4 * e + 3];
-      const int32_t va[6] = {v0, v0, v1, v0, v1, v2};
-      const int32_t vb[6] = {v1, v2, v2, v3, v3, v3};
+      const int4 sl = __ldg(reinterpret_cast<const int4 *>(tslots) + e);
+      const int32_t va[6] = {sl.x, sl.x, sl.y, sl.x, sl.y, sl.z};
+      const int32_t vb[6] = {sl.y, sl.z, sl.z, sl.w, sl.w, sl.w};
 #pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        // load_edge(a, b) = x_a - x_b (types.h:210-216); aMb_sym (types.h:165-171)
-        const double ex = xyz[3 * (int64_t)va[k] + 0] - xyz[3 * (int64_t)vb[k] + 0];
-        const double ey = xyz[3 * (int64_t)va[k] + 1] - xyz[3 * (int64_t)vb[k] + 1];
-        const double ez = xyz[3 * (int64_t)va[k] + 2] - xyz[3 * (int64_t)vb[k] + 2];
-        g[k] = (M0*ex + M1*ey + M2*ez)*ex + (M1*ex + M3*ey + M4*ez)*ey + (M2*ex + M4*ey + M5*ez)*ez;
-      }
+      for (int i = 0; i < 18; ++i) ev[i] = xyz[3 * (int64_t)va[i / 3] + i % 3] - xyz[3 * (int64_t)vb[i / 3] + i % 3];
     }
+    double g[6];
+    bool redo = !plane;
+    if (plane) {
+      if (axis) tet_norms<2>(vf, vs, f0, f1, f2, ev, g);
+      else tet_norms<1>(vf, vs, f0, f1, f2, ev, g);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) redo = redo || !dpos_finite(g[k]);
+    }
+    if (redo) tet_norms<0>(vf, vs, f0, f1, f2, ev, g);
     // scale 2^-k (k even) of the float screen record: edge norms O(1).  The
     // largest norm by its bit pattern (the order of non-negative doubles;
     // a negative or NaN norm only turns the scaling off), its binary
@@ -127,6 +168,17 @@ __global__ void fim_metric_kernel(const int32_t *__restrict__ tslots, const int6
       gsc[k] = d2f_pow2(g[k], ks);  // (float)(g * 2^-ks)
       len[k] = sqrtf(gsc[k]) * tk;
     }
+    float emax = 0.f;
+    bool finite = ok;
+    Re S[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      emax = fmaxf(emax, gsc[k]);
+      finite = finite && isfinite(gsc[k]);
+      S[k] = re_in(gsc[k]);
+    }
+    FaceTerms F;
+    face_terms(S, F);
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const int64_t c = cidx[4 * e + t];
@@ -135,13 +187,11 @@ __global__ void fim_metric_kernel(const int32_t *__restrict__ tslots, const int6
       o[1] = make_double2(g[sel_of(t, 2)], g[sel_of(t, 3)]);
       o[2] = make_double2(g[sel_of(t, 4)], g[sel_of(t, 5)]);
       float4 *of = reinterpret_cast<float4 *>(cgf + kCgfStride * c);
-      const float gs[6] = {gsc[sel_of(t, 0)], gsc[sel_of(t, 1)], gsc[sel_of(t, 2)],
-                           gsc[sel_of(t, 3)], gsc[sel_of(t, 4)], gsc[sel_of(t, 5)]};
       float hb[4];
-      corner_bounds(gs, ok ? ks : 0, hb);
-      if (!ok) hb[0] = hb[1] = hb[2] = hb[3] = 0.f;
-      of[0] = make_float4(gs[0], gs[1], gs[2], gs[3]);
-      of[1] = make_float4(gs[4], gs[5], (float)ks, 0.f);
+      corner_bounds(S, F, t, emax, tk, hb);
+      if (!(finite && emax > 0.f)) hb[0] = hb[1] = hb[2] = hb[3] = 0.f;
+      of[0] = make_float4(gsc[sel_of(t, 0)], gsc[sel_of(t, 1)], gsc[sel_of(t, 2)], gsc[sel_of(t, 3)]);
+      of[1] = make_float4(gsc[sel_of(t, 4)], gsc[sel_of(t, 5)], (float)ks, 0.f);
       // first-read record: the lengths and the bounds (fp16, rounded down, so
       // still lower bounds); its ids were written at mesh staging
       uint4 *rc = crec + kCrecWords * c;
@@ -160,7 +210,7 @@ cudaError_t launch_metric(const int32_t *tslots, const int64_t *cidx, const doub
                           double *cgeo, float *cgf, uint4 *crec, unsigned long long *bad, cudaStream_t stream)
 {
   if (e1 <= e0) return cudaSuccess;
-  const int block = 256;
+  const int block = kMetricBlock;
   int64_t grid = (e1 - e0 + block - 1) / block;
   if (grid > 152 * 64) grid = 152 * 64;
   fim_metric_kernel<<<(unsigned)grid, block, 0, stream>>>(tslots, cidx, xyz, evec, nT, fib, cf, ct, e0, e1, cgeo, cgf,

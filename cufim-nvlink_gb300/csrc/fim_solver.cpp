@@ -553,10 +553,9 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
   return FIM_OK;
 }
 
-// Uploads a conduction field and runs the metric kernel.  The arrays (host
-// or device, by `host`) are copied over the copy stream in chunks, and each
-// chunk's metric launch waits only for its own copy, so the transfers
-// overlap the FP64 metric work.  The
+// Uploads a conduction field and runs the metric kernel.  Host arrays are
+// copied over the copy stream in chunks, and each chunk's metric launch waits
+// only for its own copy, so the transfers overlap the FP64 metric work.  The
 // kernel also checks the field (positive finite speeds, finite fibres): on a
 // bad tet the call fails and the solver has no conduction until a later call
 // succeeds.
@@ -573,16 +572,36 @@ static int run_metric(fim_solver *s, const double *fib, const double *cf, const 
   // the copies overwrite arrays that earlier work on the working stream may read
   CUDA_TRY(s, cudaEventRecord(s->ev_dep, s->stream));
   CUDA_TRY(s, cudaStreamWaitEvent(cs, s->ev_dep, 0));
-  for (int i = 0; i < nch; ++i) {
-    const int64_t e0 = nT * i / nch, e1 = nT * (i + 1) / nch;
-    CUDA_TRY(s, cudaMemcpyAsync(s->fib.p + 3 * e0, fib + 3 * e0, sizeof(double) * 3 * (e1 - e0), kind, cs));
-    CUDA_TRY(s, cudaMemcpyAsync(s->cf.p + e0, cf + e0, sizeof(double) * (e1 - e0), kind, cs));
-    CUDA_TRY(s, cudaMemcpyAsync(s->ct.p + e0, ct + e0, sizeof(double) * (e1 - e0), kind, cs));
-    CUDA_TRY(s, cudaEventRecord(s->ev_chunk[i], cs));
-    CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_chunk[i], 0));
-    if (i == 0) CUDA_TRY(s, cudaEventRecord(s->ev0, s->stream));
-    CUDA_TRY(s, launch_metric(s->tslots.p, s->cidx.p, s->xyz.p, s->evec.p, s->nT, s->fib.p, s->cf.p, s->ct.p, e0,
-                              e1, s->cgeo.p, s->cgf.p, s->crec.p, s->bad.p, s->stream));
+  const auto copy = [&](int64_t e0, int64_t e1) {
+    cudaError_t e = cudaMemcpyAsync(s->fib.p + 3 * e0, fib + 3 * e0, sizeof(double) * 3 * (e1 - e0), kind, cs);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(s->cf.p + e0, cf + e0, sizeof(double) * (e1 - e0), kind, cs);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(s->ct.p + e0, ct + e0, sizeof(double) * (e1 - e0), kind, cs);
+    return e;
+  };
+  const auto aligned = [](const double *p) { return reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0; };
+  if (!host && aligned(fib) && aligned(cf) && aligned(ct)) {
+    // a field on the device: one launch reads it where it is, beside the
+    // copies that the solver keeps (each of several chunked launches ends in
+    // a partial wave).  Like the copies it starts after the copy stream's
+    // implicit wait for the legacy default stream.
+    CUDA_TRY(s, cudaEventRecord(s->ev_chunk[0], cs));
+    CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_chunk[0], 0));
+    CUDA_TRY(s, cudaEventRecord(s->ev0, s->stream));
+    CUDA_TRY(s, launch_metric(s->tslots.p, s->cidx.p, s->xyz.p, s->evec.p, s->nT, fib, cf, ct, 0, nT, s->cgeo.p,
+                              s->cgf.p, s->crec.p, s->bad.p, s->stream));
+    CUDA_TRY(s, copy(0, nT));
+    CUDA_TRY(s, cudaEventRecord(s->ev_chunk[1], cs));
+    CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_chunk[1], 0));
+  } else {
+    for (int i = 0; i < nch; ++i) {
+      const int64_t e0 = nT * i / nch, e1 = nT * (i + 1) / nch;
+      CUDA_TRY(s, copy(e0, e1));
+      CUDA_TRY(s, cudaEventRecord(s->ev_chunk[i], cs));
+      CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_chunk[i], 0));
+      if (i == 0) CUDA_TRY(s, cudaEventRecord(s->ev0, s->stream));
+      CUDA_TRY(s, launch_metric(s->tslots.p, s->cidx.p, s->xyz.p, s->evec.p, s->nT, s->fib.p, s->cf.p, s->ct.p, e0,
+                                e1, s->cgeo.p, s->cgf.p, s->crec.p, s->bad.p, s->stream));
+    }
   }
   CUDA_TRY(s, cudaEventRecord(s->ev1, s->stream));
   CUDA_TRY(s, cudaEventSynchronize(s->ev1));

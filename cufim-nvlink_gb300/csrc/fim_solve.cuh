@@ -152,7 +152,7 @@ struct BatchSh {
   union {
     struct {
       float pf[kCornerCap][3];      // their float times
-      float lbv[kCornerCap][4];     // lower bounds of the triangle pairs (1,2), (2,3), (1,3) and the tet (+inf: not valid)
+      alignas(16) float lbv[kCornerCap][4];  // lower bounds of the triangle pairs (1,2), (2,3), (1,3) and the tet (+inf: not valid)
       float elo[kCornerCap];        // smallest lower bound of the corner's valid edges (+inf: none)
     };
     double dag[kDagGroups][kDagSlots];  // phase D (where pf and sf are dead): scratch of the tet prefix groups
@@ -170,7 +170,8 @@ struct BatchSh {
     };
     int32_t ids[kIdsCap][3];        // batches of up to kIdsCap corners without queues (direct): the corners' other vertices
   };
-  int ntri, ntet, nedge, nq[3];
+  int nlist[3];                     // triangles, tets and edge corners listed
+  int nq[3];
   int next_item;                    // next unclaimed screen item (phase S)
   int wsum[kSlots / 32];            // corner counts of each warp's 32 slots (setup)
   int nfit;                         // slots whose corners end within kCornerCap (setup)
@@ -186,6 +187,9 @@ static_assert(kSlots <= 256 && kCornerCap <= (1 << 14), "queue item and screen l
 // whole warps over the slots
 static_assert(kSlots % 32 == 0 && kSlots <= kThreads, "slots must fill whole warps of the block");
 static_assert(kCornerCap % 32 == 0, "corner capacity in whole warps");
+// phase B: five bits per corner and thread, ten-bit counts per warp
+static_assert(5 * ((kCornerCap + kThreads - 1) / kThreads) <= 64 &&
+              96 * ((kCornerCap + kThreads - 1) / kThreads) < 1024, "phase B's bits and counts");
 static_assert(kDagWarps >= 1 && 32 * kDagWarps <= kThreads, "tet prefix warps within the block");
 __device__ __forceinline__ uint32_t make_item(int slot, int kind, int j)
 {
@@ -557,7 +561,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     if (tid == 0) {
       sh.cp[0] = 0;
       sh.nfit = 0;
-      sh.ntri = 0; sh.ntet = 0; sh.nedge = 0; sh.nq[0] = 0; sh.nq[1] = 0; sh.nq[2] = 0; sh.next_item = 0; sh.nfz = 0;
+      sh.nlist[0] = 0; sh.nlist[1] = 0; sh.nlist[2] = 0; sh.nq[0] = 0; sh.nq[1] = 0; sh.nq[2] = 0; sh.next_item = 0; sh.nfz = 0;
     }
     __syncthreads();
     // corner prefix over the slots: each warp scans its 32 slots, the warp
@@ -670,62 +674,55 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     __syncthreads();
     PROBE(kPrA);
 
-    // B: screen lists
-    for (int jb = 0; jb < kept; jb += kThreads) {
-      const int j = jb + tid;
-      const bool in = j < kept;
-      int slot = 0;
-      uint32_t m = 0;
-      float bhi = 0.f, lb[4] = {0.f, 0.f, 0.f, 0.f}, elo = 0.f;
-      if (in) {
-        slot = sh.cs[j];
-        m = sh.vm[j];
-        bhi = funkey(sh.bhi[slot]);
-        lb[0] = sh.lbv[j][0]; lb[1] = sh.lbv[j][1]; lb[2] = sh.lbv[j][2]; lb[3] = sh.lbv[j][3];
-        elo = sh.elo[j];
+    // B: screen lists.  Every thread first notes which solves of its corners
+    // are to be listed (five bits a corner) and counts them; one atomic per
+    // warp then reserves the warp's places in all three lists (instead of
+    // three dependent ones for every 32 corners), and the items are written
+    // round by round.
+    {
+      uint64_t bits = 0;
+      uint32_t counts = 0;  // triangles, tets << 10, edges << 20
+      for (int j = tid, sft = 0; j < kept; j += kThreads, sft += 5) {
+        const float bhi = funkey(sh.bhi[sh.cs[j]]);
+        const uint32_t m = sh.vm[j];
+        const float4 lb = *reinterpret_cast<const float4 *>(sh.lbv[j]);
+        const float elo = sh.elo[j];
+        // pairs (1,2), (2,3), (1,3), the tet, and the corners with an edge
+        // that can still be the minimum: the smallest edge lower bound (phase
+        // A) against bhi; the FP32 mode lists every corner with a valid edge
+        const uint32_t t0 = (m & 3u) == 3u && !(lb.x > bhi), t1 = (m & 6u) == 6u && !(lb.y > bhi);
+        const uint32_t t2 = (m & 5u) == 5u && !(lb.z > bhi), t3 = m == 7u && !(lb.w > bhi);
+        const uint32_t t4 = fp32 ? m != 0u : !(elo > bhi);
+        bits |= (uint64_t)(t0 | (t1 << 1) | (t2 << 2) | (t3 << 3) | (t4 << 4)) << sft;
+        counts += t0 + t1 + t2 + (t3 << 10) + (t4 << 20);
       }
-      // triangle pairs (1,2), (2,3), (1,3), appended together (one atomic
-      // per warp for the three), then the tet
-      bool need[3];
-      unsigned msk[3];
+      const uint32_t total_w = __reduce_add_sync(FULL_MASK, counts);
+      int base = 0;
+      if (total_w != 0 && lane < 3) base = atomicAdd(&sh.nlist[lane], (int)((total_w >> (10 * lane)) & 1023u));
+      int pt = __shfl_sync(FULL_MASK, base, 0), pq = __shfl_sync(FULL_MASK, base, 1);
+      int pe = __shfl_sync(FULL_MASK, base, 2);
+      if (total_w != 0)
+        for (int jb = 0; jb < kept; jb += kThreads, bits >>= 5) {
+          const int j = jb + tid;
+          const uint32_t nb = (uint32_t)bits & 31u;
+          const unsigned below = (1u << lane) - 1u;
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int a = k == 1 ? 1 : 0, b = k == 0 ? 1 : 2;
-        need[k] = in && ((m >> a) & 1u) && ((m >> b) & 1u) && !(lb[k] > bhi);
-        msk[k] = __ballot_sync(FULL_MASK, need[k]);
-      }
-      const int n0 = __popc(msk[0]), n1 = __popc(msk[1]), n2 = __popc(msk[2]);
-      if (n0 + n1 + n2 > 0) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&sh.ntri, n0 + n1 + n2);
-        base = __shfl_sync(FULL_MASK, base, 0);
-        const unsigned below = (1u << lane) - 1u;
-        const int first[3] = {base, base + n0, base + n0 + n1};  // the warp's pair-0 items, then 1, then 2
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          if (!need[k]) continue;
-          const int p = first[k] + __popc(msk[k] & below);
-          if (p < kTriCap) {
-            sh.tri[p] = (uint16_t)(j | (k << 14));
-          } else {  // list full: screen here
-            tri_list_full(d, ph, sh, j, k, slot, bhi, exact_all);
+          for (int k = 0; k < 3; ++k) {
+            const unsigned msk = __ballot_sync(FULL_MASK, (nb >> k) & 1u);
+            if ((nb >> k) & 1u) {
+              const int p = pt + __popc(msk & below);
+              if (p < kTriCap) sh.tri[p] = (uint16_t)(j | (k << 14));
+              else tri_list_full(d, ph, sh, j, k, sh.cs[j], funkey(sh.bhi[sh.cs[j]]), exact_all);  // screen here
+            }
+            pt += __popc(msk);
           }
+          const unsigned mq = __ballot_sync(FULL_MASK, (nb >> 3) & 1u);
+          if ((nb >> 3) & 1u) sh.tet[pq + __popc(mq & below)] = (uint16_t)j;  // kTetCap == kCornerCap: never full
+          pq += __popc(mq);
+          const unsigned me = __ballot_sync(FULL_MASK, (nb >> 4) & 1u);
+          if ((nb >> 4) & 1u) sh.edg[pe + __popc(me & below)] = (uint16_t)j;  // one entry per corner at most: never full
+          pe += __popc(me);
         }
-      }
-      {
-        const bool need = in && m == 7u && !(lb[3] > bhi);
-        const int p = warp_append(&sh.ntet, need, lane);
-        if (p >= 0) sh.tet[p] = (uint16_t)j;  // kTetCap == kCornerCap: never full
-      }
-      {
-        // the corners with an edge that can still be the minimum: the
-        // smallest edge lower bound (phase A) against bhi; the FP32 mode
-        // lists every corner with a valid edge
-        bool need = false;
-        if (in) need = fp32 ? m != 0u : !(elo > bhi);
-        const int p = warp_append(&sh.nedge, need, lane);
-        if (p >= 0) sh.edg[p] = (uint16_t)j;  // one entry per corner at most: never full
-      }
     }
     __syncthreads();
     PROBE(kPrB);
@@ -733,8 +730,8 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     // Few listed solves go to phase D as they are (direct): the screens' chain
     // is as long for one solve as for 32, and so is that of the FP64 solves,
     // so dropping the screens shortens the phase.
-    const bool direct = !exact_all && !fp32 && sh.ntri <= kTriCap &&
-                        fp64_cost(sh.ntet, sh.ntri, 3 * sh.nedge, dag_warps) <= kDirectCost;
+    const bool direct = !exact_all && !fp32 && sh.nlist[0] <= kTriCap &&
+                        fp64_cost(sh.nlist[1], sh.nlist[0], 3 * sh.nlist[2], dag_warps) <= kDirectCost;
 
     // S: screens over the compacted lists, handed out in chunks to whichever
     // warp is free -- tets first (32 per chunk, one per lane), then triangles
@@ -745,10 +742,10 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     // queued at once (bhi only decreases: phase D rechecks against the final
     // bound)
     if (!direct) {
-      const int ntet = min(sh.ntet, kTetCap), ntri = min(sh.ntri, kTriCap);
+      const int ntet = min(sh.nlist[1], kTetCap), ntri = min(sh.nlist[0], kTriCap);
       const int tri0 = (ntet + 31) & ~31;
       const int edge_c0 = tri0 + ((ntri + 63) / 64) * 32;  // claim index of the first edge chunk
-      const int nedge = sh.nedge;
+      const int nedge = sh.nlist[2];
       const int nclaim = edge_c0 + ((nedge + 31) & ~31);
       for (;;) {
         // claims of 32: tet chunks, then triangle chunks of 64 (two per
@@ -888,8 +885,8 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     {
       // (direct: the screen lists, with every edge of a listed corner; their
       // lower bounds are at most bhi, which phase A left final)
-      const int ntet = direct ? sh.ntet : min(sh.nq[0], kQcap), ntri = direct ? sh.ntri : min(sh.nq[1], kQcap);
-      const int nedge = direct ? 3 * sh.nedge : min(sh.nq[2], kQcap);
+      const int ntet = direct ? sh.nlist[1] : min(sh.nq[0], kQcap), ntri = direct ? sh.nlist[0] : min(sh.nq[1], kQcap);
+      const int nedge = direct ? 3 * sh.nlist[2] : min(sh.nq[2], kQcap);
       const bool shared_ids = direct && kept <= kIdsCap;
       // tets: one group of kDagLanes lanes per tet runs the prefix
       // (tet_dag_prefix); then the roots, two per tet, on consecutive

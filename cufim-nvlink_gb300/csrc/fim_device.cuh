@@ -71,6 +71,15 @@ __device__ __forceinline__ float d2f_pow2(double x, int s)
   return (float)(x * ldexp(1.0, -s));
 }
 
+// The float copy of a time: rounded to nearest, +inf only for FIM_INF (a
+// larger finite time than a float holds gives NaN, "ask the FP64 time"), so
+// that a vertex without a time shows by its copy alone.
+__device__ __forceinline__ float time_f(double x)
+{
+  const float f = (float)x;
+  return f == INFINITY && x < FIM_INF ? __int_as_float(0x7fffffff) : f;
+}
+
 // x > 0 (false for zeros and NaN)
 __device__ __forceinline__ bool dgt0(double x)
 {

@@ -56,6 +56,14 @@ struct FimCtl {
   unsigned long long iters_total;   // submesh sweeps: iterations of all windows
 };
 
+// The float copy of a vertex copy's next time and its state word: state (low
+// 8 bits) | iteration stamp of "marked" << 8.  Side by side, because the
+// re-solve phase gathers both of every neighbour.
+struct alignas(8) VState {
+  float f2;
+  uint32_t sw;
+};
+
 // Everything the persistent kernel touches, as device pointers.
 //
 // Vertices of the kernel are vertex *copies*: with submesh tags every
@@ -77,14 +85,13 @@ struct FimDev {
   const uint4 *crec;          // [kCrecWords*nC] first-read record of each corner (kCrecWords)
   const double *cgeo;         // [nC*kCgeoStride] FP64 e13, e23, e34, e12, e14, e24
   const float *cgf;           // [nC*kCgfStride] float screen record: e13..e24 * 2^-k, k, unused
-  float *phi_f;               // float copy (round to nearest) of phi, kept in step with it
-  float *phi2_f;              // float copy of phi2
+  float *phi_f;               // float copy (time_f) of phi, kept in step with it
   const int64_t *nptr;        // [nV+1] vertex neighbourhood (self included)
   const int32_t *nbr;
   // state
   double *phi;                // current times
   double *phi2;               // next times (equal to phi outside the updated lists)
-  uint32_t *sw;               // state word: state (low 8 bits) | iteration stamp of "marked" << 8
+  VState *vs;                 // float copy of phi2 and state word
   uint8_t *st;                // states as bytes, written at the end of a solve (the result)
   uint8_t *tst;               // reference tmp_state
   int32_t *list[3];           // rotating narrow lists
@@ -233,9 +240,9 @@ constexpr int64_t kStaticMaxSeedEntries = 32768;   // stimulus entries expanded 
 // Pointers into the fixed scratch of one device.
 struct NoallocScratch {
   double *phi, *phi2;
-  uint32_t *sw;
+  VState *vs;
   int32_t *list[3], *lfrozen, *lmarked;
-  float *phi_f, *phi2_f;
+  float *phi_f;
   uint8_t *st, *tst, *dec, *st_out;
   unsigned long long *key;   // per mesh vertex: earliest stimulus time (order-preserving key)
   int64_t *raw_v;            // stimuli as given

@@ -280,7 +280,7 @@ __global__ void fim_support_kernel(FimDev d, double lower, float lower_lo, float
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         const Re P = re_in(__ldcg(d.phi_f + nb[i]));
-        bool valid = (__ldcg(d.sw + nb[i]) & 0xffu) >= ST_NARROW;
+        bool valid = (__ldcg(&d.vs[nb[i]].sw) & 0xffu) >= ST_NARROW;
         if (valid) {
           if (re_lo(P) > lower_hi) valid = true;
           else if (re_hi(P) <= lower_lo) valid = false;
@@ -317,10 +317,10 @@ __global__ void fim_warm_reset_kernel(FimDev d, double tmin)
     d.tst[v] = ST_FAR;
     if (x >= tmin) {
       d.phi[v] = FIM_INF; d.phi2[v] = FIM_INF;
-      d.phi_f[v] = (float)FIM_INF; d.phi2_f[v] = (float)FIM_INF;
-      d.sw[v] = ST_FAR;
+      d.phi_f[v] = INFINITY;
+      d.vs[v] = VState{INFINITY, ST_FAR};
     } else if (x < FIM_INF) {
-      d.sw[v] = ST_NARROW;
+      d.vs[v].sw = ST_NARROW;
     }
   }
 }
@@ -331,8 +331,8 @@ __global__ void fim_reseed_kernel(FimDev d)
     const int32_t v = d.seed_v[i];
     const double x = d.seed_t[i];
     d.phi[v] = x; d.phi2[v] = x;
-    d.phi_f[v] = (float)x; d.phi2_f[v] = (float)x;
-    d.sw[v] = ST_NARROW;
+    d.phi_f[v] = time_f(x);
+    d.vs[v] = VState{time_f(x), ST_NARROW};
   }
 }
 

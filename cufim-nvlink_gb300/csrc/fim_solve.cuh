@@ -396,7 +396,7 @@ __device__ __noinline__ int64_t excess_corners(const FimDev &d, const double *ph
     uint32_t m = 0;
     for (int i = 0; i < 3; ++i) {
       const double p = __ldcg(ph + nb[i]);
-      if (sw_seen(__ldcg(d.sw + nb[i]), marked_mode, stamp) >= ST_NARROW && p > lower) {
+      if (sw_seen(__ldcg(&d.vs[nb[i]].sw), marked_mode, stamp) >= ST_NARROW && p > lower) {
         m |= 1u << i;
         atomicMin(&sh.res[slot], dkey(p + sqrt(__ldg(d.cgeo + kCgeoStride * c + edge_slot(i)))));
       }
@@ -412,18 +412,23 @@ __device__ __noinline__ int64_t excess_corners(const FimDev &d, const double *ph
   return n_valid;
 }
 
+__device__ __forceinline__ VState ld_vs(const FimDev &d, int64_t v)
+{
+  const uint2 q = __ldcg(reinterpret_cast<const uint2 *>(d.vs + v));
+  return VState{__uint_as_float(q.x), q.y};
+}
 // Writes a time and its float copy.
 __device__ __forceinline__ void set_phi(const FimDev &d, int64_t v, double x)
 {
   d.phi[v] = x;
-  d.phi_f[v] = (float)x;
+  d.phi_f[v] = time_f(x);
 }
 // Writes a time into both time buffers and their float copies.
 __device__ __forceinline__ void set_phi_both(const FimDev &d, int64_t v, double x)
 {
-  const float f = (float)x;
+  const float f = time_f(x);
   d.phi[v] = x; d.phi_f[v] = f;
-  d.phi2[v] = x; d.phi2_f[v] = f;
+  d.phi2[v] = x; d.vs[v].f2 = f;
 }
 
 // Work of another list that runs inside a phase: load() starts its loads
@@ -451,10 +456,11 @@ struct ApplySide {
   {
     if (!pending || i < 0) return;
     v = lst[i];
-    w = __ldcg(d.sw + v);
+    const VState q = ld_vs(d, v);
+    w = q.sw;
+    xf = q.f2;
     tv = __ldcg(d.tst + v);
     x = __ldcg(d.phi2 + v);
-    xf = __ldcg(d.phi2_f + v);
   }
   __device__ __forceinline__ void store()
   {
@@ -465,7 +471,7 @@ struct ApplySide {
       d.phi[v] = x;
       d.phi_f[v] = xf;
       if (sw_state(w) == ST_NARROW) {
-        if (tv == ST_FROZEN) d.sw[v] = ST_FROZEN;
+        if (tv == ST_FROZEN) d.vs[v].sw = ST_FROZEN;
         else push = true;
       }
     }
@@ -531,7 +537,6 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
 {
   constexpr bool kMarkedMode = is_marked_mode(MODE);
   const double *ph = MODE == kMarked2 ? d.phi2 : d.phi;      // times this phase reads
-  const float *phf = MODE == kMarked2 ? d.phi2_f : d.phi_f;
   const int tid = threadIdx.x, lane = tid & 31;
   const int64_t per_block = lo_.local ? (int64_t)n : ((int64_t)n + gridDim.x - 1) / gridDim.x;
   const int64_t lbeg = lo_.local ? 0 : min((int64_t)n, (int64_t)blockIdx.x * per_block);
@@ -550,7 +555,8 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
       sh.cnt[tid] = (int32_t)(d.cptr[v + 1] - d.cptr[v]);
       sh.old[tid] = old;
       sh.res[tid] = dkey(old);
-      sh.bhi[tid] = fkey(exact_all ? INFINITY : re_hi(re_in(__ldcg(phf + v))));
+      const float oh = re_hi(re_in(MODE == kMarked2 ? __ldcg(&d.vs[v].f2) : __ldcg(d.phi_f + v)));
+      sh.bhi[tid] = fkey(exact_all || !(oh == oh) ? INFINITY : oh);
       if (MODE == kNarrow2) {
         const int64_t a = d.nptr[v];
         sh.n0[tid] = a;
@@ -625,8 +631,19 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
         const int32_t nbs[3] = {(int32_t)h0.x, (int32_t)h0.y, (int32_t)h0.z};
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-          pf[i] = __ldcg(phf + nbs[i]);
-          stn[i] = (uint8_t)sw_seen(__ldcg(d.sw + nbs[i]), kMarkedMode, stamp);
+          // Only the re-solves need the neighbours' words: they ignore the
+          // vertices marked in this iteration.  Otherwise a neighbour counts
+          // (state >= narrow) exactly when it has a time, since a far vertex
+          // has none.
+          if (MODE == kMarked2) {
+            const VState q = ld_vs(d, nbs[i]);
+            pf[i] = q.f2;
+            stn[i] = (uint8_t)sw_seen(q.sw, true, stamp);
+          } else {
+            pf[i] = __ldcg(d.phi_f + nbs[i]);
+            stn[i] = kMarkedMode ? (uint8_t)sw_seen(__ldcg(&d.vs[nbs[i]].sw), true, stamp)
+                                 : (uint8_t)(pf[i] == INFINITY ? ST_FAR : ST_NARROW);
+          }
         }
         const float len[3] = {__uint_as_float(h1.x), __uint_as_float(h1.y), __uint_as_float(h1.z)};
         uint32_t m = 0;
@@ -634,8 +651,9 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           const Re P = re_in(pf[i]);
-          lo[i] = re_lo(P);
-          hi[i] = re_hi(P);
+          const bool known = pf[i] == pf[i];  // else beyond the floats (time_f): no bounds
+          lo[i] = known ? re_lo(P) : -INFINITY;
+          hi[i] = known ? re_hi(P) : INFINITY;
           bool ok = stn[i] >= ST_NARROW;
           if (ok) {
             if (lo[i] > lower_hi) ok = true;
@@ -646,7 +664,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
             m |= 1u << i;
             const Re E = P + re_len(len[i]);
             ub = fminf(ub, re_hi(E));
-            elo = fminf(elo, re_lo(E));
+            elo = known ? fminf(elo, re_lo(E)) : -INFINITY;
           }
           sh.pf[j][i] = pf[i];
           if (kept <= kIdsCap) sh.ids[j][i] = nbs[i];
@@ -1004,7 +1022,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
         if (MODE == kNarrow4) {
           d.tst[v] = ST_FAR;
           if (nw - phi_start > dt) {
-            d.sw[v] = ST_NEXT;
+            d.vs[v].sw = ST_NEXT;
           } else if (fabs(old - nw) < (1e-6 * (1 + (old + nw) * .5))) {
             d.tst[v] = ST_FROZEN;
             if (lo_.local) lo_.frozen[atomicAdd(lo_.n_frozen, 1)] = v;
@@ -1022,7 +1040,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
         const double old = sh.old[slot];
         const double nw = dunkey(sh.res[slot]);
         d.phi2[v] = nw;
-        d.phi2_f[v] = (float)nw;
+        d.vs[v].f2 = time_f(nw);
         uint8_t t = ST_FAR;
         if (fabs(old - nw) < (1e-6 * (1 + (old + nw) * .5))) {
           t = ST_FROZEN;
@@ -1050,13 +1068,13 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
           for (int h = 0; h < 2; ++h) v[h] = kk[h] < k1 ? __ldg(d.nbr + kk[h]) : -1;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            w[h] = v[h] >= 0 ? __ldcg(d.sw + v[h]) : 0u;
+            w[h] = v[h] >= 0 ? __ldcg(&d.vs[v[h]].sw) : 0u;
             pv[h] = v[h] >= 0 ? __ldcg(d.phi2 + v[h]) : 0.0;
           }
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (v[h] >= 0 && sw_state(w[h]) != ST_NARROW && sw_stamp(w[h]) != stamp && pn < pv[h]) {
-              if (atomicCAS(d.sw + v[h], w[h], sw_make(sw_state(w[h]), stamp)) == w[h]) {
+              if (atomicCAS(&d.vs[v[h]].sw, w[h], sw_make(sw_state(w[h]), stamp)) == w[h]) {
                 d.tst[v[h]] = (uint8_t)sw_state(w[h]);
                 append_active(lo_.marked, lo_.word, v[h]);
               }
@@ -1079,7 +1097,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
             if (tv == ST_FROZEN) sv = ST_FROZEN;
             else push = true;
           }
-          d.sw[v] = sw_make(sv, stamp);  // still marked for the re-solves running now
+          d.vs[v].sw = sw_make(sv, stamp);  // still marked for the re-solves running now
           set_phi_both(d, v, nw);
         }
         const int p = warp_append(lo_.word, push, lane);
@@ -1114,13 +1132,13 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
   __syncthreads();
   // update_states (cuda_fim.cu:1790-1845) on the block's copies
   for (int32_t v = c0 + tid; v < c1; v += kThreads) {
-    uint8_t stv = (uint8_t)sw_state(d.sw[v]);
-    if (stv == ST_NEXT) { stv = ST_NARROW; d.sw[v] = stv; }
+    uint8_t stv = (uint8_t)sw_state(d.vs[v].sw);
+    if (stv == ST_NEXT) { stv = ST_NARROW; d.vs[v].sw = stv; }
     else if (p.apd >= 0.0 && stv == ST_FROZEN) {
-      if (!(d.phi[v] + p.apd > cur_time)) d.sw[v] = ST_TAIL;
+      if (!(d.phi[v] + p.apd > cur_time)) d.vs[v].sw = ST_TAIL;
     } else if (p.apd >= 0.0 && stv == ST_TAIL) {
       if (!(d.phi[v] + p.apd / 0.91 > cur_time)) {
-        set_phi_both(d, v, FIM_INF); d.sw[v] = ST_FAR;
+        set_phi_both(d, v, FIM_INF); d.vs[v].sw = ST_FAR;
       }
     }
     if (stv == ST_NARROW) d.list[s][c0 + atomicAdd(&b_narrow[s], 1)] = v;
@@ -1163,10 +1181,10 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
       const double pn = __ldcg(d.phi2 + n);
       for (int64_t k = d.nptr[n] + tid % kMarkLanes; k < d.nptr[n + 1]; k += kMarkLanes) {
         const int32_t v = __ldg(d.nbr + k);
-        const uint32_t w = __ldcg(d.sw + v);
+        const uint32_t w = __ldcg(&d.vs[v].sw);
         const double pv = __ldcg(d.phi2 + v);
         if (sw_state(w) != ST_NARROW && sw_stamp(w) != stamp && pn < pv) {
-          if (atomicCAS(d.sw + v, w, sw_make(ST_NEIG, stamp)) == w) {
+          if (atomicCAS(&d.vs[v].sw, w, sw_make(ST_NEIG, stamp)) == w) {
             d.tst[v] = (uint8_t)sw_state(w);
             lo.marked[atomicAdd(&b_marked, 1)] = v;
           }
@@ -1190,14 +1208,14 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
           if (tv == ST_FROZEN) sv = ST_FROZEN;
           else lnext[atomicAdd(&b_narrow[s1], 1)] = v;
         }
-        d.sw[v] = sw_make(sv, stamp);
+        d.vs[v].sw = sw_make(sv, stamp);
       } else {
         const int32_t v = lst[i - nm];
-        const uint32_t w = __ldcg(d.sw + v);
+        const uint32_t w = __ldcg(&d.vs[v].sw);
         const uint8_t tv = __ldcg(d.tst + v);
         if (sw_stamp(w) == stamp) continue;
         if (sw_state(w) == ST_NARROW) {
-          if (tv == ST_FROZEN) d.sw[v] = ST_FROZEN;
+          if (tv == ST_FROZEN) d.vs[v].sw = ST_FROZEN;
           else lnext[atomicAdd(&b_narrow[s1], 1)] = v;
         }
       }
@@ -1249,7 +1267,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
   if (!p.resume) {
     for (int64_t v = gtid; v < d.nV; v += nthreads) {
       const double x = d.phi_init ? d.phi_init[v] : FIM_INF;
-      set_phi_both(d, v, x); d.sw[v] = x < FIM_INF ? ST_NARROW : ST_FAR; d.tst[v] = ST_FAR;
+      set_phi_both(d, v, x); d.vs[v].sw = x < FIM_INF ? ST_NARROW : ST_FAR; d.tst[v] = ST_FAR;
     }
     // failure-detection test hook: this block never arrives at the barrier (a
     // flag that nothing sets), so the others' bounded waits must expire
@@ -1257,7 +1275,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
     if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &unused)) return;
     for (int64_t i = gtid; i < d.nseed; i += nthreads) {
       const int32_t v = d.seed_v[i];
-      set_phi_both(d, v, d.seed_t[i]); d.sw[v] = ST_NARROW;
+      set_phi_both(d, v, d.seed_t[i]); d.vs[v].sw = ST_NARROW;
     }
     if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &unused)) return;
   }
@@ -1285,7 +1303,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         }
         for (int64_t k = k0; k < k1; ++k) {
           const int32_t c = d.gcopy[k];
-          if (mn < __ldcg(d.phi + c)) { set_phi_both(d, c, mn); d.sw[c] = ST_NARROW; }
+          if (mn < __ldcg(d.phi + c)) { set_phi_both(d, c, mn); d.vs[c].sw = ST_NARROW; }
         }
       }
     }
@@ -1304,13 +1322,13 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
     }
     // update_states (cuda_fim.cu:1790-1845) -> narrow list of this window
     for (int64_t v = gtid; v < d.nV; v += nthreads) {
-      uint8_t stv = (uint8_t)sw_state(d.sw[v]);
-      if (stv == ST_NEXT) { stv = ST_NARROW; d.sw[v] = stv; }
+      uint8_t stv = (uint8_t)sw_state(d.vs[v].sw);
+      if (stv == ST_NEXT) { stv = ST_NARROW; d.vs[v].sw = stv; }
       else if (p.apd >= 0.0 && stv == ST_FROZEN) {
-        if (!(d.phi[v] + p.apd > cur_time)) d.sw[v] = ST_TAIL;
+        if (!(d.phi[v] + p.apd > cur_time)) d.vs[v].sw = ST_TAIL;
       } else if (p.apd >= 0.0 && stv == ST_TAIL) {
         if (!(d.phi[v] + p.apd / 0.91 > cur_time)) {
-          set_phi_both(d, v, FIM_INF); d.sw[v] = ST_FAR;
+          set_phi_both(d, v, FIM_INF); d.vs[v].sw = ST_FAR;
         }
       }
       if (stv == ST_NARROW) append_active(d.list[s], word(), (int32_t)v);
@@ -1396,10 +1414,10 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
             // both loads at once; the word changes only by the exchange below,
             // so w is still v's word there unless another frozen vertex won
             const int32_t v = __ldg(d.nbr + k);
-            const uint32_t w = __ldcg(d.sw + v);
+            const uint32_t w = __ldcg(&d.vs[v].sw);
             const double pv = __ldcg(d.phi2 + v);
             if (sw_state(w) != ST_NARROW && sw_stamp(w) != stamp && pn < pv) {
-              if (atomicCAS(d.sw + v, w, sw_make(ST_NEIG, stamp)) == w) {
+              if (atomicCAS(&d.vs[v].sw, w, sw_make(ST_NEIG, stamp)) == w) {
                 d.tst[v] = (uint8_t)sw_state(w);
                 append_active(d.lmarked, lo.word, v);
               }
@@ -1417,11 +1435,11 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
         // valid neighbour
         for (int64_t i = gtid; i < nn; i += nthreads) {
           const int32_t v = lst[i];
-          const uint32_t w = __ldcg(d.sw + v);
+          const uint32_t w = __ldcg(&d.vs[v].sw);
           const uint8_t tv = __ldcg(d.tst + v);
           if (sw_stamp(w) == stamp) continue;  // re-solved below
           if (sw_state(w) == ST_NARROW) {
-            if (tv == ST_FROZEN) d.sw[v] = ST_FROZEN;
+            if (tv == ST_FROZEN) d.vs[v].sw = ST_FROZEN;
             else append_active(lnext, lo.word, v);
           }
         }
@@ -1444,7 +1462,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
       for (int64_t k = d.gptr[g]; k < d.gptr[g + 1]; ++k) {
         const int32_t c = d.gcopy[k];
         const double pc = __ldcg(d.phi + c);
-        const uint8_t sc = (uint8_t)sw_state(__ldcg(d.sw + c));
+        const uint8_t sc = (uint8_t)sw_state(__ldcg(&d.vs[c].sw));
         if (pc < mn) mn = pc;
         if (sc > mx) mx = sc;
       }
@@ -1452,7 +1470,7 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
       d.st_out[g] = mx;
     }
   } else {
-    for (int64_t v = gtid; v < d.nV; v += nthreads) d.st[v] = (uint8_t)sw_state(__ldcg(d.sw + v));
+    for (int64_t v = gtid; v < d.nV; v += nthreads) d.st[v] = (uint8_t)sw_state(__ldcg(&d.vs[v].sw));
   }
 
   // statistics

@@ -151,14 +151,14 @@ struct fim_solver {
   DevBuf<int64_t> cidx, cptr, nptr;
   DevBuf<uint4> crec;
   DevBuf<double> cgeo;
-  DevBuf<float> cgf, phi_f, phi2_f;
+  DevBuf<float> cgf, phi_f;
   DevBuf<int32_t> nbr;
   DevBuf<double> fib, cf, ct;
   DevBuf<unsigned long long> bad;  // first invalid tet of the last conduction upload
   // state
   DevBuf<double> phi, phi2;
   DevBuf<uint8_t> st, tst, dec;
-  DevBuf<uint32_t> sw;
+  DevBuf<VState> vs;
   DevBuf<int32_t> list0, list1, list2, lfrozen, lmarked;
   DevBuf<unsigned long long> probe;  // phase times (FIM_PROBE builds)
   DevBuf<int32_t> seed_v;
@@ -489,8 +489,8 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
     a.add(s->crec, (size_t)kCrecWords * nC); a.add(s->cgeo, (size_t)kCgeoStride * nC);
     a.add(s->cgf, (size_t)kCgfStride * nC);
     a.add(s->fib, 3 * nT); a.add(s->cf, nT); a.add(s->ct, nT);
-    a.add(s->phi, nL); a.add(s->phi_f, nL); a.add(s->phi2, nL); a.add(s->phi2_f, nL);
-    a.add(s->st, nL); a.add(s->tst, nL); a.add(s->dec, nL); a.add(s->sw, nL);
+    a.add(s->phi, nL); a.add(s->phi_f, nL); a.add(s->phi2, nL); a.add(s->vs, nL);
+    a.add(s->st, nL); a.add(s->tst, nL); a.add(s->dec, nL);
     a.add(s->list0, nL); a.add(s->list1, nL); a.add(s->list2, nL); a.add(s->lfrozen, nL); a.add(s->lmarked, nL);
     if (multi) { a.add(s->gptr, nV + 1); a.add(s->gcopy, nL); a.add(s->phi_out, nV); a.add(s->st_out, nV); }
     return a.off;
@@ -779,8 +779,8 @@ static void solve_args(const fim_solver *s, FimDev &d, FimParams &p)
   d.nV = (int32_t)s->nL; d.nG = (int32_t)s->nV; d.nT = s->nT; d.nC = s->nC;
   d.gptr = s->gptr.p; d.gcopy = s->gcopy.p; d.phi_out = s->phi_out.p; d.st_out = s->st_out.p;
   d.cptr = s->cptr.p; d.crec = s->crec.p; d.cgeo = s->cgeo.p; d.cgf = s->cgf.p; d.nptr = s->nptr.p; d.nbr = s->nbr.p;
-  d.phi_f = s->phi_f.p; d.phi2_f = s->phi2_f.p;
-  d.phi = s->phi.p; d.phi2 = s->phi2.p; d.sw = s->sw.p; d.st = s->st.p; d.tst = s->tst.p;
+  d.phi_f = s->phi_f.p;
+  d.phi = s->phi.p; d.phi2 = s->phi2.p; d.vs = s->vs.p; d.st = s->st.p; d.tst = s->tst.p;
   d.list[0] = s->list0.p; d.list[1] = s->list1.p; d.list[2] = s->list2.p;
   d.lfrozen = s->lfrozen.p; d.lmarked = s->lmarked.p; d.dec = s->dec.p;
   d.seed_v = s->seed_v.p; d.seed_t = s->seed_t.p; d.nseed = s->nseed;
@@ -1232,8 +1232,8 @@ extern "C" int fim_solve_noalloc(fim_solver *s, int64_t n, const int64_t *vertic
   d.gptr = s->gptr.p; d.gcopy = s->gcopy.p;
   d.phi_out = multi ? d_phi : nullptr; d.st_out = multi ? sc.st_out : nullptr;
   d.cptr = s->cptr.p; d.crec = s->crec.p; d.cgeo = s->cgeo.p; d.cgf = s->cgf.p; d.nptr = s->nptr.p; d.nbr = s->nbr.p;
-  d.phi_f = sc.phi_f; d.phi2_f = sc.phi2_f;
-  d.phi = sc.phi; d.phi2 = sc.phi2; d.sw = sc.sw; d.st = sc.st; d.tst = sc.tst;
+  d.phi_f = sc.phi_f;
+  d.phi = sc.phi; d.phi2 = sc.phi2; d.vs = sc.vs; d.st = sc.st; d.tst = sc.tst;
   d.list[0] = sc.list[0]; d.list[1] = sc.list[1]; d.list[2] = sc.list[2];
   d.lfrozen = sc.lfrozen; d.lmarked = sc.lmarked; d.dec = sc.dec;
   d.seed_v = sc.seed_v; d.seed_t = sc.seed_t; d.nseed = (int32_t)entries;

@@ -9,8 +9,8 @@
 // module, so it is only loaded on devices where this path is used.
 //
 // Layout (every part starts on a 256-byte boundary): per vertex copy
-// phi, phi2 (f64), sw (u32), list[3], lfrozen, lmarked (i32), phi_f,
-// phi2_f (f32), st, tst, dec (u8); per mesh vertex the gathered states st_out (u8) and
+// phi, phi2 (f64), vs (VState), list[3], lfrozen, lmarked (i32), phi_f
+// (f32), st, tst, dec (u8); per mesh vertex the gathered states st_out (u8) and
 // the stimulus keys (u64); the raw stimuli as given (i64 vertex, f64
 // time), the stimulus entries expanded to vertex copies (i32, f64); the
 // control block FimCtl.
@@ -18,7 +18,7 @@
 // What must start at zero: only the FimCtl block (phase words, error
 // word).  fim_solve_noalloc clears it with
 // cudaMemsetAsync before every launch.  Everything else is written before it
-// is read within one call: the solve kernel resets phi/phi2/sw/tst of every
+// is read within one call: the solve kernel resets phi/phi2/vs/tst of every
 // copy, the lists are filled behind their counters, and the stimulus
 // kernel sets the key of every stimulated vertex before it takes minima.
 #include "fim_internal.h"
@@ -35,15 +35,14 @@ constexpr size_t kC = (size_t)kStaticMaxCopies;
 constexpr size_t kG = (size_t)kStaticMaxVertices;
 constexpr size_t kOffPhi = 0;
 constexpr size_t kOffPhi2 = kOffPhi + align256(8 * kC);
-constexpr size_t kOffSw = kOffPhi2 + align256(8 * kC);
-constexpr size_t kOffList0 = kOffSw + align256(4 * kC);
+constexpr size_t kOffVs = kOffPhi2 + align256(8 * kC);
+constexpr size_t kOffList0 = kOffVs + align256(sizeof(VState) * kC);
 constexpr size_t kOffList1 = kOffList0 + align256(4 * kC);
 constexpr size_t kOffList2 = kOffList1 + align256(4 * kC);
 constexpr size_t kOffFrozen = kOffList2 + align256(4 * kC);
 constexpr size_t kOffMarked = kOffFrozen + align256(4 * kC);
 constexpr size_t kOffPhiF = kOffMarked + align256(4 * kC);
-constexpr size_t kOffPhi2F = kOffPhiF + align256(4 * kC);
-constexpr size_t kOffSt = kOffPhi2F + align256(4 * kC);
+constexpr size_t kOffSt = kOffPhiF + align256(4 * kC);
 constexpr size_t kOffTst = kOffSt + align256(kC);
 constexpr size_t kOffDec = kOffTst + align256(kC);
 constexpr size_t kOffStOut = kOffDec + align256(kC);
@@ -147,14 +146,13 @@ cudaError_t noalloc_scratch(int device, NoallocScratch *out)
   }
   out->phi = reinterpret_cast<double *>(base + kOffPhi);
   out->phi2 = reinterpret_cast<double *>(base + kOffPhi2);
-  out->sw = reinterpret_cast<uint32_t *>(base + kOffSw);
+  out->vs = reinterpret_cast<VState *>(base + kOffVs);
   out->list[0] = reinterpret_cast<int32_t *>(base + kOffList0);
   out->list[1] = reinterpret_cast<int32_t *>(base + kOffList1);
   out->list[2] = reinterpret_cast<int32_t *>(base + kOffList2);
   out->lfrozen = reinterpret_cast<int32_t *>(base + kOffFrozen);
   out->lmarked = reinterpret_cast<int32_t *>(base + kOffMarked);
   out->phi_f = reinterpret_cast<float *>(base + kOffPhiF);
-  out->phi2_f = reinterpret_cast<float *>(base + kOffPhi2F);
   out->st = base + kOffSt;
   out->tst = base + kOffTst;
   out->dec = base + kOffDec;

@@ -151,11 +151,44 @@ __device__ __forceinline__ double tri_ref(double e12, double e13, double e23, do
 // Where the float is not decided, or an operand is far from 1 (where the
 // bounds above could meet subnormals), tri_root_ref evaluates the root as
 // the reference does.
+//
+// The conversions are plain shifts of the bit patterns, without branches:
+// every operand whose exponent they cannot take raises `odd`, which also
+// ends in tri_root_ref.  One warp, both roots: tri_ref 3.40 us, this 2.40 us
+// (0.88 us up to the roots, 0.76 us each); 3.55 us with conversions that
+// branch to the hardware's for zeros and subnormals.
+__device__ __forceinline__ uint32_t dhi(double x) { return (uint32_t)__double2hiint(x); }
+// (double)f for a normal f (zero becomes 2^-127)
+__device__ __forceinline__ double f2d_normal(float f)
+{
+  const uint32_t u = __float_as_uint(f);
+  return __hiloint2double((int)(((u & 0x7fffffffu) >> 3) + 0x38000000u | (u & 0x80000000u)), (int)(u << 29));
+}
+// whether x lies in [2^-126, 2^127) by magnitude
+__device__ __forceinline__ bool d_float_range(double x) { return (dhi(x) & 0x7fffffffu) - 0x38100000u < 0x0fd00000u; }
+// (float)x rounded to nearest (ties to even), for d_float_range(x)
+__device__ __forceinline__ float d2f_normal(double x)
+{
+  const uint32_t hi = dhi(x), lo = (uint32_t)__double2loint(x);
+  uint32_t r = __funnelshift_l(lo, (hi & 0x7fffffffu) - 0x38000000u, 3);
+  r += (lo & 0x1fffffffu) + (r & 1u) > 0x10000000u ? 1u : 0u;
+  return __uint_as_float(r | (hi & 0x80000000u));
+}
+// x truncated to a float, for d_float_range(x); 0 below it
+__device__ __forceinline__ float d2f_trunc(double x)
+{
+  const uint32_t hi = dhi(x), m = hi & 0x7fffffffu;
+  const uint32_t r = __funnelshift_l((uint32_t)__double2loint(x), m - 0x38000000u, 3);
+  return __uint_as_float(m < 0x38100000u ? 0u : r | (hi & 0x80000000u));
+}
+
 struct TriPre {
   double a, b, c, p2, p12, bpc, stp;
   float dv;
+  bool odd;
 };
 
+// false: no root has a value
 __device__ __forceinline__ bool tri_prepare(double e12, double e13, double e23, double p1, double p2, TriPre &t)
 {
   t.a = e23;
@@ -163,12 +196,22 @@ __device__ __forceinline__ bool tri_prepare(double e12, double e13, double e23, 
   t.c = e12;
   t.p2 = p2;
   t.p12 = p2 - p1;
-  const float dv = d2f(t.p12 * t.p12 - t.c);
-  const float sv = d2f(f2d(dv) * (t.b * t.b - t.a * t.c));
+  const double dvd = t.p12 * t.p12 - t.c;
+  float dv = d2f_normal(dvd);
+  const double gram = t.b * t.b - t.a * t.c;
+  double svd = f2d_normal(dv) * gram;
+  float sv = d2f_normal(svd);
+  double dd = t.c * f2d_normal(dv);
+  t.dv = d2f_normal(dd);
+  t.odd = !(d_float_range(dvd) && d_float_range(svd) && d_float_range(dd));
+  if (t.odd) {  // rare: the conversions that take everything
+    dv = d2f(dvd);
+    sv = d2f(f2d(dv) * gram);
+    t.dv = d2f(t.c * f2d(dv));
+  }
   if (!(dv != 0.f && sv >= 0.f)) return false;
-  t.dv = d2f(t.c * f2d(dv));
   t.bpc = t.b * t.p12 * t.p12 - t.b * t.c;
-  t.stp = f2d(sqrtf(sv)) * t.p12;
+  t.stp = (t.odd ? f2d(sqrtf(sv)) : f2d_normal(sqrtf(sv))) * t.p12;
   return true;
 }
 
@@ -186,32 +229,30 @@ __device__ __forceinline__ bool mid_range(float x) { return fabsf(x) >= 0x1p-60f
 __device__ __forceinline__ double tri_root(const TriPre &t, bool second)
 {
   const double n = -(t.bpc + (second ? t.stp : -t.stp));
-  const float nf = d2f(n);
+  const float nf = d2f_trunc(n);
   const float q = __fdividef(nf, t.dv);
-  const float dl = __fdividef(d2f(fma(-f2d(q), f2d(t.dv), n)), t.dv);
+  const float dl = __fdividef(d2f_trunc(fma(-f2d_normal(q), f2d_normal(t.dv), n)), t.dv);
   const float l = q + dl, lr = dl - (l - q), lerr = fabsf(l) * 0x1p-42f;  // q + dl == l + lr
-  bool sure = mid_range(t.dv) && mid_range(nf) && fabsf(q) >= 0x1p-40f && fabsf(q) <= 0x1p40f &&
+  bool sure = !t.odd && mid_range(t.dv) && mid_range(nf) && fabsf(q) >= 0x1p-40f && fabsf(q) <= 0x1p40f &&
               l + (lr + lerr) == l && l + (lr - lerr) == l;
   if (sure) {
     if (!((l >= 0.f) && (l <= 1.f))) return FIM_INF;
-    const double ld = f2d(l);
-    const double qd = t.a + f2d(2.f * l) * t.b + f2d(l * l) * t.c;
-    const float x = d2f(qd);
+    const double ld = f2d_normal(l), l2 = __hiloint2double((int)(dhi(ld) + 0x00100000u), __double2loint(ld));  // 2 l
+    const double qd = t.a + l2 * t.b + f2d_normal(l * l) * t.c;
+    const float x = d2f_trunc(qd);
     const float rs = rsqrtf(x), s0 = x * rs;
-    const double s0d = f2d(s0);
-    const float d0 = d2f(fma(-s0d, s0d, qd)) * 0.5f * rs;
-    const double w = t.p2 - ld * t.p12 + s0d + f2d(d0);
+    const double s0d = f2d_normal(s0);
+    const float d0 = d2f_trunc(fma(-s0d, s0d, qd)) * 0.5f * rs;
+    const double w = t.p2 - ld * t.p12 + s0d + f2d_normal(d0);
     // (float)w with 2^14 of the FP64 units in the last place to spare on
     // both sides of the rounding boundary: 2^-40 |w| and more while s0 is at
     // most 4 |w|
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(w);
-    const uint32_t e = (uint32_t)(bits >> 52) & 0x7ffu, rest = (uint32_t)bits & 0x1fffffffu;
-    uint32_t r = ((e - 896u) << 23) | ((uint32_t)(bits >> 29) & 0x7fffffu);
-    r += rest > 0x10000000u ? 1u : 0u;
-    const float rf = __uint_as_float(r | ((uint32_t)(bits >> 32) & 0x80000000u));
-    sure = x >= 0x1p-60f && x <= 0x1p60f && e - 897u < 253u && rest - (0x10000000u - 0x4000u) > 0x8000u &&
+    const uint32_t hi = dhi(w), lo = (uint32_t)__double2loint(w), rest = lo & 0x1fffffffu;
+    const uint32_t r = __funnelshift_l(lo, (hi & 0x7fffffffu) - 0x38000000u, 3) + (rest > 0x10000000u ? 1u : 0u);
+    const float rf = __uint_as_float(r | (hi & 0x80000000u));
+    sure = x >= 0x1p-60f && x <= 0x1p60f && d_float_range(w) && rest - (0x10000000u - 0x4000u) > 0x8000u &&
            s0 <= 4.f * fabsf(rf);
-    if (sure) return f2d(rf);
+    if (sure) return f2d_normal(rf);
   }
   return tri_root_ref(t.a, t.b, t.c, t.p2, t.p12, n, t.dv);
 }
@@ -265,6 +306,9 @@ __device__ __forceinline__ double tet_ref(double e13, double e23, double e34, do
 // tet_ref (every node is one correctly rounded operation of the source's own
 // expression tree).
 #include "tet_dag.inc"
+// Doubles from one group's scratch to the next: half a bank row apart (mod
+// 128 B), so that two groups of a half-warp write without conflicts.
+constexpr int kDagStride = (kDagSlots + 15) / 16 * 16 + 8;
 
 // x with its sign flipped where the word `flip` has its top bit set
 __device__ __forceinline__ double flip_sign(double x, uint32_t flip)
@@ -274,28 +318,41 @@ __device__ __forceinline__ double flip_sign(double x, uint32_t flip)
 
 // Runs the level program on scratch S (leaves already stored); gl is the
 // lane's index in its group.  All lanes of the warp take part.  A lane's
-// program words are loaded four levels ahead: read level by level from
-// constant memory, with eight addresses per warp, they lengthened every level
-// of the chain.
+// program words are loaded four levels ahead (level by level from constant
+// memory, with eight addresses per warp, they lengthened every level), and
+// its operands one level ahead: the program takes a result of the level
+// before only from the lane's own register.  One warp of four tets: 1.48 us
+// (21 levels); 1.73 us with every operand from shared memory (20 levels),
+// 1.85 us where also the groups' scratch lay on the same banks.
 __device__ __forceinline__ void tet_dag_prefix(double *S, int gl)
 {
   const uint4 *prog = kTetDagProg[gl];
-  uint4 next = __ldg(prog);
+  uint4 q = __ldg(prog), qn = __ldg(prog + 1);
+  uint32_t w = q.x;
+  double A = S[w & 255u], B = S[(w >> 8) & 255u], C = S[(w >> 16) & 255u], last = 0.0;
 #pragma unroll
-  for (int l4 = 0; l4 < kDagLevels / 4; ++l4) {
-    const uint4 q = next;
-    if (l4 + 1 < kDagLevels / 4) next = __ldg(prog + l4 + 1);
-    const uint32_t ws[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t w = ws[k];
-      const double A = flip_sign(S[w & 255u], (w << 7) & 0x80000000u);
-      const double B = S[(w >> 8) & 255u];
-      const double C = flip_sign(S[(w >> 16) & 255u], (w << 5) & 0x80000000u);
-      S[kDagLeaves + (4 * l4 + k) * kDagLanes + gl] = fma(A, B, C);
+  for (int lv = 0; lv < kDagLevels; ++lv) {
+    const double r = fma(flip_sign((w & (1u << 27)) ? last : A, (w << 7) & 0x80000000u), (w & (1u << 28)) ? last : B,
+                         flip_sign((w & (1u << 29)) ? last : C, (w << 5) & 0x80000000u));
+    // while that runs: the last result out, the next level's operands (of
+    // levels up to lv - 1) in
+    if (lv > 0) {
+      S[kDagLeaves + (lv - 1) * kDagLanes + gl] = last;
       __syncwarp();
     }
+    if (lv + 1 < kDagLevels) {
+      const int k = (lv + 1) & 3;
+      if (k == 0) {
+        q = qn;
+        if ((lv + 1) / 4 + 1 < (kDagLevels + 3) / 4) qn = __ldg(prog + (lv + 1) / 4 + 1);
+      }
+      w = k == 0 ? q.x : (k == 1 ? q.y : (k == 2 ? q.z : q.w));
+      A = S[w & 255u]; B = S[(w >> 8) & 255u]; C = S[(w >> 16) & 255u];
+    }
+    last = r;
   }
+  S[kDagLeaves + (kDagLevels - 1) * kDagLanes + gl] = last;
+  __syncwarp();
 }
 
 // One root of tet_ref from the prefix in S: second = false gives its "a"

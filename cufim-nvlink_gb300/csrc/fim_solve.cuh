@@ -88,7 +88,7 @@ constexpr int kDirectCost = FIM_DIRECT_COST;
 constexpr int kIdsCap = 2 * kQcap;
 // Phase D runs the queued tets on at most FimParams::dag_warps (<=
 // kDagWarpsMax) warps, one group of kDagLanes lanes per tet (scratch:
-// kDagGroups * kDagSlots doubles).
+// kDagGroups * kDagStride doubles).
 constexpr int kDagWarps = kDagWarpsMax * 32 <= kThreads ? kDagWarpsMax : kThreads / 32;
 constexpr int kDagGroups = kDagWarps * 32 / kDagLanes;
 
@@ -155,7 +155,7 @@ struct BatchSh {
       alignas(16) float lbv[kCornerCap][4];  // lower bounds of the triangle pairs (1,2), (2,3), (1,3) and the tet (+inf: not valid)
       float elo[kCornerCap];        // smallest lower bound of the corner's valid edges (+inf: none)
     };
-    double dag[kDagGroups][kDagSlots];  // phase D (where pf and sf are dead): scratch of the tet prefix groups
+    double dag[kDagGroups][kDagStride];  // phase D (where pf and sf are dead): scratch of the tet prefix groups
   };
   uint8_t vm[kCornerCap];           // validity bits of the three neighbours
   uint8_t cs[kCornerCap];           // slot of the corner's vertex

@@ -14,9 +14,15 @@ reassociation: the tree is the one C++ builds, left to right, unary minus
 binding tightest).  Identical subexpressions are evaluated once.
 
 The nodes are list-scheduled onto kDagLanes lanes, most critical path first.
+A node may use the result of the level before only from its own lane (it is
+still in a register); other results are read from shared memory, where they
+are in time for the level after next.  So a lane can load the operands of the
+next level while it waits for the current one, and a level costs little more
+than its DFMA.
 Output: for every lane and level one word
     bits 0-7 slot of A, 8-15 slot of B, 16-23 slot of C,
-    bits 24 and 26 sign flips of A and C (no node flips B)
+    bits 24 and 26 sign flips of A and C (no node flips B),
+    bits 27-29: A, B, C is the lane's own last result instead
 and the slots of the named results.  The node of level L and lane l writes
 slot kDagLeaves + L * kDagLanes + l.
 
@@ -155,14 +161,47 @@ def schedule(dag):
     place = {}
     level = 0
     while len(place) < len(dag.nodes):
-        ready = [i for i in range(len(dag.nodes)) if i not in place and
-                 all(r[0][0] == "leaf" or (r[0][1] in place and place[r[0][1]][0] < level)
-                     for r in dag.nodes[i][1:])]
+        def lane_of(i):
+            """Lane that node i has to take at this level (None: any), or False if it is not ready."""
+            need = None
+            for r in dag.nodes[i][1:]:
+                if r[0][0] == "leaf":
+                    continue
+                if r[0][1] not in place:
+                    return False
+                lv, ln = place[r[0][1]]
+                if lv >= level:
+                    return False
+                if lv == level - 1:
+                    if need not in (None, ln):
+                        return False
+                    need = ln
+            return need
+
+        free = set(range(LANES))
+        ready = [i for i in range(len(dag.nodes)) if i not in place and lane_of(i) is not False]
         ready.sort(key=lambda i: (-hgt(i), i))
-        for lane, i in enumerate(ready[:LANES]):
-            place[i] = (level, lane)
+        wanted = {lane_of(i) for i in ready}
+        for i in ready:
+            ln = lane_of(i)
+            if ln is None:  # a lane that no more urgent successor needs, if there is one
+                pool = sorted(free, key=lambda x: (x in wanted, x))
+                if not pool:
+                    break
+                ln = pool[0]
+            if ln not in free:
+                continue
+            free.discard(ln)
+            place[i] = (level, ln)
         level += 1
     return place, level
+
+
+def depth(dag):
+    d = []
+    for _, x, y in dag.nodes:
+        d.append(1 + max([d[r[0][1]] for r in (x, y) if r[0][0] == "node"], default=0))
+    return max(d)
 
 
 def main():
@@ -170,6 +209,7 @@ def main():
     for name, src in EXPRS:
         dag.env[name] = dag.parse(src)
     place, levels = schedule(dag)
+    critical = depth(dag)
 
     def slot(ref):
         r, _ = ref
@@ -178,21 +218,30 @@ def main():
         lv, ln = place[r[1]]
         return NLEAF + lv * LANES + ln
 
+    def own(ref, lv, ln):
+        r, _ = ref
+        return r[0] == "node" and place[r[1]] == (lv - 1, ln)
+
     prog = [[0] * LANES for _ in range(levels)]
     for i, (op, x, y) in enumerate(dag.nodes):
         lv, ln = place[i]
         if op == "mul":
             a, b, c = slot(x), slot(y), NEGZERO
             flips = (x[1], y[1], False)
+            last = (own(x, lv, ln), own(y, lv, ln), False)
         else:
             a, b, c = slot(x), ONE, slot(y)
             flips = (x[1], False, y[1] != (op == "sub"))
+            last = (own(x, lv, ln), False, own(y, lv, ln))
         word = a | (b << 8) | (c << 16)
         if flips[1]:
             raise ValueError("a negated second factor")
         for k, f in enumerate(flips):
             if f:
                 word |= 1 << (24 + k)
+        for k, f in enumerate(last):
+            if f:
+                word |= 1 << (27 + k)
         prog[lv][ln] = word
     out = {}
     for name in OUTPUTS:
@@ -208,19 +257,18 @@ def main():
         "// Generated by gen_tet_dag.py -- do not edit.  Level program of the FP64",
         "// prefix of solve_tet_cu (cuda_fim.h:1302-1360): %d DFMA nodes on %d lanes"
         % (len(dag.nodes), LANES),
-        "// in %d levels (critical path %d)." % (levels, levels),
+        "// in %d levels (critical path %d)." % (levels, critical),
         "constexpr int kDagLanes = %d, kDagLevels = %d, kDagLeaves = %d;" % (LANES, levels, NLEAF),
         "constexpr int kDagSlots = kDagLeaves + kDagLevels * kDagLanes;",
         "// leaf slots: e13 e23 e34 e12 e14 e24 p1 p2 p3, then 0.5 2.0 1.0 -0.0",
         "constexpr int kDagLeafE13 = 0, kDagLeafP1 = 6, kDagLeafConst = 9;",
     ]
     lines.append("constexpr int " + ", ".join("kDagOut_%s = %d" % (n, out[n]) for n in OUTPUTS) + ";")
-    if levels % 4:
-        raise ValueError("the levels of a lane are loaded four at a time")
-    lines.append("__device__ const uint4 kTetDagProg[kDagLanes][kDagLevels / 4] = {")
+    prog += [[0] * LANES for _ in range(-levels % 4)]  # a lane's words are loaded four at a time
+    lines.append("__device__ const uint4 kTetDagProg[kDagLanes][(kDagLevels + 3) / 4] = {")
     for ln in range(LANES):
         lines.append("  {" + ",\n   ".join("{" + ", ".join("0x%08xu" % prog[lv + k][ln] for k in range(4)) + "}"
-                                           for lv in range(0, levels, 4)) + "},")
+                                           for lv in range(0, len(prog), 4)) + "},")
     lines.append("};")
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tet_dag.inc")
     with open(path, "w") as fh:

@@ -188,6 +188,15 @@ struct TriPre {
   bool odd;
 };
 
+// The floats of an odd triangle, by the conversions that take everything
+// (out of line: rare).
+static __device__ __noinline__ void tri_odd(double dvd, double gram, double c, float &dv, float &sv, float &ddv)
+{
+  dv = d2f(dvd);
+  sv = d2f(f2d(dv) * gram);
+  ddv = d2f(c * f2d(dv));
+}
+
 // false: no root has a value
 __device__ __forceinline__ bool tri_prepare(double e12, double e13, double e23, double p1, double p2, TriPre &t)
 {
@@ -204,14 +213,13 @@ __device__ __forceinline__ bool tri_prepare(double e12, double e13, double e23, 
   double dd = t.c * f2d_normal(dv);
   t.dv = d2f_normal(dd);
   t.odd = !(d_float_range(dvd) && d_float_range(svd) && d_float_range(dd));
-  if (t.odd) {  // rare: the conversions that take everything
-    dv = d2f(dvd);
-    sv = d2f(f2d(dv) * gram);
-    t.dv = d2f(t.c * f2d(dv));
-  }
+  if (t.odd) tri_odd(dvd, gram, t.c, dv, sv, t.dv);
   if (!(dv != 0.f && sv >= 0.f)) return false;
   t.bpc = t.b * t.p12 * t.p12 - t.b * t.c;
-  t.stp = (t.odd ? f2d(sqrtf(sv)) : f2d_normal(sqrtf(sv))) * t.p12;
+  const float st = sqrtf(sv);
+  double sd = f2d_normal(st);
+  if (t.odd) sd = (double)st;
+  t.stp = sd * t.p12;
   return true;
 }
 
@@ -318,7 +326,7 @@ __device__ __forceinline__ double flip_sign(double x, uint32_t flip)
 
 // Runs the level program on scratch S (leaves already stored); gl is the
 // lane's index in its group.  All lanes of the warp take part.  A lane's
-// program words are loaded four levels ahead (level by level from constant
+// program words are loaded three levels ahead (level by level from constant
 // memory, with eight addresses per warp, they lengthened every level), and
 // its operands one level ahead: the program takes a result of the level
 // before only from the lane's own register.  One warp of four tets: 1.48 us
@@ -327,32 +335,28 @@ __device__ __forceinline__ double flip_sign(double x, uint32_t flip)
 __device__ __forceinline__ void tet_dag_prefix(double *S, int gl)
 {
   const uint4 *prog = kTetDagProg[gl];
-  uint4 q = __ldg(prog), qn = __ldg(prog + 1);
+  uint4 q = __ldg(prog);
   uint32_t w = q.x;
   double A = S[w & 255u], B = S[(w >> 8) & 255u], C = S[(w >> 16) & 255u], last = 0.0;
+  double *out = S + kDagLeaves + gl;
 #pragma unroll
-  for (int lv = 0; lv < kDagLevels; ++lv) {
-    const double r = fma(flip_sign((w & (1u << 27)) ? last : A, (w << 7) & 0x80000000u), (w & (1u << 28)) ? last : B,
-                         flip_sign((w & (1u << 29)) ? last : C, (w << 5) & 0x80000000u));
-    // while that runs: the last result out, the next level's operands (of
-    // levels up to lv - 1) in
-    if (lv > 0) {
-      S[kDagLeaves + (lv - 1) * kDagLanes + gl] = last;
+  for (int r = 0; r < kDagLevels / kDagStep; ++r) {
+    const uint4 next = __ldg(prog + (r + 1 < kDagLevels / kDagStep ? r + 1 : r));
+#pragma unroll
+    for (int k = 0; k < kDagStep; ++k) {
+      const double x = fma(flip_sign((w & (1u << 27)) ? last : A, (w << 7) & 0x80000000u), (w & (1u << 28)) ? last : B,
+                           flip_sign((w & (1u << 29)) ? last : C, (w << 5) & 0x80000000u));
+      // while that runs: the next level's operands, of levels up to the last
+      // (past the end: some again)
+      w = k == 0 ? q.y : (k == 1 ? q.z : next.x);
+      A = S[w & 255u]; B = S[(w >> 8) & 255u]; C = S[(w >> 16) & 255u];
+      last = x;
+      *out = last;
+      out += kDagLanes;
       __syncwarp();
     }
-    if (lv + 1 < kDagLevels) {
-      const int k = (lv + 1) & 3;
-      if (k == 0) {
-        q = qn;
-        if ((lv + 1) / 4 + 1 < (kDagLevels + 3) / 4) qn = __ldg(prog + (lv + 1) / 4 + 1);
-      }
-      w = k == 0 ? q.x : (k == 1 ? q.y : (k == 2 ? q.z : q.w));
-      A = S[w & 255u]; B = S[(w >> 8) & 255u]; C = S[(w >> 16) & 255u];
-    }
-    last = r;
+    q = next;
   }
-  S[kDagLeaves + (kDagLevels - 1) * kDagLanes + gl] = last;
-  __syncwarp();
 }
 
 // One root of tet_ref from the prefix in S: second = false gives its "a"

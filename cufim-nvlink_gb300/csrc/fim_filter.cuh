@@ -263,7 +263,7 @@ __device__ __forceinline__ CandBound tet_screen_t(const float *gv, float p1f, fl
   float lb = INFINITY, ub = INFINITY;
   bool any = false, nan_lb = false;
   if constexpr (kBf) {
-#pragma unroll
+#pragma unroll 1  // (8 KB less code: together with the rolled listing of phase B 1M slab 10.65 -> 10.42 ms)
     for (int root = 0; root < 2; ++root) {
       const Re L2 = re_div_bf(root == 0 ? PA + SX : PA - SX, PB);
       const Re L1 = re_div_bf(-((F * L2 + E) * Q13 - (D * L2 + B) * Q23), X);

@@ -68,21 +68,17 @@ constexpr int kTetCap = kCornerCap; // tet screens per batch: never full
 constexpr int kQcap = 768;          // exact solves queued per kind and batch (more run on the spot)
 // Up to this many triangle solves of a batch run on two lanes each, one per
 // root: while they fill no more than four warps (one per sub-partition's
-// FP64 pipe) the shorter chain costs nothing (87k shell 2.26 ms with one lane
-// each, 2.19 with 64, 2.20 with 128; the other meshes within 1 %).
-#ifndef FIM_TRI_SPLIT
-#define FIM_TRI_SPLIT 64
-#endif
-constexpr int kTriSplit = FIM_TRI_SPLIT;
+// FP64 pipe) the shorter chain costs little (87k shell 1.92 ms with one lane
+// each, 1.90 with 64, 1.92 with 128; 9k cube 0.894, 0.900, 0.902; 17.7k slab
+// 1.268, 1.271, 1.333; 1M slab 10.36, 10.37, 10.48).
+constexpr int kTriSplit = 64;
 // Batches whose listed solves take at most this many FP64 warp instructions
 // (fp64_cost) skip the screens.  Solve times in ms (9k cube, 17.7k slab, 87k
-// shell, 58k windowed slab, 1M slab) without the direct path 1.30, 1.76, 2.40,
-// 5.74, 12.46; up to 200: 1.13, 1.70, 2.29, 5.16, 12.28; up to 480: 0.98,
-// 1.46, 2.19, 4.77, 12.10; up to 900: 0.97, 1.43, 2.21, 4.73, 12.13.
-#ifndef FIM_DIRECT_COST
-#define FIM_DIRECT_COST 600
-#endif
-constexpr int kDirectCost = FIM_DIRECT_COST;
+// shell, 58k windowed slab, 1M slab) without the direct path 1.07, 1.47, 2.00,
+// 4.94, 10.60; up to 200: 0.98, 1.46, 1.95, 4.60, 10.50; up to 400: 0.90,
+// 1.32, 1.90, 4.41, 10.41; up to 600: 0.90, 1.27, 1.90, 4.36, 10.37; up to
+// 900: 0.90, 1.28, 1.98, 4.41, 10.45.
+constexpr int kDirectCost = 600;
 // Corners of a batch whose vertex ids stay in shared memory (over the queues)
 // for phase D: one L2 round trip less in its chain.
 constexpr int kIdsCap = 2 * kQcap;
@@ -92,20 +88,25 @@ constexpr int kIdsCap = 2 * kQcap;
 constexpr int kDagWarps = kDagWarpsMax * 32 <= kThreads ? kDagWarpsMax : kThreads / 32;
 constexpr int kDagGroups = kDagWarps * 32 / kDagLanes;
 
-// Update phases.  With windows (finite dt) an iteration runs the reference's
-// four steps as four grid-synchronised phases: kNarrow4 (update the narrow
-// list), the apply + neighbour marking, kMarked4 (re-solve the marked
-// neighbours), the apply + next list.  With one endless window no vertex
-// can leave the narrow list for "next" inside the window, so an iteration
-// needs only two: kNarrow2 updates the narrow list and marks the downwind
-// neighbours of the vertices it freezes, kMarked2 re-solves them, applies
-// everything and builds the next list.
-// With windows the re-solve applies its own results too (kMarked3: the
-// times into both buffers, the decided state, the next list), so that
-// iteration needs three phases: a re-solved vertex is seen as "neig" by every
-// other re-solve of the phase, so nothing reads what it writes.
-enum : int { kNarrow4 = 0, kMarked4 = 1, kNarrow2 = 2, kMarked2 = 3, kMarked3 = 4 };
-__host__ __device__ constexpr bool is_marked_mode(int m) { return m == kMarked4 || m == kMarked2 || m == kMarked3; }
+// Paths of the solve kernel, one instantiation each: windows (finite dt) with
+// three grid-synchronised phases per iteration, one endless window with two,
+// submesh sweeps (blocks own whole submeshes within a window) with four phases
+// between block barriers.
+enum : int { kPathFour = 0, kPathTwo = 1, kPathLocal = 2 };
+
+// Update phases.  The reference's four steps are: update the narrow list,
+// apply it and mark neighbours, re-solve the marked neighbours, apply them and
+// build the next list.  Submesh sweeps run them as four phases.  With windows
+// the re-solve applies its own results (the times into both buffers, the
+// decided state, the next list): a re-solved vertex is seen as "neig" by every
+// other re-solve of the phase, so nothing reads what it writes.  With one
+// endless window no vertex can leave the narrow list for "next" inside the
+// window, so the update of the narrow list also marks the downwind neighbours
+// of the vertices it freezes, and the re-solve applies everything.
+//
+// Both update phases of a path are one piece of code, run with `marked` false
+// and true from one place: the kernel's code is larger than the instruction
+// caches, and this halves what a phase has to stream in.
 
 // Order-preserving map of floats to unsigned integers (for atomicMin).
 __device__ __forceinline__ unsigned int fkey(float x)
@@ -144,10 +145,10 @@ struct BatchSh {
   double old[kSlots];
   unsigned long long res[kSlots];   // dkey of the running minimum (exact values)
   unsigned int bhi[kSlots];         // fkey of a float upper bound of the new time
-  int64_t n0[kSlots];               // kNarrow2: neighbourhood range of each vertex (marking)
+  int64_t n0[kSlots];               // marking: neighbourhood range of each vertex
   int32_t ncnt[kSlots];
-  uint8_t tsv[kSlots];              // kMarked2, kMarked3: tmp_state of each vertex
-  int32_t fz[kSlots];               // kNarrow2: slots frozen in this batch
+  uint8_t tsv[kSlots];              // re-solves: tmp_state of each vertex
+  int32_t fz[kSlots];               // marking: slots frozen in this batch
   // per corner of the batch
   union {
     struct {
@@ -175,7 +176,7 @@ struct BatchSh {
   int next_item;                    // next unclaimed screen item (phase S)
   int wsum[kSlots / 32];            // corner counts of each warp's 32 slots (setup)
   int nfit;                         // slots whose corners end within kCornerCap (setup)
-  int nfz;                          // kNarrow2: frozen slots of the batch
+  int nfz;                          // marking: frozen slots of the batch
 };
 
 // (for small shapes the tet prefix scratch is the larger member of the union)
@@ -433,11 +434,7 @@ __device__ __forceinline__ void set_phi_both(const FimDev &d, int64_t v, double 
 
 // Work of another list that runs inside a phase: load() starts its loads
 // beside the first batch's, store() uses them once that batch is set up.
-struct NoSide {
-  __device__ __forceinline__ void load() {}
-  __device__ __forceinline__ void store() {}
-};
-// Phase Y's share of the narrow list: the new time of vertex lst[i] (one per
+// That is phase Y's share of the narrow list: the new time of vertex lst[i] (one per
 // thread; none for i < 0) into the times, its state, the next list.
 struct ApplySide {
   const FimDev &d;
@@ -485,11 +482,11 @@ struct ApplySide {
 // their frozen list's length in shared memory.
 struct ListOut {
   unsigned long long *word;  // the phase's word
-  int32_t *next;      // kMarked2, kMarked3: next iteration's narrow list
-  int32_t *frozen;    // kNarrow4: vertices frozen now
+  int32_t *next;      // marked: next iteration's narrow list
+  int32_t *frozen;    // narrow (windows, sweeps): vertices frozen now
   int32_t *n_frozen;  // (local)
-  int32_t *marked;    // kNarrow2: neighbours marked now
-  uint8_t *dec;       // kMarked4: decided state per position of the marked list
+  int32_t *marked;    // narrow (endless window): neighbours marked now
+  uint8_t *dec;       // marked (sweeps): decided state per position of the marked list
   bool local;         // the list is this block's own (submesh sweeps): no split over the grid
 };
 
@@ -516,27 +513,27 @@ struct ListOut {
 //  E -- the reference's per-vertex decision on the exact minimum
 //       (narrow vertices: window test (next), freeze test,
 //       cuda_fim.cu:2125-2163; re-solved neighbours: keep or restore the
-//       state, cuda_fim.cu:2255-2317), per MODE:
-//   kNarrow4 -- new time into phi2, next / frozen-now;
-//   kMarked4 -- new time into phi2, the decided state into dec;
-//   kNarrow2 -- new time into phi2; the vertices frozen now mark their
-//               downwind neighbours (cuda_fim.cu:2172-2205) at once: the
-//               mark is the iteration stamp in the state word, which the
-//               narrow updates running at the same time ignore;
-//   kMarked2 -- new time into both buffers, the state decided and the
-//               vertex appended to the next narrow list.
-// Times are read from phi (narrow modes) or phi2 (kMarked2: the narrow
+//       state, cuda_fim.cu:2255-2317), per path and phase:
+//   narrow, windows and sweeps -- new time into phi2, next / frozen-now;
+//   marked, sweeps -- new time into phi2, the decided state into dec;
+//   narrow, endless window -- new time into phi2; the vertices frozen now mark
+//       their downwind neighbours (cuda_fim.cu:2172-2205) at once: the mark
+//       is the iteration stamp in the state word, which the narrow updates
+//       running at the same time ignore;
+//   marked, windows and endless window -- new time into both buffers, the
+//       state decided and the vertex appended to the next narrow list.
+// Times are read from phi, or phi2 (marked, endless window: the narrow
 // list's new times live there until the phase applies them).  The minimum
 // over everything equals the reference's update_per_element minimum over
 // all corners (cuda_fim.h:1362-1411).
-template <int MODE, class Side = NoSide>
-__device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, int32_t n, double lower,
+template <int PATH>
+__device__ __forceinline__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, int32_t n, double lower,
                              float lower_lo, float lower_hi, double phi_start, double dt, bool exact_all, bool fp32,
                              uint32_t stamp, int dag_warps, const ListOut &lo_, int64_t &n_filtered,
-                             int64_t &n_exact, Side &side)
+                             int64_t &n_exact, bool marked, ApplySide &side)
 {
-  constexpr bool kMarkedMode = is_marked_mode(MODE);
-  const double *ph = MODE == kMarked2 ? d.phi2 : d.phi;      // times this phase reads
+  constexpr bool kTwo = PATH == kPathTwo;
+  const double *ph = kTwo && marked ? d.phi2 : d.phi;  // times this phase reads
   const int tid = threadIdx.x, lane = tid & 31;
   const int64_t per_block = lo_.local ? (int64_t)n : ((int64_t)n + gridDim.x - 1) / gridDim.x;
   const int64_t lbeg = lo_.local ? 0 : min((int64_t)n, (int64_t)blockIdx.x * per_block);
@@ -555,14 +552,14 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
       sh.cnt[tid] = (int32_t)(d.cptr[v + 1] - d.cptr[v]);
       sh.old[tid] = old;
       sh.res[tid] = dkey(old);
-      const float oh = re_hi(re_in(MODE == kMarked2 ? __ldcg(&d.vs[v].f2) : __ldcg(d.phi_f + v)));
+      const float oh = re_hi(re_in(__ldcg(kTwo && marked ? &d.vs[v].f2 : d.phi_f + v)));
       sh.bhi[tid] = fkey(exact_all || !(oh == oh) ? INFINITY : oh);
-      if (MODE == kNarrow2) {
+      if (kTwo && !marked) {
         const int64_t a = d.nptr[v];
         sh.n0[tid] = a;
         sh.ncnt[tid] = (int32_t)(d.nptr[v + 1] - a);
       }
-      if (MODE == kMarked2 || MODE == kMarked3) sh.tsv[tid] = __ldcg(d.tst + v);
+      if (PATH != kPathLocal && marked) sh.tsv[tid] = __ldcg(d.tst + v);
     }
     if (tid == 0) {
       sh.cp[0] = 0;
@@ -635,14 +632,13 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
           // vertices marked in this iteration.  Otherwise a neighbour counts
           // (state >= narrow) exactly when it has a time, since a far vertex
           // has none.
-          if (MODE == kMarked2) {
+          if (marked) {
             const VState q = ld_vs(d, nbs[i]);
-            pf[i] = q.f2;
+            pf[i] = kTwo ? q.f2 : __ldcg(d.phi_f + nbs[i]);
             stn[i] = (uint8_t)sw_seen(q.sw, true, stamp);
           } else {
             pf[i] = __ldcg(d.phi_f + nbs[i]);
-            stn[i] = kMarkedMode ? (uint8_t)sw_seen(__ldcg(&d.vs[nbs[i]].sw), true, stamp)
-                                 : (uint8_t)(pf[i] == INFINITY ? ST_FAR : ST_NARROW);
+            stn[i] = (uint8_t)(pf[i] == INFINITY ? ST_FAR : ST_NARROW);
           }
         }
         const float len[3] = {__uint_as_float(h1.x), __uint_as_float(h1.y), __uint_as_float(h1.z)};
@@ -688,7 +684,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     }
     // corners beyond kCornerCap (a single vertex with very many corners):
     // every solve of them goes to FP64
-    if (total > kept) n_filtered += excess_corners(d, ph, sh, kept, total, lower, kMarkedMode, stamp);
+    if (total > kept) n_filtered += excess_corners(d, ph, sh, kept, total, lower, marked, stamp);
     __syncthreads();
     PROBE(kPrA);
 
@@ -700,6 +696,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     {
       uint64_t bits = 0;
       uint32_t counts = 0;  // triangles, tets << 10, edges << 20
+#pragma unroll 1
       for (int j = tid, sft = 0; j < kept; j += kThreads, sft += 5) {
         const float bhi = funkey(sh.bhi[sh.cs[j]]);
         const uint32_t m = sh.vm[j];
@@ -1012,14 +1009,14 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
     PROBE(kPrD);
 
     // E: decisions
-    if (MODE == kNarrow4 || MODE == kMarked4) {
+    if (PATH == kPathLocal || (PATH == kPathFour && !marked)) {
       if (tid < nslot) {
         const int slot = tid;
         const int32_t v = sh.vtx[slot];
         const double old = sh.old[slot];
         const double nw = dunkey(sh.res[slot]);
         d.phi2[v] = nw;
-        if (MODE == kNarrow4) {
+        if (!marked) {
           d.tst[v] = ST_FAR;
           if (nw - phi_start > dt) {
             d.vs[v].sw = ST_NEXT;
@@ -1032,7 +1029,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
           lo_.dec[pos + slot] = (nw < old) ? (uint8_t)ST_NARROW : __ldcg(d.tst + v);
         }
       }
-    } else if (MODE == kNarrow2) {
+    } else if (kTwo && !marked) {
       // the window test never fires (endless window)
       if (tid < nslot) {
         const int slot = tid;
@@ -1082,7 +1079,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
           }
         }
       }
-    } else {  // kMarked2, kMarked3
+    } else {  // re-solves that apply their own results
       if (tid < kSlots) {  // whole warps: the next-list appends are warp-aggregated
         const int slot = tid;
         const bool in = slot < nslot;
@@ -1105,7 +1102,7 @@ __device__ void update_phase(const FimDev &d, BatchSh &sh, const int32_t *list, 
       }
     }
     __syncthreads();
-    PROBE(MODE == kNarrow2 ? kPrMark : kPrE);
+    PROBE(kTwo && !marked ? kPrMark : kPrE);
     pos += nslot;
   }
 }
@@ -1124,7 +1121,6 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
                              int64_t &my_evals, int64_t &my_exact, int64_t &my_updates, int where)
 {
   __shared__ int32_t b_narrow[3], b_frozen, b_marked;
-  NoSide none;
   const int tid = threadIdx.x;
   const int32_t c0 = d.blk_ptr[blockIdx.x], c1 = d.blk_ptr[blockIdx.x + 1];
   int s = (int)(it % 3);
@@ -1166,37 +1162,41 @@ __device__ bool local_window(const FimDev &d, BatchSh &sh, const FimParams &p, d
     lo.marked = d.lmarked + c0;
     lo.dec = d.dec + c0; lo.local = true;
 
-    // P1 -- update the narrow list
-    update_phase<kNarrow4>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0,
-                           p.fp32 != 0, stamp, dag, lo, my_evals, my_exact, none);
-    if (tid == 0) my_updates += nn;
-    // P2 -- apply; mark the downwind neighbours of the vertices frozen now
-    for (int32_t i = tid; i < nn; i += kThreads) {
-      const int32_t v = lst[i];
-      set_phi(d, v, __ldcg(d.phi2 + v));
-    }
-    const int32_t nf = b_frozen;
-    for (int32_t i = tid / kMarkLanes; i < nf; i += kThreads / kMarkLanes) {
-      const int32_t n = lo.frozen[i];
-      const double pn = __ldcg(d.phi2 + n);
-      for (int64_t k = d.nptr[n] + tid % kMarkLanes; k < d.nptr[n + 1]; k += kMarkLanes) {
-        const int32_t v = __ldg(d.nbr + k);
-        const uint32_t w = __ldcg(&d.vs[v].sw);
-        const double pv = __ldcg(d.phi2 + v);
-        if (sw_state(w) != ST_NARROW && sw_stamp(w) != stamp && pn < pv) {
-          if (atomicCAS(&d.vs[v].sw, w, sw_make(ST_NEIG, stamp)) == w) {
-            d.tst[v] = (uint8_t)sw_state(w);
-            lo.marked[atomicAdd(&b_marked, 1)] = v;
+    ApplySide none{d, nullptr, -1, stamp, nullptr, nullptr, false};
+    int32_t nm = 0;
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      const bool marked = half != 0;
+      // P1 -- update the narrow list; P3 -- re-solve the marked neighbours
+      const int32_t n = marked ? nm : nn;
+      update_phase<kPathLocal>(d, sh, marked ? lo.marked : lst, n, lower, lower_lo, lower_hi, phi_start, p.dt,
+                               p.exact_all != 0, p.fp32 != 0, stamp, dag, lo, my_evals, my_exact, marked, none);
+      if (tid == 0) my_updates += n;
+      if (marked) break;
+      // P2 -- apply; mark the downwind neighbours of the vertices frozen now
+      for (int32_t i = tid; i < nn; i += kThreads) {
+        const int32_t v = lst[i];
+        set_phi(d, v, __ldcg(d.phi2 + v));
+      }
+      const int32_t nf = b_frozen;
+      for (int32_t i = tid / kMarkLanes; i < nf; i += kThreads / kMarkLanes) {
+        const int32_t u = lo.frozen[i];
+        const double pn = __ldcg(d.phi2 + u);
+        for (int64_t k = d.nptr[u] + tid % kMarkLanes; k < d.nptr[u + 1]; k += kMarkLanes) {
+          const int32_t v = __ldg(d.nbr + k);
+          const uint32_t w = __ldcg(&d.vs[v].sw);
+          const double pv = __ldcg(d.phi2 + v);
+          if (sw_state(w) != ST_NARROW && sw_stamp(w) != stamp && pn < pv) {
+            if (atomicCAS(&d.vs[v].sw, w, sw_make(ST_NEIG, stamp)) == w) {
+              d.tst[v] = (uint8_t)sw_state(w);
+              lo.marked[atomicAdd(&b_marked, 1)] = v;
+            }
           }
         }
       }
+      __syncthreads();
+      nm = b_marked;
     }
-    __syncthreads();
-    // P3 -- re-solve the marked neighbours
-    const int32_t nm = b_marked;
-    update_phase<kMarked4>(d, sh, lo.marked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0,
-                           p.fp32 != 0, stamp, dag, lo, my_evals, my_exact, none);
-    if (tid == 0) my_updates += nm;
     // P4 -- apply, decided states, next narrow list
     for (int32_t i = tid; i < nm + nn; i += kThreads) {
       if (i < nm) {
@@ -1238,11 +1238,6 @@ __device__ __forceinline__ bool grid_sync_probed(const FimDev &d, uint32_t nbloc
   return ok;
 }
 
-// PATH: kPathFour -- four grid-synchronised phases per iteration (windows);
-// kPathTwo -- two (one endless window); kPathLocal -- submesh sweeps (blocks
-// own whole submeshes within a window).  One instantiation each, so that each
-// holds only the update phases it runs (no spills at 128 registers).
-enum : int { kPathFour = 0, kPathTwo = 1, kPathLocal = 2 };
 #pragma nv_diag_suppress 128  // the grid-wide window code is unreachable in the submesh-sweep instantiation
 template <int PATH>
 __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimParams p)
@@ -1254,10 +1249,9 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
   int64_t my_evals = 0, my_updates = 0, my_exact = 0;
   int where = 0;  // grid barriers passed: the phase running is where + 1
   const auto word = [&]() { return &ctl->phase[(where + 1) & 3].v; };
-  int32_t nn = 0, nm = 0, nf = 0, unused = 0;  // lengths of the narrow, marked and frozen lists
+  int32_t nn = 0, nm = 0, unused = 0;  // lengths of the narrow and the marked list
   extern __shared__ __align__(16) unsigned char fim_smem[];
   BatchSh &sh = *reinterpret_cast<BatchSh *>(fim_smem);
-  NoSide none;
   const int dag = min(max(p.dag_warps, 1), kDagWarps);
   PROBE(-1);
 
@@ -1348,69 +1342,87 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
       const int32_t *lst = d.list[s];
       int32_t *lnext = d.list[s1];
       ListOut lo;
-      lo.word = word();
       lo.next = lnext;
       lo.frozen = d.lfrozen; lo.n_frozen = nullptr;
       lo.marked = d.lmarked;
       lo.dec = d.dec; lo.local = false;
       PROBE_COUNT(kPrPhases);
 
-      if (PATH == kPathTwo) {
-        // X -- update the narrow list, mark the downwind neighbours of the
-        // vertices frozen now (cuda_fim.cu:2102-2205)
-        update_phase<kNarrow2>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
-                               lo, my_evals, my_exact, none);
-        my_updates += (gtid == 0) ? nn : 0;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nm)) return;
+      // Endless window:
+      //  X -- update the narrow list, mark the downwind neighbours of the
+      //       vertices frozen now (cuda_fim.cu:2102-2205);
+      //  Y -- apply the narrow list's times and states (the block's share of
+      //       the list, cuda_fim.cu:2291-2317) and re-solve the marked
+      //       neighbours (cuda_fim.cu:2215-2289), which read the new times
+      //       from phi2 and see every marked vertex as "neig".
+      // Windows:
+      //  P1 -- solve on elements + reduce per vertex (cuda_fim.cu:2102-2163);
+      //  P2 -- apply the narrow times, mark downwind neighbours of the
+      //       vertices frozen now (cuda_fim.cu:2172-2205);
+      //  P3 -- the narrow vertices that are not re-solved now go to the next
+      //       list (or freeze), then the marked neighbours are re-solved
+      //       (cuda_fim.cu:2215-2289), each applying its own result, decided
+      //       state and next-list entry (cuda_fim.cu:2291-2317): the two
+      //       touch disjoint vertices, and a narrow vertex's state change
+      //       leaves it a valid neighbour.
+      // One copy of update_phase serves both halves: two inlined copies are
+      // 349 KB of kernel, one is 236 KB, and the batches of a large mesh then
+      // find more of it in the instruction cache (1M slab 11.1 -> 10.4 ms,
+      // 87k shell 2.00 -> 1.90; 17.7k slab 1.265 -> 1.27, 9k cube 0.88 -> 0.90).
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        const bool marked = half != 0;
         lo.word = word();
-
-        // Y -- apply the narrow list's times and states (the block's share
-        // of the list, cuda_fim.cu:2291-2317), then re-solve the marked
-        // neighbours (cuda_fim.cu:2215-2289), which read the new times from
-        // phi2 and see every marked vertex as "neig"
-        const int64_t per_block = ((int64_t)nn + gridDim.x - 1) / gridDim.x;
-        const int64_t lbeg = min((int64_t)nn, (int64_t)blockIdx.x * per_block);
-        const int64_t lend = min((int64_t)nn, lbeg + per_block);
-        ApplySide side{d, lst, -1, stamp, lnext, lo.word, true};
-        int64_t i0 = lbeg;
-        for (; i0 + kThreads < lend; i0 += kThreads) {  // all but the last round
-          side.i = i0 + threadIdx.x;
-          side.pending = true;
-          side.load();
-          side.store();
+        ApplySide side{d, lst, -1, stamp, lnext, lo.word, false};
+        if (marked && PATH == kPathTwo) {
+          const int64_t per_block = ((int64_t)nn + gridDim.x - 1) / gridDim.x;
+          const int64_t lbeg = min((int64_t)nn, (int64_t)blockIdx.x * per_block);
+          const int64_t lend = min((int64_t)nn, lbeg + per_block);
+          int64_t i0 = lbeg;
+          for (; i0 + kThreads < lend; i0 += kThreads) {  // all but the last round
+            side.i = i0 + threadIdx.x;
+            side.pending = true;
+            side.load();
+            side.store();
+          }
+          side.i = i0 + threadIdx.x < lend ? i0 + threadIdx.x : -1;
+          side.pending = i0 < lend;
+        } else if (marked) {
+          for (int64_t i = gtid; i < nn; i += nthreads) {
+            const int32_t v = lst[i];
+            const uint32_t w = __ldcg(&d.vs[v].sw);
+            const uint8_t tv = __ldcg(d.tst + v);
+            if (sw_stamp(w) == stamp) continue;  // re-solved below
+            if (sw_state(w) == ST_NARROW) {
+              if (tv == ST_FROZEN) d.vs[v].sw = ST_FROZEN;
+              else append_active(lnext, lo.word, v);
+            }
+          }
         }
-        side.i = i0 + threadIdx.x < lend ? i0 + threadIdx.x : -1;
-        side.pending = i0 < lend;
         PROBE(kPrLight);
-        update_phase<kMarked2>(d, sh, d.lmarked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0,
-                               stamp, dag, lo, my_evals, my_exact, side);
-        side.load();  // (a block without marked vertices)
+        const int32_t n = marked ? nm : nn;
+        update_phase<PATH>(d, sh, marked ? d.lmarked : lst, n, lower, lower_lo, lower_hi, phi_start, p.dt,
+                           p.exact_all != 0, p.fp32 != 0, stamp, dag, lo, my_evals, my_exact, marked, side);
+        side.load();  // (a block without vertices)
         side.store();
-        my_updates += (gtid == 0) ? nm : 0;
-        ++it;
-        ++it_window;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nn)) return;
-      } else {
-        // P1 -- solve on elements + reduce per vertex (cuda_fim.cu:2102-2163)
-        update_phase<kNarrow4>(d, sh, lst, nn, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0, stamp, dag,
-                               lo, my_evals, my_exact, none);
-        my_updates += (gtid == 0) ? nn : 0;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nf)) return;
-        lo.word = word();
+        my_updates += (gtid == 0) ? n : 0;
+        int32_t len = 0;  // of the list that the phase appended to
+        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &len)) return;
+        if (marked) { nn = len; continue; }
+        if (PATH == kPathTwo) { nm = len; continue; }
 
-        // P2 -- apply the narrow times; mark downwind neighbours of the
-        // vertices frozen now (cuda_fim.cu:2172-2205).  The two are
-        // independent: the marking runs on groups of kMarkLanes threads from
-        // the bottom of the grid, the apply on threads from the top, so that
-        // their dependent load chains overlap.
+        // P2: the apply and the marking are independent; the marking runs on
+        // groups of kMarkLanes threads from the bottom of the grid, the apply
+        // on threads from the top, so that their dependent load chains overlap
+        lo.word = word();
         for (int64_t i = nthreads - 1 - gtid; i < nn; i += nthreads) {
           const int32_t v = lst[i];
           set_phi(d, v, __ldcg(d.phi2 + v));
         }
-        for (int64_t i = gtid / kMarkLanes; i < nf; i += nthreads / kMarkLanes) {
-          const int32_t n = d.lfrozen[i];
-          const double pn = __ldcg(d.phi2 + n);
-          for (int64_t k = d.nptr[n] + gtid % kMarkLanes; k < d.nptr[n + 1]; k += kMarkLanes) {
+        for (int64_t i = gtid / kMarkLanes; i < len; i += nthreads / kMarkLanes) {
+          const int32_t u = d.lfrozen[i];
+          const double pn = __ldcg(d.phi2 + u);
+          for (int64_t k = d.nptr[u] + gtid % kMarkLanes; k < d.nptr[u + 1]; k += kMarkLanes) {
             // both loads at once; the word changes only by the exchange below,
             // so w is still v's word there unless another frozen vertex won
             const int32_t v = __ldg(d.nbr + k);
@@ -1425,31 +1437,9 @@ __global__ void __launch_bounds__(kThreads, 1) fim_solve_kernel(FimDev d, FimPar
           }
         }
         if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nm)) return;
-        lo.word = word();
-
-        // P3 -- the narrow vertices that are not re-solved now go to the next
-        // list (or freeze), then the marked neighbours are re-solved
-        // (cuda_fim.cu:2215-2289), each applying its own result, decided
-        // state and next-list entry (cuda_fim.cu:2291-2317): the two touch
-        // disjoint vertices, and a narrow vertex's state change leaves it a
-        // valid neighbour
-        for (int64_t i = gtid; i < nn; i += nthreads) {
-          const int32_t v = lst[i];
-          const uint32_t w = __ldcg(&d.vs[v].sw);
-          const uint8_t tv = __ldcg(d.tst + v);
-          if (sw_stamp(w) == stamp) continue;  // re-solved below
-          if (sw_state(w) == ST_NARROW) {
-            if (tv == ST_FROZEN) d.vs[v].sw = ST_FROZEN;
-            else append_active(lnext, lo.word, v);
-          }
-        }
-        update_phase<kMarked3>(d, sh, d.lmarked, nm, lower, lower_lo, lower_hi, phi_start, p.dt, p.exact_all != 0, p.fp32 != 0,
-                               stamp, dag, lo, my_evals, my_exact, none);
-        my_updates += (gtid == 0) ? nm : 0;
-        ++it;
-        ++it_window;
-        if (!grid_sync_probed(d, nblocks, p.timeout_ns, ++where, &nn)) return;
       }
+      ++it;
+      ++it_window;
     }
   }
 

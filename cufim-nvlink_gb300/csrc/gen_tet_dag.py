@@ -32,6 +32,7 @@ import os
 import re
 
 LANES = 8
+STEP = 3
 # leaf slots (inputs and constants)
 LEAVES = ["e13", "e23", "e34", "e12", "e14", "e24", "p1", "p2", "p3", "c0.5", "c2.0", "c1.0", "c-0.0"]
 NLEAF = 16
@@ -264,11 +265,13 @@ def main():
         "constexpr int kDagLeafE13 = 0, kDagLeafP1 = 6, kDagLeafConst = 9;",
     ]
     lines.append("constexpr int " + ", ".join("kDagOut_%s = %d" % (n, out[n]) for n in OUTPUTS) + ";")
-    prog += [[0] * LANES for _ in range(-levels % 4)]  # a lane's words are loaded four at a time
-    lines.append("__device__ const uint4 kTetDagProg[kDagLanes][(kDagLevels + 3) / 4] = {")
+    if levels % STEP:
+        raise ValueError("the prefix runs %d levels per round" % STEP)
+    lines.append("constexpr int kDagStep = %d;  // levels per round: one uint4 of a lane's words (the last unused)" % STEP)
+    lines.append("__device__ const uint4 kTetDagProg[kDagLanes][kDagLevels / kDagStep] = {")
     for ln in range(LANES):
-        lines.append("  {" + ",\n   ".join("{" + ", ".join("0x%08xu" % prog[lv + k][ln] for k in range(4)) + "}"
-                                           for lv in range(0, len(prog), 4)) + "},")
+        lines.append("  {" + ",\n   ".join("{" + ", ".join("0x%08xu" % prog[lv + k][ln] for k in range(STEP)) + ", 0u}"
+                                           for lv in range(0, levels, STEP)) + "},")
     lines.append("};")
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tet_dag.inc")
     with open(path, "w") as fh:

@@ -91,46 +91,6 @@ struct CandBound {
   float ub;   // it certainly returns a value <= ub (+inf when not certain)
 };
 
-// solve_tri_cu(e12, e13, e23, p1, p2) in true units (the reference's float
-// intermediates make float range part of its semantics, so no rescaling: a
-// bound that leaves the float range becomes an undecided case).
-__device__ __forceinline__ CandBound tri_screen(Re e12, Re e13, Re e23, Re p1, Re p2)
-{
-  CandBound r;
-  r.some = CAND_SOME;
-  r.lb = INFINITY;
-  r.ub = INFINITY;
-  const Re P12 = p2 - p1;
-  const Re A = e23, C = e12;
-  const Re B = re_scale((e12 + e23) - e13, -0.5f);
-  const Re DV = P12 * P12 - C;                    // float divident
-  const Re SV = DV * (B * B - A * C);              // float sqrt_val
-  if (re_hi(SV) < 0.f) { r.some = CAND_NONE; return r; }
-  const bool cond_certain = (re_lo(DV) > 0.f || re_hi(DV) < 0.f) && re_lo(SV) >= 0.f;
-  const Re DV2 = C * DV;
-  const Re ST = re_sqrt(SV);                       // float sqrtTmp
-  const Re BPC = (B * P12) * P12 - B * C;
-  const Re SP = ST * P12;
-  const Re L[2] = {re_div(-(BPC - SP), DV2), re_div(-(BPC + SP), DV2)};
-  bool any = false, nan_lb = false;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const Re l = L[k];
-    if (re_hi(l) < 0.f || re_lo(l) > 1.f) continue;      // rejected root
-    const bool acc = re_lo(l) >= 0.f && re_hi(l) <= 1.f;
-    const Re Q = (A + re_scale(l, 2.f) * B) + (l * l) * C;
-    if (re_hi(Q) < 0.f) continue;                         // NaN value: dropped by fminf
-    const Re V = (p2 - l * P12) + re_sqrt(Q);
-    any = true;
-    r.lb = fminf(r.lb, re_lo(V));
-    if (cond_certain && acc && re_lo(Q) >= 0.f) r.ub = fminf(r.ub, re_hi(V));
-    if (isnan(re_lo(V))) nan_lb = true;  // an overflowed bound of either root: no bound at all
-  }
-  if (nan_lb) r.lb = NAN;
-  if (!any) r.some = CAND_NONE;
-  return r;
-}
-
 // Branch-free division and square root (hardware approximations, no
 // operand-range branches): __fdividef is within 2 ulp for divisors of
 // magnitude in [2^-126, 2^126] (elsewhere the result gets no bound: e = inf);
@@ -165,8 +125,11 @@ __device__ __forceinline__ Re re_sqrt_bf(Re a)
   return re_make(v, fmaf(v, FIM_RE_U + FIM_RE_APPROX, e + FIM_RE_TINY));
 }
 
-// tri_screen without branches (the same decisions, the two roots as
-// independent chains), for lanes that screen two pairs at once.
+// solve_tri_cu(e12, e13, e23, p1, p2) in true units (the reference's float
+// intermediates make float range part of its semantics, so no rescaling: a
+// bound that leaves the float range becomes an undecided case).  Without
+// branches, the two roots as independent chains: with branches the screens
+// took longer (1M slab 10.87 ms against 10.38, 87k shell 1.92 against 1.87).
 __device__ __forceinline__ CandBound tri_screen_bf(Re e12, Re e13, Re e23, Re p1, Re p2)
 {
   CandBound r;
@@ -263,7 +226,7 @@ __device__ __forceinline__ CandBound tet_screen_t(const float *gv, float p1f, fl
   float lb = INFINITY, ub = INFINITY;
   bool any = false, nan_lb = false;
   if constexpr (kBf) {
-#pragma unroll 1  // (8 KB less code: together with the rolled listing of phase B 1M slab 10.65 -> 10.42 ms)
+#pragma unroll 1  // (8 KB less code beats the overlap of the roots: 17.7k slab 1.280 -> 1.271 ms, 9k cube 0.904 -> 0.899)
     for (int root = 0; root < 2; ++root) {
       const Re L2 = re_div_bf(root == 0 ? PA + SX : PA - SX, PB);
       const Re L1 = re_div_bf(-((F * L2 + E) * Q13 - (D * L2 + B) * Q23), X);

@@ -360,8 +360,8 @@ __device__ __forceinline__ CandBound tri_screen_sm(const FimDev &d, const BatchS
   const float g23 = k == 0 ? g[5] : g[2];
   const float pa = k == 1 ? sh.pf[j][1] : sh.pf[j][0];
   const float pb = k == 0 ? sh.pf[j][1] : sh.pf[j][2];
-  return tri_screen(re_scale(re_in(g12), tk), re_scale(re_in(g13), tk), re_scale(re_in(g23), tk), re_in(pa),
-                    re_in(pb));
+  return tri_screen_bf(re_scale(re_in(g12), tk), re_scale(re_in(g13), tk), re_scale(re_in(g23), tk), re_in(pa),
+                       re_in(pb));
 }
 
 __device__ __forceinline__ CandBound tet_screen_sm(const FimDev &d, const BatchSh &sh, int j, int *why = nullptr)
@@ -750,21 +750,21 @@ __device__ __forceinline__ void update_phase(const FimDev &d, BatchSh &sh, const
 
     // S: screens over the compacted lists, handed out in chunks to whichever
     // warp is free -- tets first (32 per chunk, one per lane), then triangles
-    // from the next chunk boundary (64 per chunk: each lane screens two with
-    // the branch-free tri_screen_bf, so that the two chains interleave), so
-    // that every chunk holds one kind, and last the edges of 32 corners per
-    // chunk; a solve whose lower bound does not exceed the current bhi is
-    // queued at once (bhi only decreases: phase D rechecks against the final
-    // bound)
+    // from the next chunk boundary, so that every chunk holds one kind, and
+    // last the edges of 32 corners per chunk; a solve whose lower bound does
+    // not exceed the current bhi is queued at once (bhi only decreases: phase
+    // D rechecks against the final bound).  A block's chunks are few (24 for
+    // its 16 warps in a 1M slab), so their size shows at the phase's end: two
+    // triangles per lane, their chains interleaved, measured 87k shell 1.90
+    // ms, 17.7k slab 1.273, 1M slab 10.38; one 1.87, 1.266, 10.38.
     if (!direct) {
       const int ntet = min(sh.nlist[1], kTetCap), ntri = min(sh.nlist[0], kTriCap);
       const int tri0 = (ntet + 31) & ~31;
-      const int edge_c0 = tri0 + ((ntri + 63) / 64) * 32;  // claim index of the first edge chunk
+      const int edge_c0 = tri0 + ((ntri + 31) & ~31);
       const int nedge = sh.nlist[2];
       const int nclaim = edge_c0 + ((nedge + 31) & ~31);
       for (;;) {
-        // claims of 32: tet chunks, then triangle chunks of 64 (two per
-        // lane), then edge chunks of 32 corners
+        // claims of 32: tet chunks, triangle chunks, edge chunks of 32 corners
         int cl = 0;
         if (lane == 0) cl = atomicAdd(&sh.next_item, 32);
         cl = __shfl_sync(FULL_MASK, cl, 0);
@@ -803,87 +803,45 @@ __device__ __forceinline__ void update_phase(const FimDev &d, BatchSh &sh, const
           PROBE_CHUNK(13);
           continue;
         }
-        const int ib = cl < tri0 ? cl : tri0 + 2 * (cl - tri0);  // 32 claimed in the triangle range stand for 64
-        if (ib < tri0) {
-          const int i = ib + lane;
-          bool need = false;
-          int slot = 0, j = 0;
-          float lb = 0.f;
-          if (i < ntet) {
+        const bool tri = cl >= tri0;
+        const int i = cl - (tri ? tri0 : 0) + lane;
+        bool need = false;
+        int slot = 0, j = 0, k = 3;
+        float lb = 0.f;
+        if (i < (tri ? ntri : ntet)) {
+          CandBound cb;
+          if (tri) {
+            j = (int)(sh.tri[i] & 0x3fffu);
+            k = (int)(sh.tri[i] >> 14);
+            cb = tri_screen_sm(d, sh, j, k);
+          } else {
             j = (int)sh.tet[i];
-            slot = sh.cs[j];
-            CandBound cb;
-            if (exact_all) { cb.some = CAND_SOME; cb.lb = NAN; cb.ub = INFINITY; }
 #ifdef FIM_PROBE
-            else {
-              int why = 3;
-              cb = tet_screen_sm(d, sh, j, &why);
-              // outcomes: sqt < 0, sqt undecided, no accepted root, a value (pruned / queued below)
-              atomicAdd(&d.probe[blockIdx.x * kProbeSlots + 16 + (why < 3 ? why : 3)], 1ull);
-              if (why == 3 && cb.lb > funkey(sh.bhi[slot])) atomicAdd(&d.probe[blockIdx.x * kProbeSlots + 20], 1ull);
-            }
+            int why = 3;
+            cb = tet_screen_sm(d, sh, j, &why);
+            // outcomes: sqt < 0, sqt undecided, no accepted root, a value (pruned / queued below)
+            atomicAdd(&d.probe[blockIdx.x * kProbeSlots + 16 + (why < 3 ? why : 3)], 1ull);
+            if (why == 3 && cb.lb > funkey(sh.bhi[sh.cs[j]])) atomicAdd(&d.probe[blockIdx.x * kProbeSlots + 20], 1ull);
 #else
-            else cb = tet_screen_sm(d, sh, j);
+            cb = tet_screen_sm(d, sh, j);
 #endif
-            if (!exact_all && cb.some && cb.ub < INFINITY) atomicMin(&sh.bhi[slot], fkey(cb.ub));
-            lb = isnan(cb.lb) ? -INFINITY : cb.lb;
-            need = cb.some && !(lb > funkey(sh.bhi[slot]));
-            if (fp32 && need && cb.ub < INFINITY && !isnan(cb.lb)) {  // FP32 mode: conclusive screen
-              atomicMin(&sh.res[slot], dkey((double)(0.5f * (cb.lb + cb.ub))));
-              need = false;
-            }
           }
-          queue_exact(d, ph, sh, need, 0, 3, slot, j, lb, lane);
-          PROBE_CHUNK(11);
-        } else {
-          int jj[2], kk[2], sl[2];
-          bool in[2];
-          CandBound cb[2];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int i = ib + 32 * h + lane;
-            in[h] = i < tri0 + ntri;
-            const uint32_t it = in[h] ? (uint32_t)sh.tri[i - tri0] : 0u;
-            jj[h] = (int)(it & 0x3fffu);
-            kk[h] = (int)(it >> 14);
-            sl[h] = sh.cs[jj[h]];
-          }
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            float g[7];
-            screen_record(d, sh, jj[h], g);
-            const float tk = re_pow2f((int)g[6]);
-            const int k = kk[h], j = jj[h];
-            const float g12 = k == 0 ? g[3] : (k == 1 ? g[1] : g[0]);
-            const float g13 = k == 1 ? g[5] : g[4];
-            const float g23 = k == 0 ? g[5] : g[2];
-            const float pa = k == 1 ? sh.pf[j][1] : sh.pf[j][0];
-            const float pb = k == 0 ? sh.pf[j][1] : sh.pf[j][2];
-            cb[h] = tri_screen_bf(re_scale(re_in(g12), tk), re_scale(re_in(g13), tk), re_scale(re_in(g23), tk),
-                                  re_in(pa), re_in(pb));
-            if (exact_all) { cb[h].some = CAND_SOME; cb[h].lb = NAN; cb[h].ub = INFINITY; }
-          }
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            bool need = false;
-            float lb = 0.f;
-            if (in[h]) {
-              if (!exact_all && cb[h].some && cb[h].ub < INFINITY) atomicMin(&sh.bhi[sl[h]], fkey(cb[h].ub));
-              lb = isnan(cb[h].lb) ? -INFINITY : cb[h].lb;
-              need = cb[h].some && !(lb > funkey(sh.bhi[sl[h]]));
+          if (exact_all) { cb.some = CAND_SOME; cb.lb = NAN; cb.ub = INFINITY; }
+          slot = sh.cs[j];
+          if (!exact_all && cb.some && cb.ub < INFINITY) atomicMin(&sh.bhi[slot], fkey(cb.ub));
+          lb = isnan(cb.lb) ? -INFINITY : cb.lb;
+          need = cb.some && !(lb > funkey(sh.bhi[slot]));
 #ifdef FIM_PROBE
-              // triangle outcomes: no value, a value above bhi, a value below
-              atomicAdd(&d.probe[blockIdx.x * kProbeSlots + (!cb[h].some ? 21 : (need ? 23 : 22))], 1ull);
+          // triangle outcomes: no value, a value above bhi, a value below
+          if (tri) atomicAdd(&d.probe[blockIdx.x * kProbeSlots + (!cb.some ? 21 : (need ? 23 : 22))], 1ull);
 #endif
-              if (fp32 && need && cb[h].ub < INFINITY && !isnan(cb[h].lb)) {  // FP32 mode: conclusive screen
-                atomicMin(&sh.res[sl[h]], dkey((double)(0.5f * (cb[h].lb + cb[h].ub))));
-                need = false;
-              }
-            }
-            queue_exact(d, ph, sh, need, 1, kk[h], sl[h], jj[h], lb, lane);
+          if (fp32 && need && cb.ub < INFINITY && !isnan(cb.lb)) {  // FP32 mode: conclusive screen
+            atomicMin(&sh.res[slot], dkey((double)(0.5f * (cb.lb + cb.ub))));
+            need = false;
           }
-          PROBE_CHUNK(12);
         }
+        queue_exact(d, ph, sh, need, tri ? 1 : 0, k, slot, j, lb, lane);
+        PROBE_CHUNK(tri ? 12 : 11);
 #undef PROBE_CHUNK
       }
       __syncthreads();

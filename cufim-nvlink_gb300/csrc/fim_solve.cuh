@@ -535,17 +535,22 @@ __device__ __forceinline__ void update_phase(const FimDev &d, BatchSh &sh, const
   constexpr bool kTwo = PATH == kPathTwo;
   const double *ph = kTwo && marked ? d.phi2 : d.phi;  // times this phase reads
   const int tid = threadIdx.x, lane = tid & 31;
-  const int64_t per_block = lo_.local ? (int64_t)n : ((int64_t)n + gridDim.x - 1) / gridDim.x;
-  const int64_t lbeg = lo_.local ? 0 : min((int64_t)n, (int64_t)blockIdx.x * per_block);
-  const int64_t lend = min((int64_t)n, lbeg + per_block);
-  int64_t pos = lbeg;
+  // The block's share of the list: every gridDim.x-th vertex.  Neighbours in
+  // the list lie side by side in the mesh and cost alike, so contiguous shares
+  // leave some blocks with the dear ones (58k windowed slab 4.30 ms against
+  // 4.20, 17.7k slab 1.265 / 1.239, 87k shell 1.869 / 1.860, 1M slab 10.37 /
+  // 10.33; runs of 4 vertices 4.39, 1.306, 1.908, 10.40).  A submesh's list is
+  // its block's own.
+  const int64_t step = lo_.local ? 1 : (int64_t)gridDim.x, first = lo_.local ? 0 : (int64_t)blockIdx.x;
+  const int64_t lend = n > first ? (n - 1 - first) / step + 1 : 0;
+  int64_t pos = 0;
   while (pos < lend) {
     PROBE_COUNT(kPrBatches);
     // batch: the longest run of vertices with <= kCornerCap corners (>= 1 vertex)
     const int cand = (int)min((int64_t)kSlots, lend - pos);
     side.load();
     if (tid < cand) {
-      const int32_t v = __ldcg(list + pos + tid);
+      const int32_t v = __ldcg(list + first + (pos + tid) * step);
       const double old = __ldcg(ph + v);
       sh.vtx[tid] = v;
       sh.c0[tid] = d.cptr[v];

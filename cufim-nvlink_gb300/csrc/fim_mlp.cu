@@ -1,16 +1,17 @@
 // fim_mlp.cu -- the learned warm start: per-vertex features and a small
 // MLP (7 -> 128 -> 128 -> 128 -> 1, ReLU) trained and evaluated on the GPU.
 //
-// One persistent kernel, mlp_kernel, runs the whole network over 128-row
-// tiles: the three hidden layers forward and, when training, back again,
-// every product a tcgen05 MMA with BF16 operands in shared memory and an
+// One persistent kernel runs the whole network over 128-row tiles,
+// mlp_forward_kernel the three hidden layers and the output, mlp_train_kernel
+// also the way back: every product a tcgen05 MMA with BF16 operands and an
 // FP32 accumulator in tensor memory.  A tile's activations never leave the
-// SM: each layer's epilogue (bias + ReLU, or the ReLU mask) writes BF16 rows
-// back to shared memory in the layout the next MMA reads.  The weight
-// gradients accumulate in tensor memory over all tiles of a CTA, and
-// mlp_reduce_kernel adds the CTAs' sums in a fixed order and, in a training
-// step, applies Adam.  Master weights, biases, output layer, loss and bias
-// gradients are FP32; the MMAs read a BF16 copy of the weights refreshed
+// SM: each layer's epilogue (bias + ReLU, or the ReLU mask) writes them as
+// BF16 where the next MMA reads them, in tensor memory forward and in shared
+// memory in training.  The weight gradients accumulate in tensor memory over
+// all tiles of a CTA, and mlp_reduce_kernel adds the CTAs' sums in a fixed
+// order and, in a training step, applies Adam.  Master weights, biases,
+// output layer, loss and bias gradients are FP32; the MMAs read a BF16 copy
+// of the weights refreshed
 // after every update.  The input width is padded from 7 features to
 // kMlpIn = 64 columns (zeros), one 128-byte K slice.
 //
@@ -40,9 +41,9 @@ namespace {
 // weights), and an MN-major one when its rows are (weight gradients:
 // contraction over the tile's rows; data gradients: over the weights' output
 // rows), so no operand is ever transposed in memory.  Every mbarrier wait is
-// bounded (%globaltimer): a wait that runs out sets the error word, the
-// group leaves at its next barrier, and the CTA waits (bounded) for the
-// copies and MMAs it issued and frees its tensor memory.
+// bounded (%globaltimer): a wait that runs out ends the loops of the CTA's
+// warps and sets the error word, and the CTA waits (bounded) for the copies
+// and MMAs it issued and frees its tensor memory.
 constexpr int kTileM = 128, kBlkCols = 64;
 constexpr uint32_t kBlkBytes = kTileM * kBlkCols * 2;  // 16 KB
 constexpr uint64_t kMlpWaitNs = 2000000000ull;         // bound of every mbarrier wait
@@ -122,6 +123,38 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem, uint64_t a, uint64_t b,
       ::"r"(tmem), "l"(a), "l"(b), "r"(id), "r"(accumulate)
       : "memory");
 }
+// For a warp that runs in step with one lane issuing (lead): operands stay in
+// uniform registers, and a step is the MMA and an add.  Descriptors by their
+// low words (kDescHi is the other); acc += where `more`, else acc =.
+constexpr uint32_t kDescHi = (uint32_t)(kDescBase >> 32);
+template <bool kMore>
+__device__ __forceinline__ void umma_ss(bool lead, uint32_t acc, uint32_t a, uint32_t b, uint32_t id)
+{
+  asm volatile(
+      "{\n .reg .pred p, q;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %6, 0;\n"
+      " mov.b64 x, {%1, %3};\n mov.b64 y, {%2, %3};\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %4, p;\n}"
+      ::"r"(acc), "r"(a), "r"(b), "r"(kDescHi), "r"(id), "n"(kMore ? 1 : 0), "r"((uint32_t)lead)
+      : "memory");
+}
+// the same with A in tensor memory
+template <bool kMore>
+__device__ __forceinline__ void umma_ts(bool lead, uint32_t acc, uint32_t a, uint32_t b, uint32_t id)
+{
+  asm volatile(
+      "{\n .reg .pred p, q;\n .reg .b64 y;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %6, 0;\n"
+      " mov.b64 y, {%2, %3};\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %4, p;\n}"
+      ::"r"(acc), "r"(a), "r"(b), "r"(kDescHi), "r"(id), "n"(kMore ? 1 : 0), "r"((uint32_t)lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_lead(bool lead, uint32_t bar)
+{
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar), "r"((uint32_t)lead)
+      : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -163,6 +196,52 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t *v)
         "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
       : "r"(taddr), "r"(taddr + 32u)
       : "memory");
+}
+// Accumulator fragments: columns 0..63 of the warp's 32 lanes, thread T with
+// columns 8 j + 2 (T % 4) + {0, 1} of lanes T / 4 + 8 k in v[32 (k / 2) + 4 j +
+// 2 (k % 2) + {0, 1}], so that a thread needs a quarter of the biases it would
+// need with a whole row; the loads and their wait are one statement, so that
+// no use of v can move between them
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t *v)
+{
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+      "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64];\n"
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, "
+      "%44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, "
+      "[%65];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]),
+        "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]),
+        "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]),
+        "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]),
+        "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
+      : "r"(taddr), "r"(taddr + (16u << 16))
+      : "memory");
+}
+// the packed pairs of such a fragment, v[16 (k / 2) + 2 j + k % 2], as columns
+// 0..31
+__device__ __forceinline__ void tmem_st_frag(uint32_t taddr, const uint32_t *v)
+{
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%32], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+      "%13, %14, %15};\n"
+      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%33], {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, "
+      "%27, %28, %29, %30, %31};\n"
+      ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]),
+        "r"(taddr), "r"(taddr + (16u << 16))
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Index of weight i (W1 [kMlpIn x kMlpH], W2, W3 [kMlpH x kMlpH], each
 // [in x out] row-major) in the transposed copies [out x in] that the MMAs
@@ -236,39 +315,18 @@ __device__ __forceinline__ uint32_t bf2_relu(uint32_t x)
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 // ---------------------------------------------------------------------------
-// The network over 128-row tiles.  A group of warps owns a tile: warp w reads
-// tensor-memory lanes 32 (w % 4) .. + 31 (the tile's rows); the group's
-// thread 0 issues the TMA loads and the MMAs.
-//
-// Forward: four groups of four warps per CTA on tiles of their own, so that
-// one tile's MMAs (20 steps) and waits run beside the epilogues of the
-// others.  A group needs 32 KB: its activations, overwritten layer by layer;
-// the next tile's features are loaded into them while the last layer's
-// epilogue runs, which no longer touches them.
-// Training: one group of eight warps (two column halves), since a tile's
-// features and three activations (112 KB) leave no room for a second tile
-// beside the 80 KB of weights; the next tile's features are loaded a tile
-// ahead.
-//
-// Measured over 1.03M rows (features 132 MB), predict call: three GEMM
-// kernels with H1 and H2 in memory 252 us, this kernel 106 us (98 us on the
-// device: tensor pipe 39 % busy; with both operands in shared memory a
-// 128 x 128 x 16 step reads 8 KB in the 64 cycles it takes, so the MMAs alone
-// use the shared-memory bandwidth that the epilogues need too).  Two groups
-// of eight warps 125 us, four of eight 115 us.  Training step of 4,096 rows
-// (22 launches before, 2 now) 191 -> 46 us; gradients of 131,136 rows, whose
-// activations and their transposes went through memory, 500 -> 97 us.
+// Training over 128-row tiles: eight warps, warp w with tensor-memory lanes
+// 32 (w % 4) .. + 31 (the tile's rows) of a column half; thread 0 issues the
+// TMA loads and the MMAs.  One tile at a time, since a tile's features and
+// three activations (112 KB) leave no room for a second one beside the 80 KB
+// of weights; the next tile's features are loaded a tile ahead.  Step of
+// 4,096 rows (22 launches before, 2 now) 191 -> 46 us; gradients of 131,136
+// rows, whose activations and their transposes went through memory, 500 -> 97.
 constexpr uint32_t kW1Bytes = kBlkBytes, kW2Bytes = 2 * kBlkBytes;
 constexpr uint32_t kWBytes = kW1Bytes + 2 * kW2Bytes;  // the weights, [out][in]
 constexpr uint32_t kActBytes = 2 * kBlkBytes;          // 128 x 128 activations
-template <bool kTrain>
-struct MlpShape {
-  static constexpr int kGroups = kTrain ? 1 : 4;
-  static constexpr int kGroupThreads = kTrain ? 256 : 128;
-  static constexpr int kThreads = kGroups * kGroupThreads;
-  static constexpr uint32_t kGroupBytes = kTrain ? 2 * kBlkBytes + 3 * kActBytes : kActBytes;
-  static constexpr int kSmem = (int)(kWBytes + kGroups * kGroupBytes) + 1024;  // + slack to align to 1024 B
-};
+constexpr int kTrainThreads = 256;
+constexpr int kTrainSmem = (int)(kWBytes + 2 * kBlkBytes + 3 * kActBytes) + 1024;  // + slack to align to 1024 B
 constexpr int kTmemCols = 512;
 // tensor-memory columns in training: the layer's accumulator, then the
 // transposed weight gradients [out][in] of layers 3, 2, 1
@@ -277,44 +335,30 @@ constexpr uint32_t kTmW3 = 128, kTmW2 = 256, kTmW1 = 384;
 // summed squared error
 constexpr int kPartStride = (kMlpParams + 1 + 63) & ~63;
 
-template <int kThreads>
-__device__ __forceinline__ void group_sync(int g)
-{
-  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kThreads) : "memory");
-}
-
-template <bool kTrain>
-__global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
+__global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw1,
     const __grid_constant__ CUtensorMap tw2, const __grid_constant__ CUtensorMap tw3, int M,
-    const float *__restrict__ P, float *y, const float *__restrict__ tgt, float *part, volatile unsigned int *err)
+    const float *__restrict__ P, const float *__restrict__ tgt, float *part, volatile unsigned int *err)
 {
-  using S = MlpShape<kTrain>;
   extern __shared__ unsigned char mlp_smem[];
-  __shared__ __align__(8) uint64_t wfull, xfull[S::kGroups][2], mdone[S::kGroups];
+  __shared__ __align__(8) uint64_t wfull, xfull[2], mdone;
   __shared__ uint32_t tmem_base;
   __shared__ __align__(16) float s_bias[3][kMlpH], s_w4[kMlpH];
-  __shared__ float s_part[kTileM], s_dy[kTileM];  // training
-  __shared__ volatile int s_fail[S::kGroups][2];
-  const int g = threadIdx.x / S::kGroupThreads, t = threadIdx.x % S::kGroupThreads;
-  const int lane = t & 31, q = (t >> 5) & 3, h = t >> 7;  // h: column half (training; 0 forward, both halves in turn)
+  __shared__ float s_part[kTileM], s_dy[kTileM];
+  __shared__ volatile int s_fail[2];
+  const int t = threadIdx.x, lane = t & 31, q = (t >> 5) & 3, h = t >> 7;  // h: column half
   const uint32_t w1 = (smem_u32(mlp_smem) + 1023u) & ~1023u, w2 = w1 + kW1Bytes, w3 = w2 + kW2Bytes;
   unsigned char *const sm = mlp_smem + (w1 - smem_u32(mlp_smem));  // generic address of w1
-  const uint32_t xs = w1 + kWBytes + (uint32_t)g * S::kGroupBytes;
-  const uint32_t h1 = kTrain ? xs + 2 * kBlkBytes : xs;  // forward: one buffer for features and activations
-  const uint32_t h2 = kTrain ? h1 + kActBytes : h1, h3 = kTrain ? h2 + kActBytes : h1;
+  const uint32_t xs = w1 + kWBytes, h1 = xs + 2 * kBlkBytes, h2 = h1 + kActBytes, h3 = h2 + kActBytes;
   const int ntiles = (M + kTileM - 1) / kTileM;
-  const int tstep = gridDim.x * S::kGroups;
-  const int tile0 = g * gridDim.x + blockIdx.x;  // few tiles: one per CTA
+  const int tstep = gridDim.x, tile0 = blockIdx.x;
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&wfull), 1);
-    for (int i = 0; i < S::kGroups; ++i) {
-      mbar_init(smem_u32(&xfull[i][0]), 1);
-      mbar_init(smem_u32(&xfull[i][1]), 1);
-      mbar_init(smem_u32(&mdone[i]), 1);
-      s_fail[i][0] = s_fail[i][1] = 0;
-    }
+    mbar_init(smem_u32(&xfull[0]), 1);
+    mbar_init(smem_u32(&xfull[1]), 1);
+    mbar_init(smem_u32(&mdone), 1);
+    s_fail[0] = s_fail[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < 32) {
@@ -326,14 +370,13 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base + (kTrain ? 0u : (uint32_t)(g * 128));
-  const uint32_t bar_m = smem_u32(&mdone[g]);
-  const uint32_t bar_x0 = smem_u32(&xfull[g][0]), bar_x1 = smem_u32(&xfull[g][1]);
-  int issued = 0, consumed = 0;  // thread 0 of the group: feature tiles
-  // feature tile i of the group: its buffer, barrier and parity
-  const auto x_buf = [&](int i) { return xs + (kTrain ? (uint32_t)(i & 1) * kBlkBytes : 0u); };
-  const auto x_bar = [&](int i) { return kTrain && (i & 1) ? bar_x1 : bar_x0; };
-  const auto x_par = [&](int i) { return (uint32_t)(kTrain ? i >> 1 : i) & 1u; };
+  const uint32_t tmem = tmem_base;
+  const uint32_t bar_m = smem_u32(&mdone);
+  int issued = 0, consumed = 0;  // thread 0: feature tiles
+  // feature tile i of the CTA: its buffer, barrier and parity
+  const auto x_buf = [&](int i) { return xs + (uint32_t)(i & 1) * kBlkBytes; };
+  const auto x_bar = [&](int i) { return smem_u32(&xfull[i & 1]); };
+  const auto x_par = [&](int i) { return (uint32_t)(i >> 1) & 1u; };
   const auto load_x = [&](int tile) {
     mbar_expect_tx(x_bar(issued), kBlkBytes);
     tma_load_2d(x_buf(issued), &tx, 0, tile * kTileM, x_bar(issued));
@@ -348,26 +391,26 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
       tma_load_2d(w3 + s * kBlkBytes, &tw3, s * kBlkCols, 0, smem_u32(&wfull));
     }
   }
-  for (int i = threadIdx.x; i < 4 * kMlpH; i += S::kThreads) {
+  for (int i = threadIdx.x; i < 4 * kMlpH; i += kTrainThreads) {
     if (i < 3 * kMlpH) s_bias[i / kMlpH][i % kMlpH] = P[kMlpOB1 + i];
     else s_w4[i - 3 * kMlpH] = P[kMlpOW4 + i - 3 * kMlpH];
   }
   const float b4 = P[kMlpOB4];
   __syncthreads();
   bool wok = true;
-  if (t == 0) wok = mbar_wait(smem_u32(&wfull), 0);  // each group's issuer sees the weights
+  if (t == 0) wok = mbar_wait(smem_u32(&wfull), 0);
 
-  // A phase ends with the group's barrier; a wait that ran out in phase p
-  // is flagged in s_fail[g][p & 1] before that barrier and read after it, so
-  // the whole group leaves together (a later phase writes the other word).
+  // A phase ends with a barrier; a wait that ran out in phase p
+  // is flagged in s_fail[p & 1] before that barrier and read after it, so
+  // the whole CTA leaves together (a later phase writes the other word).
   int phase = 0;
   uint32_t mpar = 0;       // parity of the next MMA completion
   int commits = 0;         // thread 0: completions requested
   int waited = 0;
-  const auto fail = [&]() { s_fail[g][phase & 1] = 1; };
+  const auto fail = [&]() { s_fail[phase & 1] = 1; };
   const auto end_phase = [&]() {
-    group_sync<S::kGroupThreads>(g);
-    const bool bad = s_fail[g][phase & 1] != 0;
+    __syncthreads();
+    const bool bad = s_fail[phase & 1] != 0;
     ++phase;
     return !bad;
   };
@@ -387,14 +430,11 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
   const uint32_t tv = tmem + ((uint32_t)(q * 32) << 16);
   const int r = q * 32 + lane;  // this thread's row of the tile
   // 64 columns of the row: from the accumulator, and where they lie in an activation block
-  const auto load_acc = [&](int half, uint32_t *v) {
-    tmem_ld64(tv + 64 * half, v);
-  };
-  const auto chunk_ptr = [&](uint32_t base, int half, int c) {  // 16-byte chunk c, at chunk c ^ (row % 8)
-    return reinterpret_cast<uint4 *>(sm + (base - w1) + (uint32_t)half * kBlkBytes + (uint32_t)r * 128u +
+  const auto load_acc = [&](uint32_t *v) { tmem_ld64(tv + 64 * h, v); };
+  const auto chunk_ptr = [&](uint32_t base, int c) {  // 16-byte chunk c, at chunk c ^ (row % 8)
+    return reinterpret_cast<uint4 *>(sm + (base - w1) + (uint32_t)h * kBlkBytes + (uint32_t)r * 128u +
                                      ((uint32_t)(c ^ (r & 7)) << 4));
   };
-  const int half0 = h, half1 = kTrain ? h + 1 : 2;  // the column halves of this thread
 
   // training: sums over this thread's rows (columns 2 cp, 2 cp + 1, rows
   // 32 rg .. + 31 of every tile) of the bias gradients and of gw4; over this
@@ -422,7 +462,7 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
     const bool in = tile * kTileM + r < M;
     // layer 1
     if (t == 0) {
-      if (kTrain && tile + tstep < ntiles) load_x(tile + tstep);  // its stage was read by MMAs that have completed
+      if (tile + tstep < ntiles) load_x(tile + tstep);  // its stage was read by MMAs that have completed
       if (!wok || !mbar_wait(x_bar(j), x_par(j))) fail();
       else {
         ++consumed;
@@ -436,12 +476,11 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
 #pragma unroll 1
     for (int layer = 0; layer < 2; ++layer) {
       wait_mma();
-#pragma unroll 1
-      for (int half = half0; half < half1; ++half) {
+      {
         uint32_t v[64];
-        load_acc(half, v);
+        load_acc(v);
         const uint32_t dst = layer == 0 ? h1 : h2;
-        const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[layer][64 * half]);
+        const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[layer][64 * h]);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint32_t w[4];
@@ -452,9 +491,9 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
             const uint64_t x1 = f2_add(f2_pack(__uint_as_float(v[8 * c + 4 * k + 2]), __uint_as_float(v[8 * c + 4 * k + 3])), bb.y);
             w[2 * k] = bf2_relu(bf2(f2_lo(x0), f2_hi(x0)));
             w[2 * k + 1] = bf2_relu(bf2(f2_lo(x1), f2_hi(x1)));
-            if (kTrain && !in) w[2 * k] = w[2 * k + 1] = 0u;  // rows past the matrix take no part in the gradients
+            if (!in) w[2 * k] = w[2 * k + 1] = 0u;  // rows past the matrix take no part in the gradients
           }
-          *chunk_ptr(dst, half, c) = make_uint4(w[0], w[1], w[2], w[3]);
+          *chunk_ptr(dst, c) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
       if (!publish()) { ok = false; break; }
@@ -471,14 +510,12 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
     // layer 3 and the output layer: y = relu(.) . w4 + b4 on the BF16
     // activations, the two column halves added in a fixed order
     wait_mma();
-    if (!kTrain && t == 0 && tile + tstep < ntiles) load_x(tile + tstep);
     float ysum = 0.f;
-#pragma unroll 1
-    for (int half = half0; half < half1; ++half) {
+    {
       uint32_t v[64];
-      load_acc(half, v);
-      const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[2][64 * half]);
-      const ulonglong2 *wv = reinterpret_cast<const ulonglong2 *>(&s_w4[64 * half]);
+      load_acc(v);
+      const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[2][64 * h]);
+      const ulonglong2 *wv = reinterpret_cast<const ulonglong2 *>(&s_w4[64 * h]);
       uint64_t sum0 = 0ull, sum1 = 0ull;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -490,21 +527,17 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
           const uint64_t x1 = f2_add(f2_pack(__uint_as_float(v[8 * c + 4 * k + 2]), __uint_as_float(v[8 * c + 4 * k + 3])), bb.y);
           w[2 * k] = bf2_relu(bf2(f2_lo(x0), f2_hi(x0)));
           w[2 * k + 1] = bf2_relu(bf2(f2_lo(x1), f2_hi(x1)));
-          if (kTrain && !in) w[2 * k] = w[2 * k + 1] = 0u;
+          if (!in) w[2 * k] = w[2 * k + 1] = 0u;
           sum0 = f2_fma(f2_pack(bf_lo(w[2 * k]), bf_hi(w[2 * k])), ww.x, sum0);
           sum1 = f2_fma(f2_pack(bf_lo(w[2 * k + 1]), bf_hi(w[2 * k + 1])), ww.y, sum1);
         }
-        if (kTrain) *chunk_ptr(h3, half, c) = make_uint4(w[0], w[1], w[2], w[3]);
+        *chunk_ptr(h3, c) = make_uint4(w[0], w[1], w[2], w[3]);
       }
-      ysum += (f2_lo(sum0) + f2_hi(sum0)) + (f2_lo(sum1) + f2_hi(sum1));
+      ysum = (f2_lo(sum0) + f2_hi(sum0)) + (f2_lo(sum1) + f2_hi(sum1));
     }
     if (h == 1) s_part[r] = ysum;
-    tc_fence_before();  // (the accumulator is read: the next tile's first MMA may write it)
+    tc_fence_before();  // (the accumulator is read: the next MMA may write it)
     if (!end_phase()) { ok = false; break; }
-    if (!kTrain) {
-      if (in) y[tile * (int64_t)kTileM + r] = ysum + b4;
-      continue;
-    }
     if (h == 0) {
       float dy = 0.f;
       if (in) {
@@ -555,10 +588,10 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
       wait_mma();
       {
         uint32_t v[64];
-        load_acc(h, v);
+        load_acc(v);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          uint4 *a = chunk_ptr(hp, h, c);
+          uint4 *a = chunk_ptr(hp, c);
           const uint4 mm = *a;
           const uint32_t m[4] = {mm.x, mm.y, mm.z, mm.w};
           uint32_t w[4];
@@ -585,7 +618,7 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
     if (!end_phase()) { ok = false; break; }
   }
 
-  if (kTrain && ok && tile0 < ntiles) {
+  if (ok && tile0 < ntiles) {
     // this CTA's sums, in parameter order ([in][out]): lane = output column
     float *o = part + (size_t)blockIdx.x * kPartStride;
 #pragma unroll 1
@@ -616,8 +649,8 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
       sse += __shfl_xor_sync(0xffffffffu, sse, k);
     }
     if (lane == 0) { red[2 * (t >> 5)] = gb4; red[2 * (t >> 5) + 1] = sse; }
-    group_sync<S::kGroupThreads>(g);
-    for (int i = t; i < 4 * kMlpH; i += S::kGroupThreads)
+    __syncthreads();
+    for (int i = t; i < 4 * kMlpH; i += kTrainThreads)
       o[kMlpOB1 + i] = ((sum[i] + sum[4 * kMlpH + i]) + sum[8 * kMlpH + i]) + sum[12 * kMlpH + i];
     if (t < 2) o[kMlpOB4 + t] = ((red[t] + red[2 + t]) + red[4 + t]) + red[6 + t];
   }
@@ -628,6 +661,230 @@ __global__ void __launch_bounds__(MlpShape<kTrain>::kThreads, 1) mlp_kernel(
     for (int i = consumed; i < issued; ++i) (void)mbar_wait(x_bar(i), x_par(i));
     for (int i = waited; i < commits; ++i) (void)mbar_wait(bar_m, (uint32_t)i & 1u);
   }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Forward only: two groups of eight warps, each on a tile of its own (a warp
+// holds 32 rows of one column half), and one warp that issues every copy and
+// MMA.  A group has 128 columns of tensor memory for the accumulator and 64
+// for the BF16 activations, which the epilogue writes there as the A operand
+// of the next layer: they never pass through shared memory, where a 128 x 128
+// x 16 step then reads 4 KB in its 64 cycles instead of 8.
+//
+// Predictions of 1.03M rows (features 132 MB): three GEMM kernels with the
+// activations in memory 252 us; one kernel, four groups of four warps that
+// each issued their own MMAs on operands in shared memory, 106; this one 91
+// (the MMAs 38 us at 68 cycles a step, the features 19 us of memory time; the
+// rest is the wait from a group's epilogue to its next MMA, which one other
+// group covers only in part).  Three groups of four warps sharing the four
+// quarters of tensor memory, one MMA in flight at a time: 121.  Accumulator
+// halves of 64 columns: a step takes as long as one of 128.
+constexpr int kFwdGroups = 2, kFwdGroupThreads = 256, kFwdThreads = kFwdGroups * kFwdGroupThreads + 32;
+constexpr int kFwdSmem = (int)(kWBytes + kFwdGroups * 2 * kBlkBytes) + 1024;  // + slack to align to 1024 B
+constexpr uint32_t kTmAct = 128, kTmGroup = 256;  // the activations' columns; from group to group
+
+__global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(
+    const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw1,
+    const __grid_constant__ CUtensorMap tw2, const __grid_constant__ CUtensorMap tw3, int M,
+    const float *__restrict__ P, float *y, volatile unsigned int *err)
+{
+  extern __shared__ unsigned char mlp_smem[];
+  // xfull: a group's two feature stages; mdone: its MMA has completed; ready:
+  // its epilogue is through (the next MMA may read the activations, or after
+  // layer 3 write over them)
+  // half: the second column half's part of a result is in s_part
+  __shared__ __align__(8) uint64_t wfull, xfull[kFwdGroups][2], mdone[kFwdGroups], ready[kFwdGroups], half[kFwdGroups];
+  __shared__ float s_part[kFwdGroups][kTileM];
+  __shared__ int xloads[kFwdGroups];  // feature tiles asked for
+  __shared__ uint32_t tmem_base;
+  __shared__ __align__(16) float s_bias[3][kMlpH], s_w4[kMlpH];
+  const int g = threadIdx.x / kFwdGroupThreads, t = threadIdx.x % kFwdGroupThreads, lane = t & 31;
+  const uint32_t w1 = (smem_u32(mlp_smem) + 1023u) & ~1023u, w2 = w1 + kW1Bytes, w3 = w2 + kW2Bytes;
+  const int ntiles = (M + kTileM - 1) / kTileM, tstep = gridDim.x * kFwdGroups;
+
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&wfull), 1);
+    for (int i = 0; i < kFwdGroups; ++i) {
+      mbar_init(smem_u32(&xfull[i][0]), 1);
+      mbar_init(smem_u32(&xfull[i][1]), 1);
+      mbar_init(smem_u32(&mdone[i]), 1);
+      mbar_init(smem_u32(&ready[i]), kFwdGroupThreads);
+      mbar_init(smem_u32(&half[i]), kTileM);
+      xloads[i] = 0;
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  for (int i = threadIdx.x; i < 4 * kMlpH; i += kFwdThreads) {
+    if (i < 3 * kMlpH) s_bias[i / kMlpH][i % kMlpH] = P[kMlpOB1 + i];
+    else s_w4[i - 3 * kMlpH] = P[kMlpOW4 + i - 3 * kMlpH];
+  }
+  const float b4 = P[kMlpOB4];
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base;
+
+  bool ok = true;
+  if (g == kFwdGroups) {  // the issuing warp: in step, lane 0 issues
+    {
+      const bool lead = lane == 0;
+      const uint32_t id = idesc(128, false, false);
+      const auto desc_lo = [](uint32_t addr) { return (addr >> 4) | (1u << 16); };
+      const auto x_buf = [&](int gg, int i) { return w1 + kWBytes + (uint32_t)(2 * gg + (i & 1)) * kBlkBytes; };
+      const auto load_x = [&](int gg, int i) {  // tile i of group gg, if there is one
+        const int tile = gg * gridDim.x + blockIdx.x + i * tstep;
+        if (tile >= ntiles) return;
+        if (!lead) return;
+        ++xloads[gg];
+        mbar_expect_tx(smem_u32(&xfull[gg][i & 1]), kBlkBytes);
+        tma_load_2d(x_buf(gg, i), &tx, 0, tile * kTileM, smem_u32(&xfull[gg][i & 1]));
+      };
+      for (int gg = 0; gg < kFwdGroups; ++gg) load_x(gg, 0);
+      if (lead) {
+        mbar_expect_tx(smem_u32(&wfull), kWBytes);
+        tma_load_2d(w1, &tw1, 0, 0, smem_u32(&wfull));
+        for (int s = 0; s < 2; ++s) {
+          tma_load_2d(w2 + s * kBlkBytes, &tw2, s * kBlkCols, 0, smem_u32(&wfull));
+          tma_load_2d(w3 + s * kBlkBytes, &tw3, s * kBlkCols, 0, smem_u32(&wfull));
+        }
+      }
+      for (int gg = 0; gg < kFwdGroups; ++gg) load_x(gg, 1);
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&wfull), 0));
+      int issued[kFwdGroups] = {};
+      for (int i = 0; ok && (int)blockIdx.x + i * tstep < ntiles; ++i) {
+#pragma unroll
+        for (int layer = 0; layer < 3; ++layer) {
+#pragma unroll
+          for (int gg = 0; gg < kFwdGroups; ++gg) {
+            const int n = 3 * i + layer;
+            if (!ok || (int)(gg * gridDim.x + blockIdx.x) + i * tstep >= ntiles) continue;
+            // the group is through with its last epilogue
+            ok = __all_sync(0xffffffffu,
+                            (n == 0 || mbar_wait(smem_u32(&ready[gg]), (uint32_t)(n - 1) & 1u)) &&
+                                (layer != 0 || mbar_wait(smem_u32(&xfull[gg][i & 1]), (uint32_t)(i >> 1) & 1u)));
+            if (!ok) continue;
+            tc_fence_after();
+            const uint32_t acc = tmem + gg * kTmGroup;
+            if (layer == 0) {
+              const uint32_t a = desc_lo(x_buf(gg, i)), b = desc_lo(w1);
+              umma_ss<false>(lead, acc, a, b, id);
+#pragma unroll
+              for (int c = 1; c < kBlkCols / 16; ++c) umma_ss<true>(lead, acc, a + 2 * c, b + 2 * c, id);
+            } else {
+              const uint32_t a = acc + kTmAct, b = desc_lo(layer == 1 ? w2 : w3);
+              umma_ts<false>(lead, acc, a, b, id);
+#pragma unroll
+              for (int c = 1; c < kMlpH / 16; ++c)
+                umma_ts<true>(lead, acc, a + 8 * c, b + (c / 4) * (kBlkBytes >> 4) + 2 * (c % 4), id);
+            }
+            umma_commit_lead(lead, smem_u32(&mdone[gg]));
+            issued[gg] = n + 1;
+            if (layer == 1) load_x(gg, i + 2);  // layer 1 has read the stage
+            __syncwarp();
+          }
+        }
+      }
+      if (!ok && lead) {  // what is still in flight lands before the CTA leaves (bounded)
+        (void)mbar_wait(smem_u32(&wfull), 0);
+        for (int gg = 0; gg < kFwdGroups; ++gg) {
+          if (issued[gg]) (void)mbar_wait(smem_u32(&mdone[gg]), (uint32_t)(issued[gg] - 1) & 1u);
+          for (int j = max(0, xloads[gg] - 2); j < xloads[gg]; ++j)
+            (void)mbar_wait(smem_u32(&xfull[gg][j & 1]), (uint32_t)(j >> 1) & 1u);
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    const int row = (t & 96) + (lane >> 2) + 8 * (lane & 3);  // the row whose result this thread sums
+    const int h = t >> 7;                                     // column half
+    const uint32_t acc = tmem + g * kTmGroup + ((uint32_t)(t & 96) << 16) + 64 * h;
+    const uint32_t act = tmem + g * kTmGroup + ((uint32_t)(t & 96) << 16) + kTmAct + 32 * h;
+    const uint32_t bar_m = smem_u32(&mdone[g]), bar_r = smem_u32(&ready[g]), bar_h = smem_u32(&half[g]);
+    // bias and ReLU of a pair of columns
+    const auto relu = [&](uint32_t lo, uint32_t hi, uint64_t bias) {
+      const uint64_t x = f2_add(f2_pack(__uint_as_float(lo), __uint_as_float(hi)), bias);
+      return bf2_relu(bf2(f2_lo(x), f2_hi(x)));
+    };
+    const auto pair = [&](const float *p, int j) {  // columns 8 j + 2 (lane % 4) + {0, 1} of the half
+      return *reinterpret_cast<const uint64_t *>(p + 64 * h + 8 * j + 2 * (lane & 3));
+    };
+    int n = 0;  // the group's MMAs
+    for (int tile = g * gridDim.x + blockIdx.x, i = 0; ok && tile < ntiles; tile += tstep, ++i) {
+#pragma unroll 1
+      for (int layer = 0; layer < 2; ++layer, ++n) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_m, (uint32_t)n & 1u));
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t v[64], w[32];
+        tmem_ld_frag(acc, v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint64_t bb = pair(s_bias[layer], j);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int e = 32 * (k >> 1) + 4 * j + 2 * (k & 1);
+            w[16 * (k >> 1) + 2 * j + (k & 1)] = relu(v[e], v[e + 1], bb);
+          }
+        }
+        tmem_st_frag(act, w);
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(bar_r);
+      }
+      if (!ok) break;
+      // layer 3 and the output layer: y = relu(.) . w4 + b4 on the BF16
+      // activations: a thread's 16 columns of four rows, the sums of the four
+      // threads that share the rows, then the two column halves
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_m, (uint32_t)n & 1u));
+      if (!ok) break;
+      ++n;
+      tc_fence_after();
+      uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};
+      {
+        uint32_t v[64];
+        tmem_ld_frag(acc, v);
+        tc_fence_before();
+        mbar_arrive(bar_r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint64_t bb = pair(s_bias[2], j), ww = pair(s_w4, j);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int e = 32 * (k >> 1) + 4 * j + 2 * (k & 1);
+            const uint32_t a = relu(v[e], v[e + 1], bb);
+            sum[k] = f2_fma(f2_pack(bf_lo(a), bf_hi(a)), ww, sum[k]);
+          }
+        }
+      }
+      float ys = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float x = f2_lo(sum[k]) + f2_hi(sum[k]);
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        x += __shfl_xor_sync(0xffffffffu, x, 2);
+        if ((lane & 3) == k) ys = x;
+      }
+      // (the next tile's part is written after both halves have been ready for its layers)
+      if (h == 1) {
+        s_part[g][row] = ys;
+        mbar_arrive(bar_h);
+      } else {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_h, (uint32_t)i & 1u));
+        if (ok && tile * kTileM + row < M) y[tile * (int64_t)kTileM + row] = (ys + s_part[g][row]) + b4;
+      }
+    }
+  }
+  if (!ok && lane == 0) *err = 1u;
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x < 32)
@@ -889,17 +1146,18 @@ int mlp_check_n(int64_t n, const char *who)
 
 // Launches the network over n rows of X: predictions into y, or with targets
 // the partial gradients of *ctas CTAs into m->part.
-template <bool kTrain>
 cudaError_t mlp_launch(fim_mlp *m, int n, const void *X, float *y, const float *tgt, int *ctas)
 {
-  using S = MlpShape<kTrain>;
   CUtensorMap tx;
   if (!make_map(&tx, X, kMlpIn, (uint64_t)n)) return cudaErrorInvalidValue;
   const int ntiles = (n + kTileM - 1) / kTileM;
   const int grid = std::min(ntiles, m->sms);
   if (ctas) *ctas = grid;
-  mlp_kernel<kTrain><<<grid, S::kThreads, S::kSmem, m->st>>>(tx, m->tw1, m->tw2, m->tw3, n, m->P, y, tgt, m->part,
-                                                             &m->d_res->err);
+  if (tgt)
+    mlp_train_kernel<<<grid, kTrainThreads, kTrainSmem, m->st>>>(tx, m->tw1, m->tw2, m->tw3, n, m->P, tgt, m->part,
+                                                                 &m->d_res->err);
+  else
+    mlp_forward_kernel<<<grid, kFwdThreads, kFwdSmem, m->st>>>(tx, m->tw1, m->tw2, m->tw3, n, m->P, y, &m->d_res->err);
   return cudaGetLastError();
 }
 
@@ -915,7 +1173,7 @@ int mlp_gradients(fim_mlp *m, int64_t n, const void *X, const float *tgt, float 
     c2 = 1.f - std::pow(b2, (float)m->steps);
   }
   int ctas = 0;
-  MLP_TRY(who, mlp_launch<true>(m, (int)n, X, nullptr, tgt, &ctas));
+  MLP_TRY(who, mlp_launch(m, (int)n, X, nullptr, tgt, &ctas));
   mlp_reduce_kernel<<<kPartStride / kRedParams, 4 * kRedParams, 0, m->st>>>(
       ctas, m->part, (int)n, m->G, &m->d_res->loss, m->P, m->M, m->V, lr, b1, b2, 1e-8f, c1, c2, m->W16T);
   MLP_TRY(who, cudaGetLastError());
@@ -960,10 +1218,10 @@ extern "C" int fim_mlp_create(int device, uint64_t seed, fim_mlp **out)
   m->h_res->err = 0;
   void *d = nullptr;
   if ((e = cudaHostGetDevicePointer(&d, h, 0)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(mlp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                MlpShape<false>::kSmem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(mlp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                MlpShape<true>::kSmem)) != cudaSuccess)
+      (e = cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem)) !=
+          cudaSuccess ||
+      (e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem)) !=
+          cudaSuccess)
     return fail(mlp_fail("fim_mlp_create", e));
   m->d_res = static_cast<fim_mlp::Result *>(d);
   if (!make_map(&m->tw1, m->W16T + kMlpOW1, kMlpIn, kMlpH) || !make_map(&m->tw2, m->W16T + kMlpOW2, kMlpH, kMlpH) ||
@@ -1064,7 +1322,7 @@ extern "C" int fim_mlp_predict(fim_mlp *m, int64_t n, const void *d_features, fl
     MLP_TRY("fim_mlp: activations", cudaMalloc(&m->y, sizeof(float) * n));
     m->y_cap = n;
   }
-  MLP_TRY("fim_mlp_predict: forward", mlp_launch<false>(m, (int)n, d_features, direct ? d_out : m->y, nullptr, nullptr));
+  MLP_TRY("fim_mlp_predict: forward", mlp_launch(m, (int)n, d_features, direct ? d_out : m->y, nullptr, nullptr));
   if (!direct)
     MLP_TRY("fim_mlp_predict", cudaMemcpyAsync(d_out, m->y, sizeof(float) * n, cudaMemcpyDeviceToDevice, m->st));
   MLP_TRY("fim_mlp_predict", cudaStreamSynchronize(m->st));

@@ -186,3 +186,24 @@ def test_prediction_into_its_own_features_or_an_odd_address(F, torch_cuda):
         mlp.predict(n, dX.data_ptr(), dX.data_ptr())
         over = dX.cpu().numpy().reshape(-1)[:2 * n].copy().view(np.float32)
         assert np.array_equal(over, y.cpu().numpy())
+
+
+@pytest.mark.parametrize("tiles", [153, 304, 305, 456, 457, 761, 3 * 456 + 300])
+def test_prediction_rounds_with_few_tiles(F, torch_cuda, tiles):
+    """Last rounds in which only some CTAs or only one or two of a CTA's three
+    groups have a tile (152 CTAs), the last tile half full: against the
+    restatement, the bounds of the other predictions."""
+    from oracle import mlp_oracle as M
+    torch = torch_cuda
+    n = 128 * tiles - 64
+    p, X, _ = _random_problem(M, n, 7)
+    with F.Mlp(seed=3) as mlp:
+        mlp.set_params(p)
+        dX = _to_device_bf16(torch, X)
+        y = torch.full((n + 1,), 7.0, dtype=torch.float32, device="cuda")
+        mlp.predict(n, dX.data_ptr(), y.data_ptr())
+    _, _, _, y_o = M.forward(p, X)
+    yg = y.cpu().numpy()
+    assert yg[n] == 7.0
+    assert (~np.isclose(yg[:n], y_o, rtol=1e-3, atol=1e-3)).mean() < 0.01
+    assert np.abs(yg[:n] - y_o).max() < 0.05 * np.abs(y_o).max()

@@ -176,27 +176,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *v)
       : "r"(taddr)
       : "memory");
 }
-// 64 consecutive FP32 columns of this thread's tensor-memory lane; the load
-// and its wait are one statement, so that no use of v can move between them
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t *v)
-{
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64];\n"
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
-      "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%65];\n"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]),
-        "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]),
-        "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]),
-        "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]),
-        "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
-      : "r"(taddr), "r"(taddr + 32u)
-      : "memory");
-}
 // Accumulator fragments: columns 0..63 of the warp's 32 lanes, thread T with
 // columns 8 j + 2 (T % 4) + {0, 1} of lanes T / 4 + 8 k in v[32 (k / 2) + 4 j +
 // 2 (k % 2) + {0, 1}], so that a thread needs a quarter of the biases it would
@@ -315,17 +294,18 @@ __device__ __forceinline__ uint32_t bf2_relu(uint32_t x)
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 // ---------------------------------------------------------------------------
-// Training over 128-row tiles: eight warps, warp w with tensor-memory lanes
-// 32 (w % 4) .. + 31 (the tile's rows) of a column half; thread 0 issues the
-// TMA loads and the MMAs.  One tile at a time, since a tile's features and
+// Training over 128-row tiles: sixteen warps, warp w with tensor-memory lanes
+// 32 (w % 4) .. + 31 (the tile's rows) of a quarter of the columns; thread 0
+// issues the TMA loads and the MMAs.  One tile at a time, since a tile's features and
 // three activations (112 KB) leave no room for a second one beside the 80 KB
 // of weights; the next tile's features are loaded a tile ahead.  Step of
-// 4,096 rows (22 launches before, 2 now) 191 -> 46 us; gradients of 131,136
-// rows, whose activations and their transposes went through memory, 500 -> 97.
+// 4,096 rows (22 launches before, 2 now) 191 -> 44 us; gradients of 131,136
+// rows, whose activations and their transposes went through memory, 500 -> 91
+// (eight warps with half of the columns each: 45.5 and 96 us).
 constexpr uint32_t kW1Bytes = kBlkBytes, kW2Bytes = 2 * kBlkBytes;
 constexpr uint32_t kWBytes = kW1Bytes + 2 * kW2Bytes;  // the weights, [out][in]
 constexpr uint32_t kActBytes = 2 * kBlkBytes;          // 128 x 128 activations
-constexpr int kTrainThreads = 256;
+constexpr int kTrainThreads = 512, kColParts = kTrainThreads / kTileM, kCols = kMlpH / kColParts;
 constexpr int kTrainSmem = (int)(kWBytes + 2 * kBlkBytes + 3 * kActBytes) + 1024;  // + slack to align to 1024 B
 constexpr int kTmemCols = 512;
 // tensor-memory columns in training: the layer's accumulator, then the
@@ -344,9 +324,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   __shared__ __align__(8) uint64_t wfull, xfull[2], mdone;
   __shared__ uint32_t tmem_base;
   __shared__ __align__(16) float s_bias[3][kMlpH], s_w4[kMlpH];
-  __shared__ float s_part[kTileM], s_dy[kTileM];
+  __shared__ float s_part[kColParts - 1][kTileM], s_dy[kTileM];
   __shared__ volatile int s_fail[2];
-  const int t = threadIdx.x, lane = t & 31, q = (t >> 5) & 3, h = t >> 7;  // h: column half
+  const int t = threadIdx.x, lane = t & 31, q = (t >> 5) & 3, h = t >> 7;  // h: column part
   const uint32_t w1 = (smem_u32(mlp_smem) + 1023u) & ~1023u, w2 = w1 + kW1Bytes, w3 = w2 + kW2Bytes;
   unsigned char *const sm = mlp_smem + (w1 - smem_u32(mlp_smem));  // generic address of w1
   const uint32_t xs = w1 + kWBytes, h1 = xs + 2 * kBlkBytes, h2 = h1 + kActBytes, h3 = h2 + kActBytes;
@@ -430,15 +410,16 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   const uint32_t tv = tmem + ((uint32_t)(q * 32) << 16);
   const int r = q * 32 + lane;  // this thread's row of the tile
   // 64 columns of the row: from the accumulator, and where they lie in an activation block
-  const auto load_acc = [&](uint32_t *v) { tmem_ld64(tv + 64 * h, v); };
+  const auto load_acc = [&](uint32_t *v) { tmem_ld32(tv + kCols * h, v); };
   const auto chunk_ptr = [&](uint32_t base, int c) {  // 16-byte chunk c, at chunk c ^ (row % 8)
-    return reinterpret_cast<uint4 *>(sm + (base - w1) + (uint32_t)h * kBlkBytes + (uint32_t)r * 128u +
-                                     ((uint32_t)(c ^ (r & 7)) << 4));
+    return reinterpret_cast<uint4 *>(sm + (base - w1) + (uint32_t)(h >> 1) * kBlkBytes + (uint32_t)r * 128u +
+                                     ((uint32_t)((4 * (h & 1) + c) ^ (r & 7)) << 4));
   };
 
   // training: sums over this thread's rows (columns 2 cp, 2 cp + 1, rows
-  // 32 rg .. + 31 of every tile) of the bias gradients and of gw4; over this
+  // kRgRows rg .. of every tile) of the bias gradients and of gw4; over this
   // thread's own row of dy and of the squared error
+  constexpr int kRowGroups = kTrainThreads / 64, kRgRows = kTileM / kRowGroups;
   const int cp = t & 63, rg = t >> 6;
   float gb1[2] = {0.f, 0.f}, gb2[2] = {0.f, 0.f}, gb3[2] = {0.f, 0.f}, gw4[2] = {0.f, 0.f};
   float gb4 = 0.f, sse = 0.f;
@@ -449,8 +430,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   };
   const auto colsum = [&](uint32_t base, float *s) {
 #pragma unroll 16
-    for (int i = 0; i < 32; ++i) {
-      const uint32_t w = *pair_ptr(base, 32 * rg + i);
+    for (int i = 0; i < kRgRows; ++i) {
+      const uint32_t w = *pair_ptr(base, kRgRows * rg + i);
       s[0] += bf_lo(w);
       s[1] += bf_hi(w);
     }
@@ -477,12 +458,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     for (int layer = 0; layer < 2; ++layer) {
       wait_mma();
       {
-        uint32_t v[64];
+        uint32_t v[kCols];
         load_acc(v);
         const uint32_t dst = layer == 0 ? h1 : h2;
-        const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[layer][64 * h]);
+        const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[layer][kCols * h]);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < kCols / 8; ++c) {
           uint32_t w[4];
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
@@ -508,17 +489,17 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     }
     if (!ok) break;
     // layer 3 and the output layer: y = relu(.) . w4 + b4 on the BF16
-    // activations, the two column halves added in a fixed order
+    // activations, the column parts added in a fixed order
     wait_mma();
     float ysum = 0.f;
     {
-      uint32_t v[64];
+      uint32_t v[kCols];
       load_acc(v);
-      const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[2][64 * h]);
-      const ulonglong2 *wv = reinterpret_cast<const ulonglong2 *>(&s_w4[64 * h]);
+      const ulonglong2 *bias = reinterpret_cast<const ulonglong2 *>(&s_bias[2][kCols * h]);
+      const ulonglong2 *wv = reinterpret_cast<const ulonglong2 *>(&s_w4[kCols * h]);
       uint64_t sum0 = 0ull, sum1 = 0ull;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < kCols / 8; ++c) {
         uint32_t w[4];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -535,13 +516,13 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
       }
       ysum = (f2_lo(sum0) + f2_hi(sum0)) + (f2_lo(sum1) + f2_hi(sum1));
     }
-    if (h == 1) s_part[r] = ysum;
+    if (h > 0) s_part[h - 1][r] = ysum;
     tc_fence_before();  // (the accumulator is read: the next MMA may write it)
     if (!end_phase()) { ok = false; break; }
     if (h == 0) {
       float dy = 0.f;
       if (in) {
-        const float e = ((ysum + s_part[r]) + b4) - tgt[tile * (int64_t)kTileM + r];
+        const float e = ((((ysum + s_part[0][r]) + s_part[1][r]) + s_part[2][r]) + b4) - tgt[tile * (int64_t)kTileM + r];
         dy = 2.f * e / (float)M;
         sse += e * e;
         gb4 += dy;
@@ -552,14 +533,13 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     // dZ3 = bf16(dy w4) where H3 > 0, in place; sums of gw4 and gb3
     {
       const float wa = s_w4[2 * cp], wb = s_w4[2 * cp + 1];
-#pragma unroll 1
-      for (int i0 = 0; i0 < 32; i0 += 16) {
-        uint32_t w[16];
+      {
+        uint32_t w[kRgRows];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) w[i] = *pair_ptr(h3, 32 * rg + i0 + i);
+        for (int i = 0; i < kRgRows; ++i) w[i] = *pair_ptr(h3, kRgRows * rg + i);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float dy = s_dy[32 * rg + i0 + i], x0 = bf_lo(w[i]), x1 = bf_hi(w[i]);
+        for (int i = 0; i < kRgRows; ++i) {
+          const float dy = s_dy[kRgRows * rg + i], x0 = bf_lo(w[i]), x1 = bf_hi(w[i]);
           gw4[0] += x0 * dy;
           gw4[1] += x1 * dy;
           w[i] = bf2(x0 > 0.f ? dy * wa : 0.f, x1 > 0.f ? dy * wb : 0.f);
@@ -567,7 +547,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
           gb3[1] += bf_hi(w[i]);
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) *pair_ptr(h3, 32 * rg + i0 + i) = w[i];
+        for (int i = 0; i < kRgRows; ++i) *pair_ptr(h3, kRgRows * rg + i) = w[i];
       }
     }
     if (!publish()) { ok = false; break; }
@@ -587,10 +567,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
       if (layer == 1) colsum(h2, gb2);
       wait_mma();
       {
-        uint32_t v[64];
+        uint32_t v[kCols];
         load_acc(v);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < kCols / 8; ++c) {
           uint4 *a = chunk_ptr(hp, c);
           const uint4 mm = *a;
           const uint32_t m[4] = {mm.x, mm.y, mm.z, mm.w};
@@ -623,17 +603,16 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     float *o = part + (size_t)blockIdx.x * kPartStride;
 #pragma unroll 1
     for (int w = 0; w < 3; ++w) {
-      const int nin = w == 2 ? 32 : 64, in0 = nin * h;
+      const int in0 = kCols * h;
+      if (w == 2 && in0 >= kMlpIn) break;
       float *dst = o + (w == 0 ? kMlpOW3 : (w == 1 ? kMlpOW2 : kMlpOW1)) + r;
       const uint32_t src = tmem + (w == 0 ? kTmW3 : (w == 1 ? kTmW2 : kTmW1)) + ((uint32_t)(q * 32) << 16) + in0;
-      for (int c = 0; c < nin; c += 32) {
-        uint32_t v[32];
-        tmem_ld32(src + c, v);
+      uint32_t v[kCols];
+      tmem_ld32(src, v);
 #pragma unroll
-        for (int k = 0; k < 32; ++k) dst[(in0 + c + k) * kMlpH] = __uint_as_float(v[k]);
-      }
+      for (int k = 0; k < kCols; ++k) dst[(in0 + k) * kMlpH] = __uint_as_float(v[k]);
     }
-    // the four row groups' column sums, in order; the features' stages are free
+    // the row groups' column sums, in order; the features' stages are free
     float *sum = reinterpret_cast<float *>(mlp_smem + (xs - smem_u32(mlp_smem)));
     float *mine = sum + rg * 4 * kMlpH + 2 * cp;
     const float *src[4] = {gb1, gb2, gb3, gw4};
@@ -642,7 +621,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
       mine[k * kMlpH] = src[k][0];
       mine[k * kMlpH + 1] = src[k][1];
     }
-    float *red = sum + 16 * kMlpH;
+    float *red = sum + kRowGroups * 4 * kMlpH;
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) {
       gb4 += __shfl_xor_sync(0xffffffffu, gb4, k);
@@ -650,8 +629,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     }
     if (lane == 0) { red[2 * (t >> 5)] = gb4; red[2 * (t >> 5) + 1] = sse; }
     __syncthreads();
-    for (int i = t; i < 4 * kMlpH; i += kTrainThreads)
-      o[kMlpOB1 + i] = ((sum[i] + sum[4 * kMlpH + i]) + sum[8 * kMlpH + i]) + sum[12 * kMlpH + i];
+    for (int i = t; i < 4 * kMlpH; i += kTrainThreads) {
+      float a = sum[i];
+#pragma unroll
+      for (int k = 1; k < kRowGroups; ++k) a += sum[4 * kMlpH * k + i];
+      o[kMlpOB1 + i] = a;
+    }
     if (t < 2) o[kMlpOB4 + t] = ((red[t] + red[2 + t]) + red[4 + t]) + red[6 + t];
   }
   if (t == 0 && (!ok || !wok)) {

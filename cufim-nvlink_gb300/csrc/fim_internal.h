@@ -223,12 +223,12 @@ constexpr int kMlpOB1 = kMlpW16, kMlpOB2 = kMlpOB1 + kMlpH, kMlpOB3 = kMlpOB2 + 
 constexpr int kMlpOW4 = kMlpOB3 + kMlpH, kMlpOB4 = kMlpOW4 + kMlpH;
 constexpr int kMlpParams = kMlpOB4 + 1;
 
-// Feature rows of the learned warm start (fim_mlp.cu); red receives the
+// Feature rows of the learned warm start (fim_mlp.cu); *red points to the
 // bounding box and the largest stimulus distance (features_scale reads it).
+size_t features_scratch(int nV);  // floats of scratch, 32-byte aligned
 cudaError_t launch_features(int nV, int64_t nT, const double *xyz, const int32_t *tslots, const double *fib,
                             const double *cf, const double *ct, int nseed, const int32_t *seed_v,
-                            const double *seed_t, float *acc, float *dist, unsigned int *red, void *X,
-                            cudaStream_t st);
+                            const double *seed_t, float *scratch, unsigned int **red, void *X, cudaStream_t st);
 float features_scale(const unsigned int *host_red);
 
 // ---- fixed scratch of fim_solve_noalloc (fim_static.cu) ----

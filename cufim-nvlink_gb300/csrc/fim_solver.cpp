@@ -1478,15 +1478,13 @@ extern "C" int fim_features(fim_solver *s, void *d_features, float *time_scale)
     return set_err(s, FIM_ERR_NOT_READY, "fim_features: mesh, conduction and stimuli must be set first");
   if (s->gptr.p) return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_features: meshes with submesh tags are not supported");
   CUDA_TRY(s, cudaSetDevice(s->device));
-  DevBuf<float> acc, dist;
-  DevBuf<unsigned int> red;
-  CUDA_TRY(s, acc.alloc(6 * (size_t)s->nV));
-  CUDA_TRY(s, dist.alloc((size_t)s->nV));
-  CUDA_TRY(s, red.alloc(8));
+  DevBuf<float> scratch;
+  unsigned int *red = nullptr;
+  CUDA_TRY(s, scratch.alloc(features_scratch((int)s->nV)));
   CUDA_TRY(s, launch_features((int)s->nV, s->nT, s->xyz.p, s->tslots.p, s->fib.p, s->cf.p, s->ct.p, s->nseed,
-                              s->seed_v.p, s->seed_t.p, acc.p, dist.p, red.p, d_features, s->stream));
+                              s->seed_v.p, s->seed_t.p, scratch.p, &red, d_features, s->stream));
   unsigned int h[8] = {};
-  CUDA_TRY(s, cudaMemcpyAsync(h, red.p, sizeof(unsigned int) * 7, cudaMemcpyDeviceToHost, s->stream));
+  CUDA_TRY(s, cudaMemcpyAsync(h, red, sizeof(unsigned int) * 7, cudaMemcpyDeviceToHost, s->stream));
   CUDA_TRY(s, cudaStreamSynchronize(s->stream));
   if (time_scale) *time_scale = features_scale(h);
   return FIM_OK;

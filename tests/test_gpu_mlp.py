@@ -207,3 +207,44 @@ def test_prediction_rounds_with_few_tiles(F, torch_cuda, tiles):
     assert yg[n] == 7.0
     assert (~np.isclose(yg[:n], y_o, rtol=1e-3, atol=1e-3)).mean() < 0.01
     assert np.abs(yg[:n] - y_o).max() < 0.05 * np.abs(y_o).max()
+
+
+@pytest.mark.parametrize("cells,offset", [((1, 1, 1), 0), ((3, 2, 1), 2), ((9, 7, 3), 0), ((9, 7, 3), 6), ((31, 16, 5), 0)])
+def test_features_against_their_definition(F, torch_cuda, cells, offset):
+    """Every feature from its definition in float64, on a 16-byte boundary and
+    off it.  Features are BF16 (relative half step 2^-9; 2^-7 leaves room for
+    the FP32 sums before the rounding); the angle and the coordinates lie in
+    [-1, 1] and may pass through zero: 2^-8 absolute."""
+    import fim_mesh
+    torch = torch_cuda
+    c = fim_mesh.slab_case(cells=cells, size=(2.0, 1.5, 0.5), seed=11, cf=0.6, ct=0.25, angle=50.0, scar_radius=0.2,
+                           n_stim=3, t0_max=5.0)
+    xyz, tets = np.asarray(c["xyz"], float), np.asarray(c["tets"])
+    nV = xyz.shape[0]
+    buf = torch.full((nV * 64 + 16,), 77, dtype=torch.int16, device="cuda")
+    with F.Solver() as s:
+        s.set_mesh(xyz, tets)
+        s.set_conduction(c["fib"], c["cf"], c["ct"])
+        s.set_stimuli(c["seed_v"], c["seed_t"])
+        scale = s.features(buf.data_ptr() + offset)
+    raw = buf.cpu().numpy().view(np.uint16)
+    lo = offset // 2
+    assert (raw[:lo] == 77).all() and (raw[lo + nV * 64:] == 77).all()
+    X = (raw[lo:lo + nV * 64].astype(np.uint32) << 16).view(np.float32).reshape(nV, 64).astype(float)
+    sums = np.zeros((nV, 6))
+    per_tet = np.column_stack([np.asarray(c["fib"], float), c["cf"], c["ct"], np.ones(len(tets))])
+    for k in range(4):
+        np.add.at(sums, tets[:, k], per_tet)
+    f = sums[:, :3] / np.linalg.norm(sums[:, :3], axis=1, keepdims=True)
+    cf, ct = sums[:, 3] / sums[:, 5], sums[:, 4] / sums[:, 5]
+    d = xyz[:, None, :] - xyz[np.asarray(c["seed_v"])][None]
+    along = np.einsum("vsk,vk->vs", d, f)
+    d2 = along ** 2 / cf[:, None] ** 2 + ((d ** 2).sum(-1) - along ** 2) / ct[:, None] ** 2
+    dist = (np.asarray(c["seed_t"], float)[None] + np.sqrt(np.maximum(d2, 0))).min(1)
+    mid, half = (xyz.max(0) + xyz.min(0)) / 2, (xyz.max(0) - xyz.min(0)) / 2
+    assert scale == pytest.approx(dist.max(), rel=1e-5)
+    assert np.allclose(X[:, :3], (xyz - mid) / half, rtol=0, atol=2.0 ** -8)
+    for k, want in ((3, dist / dist.max()), (4, cf), (5, ct)):
+        assert np.allclose(X[:, k], want, rtol=2.0 ** -7, atol=2.0 ** -12), k
+    assert np.allclose(X[:, 6], np.arctan2(f[:, 1], f[:, 0]) / np.pi, rtol=0, atol=2.0 ** -8)
+    assert (X[:, 7:] == 0).all()

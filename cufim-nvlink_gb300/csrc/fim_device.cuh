@@ -448,8 +448,9 @@ static __device__ bool grid_sync(FimCtl *ctl, uint32_t nblocks, uint64_t timeout
     unsigned long long *word = &ctl->phase[k & 3].v;
     // the word of phase k + 2, last used by barrier k - 2, which every block has left
     if (blockIdx.x == 0) ctl->phase[(k + 2) & 3].v = 0ull;
-    __threadfence();
-    atomicAdd(word, 1ull);
+    // (a release on the arrival itself: with a full fence before a relaxed one
+    // the 58k windowed slab took 4.25 ms instead of 4.17)
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(1ull) : "memory");
     const uint64_t t0 = global_timer();
     uint32_t spins = 0;
     int ok = 1;

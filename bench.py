@@ -38,14 +38,8 @@ import numpy as np  # noqa: E402
 SLAB_CELLS = (266, 93, 40)
 # DRAM bytes (read + write) of one fim_solve_kernel launch per vertex update,
 # from ncu dram__bytes_read.sum + dram__bytes_write.sum on this workload
-# (ncu measurement: 4.294 GB for 4,689,493 vertex updates, two-phase kernel, 192x4096 batches)
-NCU_DRAM_BYTES_PER_VERTEX_UPDATE = 4.294e9 / 4689493
-
-
-def metric_launches(nT):
-    """fim_metric_kernel launches per conduction upload: the field goes up in
-    up to 8 chunks of at least 2^18 tets (fim_solver.cpp, run_metric)."""
-    return max(1, min(8, nT >> 18))
+# (ncu measurement: 4.551 GB for 4,689,493 vertex updates, two-phase kernel, 192x4096 batches)
+NCU_DRAM_BYTES_PER_VERTEX_UPDATE = 4.551e9 / 4689493
 METRICS = {
     "slab": "slab solves/s (1.03M-vertex anisotropic FIM, bit-exact vs FP64 oracle)",
     "cube": "cube solves/s (9,261-vertex plain FIM, bit-exact vs FP64 oracle)",
@@ -370,7 +364,7 @@ def run_mine(args):
                               "latency of its per-batch phase chain (FP64 solves, block barriers), not by HBM")},
         "e2e": {"value": world * e2e_steps / e2e_s, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h)},
-        "gpu_launches": (metric_launches(nT) + 1) * args.steps,
+        "gpu_launches": 2 * args.steps,  # metric and solve
         "clocks": clk,
         "autotune": {"batch_vertices": tune["batch_slots"], "batch_corners": tune["batch_corners"],
                      "grid_blocks": tune["grid_blocks"], "fp64_tet_warps": tune["dag_warps"],

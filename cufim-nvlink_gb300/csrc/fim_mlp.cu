@@ -98,15 +98,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 // offset), leading byte offset unused.  MN-major: 64-column blocks kBlkBytes
 // apart (leading byte offset), 8-row groups (of the contraction) 1024 B
 // apart (stride byte offset).
-constexpr uint64_t kDescBase = ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-__device__ __forceinline__ uint64_t desc_k(uint32_t addr)
-{
-  return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | kDescBase;
-}
-__device__ __forceinline__ uint64_t desc_mn(uint32_t addr)
-{
-  return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)(kBlkBytes >> 4) << 16) | kDescBase;
-}
+// Descriptors are kept as their low words: the high one is kDescHi for both.
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_k(uint32_t addr) { return (addr >> 4) | (1u << 16); }
+__device__ __forceinline__ uint32_t desc_mn(uint32_t addr) { return (addr >> 4) | ((kBlkBytes >> 4) << 16); }
 // Instruction descriptor of tcgen05.mma kind::f16: FP32 accumulator (bits
 // 4-5 = 1), BF16 A and B (bits 7-9, 10-12 = 1), A / B MN-major (bits 15,
 // 16), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
@@ -115,44 +110,36 @@ __host__ __device__ constexpr uint32_t idesc(int n, bool a_mn, bool b_mn)
   return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate)
+// One lane of a warp in step issues the MMAs (elect_one, after a branch on a
+// warp index that is known to be uniform): operands then stay in uniform
+// registers.  Issued by a thread of a divergent branch a step took 80 cycles
+// of the issuing thread, more than the 64 of the tensor pipe (predictions of
+// 1.03M rows 90 us, 79 this way).
+__device__ __forceinline__ bool elect_one()
 {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(tmem), "l"(a), "l"(b), "r"(id), "r"(accumulate)
-      : "memory");
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+  return e != 0;
 }
-// For a warp that runs in step with one lane issuing (lead): operands stay in
-// uniform registers, and a step is the MMA and an add.  Descriptors by their
-// low words (kDescHi is the other); acc += where `more`, else acc =.
-constexpr uint32_t kDescHi = (uint32_t)(kDescBase >> 32);
-template <bool kMore>
-__device__ __forceinline__ void umma_ss(bool lead, uint32_t acc, uint32_t a, uint32_t b, uint32_t id)
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x / 32, 0); }
+// acc (+)= A B; A and B in shared memory
+__device__ __forceinline__ void umma_ss(uint32_t acc, uint32_t a, uint32_t b, uint32_t id, bool more)
 {
   asm volatile(
-      "{\n .reg .pred p, q;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %6, 0;\n"
+      "{\n .reg .pred p;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n"
       " mov.b64 x, {%1, %3};\n mov.b64 y, {%2, %3};\n"
-      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %4, p;\n}"
-      ::"r"(acc), "r"(a), "r"(b), "r"(kDescHi), "r"(id), "n"(kMore ? 1 : 0), "r"((uint32_t)lead)
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %4, p;\n}"
+      ::"r"(acc), "r"(a), "r"(b), "r"(kDescHi), "r"(id), "r"((uint32_t)more)
       : "memory");
 }
 // the same with A in tensor memory
-template <bool kMore>
-__device__ __forceinline__ void umma_ts(bool lead, uint32_t acc, uint32_t a, uint32_t b, uint32_t id)
+__device__ __forceinline__ void umma_ts(uint32_t acc, uint32_t a, uint32_t b, uint32_t id, bool more)
 {
   asm volatile(
-      "{\n .reg .pred p, q;\n .reg .b64 y;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %6, 0;\n"
+      "{\n .reg .pred p;\n .reg .b64 y;\n setp.ne.b32 p, %5, 0;\n"
       " mov.b64 y, {%2, %3};\n"
-      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %4, p;\n}"
-      ::"r"(acc), "r"(a), "r"(b), "r"(kDescHi), "r"(id), "n"(kMore ? 1 : 0), "r"((uint32_t)lead)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_lead(bool lead, uint32_t bar)
-{
-  asm volatile(
-      "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
-      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar), "r"((uint32_t)lead)
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], y, %4, p;\n}"
+      ::"r"(acc), "r"(a), "r"(b), "r"(kDescHi), "r"(id), "r"((uint32_t)more)
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar)
@@ -232,15 +219,23 @@ __device__ __forceinline__ int transposed_index(int i)
   return off + (k % kMlpH) * kMlpH + k / kMlpH;
 }
 
-// acc (tile rows x 128) = A (K-major, kblk blocks of 64 columns) times the
-// K-major 128 x 64 kblk operand B, transposed
-__device__ __forceinline__ void mma_rows(uint32_t acc, uint32_t a, uint32_t b, int kblk)
+// acc (tile rows x 128) = A (K-major, kBlocks blocks of 64 columns) times the
+// K-major 128 x 64 kBlocks operand B, transposed
+template <int kBlocks>
+__device__ __forceinline__ void mma_rows(uint32_t acc, uint32_t a, uint32_t b)
 {
-  for (int s = 0; s < kblk; ++s)
 #pragma unroll
-    for (int k = 0; k < kBlkCols / 16; ++k)
-      umma_bf16(acc, desc_k(a + s * kBlkBytes + 32 * k), desc_k(b + s * kBlkBytes + 32 * k), idesc(128, false, false),
-                (uint32_t)(s | k));
+  for (int k = 0; k < kBlocks * kBlkCols / 16; ++k) {
+    const uint32_t at = (k / 4) * (kBlkBytes >> 4) + 2 * (k % 4);
+    umma_ss(acc, desc_k(a) + at, desc_k(b) + at, idesc(128, false, false), k != 0);
+  }
+}
+// the same for 128 columns with A in tensor memory, two BF16 to a 32-bit column
+__device__ __forceinline__ void mma_rows_tmem(uint32_t acc, uint32_t a, uint32_t b)
+{
+#pragma unroll
+  for (int k = 0; k < 128 / 16; ++k)
+    umma_ts(acc, a + 8 * k, desc_k(b) + (k / 4) * (kBlkBytes >> 4) + 2 * (k % 4), idesc(128, false, false), k != 0);
 }
 // acc (tile rows x 128) = A (K-major, 128 columns) times W (128 rows x 128
 // columns, contraction over its rows)
@@ -248,16 +243,16 @@ __device__ __forceinline__ void mma_data(uint32_t acc, uint32_t a, uint32_t w)
 {
 #pragma unroll
   for (int k = 0; k < 128 / 16; ++k)
-    umma_bf16(acc, desc_k(a + (uint32_t)(k / 4) * kBlkBytes + 32 * (k % 4)), desc_mn(w + 2048 * k),
-              idesc(128, false, true), (uint32_t)k);
+    umma_ss(acc, desc_k(a) + (k / 4) * (kBlkBytes >> 4) + 2 * (k % 4), desc_mn(w) + (2048 >> 4) * k,
+            idesc(128, false, true), k != 0);
 }
 // acc (128 x n) (+)= D^T H over the tile's rows: D 128 columns, H n columns
-__device__ __forceinline__ void mma_weight(uint32_t acc, uint32_t d, uint32_t h, int n, bool first)
+template <int n>
+__device__ __forceinline__ void mma_weight(uint32_t acc, uint32_t d, uint32_t h, bool first)
 {
-  const uint32_t id = n == 128 ? idesc(128, true, true) : idesc(64, true, true);
 #pragma unroll
   for (int k = 0; k < kTileM / 16; ++k)
-    umma_bf16(acc, desc_mn(d + 2048 * k), desc_mn(h + 2048 * k), id, (first && k == 0) ? 0u : 1u);
+    umma_ss(acc, desc_mn(d) + (2048 >> 4) * k, desc_mn(h) + (2048 >> 4) * k, idesc(n, true, true), !(first && k == 0));
 }
 
 __device__ __forceinline__ uint64_t f2_pack(float x, float y)
@@ -295,7 +290,7 @@ __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w <<
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 // ---------------------------------------------------------------------------
 // Training over 128-row tiles: sixteen warps, warp w with tensor-memory lanes
-// 32 (w % 4) .. + 31 (the tile's rows) of a quarter of the columns; thread 0
+// 32 (w % 4) .. + 31 (the tile's rows) of a quarter of the columns; warp 0
 // issues the TMA loads and the MMAs.  One tile at a time, since a tile's features and
 // three activations (112 KB) leave no room for a second one beside the 80 KB
 // of weights; the next tile's features are loaded a tile ahead.  Step of
@@ -350,19 +345,22 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+  const int warp = warp_index();
   const uint32_t bar_m = smem_u32(&mdone);
-  int issued = 0, consumed = 0;  // thread 0: feature tiles
+  int issued = 0, consumed = 0;  // warp 0: feature tiles
   // feature tile i of the CTA: its buffer, barrier and parity
   const auto x_buf = [&](int i) { return xs + (uint32_t)(i & 1) * kBlkBytes; };
   const auto x_bar = [&](int i) { return smem_u32(&xfull[i & 1]); };
   const auto x_par = [&](int i) { return (uint32_t)(i >> 1) & 1u; };
   const auto load_x = [&](int tile) {
-    mbar_expect_tx(x_bar(issued), kBlkBytes);
-    tma_load_2d(x_buf(issued), &tx, 0, tile * kTileM, x_bar(issued));
+    if (lane == 0) {
+      mbar_expect_tx(x_bar(issued), kBlkBytes);
+      tma_load_2d(x_buf(issued), &tx, 0, tile * kTileM, x_bar(issued));
+    }
     ++issued;
   };
-  if (t == 0 && tile0 < ntiles) load_x(tile0);
+  if (warp == 0 && tile0 < ntiles) load_x(tile0);
   if (threadIdx.x == 0) {
     mbar_expect_tx(smem_u32(&wfull), kWBytes);
     tma_load_2d(w1, &tw1, 0, 0, smem_u32(&wfull));
@@ -378,14 +376,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   const float b4 = P[kMlpOB4];
   __syncthreads();
   bool wok = true;
-  if (t == 0) wok = mbar_wait(smem_u32(&wfull), 0);
+  if (warp == 0) wok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&wfull), 0));
 
   // A phase ends with a barrier; a wait that ran out in phase p
   // is flagged in s_fail[p & 1] before that barrier and read after it, so
   // the whole CTA leaves together (a later phase writes the other word).
   int phase = 0;
   uint32_t mpar = 0;       // parity of the next MMA completion
-  int commits = 0;         // thread 0: completions requested
+  int commits = 0;         // warp 0: completions requested
   int waited = 0;
   const auto fail = [&]() { s_fail[phase & 1] = 1; };
   const auto end_phase = [&]() {
@@ -442,18 +440,20 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   for (int tile = tile0; tile < ntiles; tile += tstep, ++j) {
     const bool in = tile * kTileM + r < M;
     // layer 1
-    if (t == 0) {
+    if (warp == 0) {
       if (tile + tstep < ntiles) load_x(tile + tstep);  // its stage was read by MMAs that have completed
-      if (!wok || !mbar_wait(x_bar(j), x_par(j))) fail();
+      if (!__all_sync(0xffffffffu, wok && mbar_wait(x_bar(j), x_par(j)))) fail();
       else {
         ++consumed;
         tc_fence_after();
-        mma_rows(tmem, x_buf(j), w1, 1);
-        umma_commit(bar_m);
+        if (elect_one()) {
+          mma_rows<1>(tmem, x_buf(j), w1);
+          umma_commit(bar_m);
+        }
         ++commits;
       }
+      __syncwarp();
     }
-    __syncwarp();
 #pragma unroll 1
     for (int layer = 0; layer < 2; ++layer) {
       wait_mma();
@@ -478,14 +478,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
         }
       }
       if (!publish()) { ok = false; break; }
-      if (t == 0) {
+      if (warp == 0) {
         tc_fence_after();
-        if (layer == 0) mma_rows(tmem, h1, w2, 2);
-        else mma_rows(tmem, h2, w3, 2);
-        umma_commit(bar_m);
+        if (elect_one()) {
+          mma_rows<2>(tmem, layer == 0 ? h1 : h2, layer == 0 ? w2 : w3);
+          umma_commit(bar_m);
+        }
         ++commits;
+        __syncwarp();
       }
-      __syncwarp();
     }
     if (!ok) break;
     // layer 3 and the output layer: y = relu(.) . w4 + b4 on the BF16
@@ -556,14 +557,16 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
 #pragma unroll 1
     for (int layer = 0; layer < 2; ++layer) {
       const uint32_t dz = layer == 0 ? h3 : h2, hp = layer == 0 ? h2 : h1;
-      if (t == 0) {
+      if (warp == 0) {
         tc_fence_after();
-        mma_data(tmem, dz, layer == 0 ? w3 : w2);
-        mma_weight(tmem + (layer == 0 ? kTmW3 : kTmW2), dz, hp, 128, j == 0);
-        umma_commit(bar_m);
+        if (elect_one()) {
+          mma_data(tmem, dz, layer == 0 ? w3 : w2);
+          mma_weight<128>(tmem + (layer == 0 ? kTmW3 : kTmW2), dz, hp, j == 0);
+          umma_commit(bar_m);
+        }
         ++commits;
+        __syncwarp();
       }
-      __syncwarp();
       if (layer == 1) colsum(h2, gb2);
       wait_mma();
       {
@@ -586,13 +589,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     }
     if (!ok) break;
     // dW1 = X^T dZ1
-    if (t == 0) {
+    if (warp == 0) {
       tc_fence_after();
-      mma_weight(tmem + kTmW1, h1, x_buf(j), 64, j == 0);
-      umma_commit(bar_m);
+      if (elect_one()) {
+        mma_weight<64>(tmem + kTmW1, h1, x_buf(j), j == 0);
+        umma_commit(bar_m);
+      }
       ++commits;
+      __syncwarp();
     }
-    __syncwarp();
     colsum(h1, gb1);
     wait_mma();
     if (!end_phase()) { ok = false; break; }
@@ -685,7 +690,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(
   __shared__ int xloads[kFwdGroups];  // feature tiles asked for
   __shared__ uint32_t tmem_base;
   __shared__ __align__(16) float s_bias[3][kMlpH], s_w4[kMlpH];
-  const int g = threadIdx.x / kFwdGroupThreads, t = threadIdx.x % kFwdGroupThreads, lane = t & 31;
+  const int g = warp_index() / (kFwdGroupThreads / 32);
+  const int t = threadIdx.x % kFwdGroupThreads, lane = t & 31;
   const uint32_t w1 = (smem_u32(mlp_smem) + 1023u) & ~1023u, w2 = w1 + kW1Bytes, w3 = w2 + kW2Bytes;
   const int ntiles = (M + kTileM - 1) / kTileM, tstep = gridDim.x * kFwdGroups;
 
@@ -715,14 +721,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
 
   bool ok = true;
   if (g == kFwdGroups) {  // the issuing warp: in step, lane 0 issues
     {
-      const bool lead = lane == 0;
-      const uint32_t id = idesc(128, false, false);
-      const auto desc_lo = [](uint32_t addr) { return (addr >> 4) | (1u << 16); };
+      const bool lead = elect_one();
       const auto x_buf = [&](int gg, int i) { return w1 + kWBytes + (uint32_t)(2 * gg + (i & 1)) * kBlkBytes; };
       const auto load_x = [&](int gg, int i) {  // tile i of group gg, if there is one
         const int tile = gg * gridDim.x + blockIdx.x + i * tstep;
@@ -757,20 +761,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(
                                 (layer != 0 || mbar_wait(smem_u32(&xfull[gg][i & 1]), (uint32_t)(i >> 1) & 1u)));
             if (!ok) continue;
             tc_fence_after();
-            const uint32_t acc = tmem + gg * kTmGroup;
-            if (layer == 0) {
-              const uint32_t a = desc_lo(x_buf(gg, i)), b = desc_lo(w1);
-              umma_ss<false>(lead, acc, a, b, id);
-#pragma unroll
-              for (int c = 1; c < kBlkCols / 16; ++c) umma_ss<true>(lead, acc, a + 2 * c, b + 2 * c, id);
-            } else {
-              const uint32_t a = acc + kTmAct, b = desc_lo(layer == 1 ? w2 : w3);
-              umma_ts<false>(lead, acc, a, b, id);
-#pragma unroll
-              for (int c = 1; c < kMlpH / 16; ++c)
-                umma_ts<true>(lead, acc, a + 8 * c, b + (c / 4) * (kBlkBytes >> 4) + 2 * (c % 4), id);
+            if (lead) {
+              const uint32_t acc = tmem + gg * kTmGroup;
+              if (layer == 0) mma_rows<1>(acc, x_buf(gg, i), w1);
+              else mma_rows_tmem(acc, acc + kTmAct, layer == 1 ? w2 : w3);
+              umma_commit(smem_u32(&mdone[gg]));
             }
-            umma_commit_lead(lead, smem_u32(&mdone[gg]));
             issued[gg] = n + 1;
             if (layer == 1) load_x(gg, i + 2);  // layer 1 has read the stage
             __syncwarp();

@@ -294,9 +294,9 @@ __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 
 // issues the TMA loads and the MMAs.  One tile at a time, since a tile's features and
 // three activations (112 KB) leave no room for a second one beside the 80 KB
 // of weights; the next tile's features are loaded a tile ahead.  Step of
-// 4,096 rows (22 launches before, 2 now) 191 -> 44 us; gradients of 131,136
-// rows, whose activations and their transposes went through memory, 500 -> 91
-// (eight warps with half of the columns each: 45.5 and 96 us).
+// 4,096 rows (22 launches before, 2 now) 191 -> 43 us; gradients of 131,136
+// rows, whose activations and their transposes went through memory, 500 -> 85
+// (eight warps with half of the columns each: 96 against 91 us at the time).
 constexpr uint32_t kW1Bytes = kBlkBytes, kW2Bytes = 2 * kBlkBytes;
 constexpr uint32_t kWBytes = kW1Bytes + 2 * kW2Bytes;  // the weights, [out][in]
 constexpr uint32_t kActBytes = 2 * kBlkBytes;          // 128 x 128 activations
@@ -665,12 +665,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
 //
 // Predictions of 1.03M rows (features 132 MB): three GEMM kernels with the
 // activations in memory 252 us; one kernel, four groups of four warps that
-// each issued their own MMAs on operands in shared memory, 106; this one 91
-// (the MMAs 38 us at 68 cycles a step, the features 19 us of memory time; the
-// rest is the wait from a group's epilogue to its next MMA, which one other
-// group covers only in part).  Three groups of four warps sharing the four
-// quarters of tensor memory, one MMA in flight at a time: 121.  Accumulator
-// halves of 64 columns: a step takes as long as one of 128.
+// each issued their own MMAs on operands in shared memory, 106; this one 80
+// (73 on the device: the MMAs 38 at 68 cycles a step, the features 19 of
+// memory time; no pipe is busy for much more than half of it, and a group
+// waits for the other's part of the tensor pipe and of the issue slots).
+// Three groups, the third with its activations in shared memory (four warps
+// each, or eight on 32 columns at a time): 80 and 79.  An issuing warp per
+// group: their MMAs interleave and both groups wait longer, 97 against 92 at
+// the time.  Accumulator halves of 64 columns: a step takes as long as one
+// of 128.
 constexpr int kFwdGroups = 2, kFwdGroupThreads = 256, kFwdThreads = kFwdGroups * kFwdGroupThreads + 32;
 constexpr int kFwdSmem = (int)(kWBytes + kFwdGroups * 2 * kBlkBytes) + 1024;  // + slack to align to 1024 B
 constexpr uint32_t kTmAct = 128, kTmGroup = 256;  // the activations' columns; from group to group

@@ -197,10 +197,13 @@ struct StageLists {
 };
 // Checks tets (device, 4 nT ids) and xyz (device) into ctl; first (or
 // nullptr) receives every vertex's first appearance.
-cudaError_t launch_stage_check(int64_t nV, int64_t nT, const int64_t *tets, const double *xyz, uint32_t *first,
+// (Id: int64_t or int32_t)
+template <typename Id>
+cudaError_t launch_stage_check(int64_t nV, int64_t nT, const Id *tets, const double *xyz, uint32_t *first,
                                StageCtl *ctl, cudaStream_t st);
 // Slots of a mesh with one submesh, from checked tets.
-cudaError_t launch_stage_slots(int64_t nT, const int64_t *tets, const uint32_t *first, int32_t *slots,
+template <typename Id>
+cudaError_t launch_stage_slots(int64_t nT, const Id *tets, const uint32_t *first, int32_t *slots,
                                cudaStream_t st);
 // Corners of every vertex copy (increasing tet index) and the lengths of the
 // neighbourhoods; launch_stage_compact then writes the neighbourhoods.

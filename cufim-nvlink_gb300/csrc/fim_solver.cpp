@@ -411,8 +411,9 @@ struct Parts {
 
 }  // namespace
 
-extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, const int64_t *tets,
-                            const int32_t *atags)
+// Mesh of ids of 64 or 32 bits.
+template <typename Id>
+static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, const Id *tets, const int32_t *atags)
 {
   if (!s) return set_err(nullptr, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: solver is NULL");
   if (nV <= 0 || nT <= 0 || !xyz || !tets)
@@ -427,7 +428,7 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
   // previous mesh is still in place (a rejected mesh leaves it usable).
   // Staging buffer: control words, tets, coordinates, first appearances.
   const auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const size_t o_tets = up(sizeof(StageCtl)), o_xyz = o_tets + up(sizeof(int64_t) * 4 * nT);
+  const size_t o_tets = up(sizeof(StageCtl)), o_xyz = o_tets + up(sizeof(Id) * 4 * nT);
   const size_t o_first = o_xyz + up(sizeof(double) * 3 * nV);
   CUDA_TRY(s, s->stage.reserve(o_first + up(sizeof(uint32_t) * nV)));
   struct StageGuard {  // a large staging buffer is given back when the call ends
@@ -435,10 +436,10 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
     ~StageGuard() { if (b.n > (size_t(64) << 20)) b.release(); }
   } guard{s->stage};
   StageCtl *d_ctl = reinterpret_cast<StageCtl *>(s->stage.p);
-  int64_t *d_tets = reinterpret_cast<int64_t *>(s->stage.p + o_tets);
+  Id *d_tets = reinterpret_cast<Id *>(s->stage.p + o_tets);
   double *d_xyz = reinterpret_cast<double *>(s->stage.p + o_xyz);
   uint32_t *d_first = reinterpret_cast<uint32_t *>(s->stage.p + o_first);
-  CUDA_TRY(s, cudaMemcpyAsync(d_tets, tets, sizeof(int64_t) * 4 * nT, cudaMemcpyHostToDevice, st));
+  CUDA_TRY(s, cudaMemcpyAsync(d_tets, tets, sizeof(Id) * 4 * nT, cudaMemcpyHostToDevice, st));
   CUDA_TRY(s, cudaMemcpyAsync(d_xyz, xyz, sizeof(double) * 3 * nV, cudaMemcpyHostToDevice, st));
   CUDA_TRY(s, launch_stage_check(nV, nT, d_tets, d_xyz, d_first, d_ctl, st));
   StageCtl h{};
@@ -457,8 +458,14 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
   {
     std::vector<int32_t> agg;
     const int32_t nagg = atags ? aggregates(nT, atags, agg) : 1;
-    if (nagg > 1) reference_slots(nV, nT, tets, agg, nagg, S);
-    else {
+    if (nagg > 1) {
+      if constexpr (sizeof(Id) == sizeof(int64_t)) {
+        reference_slots(nV, nT, tets, agg, nagg, S);
+      } else {
+        const std::vector<int64_t> wide(tets, tets + 4 * nT);
+        reference_slots(nV, nT, wide.data(), agg, nagg, S);
+      }
+    } else {
       S.n_copies = nV;
       S.sub_ptr.push_back(0);
     }
@@ -551,6 +558,21 @@ extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_
   s->stats.n_corners = nC;
   s->have_mesh = true;
   return FIM_OK;
+}
+
+extern "C" int fim_set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, const int64_t *tets,
+                            const int32_t *atags)
+{
+  return set_mesh(s, nV, xyz, nT, tets, atags);
+}
+
+// For the Python binding, whose meshes mostly have 32-bit ids: widening them
+// on the host took 1.1 ms of a 135k-vertex one-shot solve (not part of
+// include/fim.h).
+extern "C" int fim_set_mesh_i32(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, const int32_t *tets,
+                                const int32_t *atags)
+{
+  return set_mesh(s, nV, xyz, nT, tets, atags);
 }
 
 // Uploads a conduction field and runs the metric kernel.  Host arrays are

@@ -39,16 +39,29 @@ __device__ __forceinline__ void cswap_by(uint32_t &ka, int &a, uint32_t &kb, int
   }
 }
 
+// The four ids of tet e, of 64 or 32 bits.
+__device__ __forceinline__ void load_ids(const int64_t *tets, int64_t e, long long *id)
+{
+  const longlong2 *p = reinterpret_cast<const longlong2 *>(tets);
+  const longlong2 a = __ldg(p + 2 * e), b = __ldg(p + 2 * e + 1);
+  id[0] = a.x; id[1] = a.y; id[2] = b.x; id[3] = b.y;
+}
+__device__ __forceinline__ void load_ids(const int32_t *tets, int64_t e, long long *id)
+{
+  const int4 a = __ldg(reinterpret_cast<const int4 *>(tets) + e);
+  id[0] = a.x; id[1] = a.y; id[2] = a.z; id[3] = a.w;
+}
+
 // Tets: every id in [0, nV), no vertex twice; the first offender of each
 // kind goes to ctl.  first[v] receives the smallest 4 e + (position of v
 // among tet e's ids in ascending order): the order of first appearance by
 // which the reference numbers a submesh's vertices (types.cpp:331-345).
-__global__ void check_tets_kernel(int64_t nV, int64_t nT, const longlong2 *__restrict__ tets, uint32_t *first,
-                                  StageCtl *ctl)
+template <typename Id>
+__global__ void check_tets_kernel(int64_t nV, int64_t nT, const Id *__restrict__ tets, uint32_t *first, StageCtl *ctl)
 {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nT; e += (int64_t)gridDim.x * blockDim.x) {
-    const longlong2 a = __ldg(tets + 2 * e), b = __ldg(tets + 2 * e + 1);
-    const long long id[4] = {a.x, a.y, b.x, b.y};
+    long long id[4];
+    load_ids(tets, e, id);
     bool in = true;
 #pragma unroll
     for (int j = 3; j >= 0; --j)
@@ -82,12 +95,14 @@ __global__ void check_xyz_kernel(int64_t n, const double *__restrict__ xyz, Stag
 
 // One submesh: the slots of every tet are its ids in the order of first
 // appearance (types.cpp:383-398, 473).
-__global__ void slots_kernel(int64_t nT, const longlong2 *__restrict__ tets, const uint32_t *__restrict__ first,
+template <typename Id>
+__global__ void slots_kernel(int64_t nT, const Id *__restrict__ tets, const uint32_t *__restrict__ first,
                              int4 *__restrict__ slots)
 {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nT; e += (int64_t)gridDim.x * blockDim.x) {
-    const longlong2 a = __ldg(tets + 2 * e), b = __ldg(tets + 2 * e + 1);
-    int v[4] = {(int)a.x, (int)a.y, (int)b.x, (int)b.y};
+    long long id[4];
+    load_ids(tets, e, id);
+    int v[4] = {(int)id[0], (int)id[1], (int)id[2], (int)id[3]};
     uint32_t k[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) k[j] = __ldg(first + v[j]);
@@ -378,7 +393,8 @@ cudaError_t scan(int64_t n, const int32_t *cnt, int64_t *out, long long *tile_su
 
 }  // namespace
 
-cudaError_t launch_stage_check(int64_t nV, int64_t nT, const int64_t *tets, const double *xyz, uint32_t *first,
+template <typename Id>
+cudaError_t launch_stage_check(int64_t nV, int64_t nT, const Id *tets, const double *xyz, uint32_t *first,
                                StageCtl *ctl, cudaStream_t st)
 {
   cudaError_t e;
@@ -386,18 +402,25 @@ cudaError_t launch_stage_check(int64_t nV, int64_t nT, const int64_t *tets, cons
   if ((e = cudaMemsetAsync(&ctl->max_edge2, 0, sizeof(StageCtl) - offsetof(StageCtl, max_edge2), st)) != cudaSuccess)
     return e;
   if (first && (e = cudaMemsetAsync(first, 0xff, sizeof(uint32_t) * (size_t)nV, st)) != cudaSuccess) return e;
-  check_tets_kernel<<<stage_grid(nT, kStageThreads), kStageThreads, 0, st>>>(
-      nV, nT, reinterpret_cast<const longlong2 *>(tets), first, ctl);
+  check_tets_kernel<<<stage_grid(nT, kStageThreads), kStageThreads, 0, st>>>(nV, nT, tets, first, ctl);
   check_xyz_kernel<<<stage_grid(3 * nV, kStageThreads), kStageThreads, 0, st>>>(3 * nV, xyz, ctl);
   return cudaGetLastError();
 }
 
-cudaError_t launch_stage_slots(int64_t nT, const int64_t *tets, const uint32_t *first, int32_t *slots, cudaStream_t st)
+template <typename Id>
+cudaError_t launch_stage_slots(int64_t nT, const Id *tets, const uint32_t *first, int32_t *slots, cudaStream_t st)
 {
-  slots_kernel<<<stage_grid(nT, kStageThreads), kStageThreads, 0, st>>>(
-      nT, reinterpret_cast<const longlong2 *>(tets), first, reinterpret_cast<int4 *>(slots));
+  slots_kernel<<<stage_grid(nT, kStageThreads), kStageThreads, 0, st>>>(nT, tets, first,
+                                                                        reinterpret_cast<int4 *>(slots));
   return cudaGetLastError();
 }
+
+template cudaError_t launch_stage_check(int64_t, int64_t, const int64_t *, const double *, uint32_t *, StageCtl *,
+                                        cudaStream_t);
+template cudaError_t launch_stage_check(int64_t, int64_t, const int32_t *, const double *, uint32_t *, StageCtl *,
+                                        cudaStream_t);
+template cudaError_t launch_stage_slots(int64_t, const int64_t *, const uint32_t *, int32_t *, cudaStream_t);
+template cudaError_t launch_stage_slots(int64_t, const int32_t *, const uint32_t *, int32_t *, cudaStream_t);
 
 cudaError_t launch_stage_lists(int64_t nL, int64_t nT, const StageLists &x, StageCtl *ctl, cudaStream_t st)
 {

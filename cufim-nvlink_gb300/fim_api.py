@@ -88,6 +88,7 @@ def lib():
         L.fim_last_error.argtypes = [vp]
         L.fim_last_error.restype = C.c_char_p
         L.fim_set_mesh.argtypes = [vp, i64, P(d), i64, P(i64), P(i32)]
+        L.fim_set_mesh_i32.argtypes = [vp, i64, P(d), i64, P(i32), P(i32)]
         L.fim_set_conduction.argtypes = [vp, P(d), P(d), P(d)]
         L.fim_set_conduction_device.argtypes = [vp, vp, vp, vp]
         L.fim_set_stimuli.argtypes = [vp, i64, P(i64), P(d)]
@@ -187,12 +188,14 @@ class Solver:
 
     def set_mesh(self, xyz, tets, atags=None):
         xyz = np.ascontiguousarray(xyz, dtype=np.float64)
-        tets = np.ascontiguousarray(tets, dtype=np.int64)
+        tets = np.asarray(tets)
+        narrow = tets.dtype == np.int32  # taken as they are: widening costs more than staging
+        tets = np.ascontiguousarray(tets, dtype=np.int32 if narrow else np.int64)
         at = None if atags is None else np.ascontiguousarray(atags, dtype=np.int32)
         self.nV = xyz.shape[0]
         self.nT = tets.shape[0]
-        _check(lib().fim_set_mesh(self.h, self.nV, _ptr(xyz, C.c_double), self.nT, _ptr(tets, C.c_int64),
-                                  _ptr(at, C.c_int32)), self.h)
+        call, ids = (lib().fim_set_mesh_i32, C.c_int32) if narrow else (lib().fim_set_mesh, C.c_int64)
+        _check(call(self.h, self.nV, _ptr(xyz, C.c_double), self.nT, _ptr(tets, ids), _ptr(at, C.c_int32)), self.h)
 
     def set_conduction(self, fib, cf, ct):
         fib = np.ascontiguousarray(fib, dtype=np.float64)

@@ -111,3 +111,31 @@ def test_rejected_mesh_leaves_the_previous_one(F, O):
         s.nV, s.nT = len(xyz), len(tets)
         s.solve()
         assert np.array_equal(s.times(with_state=False), phi)
+
+
+@pytest.mark.parametrize("tagged", [False, True])
+def test_ids_of_32_and_64_bits(F, O, tagged):
+    """Meshes with ids of either width, in any layout, solve to the same bits;
+    a bad id is reported the same way."""
+    import fim_mesh
+    xyz, tets = fim_mesh.kuhn_box(9, 5, 4, 1.0, 0.6, 0.5, seed=2)
+    c = case_of(xyz, np.asarray(tets, dtype=np.int64))
+    tags = (np.arange(len(tets)) * 3 // len(tets)).astype(np.int32) if tagged else None
+    wide = np.asarray(tets, dtype=np.int64)
+    strided = np.zeros((len(tets), 8), dtype=np.int32)
+    strided[:, ::2] = wide
+    got = []
+    for ids in (wide, wide.astype(np.int32), strided[:, ::2], np.asfortranarray(wide.astype(np.int32)),
+                wide.astype(np.uint32), wide.astype(np.int16)):
+        with F.Solver() as s:
+            s.set_mesh(xyz, ids, tags)
+            s.set_conduction(c["fib"], c["cf"], c["ct"])
+            s.set_stimuli(c["seed_v"], c["seed_t"])
+            s.solve()
+            got.append(s.times())
+            bad = np.array(ids)
+            bad[5, 3] = len(xyz)
+            with pytest.raises(F.FimError, match=f"tet 5 has vertex {len(xyz)}"):
+                s.set_mesh(xyz, bad, tags)
+    for phi, st in got[1:]:
+        assert np.array_equal(phi, got[0][0]) and np.array_equal(st, got[0][1])

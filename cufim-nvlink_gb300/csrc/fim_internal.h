@@ -160,6 +160,8 @@ cudaError_t solve_prepare(int shape, int device, int block, int *max_grid);
 cudaError_t launch_solve(const FimDev &d, const FimParams &p, int shape, int grid, int block, cudaStream_t stream);
 // Writes phi (any order) into out.
 cudaError_t launch_copy(const double *src, double *dst, int64_t n, cudaStream_t stream);
+// src on a 4-byte, dst on a 16-byte boundary
+cudaError_t launch_widen(const uint8_t *src, int32_t *dst, int64_t n, cudaStream_t stream);
 // Support check of a finished solve (fim_kernels.cu): every reached vertex
 // that is not a seed (is_seed[v] == 0) and whose time lies below a rigorous
 // lower bound of every candidate of its neighbours counts into ctl->n_bad

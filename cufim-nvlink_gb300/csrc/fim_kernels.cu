@@ -386,6 +386,26 @@ __global__ void fim_copy_kernel(const double *__restrict__ src, double *__restri
     dst[i] = __ldcg(src + i);
 }
 
+// States as the 32-bit integers callers read (fim_get_times).
+__global__ void fim_widen_kernel(const uint8_t *__restrict__ src, int32_t *__restrict__ dst, int64_t n)
+{
+  for (int64_t i = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n; i += 4 * (int64_t)gridDim.x * blockDim.x) {
+    if (i + 4 <= n) {
+      const uchar4 a = __ldcg(reinterpret_cast<const uchar4 *>(src + i));
+      *reinterpret_cast<int4 *>(dst + i) = make_int4(a.x, a.y, a.z, a.w);
+    } else {
+      for (int64_t k = i; k < n; ++k) dst[k] = src[k];
+    }
+  }
+}
+
+cudaError_t launch_widen(const uint8_t *src, int32_t *dst, int64_t n, cudaStream_t stream)
+{
+  if (n <= 0) return cudaSuccess;
+  fim_widen_kernel<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 152 * 8), 256, 0, stream>>>(src, dst, n);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_copy(const double *src, double *dst, int64_t n, cudaStream_t stream)
 {
   if (n <= 0) return cudaSuccess;

@@ -139,3 +139,27 @@ def test_ids_of_32_and_64_bits(F, O, tagged):
                 s.set_mesh(xyz, bad, tags)
     for phi, st in got[1:]:
         assert np.array_equal(phi, got[0][0]) and np.array_equal(st, got[0][1])
+
+
+@pytest.mark.parametrize("extra", [0, 3, 16384, 16387, 40000])  # states are widened on the device above 16,384 vertices
+def test_states_of_vertices_in_no_tet(F, extra):
+    """States come back for every vertex: with tags and more vertices in no
+    tet than vertex copies too (they stay far, and unreached)."""
+    import fim_mesh
+    xyz, tets = fim_mesh.kuhn_box(5, 4, 3, 1.0, 0.8, 0.6, seed=3)
+    n = len(xyz)
+    c = case_of(xyz, np.asarray(tets, dtype=np.int64))
+    tags = (np.arange(len(tets)) * 2 // len(tets)).astype(np.int32)
+    far = np.concatenate([xyz, np.full((extra, 3), 9.0)])
+    for at in (None, tags):
+        got = []
+        for points in (xyz, far):
+            with F.Solver() as s:
+                s.set_mesh(points, c["tets"], at)
+                s.set_conduction(c["fib"], c["cf"], c["ct"])
+                s.set_stimuli(c["seed_v"], c["seed_t"])
+                s.solve()
+                got.append(s.times())
+        assert np.array_equal(got[1][0][:n], got[0][0]) and np.array_equal(got[1][1][:n], got[0][1])
+        assert (got[1][1][n:] == F.FAR).all() and (got[1][0][n:] > 1e300).all()
+        assert len(np.unique(got[0][1])) >= 1 and got[0][1].min() >= 0

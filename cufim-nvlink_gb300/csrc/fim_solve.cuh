@@ -57,9 +57,12 @@ constexpr int kThreads = kSolveThreads;  // threads per block of the solve kerne
 #endif
 constexpr int kMarkLanes = FIM_MARK_LANES;  // threads per frozen vertex in the neighbour marking
 static_assert(kThreads % kMarkLanes == 0, "marking groups must tile the grid");
-// the two-phase path's marking (phase X): groups of kMarkLanesX threads,
-// two neighbours per thread and round
-constexpr int kMarkLanesX = 8;
+// the two-phase path's marking (phase X): groups of kMarkLanesX threads, one
+// neighbour per thread and round, so that a vertex with 15 neighbours takes
+// one (9k cube 0.871 ms, 17.7k slab 1.210, 87k shell 1.818, 1M slab 10.31; 8
+// threads with two neighbours each 0.898, 1.241, 1.864, 10.39; 32 threads
+// 0.869, 1.208, 1.843, 10.61)
+constexpr int kMarkLanesX = 16;
 static_assert(kThreads % kMarkLanesX == 0, "marking groups must tile the block");
 constexpr int kSlots = FIM_SLOTS;             // vertices per batch (at most)
 constexpr int kCornerCap = FIM_CORNER_CAP;    // corners per batch
@@ -1012,32 +1015,20 @@ __device__ __forceinline__ void update_phase(const FimDev &d, BatchSh &sh, const
       PROBE(kPrE);
       // the downwind neighbours of the vertices frozen now (not narrow, later
       // time): stamped in their state word, first stamp wins; a group of
-      // kMarkLanesX threads per frozen vertex, two neighbours per thread and
-      // round with their loads issued together
+      // kMarkLanesX threads per frozen vertex
       const int nfz = sh.nfz;
       for (int g = tid / kMarkLanesX; g < nfz; g += kThreads / kMarkLanesX) {
         const int slot = sh.fz[g];
         const double pn = dunkey(sh.res[slot]);
         const int64_t k0 = sh.n0[slot], k1 = k0 + sh.ncnt[slot];
-        for (int64_t k = k0 + tid % kMarkLanesX; k < k1; k += 2 * kMarkLanesX) {
-          const int64_t kk[2] = {k, k + kMarkLanesX};
-          int32_t v[2];
-          uint32_t w[2];
-          double pv[2];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) v[h] = kk[h] < k1 ? __ldg(d.nbr + kk[h]) : -1;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            w[h] = v[h] >= 0 ? __ldcg(&d.vs[v[h]].sw) : 0u;
-            pv[h] = v[h] >= 0 ? __ldcg(d.phi2 + v[h]) : 0.0;
-          }
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (v[h] >= 0 && sw_state(w[h]) != ST_NARROW && sw_stamp(w[h]) != stamp && pn < pv[h]) {
-              if (atomicCAS(&d.vs[v[h]].sw, w[h], sw_make(sw_state(w[h]), stamp)) == w[h]) {
-                d.tst[v[h]] = (uint8_t)sw_state(w[h]);
-                append_active(lo_.marked, lo_.word, v[h]);
-              }
+        for (int64_t k = k0 + tid % kMarkLanesX; k < k1; k += kMarkLanesX) {
+          const int32_t v = __ldg(d.nbr + k);
+          const uint32_t w = __ldcg(&d.vs[v].sw);
+          const double pv = __ldcg(d.phi2 + v);
+          if (sw_state(w) != ST_NARROW && sw_stamp(w) != stamp && pn < pv) {
+            if (atomicCAS(&d.vs[v].sw, w, sw_make(sw_state(w), stamp)) == w) {
+              d.tst[v] = (uint8_t)sw_state(w);
+              append_active(lo_.marked, lo_.word, v);
             }
           }
         }

@@ -192,10 +192,12 @@ class Solver:
         narrow = tets.dtype == np.int32  # taken as they are: widening costs more than staging
         tets = np.ascontiguousarray(tets, dtype=np.int32 if narrow else np.int64)
         at = None if atags is None else np.ascontiguousarray(atags, dtype=np.int32)
+        call, ids = (lib().fim_set_mesh_i32, C.c_int32) if narrow else (lib().fim_set_mesh, C.c_int64)
+        _check(call(self.h, xyz.shape[0], _ptr(xyz, C.c_double), tets.shape[0], _ptr(tets, ids), _ptr(at, C.c_int32)),
+               self.h)
+        # (only now: a rejected mesh leaves the previous one, whose size times() needs)
         self.nV = xyz.shape[0]
         self.nT = tets.shape[0]
-        call, ids = (lib().fim_set_mesh_i32, C.c_int32) if narrow else (lib().fim_set_mesh, C.c_int64)
-        _check(call(self.h, self.nV, _ptr(xyz, C.c_double), self.nT, _ptr(tets, ids), _ptr(at, C.c_int32)), self.h)
 
     def set_conduction(self, fib, cf, ct):
         fib = np.ascontiguousarray(fib, dtype=np.float64)

@@ -1212,12 +1212,8 @@ int mlp_gradients(fim_mlp *m, int64_t n, const void *X, const float *tgt, float 
                   const char *who)
 {
   const float b1 = 0.9f, b2 = 0.999f;
-  float c1 = 1.f, c2 = 1.f;
-  if (lr > 0.f) {
-    ++m->steps;
-    c1 = 1.f - std::pow(b1, (float)m->steps);
-    c2 = 1.f - std::pow(b2, (float)m->steps);
-  }
+  const int64_t step = m->steps + (lr > 0.f ? 1 : 0);  // counted once its update has been launched
+  const float c1 = 1.f - std::pow(b1, (float)step), c2 = 1.f - std::pow(b2, (float)step);  // (unused without an update)
   int ctas = 0;
   MLP_TRY(who, mlp_launch(m, (int)n, X, nullptr, tgt, &ctas));
   // the launch of the sums is prepared while the training kernel runs (step of
@@ -1234,6 +1230,7 @@ int mlp_gradients(fim_mlp *m, int64_t n, const void *X, const float *tgt, float 
   cfg.numAttrs = 1;
   MLP_TRY(who, cudaLaunchKernelEx(&cfg, mlp_reduce_kernel, ctas, (const float *)m->part, (int)n, m->G, &m->d_res->loss,
                                   m->P, m->M, m->V, lr, b1, b2, 1e-8f, c1, c2, m->W16T));
+  m->steps = step;
   if (grads)
     MLP_TRY(who, cudaMemcpyAsync(grads, m->G, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->st));
   MLP_TRY(who, cudaStreamSynchronize(m->st));

@@ -248,3 +248,25 @@ def test_features_against_their_definition(F, torch_cuda, cells, offset):
         assert np.allclose(X[:, k], want, rtol=2.0 ** -7, atol=2.0 ** -12), k
     assert np.allclose(X[:, 6], np.arctan2(f[:, 1], f[:, 0]) / np.pi, rtol=0, atol=2.0 ** -8)
     assert (X[:, 7:] == 0).all()
+
+
+def test_a_refused_training_step_counts_for_nothing(F, torch_cuda):
+    """A training step that is refused before anything runs (features off the
+    16-byte boundary of the copies) leaves the network as it was, Adam's step
+    count included: the next step is the first step's bits."""
+    from oracle import mlp_oracle as M
+    torch = torch_cuda
+    n = 128
+    p, X, t = _random_problem(M, n, 8)
+    dX, dt = _to_device_bf16(torch, np.concatenate([X, X[:1]])), torch.from_numpy(t).cuda()
+    got = []
+    for refused in (0, 3):
+        with F.Mlp(seed=3) as mlp:
+            mlp.set_params(p)
+            for _ in range(refused):
+                with pytest.raises(F.FimError):
+                    mlp.train_step(n, dX.data_ptr() + 2, dt.data_ptr(), 1e-2)
+                assert np.array_equal(mlp.get_params(), p)
+            got.append([(mlp.train_step(n, dX.data_ptr(), dt.data_ptr(), 1e-2), mlp.get_params()) for _ in range(2)])
+    for (loss, params), (loss_ref, params_ref) in zip(got[1], got[0]):
+        assert loss == loss_ref and np.array_equal(params, params_ref)

@@ -313,7 +313,8 @@ constexpr int kPartStride = (kMlpParams + 1 + 63) & ~63;
 __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
     const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw1,
     const __grid_constant__ CUtensorMap tw2, const __grid_constant__ CUtensorMap tw3, int M,
-    const float *__restrict__ P, const float *__restrict__ tgt, float *part, volatile unsigned int *err)
+    const float *__restrict__ P, const float *__restrict__ tgt, float *part, unsigned int *bad,
+    volatile unsigned int *err)
 {
   extern __shared__ unsigned char mlp_smem[];
   __shared__ __align__(8) uint64_t wfull, xfull[2], mdone;
@@ -644,6 +645,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   }
   if (t == 0 && (!ok || !wok)) {
     *err = 1u;
+    *bad = 1u;  // this CTA's sums are missing: mlp_reduce_kernel leaves everything as it is
     // copies and MMAs still in flight land before the CTA leaves (bounded)
     (void)mbar_wait(smem_u32(&wfull), 0);
     for (int i = consumed; i < issued; ++i) (void)mbar_wait(x_bar(i), x_par(i));
@@ -876,12 +878,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(
 // Sums of the CTAs' partial gradients, in a fixed order (four threads per
 // parameter take a quarter of the CTAs each), into G; the mean squared error
 // into *loss.  With lr > 0 also Adam (bias-corrected) on every parameter and
-// the BF16 copies of the weight matrices, transposed to [out][in].
+// the BF16 copies of the weight matrices, transposed to [out][in].  Where a
+// CTA's wait ran out (*bad) its sums are missing, and nothing is written.
 constexpr int kRedParams = 64;
 __global__ void __launch_bounds__(4 * kRedParams) mlp_reduce_kernel(int ctas, const float *__restrict__ part, int rows,
                                                                     float *G, float *loss, float *P, float *m, float *v,
                                                                     float lr, float b1, float b2, float eps, float c1,
-                                                                    float c2, __nv_bfloat16 *W16T)
+                                                                    float c2, __nv_bfloat16 *W16T,
+                                                                    const unsigned int *bad)
 {
   __shared__ float s[4][kRedParams];
   const int k = threadIdx.x / kRedParams, l = threadIdx.x % kRedParams;
@@ -890,6 +894,7 @@ __global__ void __launch_bounds__(4 * kRedParams) mlp_reduce_kernel(int ctas, co
   // (launched while the training kernel still runs: it is through, with its
   // writes visible, after this wait)
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  const unsigned int missing = __ldcg(bad);
   float a = 0.f;
   if (i <= kMlpParams) {
 #pragma unroll 8
@@ -897,7 +902,7 @@ __global__ void __launch_bounds__(4 * kRedParams) mlp_reduce_kernel(int ctas, co
   }
   s[k][l] = a;
   __syncthreads();
-  if (k != 0 || i > kMlpParams) return;
+  if (k != 0 || i > kMlpParams || missing != 0u) return;
   const float g = ((s[0][l] + s[1][l]) + s[2][l]) + s[3][l];
   if (i == kMlpParams) {
     *loss = g / (float)rows;
@@ -1145,6 +1150,7 @@ struct fim_mlp {
   __nv_bfloat16 *W16T = nullptr;     // BF16 weights, [out][in]
   CUtensorMap tw1, tw2, tw3;
   float *part = nullptr;             // partial gradients of up to sms CTAs
+  unsigned int *bad = nullptr;       // (behind them) set by a training CTA whose bounded wait ran out
   // mapped host memory: the loss of the last reduction, and a word set by a
   // kernel whose bounded wait ran out (read after the stream has drained)
   struct Result { float loss; unsigned int err; };
@@ -1175,6 +1181,7 @@ int mlp_status(fim_mlp *m, const char *who)
 {
   if (m->h_res->err == 0) return FIM_OK;
   m->h_res->err = 0;
+  MLP_TRY(who, cudaMemsetAsync(m->bad, 0, sizeof *m->bad, m->st));
   std::string msg = std::string(who) + ": a tensor-core GEMM wait ran out (results discarded)";
   set_last_error(msg.c_str());
   return FIM_ERR_TIMEOUT;
@@ -1201,7 +1208,7 @@ cudaError_t mlp_launch(fim_mlp *m, int n, const void *X, float *y, const float *
   if (ctas) *ctas = grid;
   if (tgt)
     mlp_train_kernel<<<grid, kTrainThreads, kTrainSmem, m->st>>>(tx, m->tw1, m->tw2, m->tw3, n, m->P, tgt, m->part,
-                                                                 &m->d_res->err);
+                                                                 m->bad, &m->d_res->err);
   else
     mlp_forward_kernel<<<grid, kFwdThreads, kFwdSmem, m->st>>>(tx, m->tw1, m->tw2, m->tw3, n, m->P, y, &m->d_res->err);
   return cudaGetLastError();
@@ -1212,7 +1219,7 @@ int mlp_gradients(fim_mlp *m, int64_t n, const void *X, const float *tgt, float 
                   const char *who)
 {
   const float b1 = 0.9f, b2 = 0.999f;
-  const int64_t step = m->steps + (lr > 0.f ? 1 : 0);  // counted once its update has been launched
+  const int64_t step = m->steps + (lr > 0.f ? 1 : 0);  // counted once its update is made
   const float c1 = 1.f - std::pow(b1, (float)step), c2 = 1.f - std::pow(b2, (float)step);  // (unused without an update)
   int ctas = 0;
   MLP_TRY(who, mlp_launch(m, (int)n, X, nullptr, tgt, &ctas));
@@ -1229,13 +1236,15 @@ int mlp_gradients(fim_mlp *m, int64_t n, const void *X, const float *tgt, float 
   cfg.attrs = early;
   cfg.numAttrs = 1;
   MLP_TRY(who, cudaLaunchKernelEx(&cfg, mlp_reduce_kernel, ctas, (const float *)m->part, (int)n, m->G, &m->d_res->loss,
-                                  m->P, m->M, m->V, lr, b1, b2, 1e-8f, c1, c2, m->W16T));
-  m->steps = step;
+                                  m->P, m->M, m->V, lr, b1, b2, 1e-8f, c1, c2, m->W16T,
+                                  (const unsigned int *)m->bad));
   if (grads)
     MLP_TRY(who, cudaMemcpyAsync(grads, m->G, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->st));
   MLP_TRY(who, cudaStreamSynchronize(m->st));
   if (loss) *loss = m->h_res->loss;
-  return mlp_status(m, who);
+  const int rc = mlp_status(m, who);
+  if (rc == FIM_OK) m->steps = step;
+  return rc;
 }
 
 }  // namespace
@@ -1264,9 +1273,11 @@ extern "C" int fim_mlp_create(int device, uint64_t seed, fim_mlp **out)
       (e = cudaMalloc(&m->M, sizeof(float) * kMlpParams)) != cudaSuccess ||
       (e = cudaMalloc(&m->V, sizeof(float) * kMlpParams)) != cudaSuccess ||
       (e = cudaMalloc(&m->W16T, sizeof(__nv_bfloat16) * kMlpW16)) != cudaSuccess ||
-      (e = cudaMalloc(&m->part, sizeof(float) * kPartStride * (size_t)m->sms)) != cudaSuccess ||
+      (e = cudaMalloc(&m->part, sizeof(float) * (kPartStride * (size_t)m->sms + 1))) != cudaSuccess ||
       (e = cudaHostAlloc(&h, sizeof(fim_mlp::Result), cudaHostAllocMapped)) != cudaSuccess)
     return fail(mlp_fail("fim_mlp_create", e));
+  m->bad = reinterpret_cast<unsigned int *>(m->part + kPartStride * (size_t)m->sms);
+  if ((e = cudaMemsetAsync(m->bad, 0, sizeof *m->bad, m->st)) != cudaSuccess) return fail(mlp_fail("fim_mlp_create", e));
   m->h_res = static_cast<volatile fim_mlp::Result *>(h);
   m->h_res->loss = 0.f;
   m->h_res->err = 0;
@@ -1356,6 +1367,19 @@ extern "C" int fim_mlp_train_step(fim_mlp *m, int64_t n, const void *d_features,
   if ((rc = mlp_check_n(n, "fim_mlp_train_step")) != FIM_OK) return rc;
   MLP_TRY("fim_mlp_train_step: set device", cudaSetDevice(m->device));
   return mlp_gradients(m, n, d_features, d_targets, lr, nullptr, loss, "fim_mlp_train_step");
+}
+
+// Test hook (not part of include/fim.h): leaves the error words as a training
+// CTA whose wait ran out does, so that the next training call finds them.
+extern "C" int fim_mlp_test_timeout(fim_mlp *m)
+{
+  if (!m) { set_last_error("fim_mlp_test_timeout: NULL argument"); return FIM_ERR_INVALID_ARGUMENT; }
+  MLP_TRY("fim_mlp_test_timeout: set device", cudaSetDevice(m->device));
+  const unsigned int one = 1u;
+  MLP_TRY("fim_mlp_test_timeout", cudaMemcpyAsync(m->bad, &one, sizeof one, cudaMemcpyHostToDevice, m->st));
+  MLP_TRY("fim_mlp_test_timeout", cudaStreamSynchronize(m->st));
+  m->h_res->err = 1;
+  return FIM_OK;
 }
 
 extern "C" int fim_mlp_predict(fim_mlp *m, int64_t n, const void *d_features, float *d_out)

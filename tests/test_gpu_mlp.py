@@ -270,3 +270,36 @@ def test_a_refused_training_step_counts_for_nothing(F, torch_cuda):
             got.append([(mlp.train_step(n, dX.data_ptr(), dt.data_ptr(), 1e-2), mlp.get_params()) for _ in range(2)])
     for (loss, params), (loss_ref, params_ref) in zip(got[1], got[0]):
         assert loss == loss_ref and np.array_equal(params, params_ref)
+
+
+def test_a_training_step_whose_wait_ran_out_changes_nothing(F, torch_cuda):
+    """With the error words as a CTA whose bounded wait ran out leaves them
+    (its sums are missing) the call reports it and parameters, moments and
+    step count stay: the steps after it are those of a network without it."""
+    import ctypes as C
+    from oracle import mlp_oracle as M
+    torch = torch_cuda
+    n = 512
+    p, X, t = _random_problem(M, n, 9)
+    dX, dt = _to_device_bf16(torch, X), torch.from_numpy(t).cuda()
+    timeout = F.lib().fim_mlp_test_timeout
+    timeout.argtypes = [C.c_void_p]
+    got = []
+    for hit in (False, True):
+        with F.Mlp(seed=3) as mlp:
+            mlp.set_params(p)
+            steps = []
+            for i in range(3):
+                if hit:
+                    before = mlp.get_params()
+                    assert timeout(mlp.h) == 0
+                    with pytest.raises(F.FimError) as e:
+                        mlp.train_step(n, dX.data_ptr(), dt.data_ptr(), 1e-2)
+                    assert F.STATUS[e.value.code] == "FIM_ERR_TIMEOUT"
+                    assert np.array_equal(mlp.get_params(), before)
+                steps.append((mlp.train_step(n, dX.data_ptr(), dt.data_ptr(), 1e-2), mlp.get_params()))
+            g, loss = mlp.gradients(n, dX.data_ptr(), dt.data_ptr())
+            steps.append((loss, g))
+            got.append(steps)
+    for (loss, v), (loss_ref, v_ref) in zip(got[1], got[0]):
+        assert loss == loss_ref and np.array_equal(v, v_ref)

@@ -1165,6 +1165,7 @@ namespace {
 
 int mlp_fail(const char *what, cudaError_t e)
 {
+  cudaGetLastError();  // reported here, not again by the next launch's check
   std::string m = std::string(what) + ": " + cudaGetErrorString(e);
   set_last_error(m.c_str());
   return e == cudaErrorMemoryAllocation ? FIM_ERR_OUT_OF_MEMORY : FIM_ERR_CUDA;

@@ -46,8 +46,12 @@ struct DevBuf {
     release();
     if (count == 0) count = 1;
     cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-    if (e == cudaSuccess) n = count;
-    else p = nullptr;
+    if (e == cudaSuccess) {
+      n = count;
+    } else {
+      p = nullptr;
+      cudaGetLastError();  // (the caller's to report: not again by the next launch's check)
+    }
     return e;
   }
   // keeps the buffer when it already holds count elements
@@ -187,6 +191,7 @@ static int set_err(fim_solver *s, int code, const char *fmt, ...)
   do {                                                                                        \
     cudaError_t _e = (call);                                                                  \
     if (_e != cudaSuccess) {                                                                  \
+      cudaGetLastError(); /* reported here, not again by the next launch's check */           \
       return set_err((s), _e == cudaErrorMemoryAllocation ? FIM_ERR_OUT_OF_MEMORY : FIM_ERR_CUDA, \
                      "%s failed: %s (%s:%d)", #call, cudaGetErrorString(_e), __FILE__, __LINE__); \
     }                                                                                         \
@@ -523,10 +528,7 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
   }
   // the edge vectors for the metric kernel (144 B per tet); without room
   // for them the kernel forms them from xyz
-  if (reserve_near(s->evec, (size_t)18 * nT) != cudaSuccess) {
-    cudaGetLastError();
-    s->evec.release();
-  }
+  (void)reserve_near(s->evec, (size_t)18 * nT);
   CUDA_TRY(s, launch_edge_vectors(s->tslots.p, s->xyz.p, nT, s->evec.p, d_ctl, st));
   // corners and neighbourhoods; arrays that are not in use before the first
   // conduction upload or solve serve as scratch

@@ -526,10 +526,6 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
     CUDA_TRY(s, launch_stage_slots(nT, d_tets, d_first, s->tslots.p, st));
     ls.cslots = s->tslots.p;
   }
-  // the edge vectors for the metric kernel (144 B per tet); without room
-  // for them the kernel forms them from xyz
-  (void)reserve_near(s->evec, (size_t)18 * nT);
-  CUDA_TRY(s, launch_edge_vectors(s->tslots.p, s->xyz.p, nT, s->evec.p, d_ctl, st));
   // corners and neighbourhoods; arrays that are not in use before the first
   // conduction upload or solve serve as scratch
   ls.cptr = s->cptr.p; ls.nptr = s->nptr.p; ls.crec = s->crec.p; ls.cidx = s->cidx.p;
@@ -540,14 +536,15 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
   CUDA_TRY(s, launch_stage_lists(nL, nT, ls, d_ctl, st));
   int64_t n_nbr = 0;
   CUDA_TRY(s, cudaMemcpyAsync(&n_nbr, s->nptr.p + nL, sizeof n_nbr, cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(s, cudaMemcpyAsync(&h, d_ctl, sizeof h, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(s, cudaStreamSynchronize(st));
   CUDA_TRY(s, reserve_near(s->nbr, (size_t)n_nbr));
   CUDA_TRY(s, launch_stage_compact(nL, ls, s->nbr.p, st));
-  // reference front width: 1.01 * longest edge / 0.6 (compute_dwf, cuda_fim.h:1536-1576)
-  double maxe2;
-  std::memcpy(&maxe2, &h.max_edge2, sizeof maxe2);
-  s->front_width = 1.01 * std::sqrt(maxe2) / 0.6;
+  // the edge vectors for the metric kernel (144 B per tet), after everything
+  // that a mesh cannot do without: where they find no room the metric kernel
+  // forms them from xyz
+  (void)reserve_near(s->evec, (size_t)18 * nT);
+  CUDA_TRY(s, launch_edge_vectors(s->tslots.p, s->xyz.p, nT, s->evec.p, d_ctl, st));
+  CUDA_TRY(s, cudaMemcpyAsync(&h, d_ctl, sizeof h, cudaMemcpyDeviceToHost, st));
   // vertices in at least one tet (seeds elsewhere are dropped, as the
   // reference seeds through submeshes only)
   s->in_tet.resize(nV);
@@ -558,6 +555,10 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
     CUDA_TRY(s, cudaMemcpyAsync(s->in_tet.data(), s->dec.p, nV, cudaMemcpyDeviceToHost, st));
   }
   CUDA_TRY(s, cudaStreamSynchronize(st));
+  // reference front width: 1.01 * longest edge / 0.6 (compute_dwf, cuda_fim.h:1536-1576)
+  double maxe2;
+  std::memcpy(&maxe2, &h.max_edge2, sizeof maxe2);
+  s->front_width = 1.01 * std::sqrt(maxe2) / 0.6;
   s->stats.n_corners = nC;
   s->have_mesh = true;
   return FIM_OK;

@@ -119,3 +119,20 @@ def test_a_failed_allocation_is_reported_once(L):
         s.solve(nV, nT)
         s.times(nV)
         assert s.set_mesh(small) == 0, L.fim_last_error(s.h)
+
+
+@pytest.mark.parametrize("tagged", [False, True])
+@pytest.mark.parametrize("short", ["evec", "nbr"])
+def test_edge_vectors_give_way(L, tagged, short):
+    """The edge vectors are optional: a mesh for which they leave no room, or
+    which leaves none for them, is staged without them, with the same lists."""
+    m = mesh((7, 5, 4), tagged=tagged)
+    with Solver(L) as s:
+        assert s.set_mesh(m) == 0
+        want, need = s.lists(), [s.bytes(k) for k in range(4)]
+    assert need[EVEC] == 144 * len(m[1])
+    with Solver(L) as s:
+        # all but one byte of what everything takes, and all but the edge vectors
+        s.room(sum(need) - 1 if short == "evec" else sum(need) - need[EVEC])
+        assert s.set_mesh(m) == 0, L.fim_last_error(s.h)
+        assert s.bytes(EVEC) == 0 and s.lists() == want

@@ -415,6 +415,23 @@ struct Parts {
   }
 };
 
+// launch_stage_check on the host: the first offenders of a mesh.
+template <typename Id>
+StageCtl host_check(int64_t nV, int64_t nT, const Id *tets, const double *xyz)
+{
+  StageCtl h{~0ull, ~0ull, ~0ull, 0, 0, 0};
+  for (int64_t i = 0; i < 4 * nT && h.bad_id == ~0ull; ++i)
+    if (tets[i] < 0 || tets[i] >= nV) h.bad_id = (unsigned long long)i;
+  for (int64_t e = 0; e < nT && h.bad_tet == ~0ull; ++e) {
+    const Id *t = tets + 4 * e;
+    if (t[0] == t[1] || t[0] == t[2] || t[0] == t[3] || t[1] == t[2] || t[1] == t[3] || t[2] == t[3])
+      h.bad_tet = (unsigned long long)e;
+  }
+  for (int64_t i = 0; i < 3 * nV && h.bad_xyz == ~0ull; ++i)
+    if (!std::isfinite(xyz[i])) h.bad_xyz = (unsigned long long)i;
+  return h;
+}
+
 }  // namespace
 
 // Mesh of ids of 64 or 32 bits.
@@ -435,8 +452,14 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
   // Staging buffer: control words, tets, coordinates, first appearances.
   const auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t o_tets = up(sizeof(StageCtl)), o_xyz = o_tets + up(sizeof(Id) * 4 * nT);
-  const size_t o_first = o_xyz + up(sizeof(double) * 3 * nV);
-  CUDA_TRY(s, s->stage.reserve(o_first + up(sizeof(uint32_t) * nV)));
+  const size_t o_first = o_xyz + up(sizeof(double) * 3 * nV), stage_bytes = o_first + up(sizeof(uint32_t) * nV);
+  // (where it finds no room, even without the edge vectors, the mesh is
+  // checked here and staged from inside its own arrays)
+  bool staged = s->stage.reserve(stage_bytes) == cudaSuccess;
+  if (!staged && s->evec.p) {
+    s->evec.release();
+    staged = s->stage.reserve(stage_bytes) == cudaSuccess;
+  }
   struct StageGuard {  // a large staging buffer is given back when the call ends
     DevBuf<unsigned char> &b;
     ~StageGuard() { if (b.n > (size_t(64) << 20)) b.release(); }
@@ -445,12 +468,20 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
   Id *d_tets = reinterpret_cast<Id *>(s->stage.p + o_tets);
   double *d_xyz = reinterpret_cast<double *>(s->stage.p + o_xyz);
   uint32_t *d_first = reinterpret_cast<uint32_t *>(s->stage.p + o_first);
-  CUDA_TRY(s, cudaMemcpyAsync(d_tets, tets, sizeof(Id) * 4 * nT, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(s, cudaMemcpyAsync(d_xyz, xyz, sizeof(double) * 3 * nV, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(s, launch_stage_check(nV, nT, d_tets, d_xyz, d_first, d_ctl, st));
+  const auto upload = [&](bool first) {
+    cudaError_t e = cudaMemcpyAsync(d_tets, tets, sizeof(Id) * 4 * nT, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_xyz, xyz, sizeof(double) * 3 * nV, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = launch_stage_check(nV, nT, d_tets, d_xyz, first ? d_first : nullptr, d_ctl, st);
+    return e;
+  };
   StageCtl h{};
-  CUDA_TRY(s, cudaMemcpyAsync(&h, d_ctl, sizeof h, cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(s, cudaStreamSynchronize(st));
+  if (staged) {
+    CUDA_TRY(s, upload(true));
+    CUDA_TRY(s, cudaMemcpyAsync(&h, d_ctl, sizeof h, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(s, cudaStreamSynchronize(st));
+  } else {
+    h = host_check(nV, nT, tets, xyz);
+  }
   if (h.bad_id != ~0ull)
     return set_err(s, FIM_ERR_INVALID_ARGUMENT, "fim_set_mesh: tet %lld has vertex %lld outside [0,%lld)",
                    (long long)(h.bad_id / 4), (long long)tets[h.bad_id], (long long)nV);
@@ -509,10 +540,41 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
     return a.off;
   };
   s->gptr.release(); s->gcopy.release(); s->phi_out.release(); s->st_out.release();
-  CUDA_TRY(s, reserve_near(s->arena, parts(nullptr)));
+  // What a mesh cannot do without comes before what is left of the previous
+  // one, before the staging buffer, and both before the edge vectors.
+  const auto free_stage = [&]() {
+    if (!staged) return false;
+    s->stage.release();
+    staged = false;
+    return true;
+  };
+  const size_t arena_bytes = parts(nullptr);
+  cudaError_t e = reserve_near(s->arena, arena_bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    s->nbr.release();
+    s->evec.release();
+    e = reserve_near(s->arena, arena_bytes);
+  }
+  if (e == cudaErrorMemoryAllocation && free_stage()) e = reserve_near(s->arena, arena_bytes);
+  CUDA_TRY(s, e);
   parts(s->arena.p);
-
-  CUDA_TRY(s, cudaMemcpyAsync(s->xyz.p, d_xyz, sizeof(double) * 3 * nV, cudaMemcpyDeviceToDevice, st));
+  // The control words' and the ids' place without a staging buffer: arrays
+  // that are not in use yet (fib and phi until after this call; of cgeo, 192 B
+  // per tet, launch_stage_lists overwrites the first 64).
+  const auto place_in_arena = [&]() {
+    static_assert(sizeof(StageCtl) <= 256, "the smallest part of an arena");
+    static_assert(kCgeoStride * 4 * sizeof(double) >= 16 * sizeof(int32_t) + 4 * sizeof(int64_t), "room beside scratch");
+    d_ctl = reinterpret_cast<StageCtl *>(s->fib.p);
+    d_tets = reinterpret_cast<Id *>(s->cgeo.p + 8 * nT);
+    d_xyz = s->xyz.p;
+    d_first = reinterpret_cast<uint32_t *>(s->phi.p);
+  };
+  if (staged) {
+    CUDA_TRY(s, cudaMemcpyAsync(s->xyz.p, d_xyz, sizeof(double) * 3 * nV, cudaMemcpyDeviceToDevice, st));
+  } else {
+    place_in_arena();
+    CUDA_TRY(s, upload(!multi));  // (with tags phi may be shorter than the vertices; the host has numbered them)
+  }
   StageLists ls{};
   if (multi) {
     // (the tets on the device have served their purpose: the copies' slots
@@ -537,12 +599,24 @@ static int set_mesh(fim_solver *s, int64_t nV, const double *xyz, int64_t nT, co
   int64_t n_nbr = 0;
   CUDA_TRY(s, cudaMemcpyAsync(&n_nbr, s->nptr.p + nL, sizeof n_nbr, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(s, cudaStreamSynchronize(st));
-  CUDA_TRY(s, reserve_near(s->nbr, (size_t)n_nbr));
+  const auto leave_stage = [&]() {  // gives the staging buffer up: only its control words are still needed
+    if (!free_stage()) return false;
+    place_in_arena();
+    e = cudaMemsetAsync(d_ctl, 0, sizeof(StageCtl), st);
+    return e == cudaSuccess;
+  };
+  if (reserve_near(s->nbr, (size_t)n_nbr) != cudaSuccess) {
+    s->evec.release();
+    if (reserve_near(s->nbr, (size_t)n_nbr) != cudaSuccess) {
+      leave_stage();
+      CUDA_TRY(s, reserve_near(s->nbr, (size_t)n_nbr));
+    }
+  }
   CUDA_TRY(s, launch_stage_compact(nL, ls, s->nbr.p, st));
   // the edge vectors for the metric kernel (144 B per tet), after everything
   // that a mesh cannot do without: where they find no room the metric kernel
   // forms them from xyz
-  (void)reserve_near(s->evec, (size_t)18 * nT);
+  if (reserve_near(s->evec, (size_t)18 * nT) != cudaSuccess && leave_stage()) (void)reserve_near(s->evec, (size_t)18 * nT);
   CUDA_TRY(s, launch_edge_vectors(s->tslots.p, s->xyz.p, nT, s->evec.p, d_ctl, st));
   CUDA_TRY(s, cudaMemcpyAsync(&h, d_ctl, sizeof h, cudaMemcpyDeviceToHost, st));
   // vertices in at least one tet (seeds elsewhere are dropped, as the

@@ -134,6 +134,9 @@ constexpr int kDagWarpsMax = 12;
 
 // Records the message returned by fim_last_error(NULL) on this thread.
 void set_last_error(const char *msg);
+// Whether kernels on the device may read and write p: its own memory, or
+// managed.  Memory of another device needs a copy.
+bool on_device(const void *p, int device);
 
 // ---- kernels (fim_kernels.cu) ----
 // FP64 metric + edge norms of tets [e0, e1) scattered into the corner

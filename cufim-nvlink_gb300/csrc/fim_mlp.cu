@@ -1390,10 +1390,10 @@ extern "C" int fim_mlp_predict(fim_mlp *m, int64_t n, const void *d_features, fl
   if ((rc = mlp_check_n(n, "fim_mlp_predict")) != FIM_OK) return rc;
   MLP_TRY("fim_mlp_predict: set device", cudaSetDevice(m->device));
   // The kernel writes the predictions in place unless d_out is not aligned
-  // to a float or overlaps the features it still reads.
+  // to a float, overlaps the features it still reads, or is not on the device.
   const uintptr_t x = reinterpret_cast<uintptr_t>(d_features), o = reinterpret_cast<uintptr_t>(d_out);
   const uintptr_t xn = sizeof(__nv_bfloat16) * kMlpIn * (uintptr_t)n, on = sizeof(float) * (uintptr_t)n;
-  const bool direct = o % sizeof(float) == 0 && (o + on <= x || x + xn <= o);
+  const bool direct = o % sizeof(float) == 0 && (o + on <= x || x + xn <= o) && on_device(d_out, m->device);
   if (!direct && n > m->y_cap) {
     cudaFree(m->y);
     m->y = nullptr;

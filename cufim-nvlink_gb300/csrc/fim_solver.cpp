@@ -90,6 +90,16 @@ cudaError_t reserve_near(DevBuf<T> &b, size_t count)
 
 void fimgb::set_last_error(const char *msg) { g_last_error = msg; }
 
+bool fimgb::on_device(const void *p, int device)
+{
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeDevice && a.device == device);
+}
+
 // fim_set_conduction uploads the field in up to kCondChunks pieces of at
 // least kCondChunkMin tets.
 constexpr int kCondChunks = 8;
@@ -678,12 +688,15 @@ static int run_metric(fim_solver *s, const double *fib, const double *cf, const 
     if (e == cudaSuccess) e = cudaMemcpyAsync(s->ct.p + e0, ct + e0, sizeof(double) * (e1 - e0), kind, cs);
     return e;
   };
-  const auto aligned = [](const double *p) { return reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0; };
-  if (!host && aligned(fib) && aligned(cf) && aligned(ct)) {
+  const auto readable = [s](const double *p) {
+    return reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0 && on_device(p, s->device);
+  };
+  if (!host && readable(fib) && readable(cf) && readable(ct)) {
     // a field on the device: one launch reads it where it is, beside the
     // copies that the solver keeps (each of several chunked launches ends in
     // a partial wave).  Like the copies it starts after the copy stream's
-    // implicit wait for the legacy default stream.
+    // implicit wait for the legacy default stream.  (Memory elsewhere, on
+    // another device say, is within the copies' reach only.)
     CUDA_TRY(s, cudaEventRecord(s->ev_chunk[0], cs));
     CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_chunk[0], 0));
     CUDA_TRY(s, cudaEventRecord(s->ev0, s->stream));

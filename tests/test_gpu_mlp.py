@@ -303,3 +303,19 @@ def test_a_training_step_whose_wait_ran_out_changes_nothing(F, torch_cuda):
             got.append(steps)
     for (loss, v), (loss_ref, v_ref) in zip(got[1], got[0]):
         assert loss == loss_ref and np.array_equal(v, v_ref)
+
+
+def test_prediction_into_pinned_host_memory(F, torch_cuda):
+    """Outputs that are not on the device take the copy too."""
+    from oracle import mlp_oracle as M
+    torch = torch_cuda
+    n = 1024
+    p, X, _ = _random_problem(M, n, 10)
+    with F.Mlp(seed=3) as mlp:
+        mlp.set_params(p)
+        dX = _to_device_bf16(torch, X)
+        y = torch.empty(n, dtype=torch.float32, device="cuda")
+        h = torch.empty(n, dtype=torch.float32).pin_memory()
+        mlp.predict(n, dX.data_ptr(), y.data_ptr())
+        mlp.predict(n, dX.data_ptr(), h.data_ptr())
+        assert np.array_equal(h.numpy(), y.cpu().numpy())

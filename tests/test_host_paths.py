@@ -195,3 +195,17 @@ def test_a_larger_mesh_replaces_a_smaller_one(L):
         assert s.set_mesh(a) == 0 and s.bytes(EVEC) > 0 and s.bytes(STAGE) > 0
         assert s.set_mesh(b) == 0, L.fim_last_error(s.h)
         assert s.lists() == want
+
+
+@pytest.mark.parametrize("device,in_place", [(0, True), (1, False)])
+def test_a_field_on_another_device_is_copied(L, device, in_place):
+    """The metric kernel reads a field where it is only on the solver's own
+    device; from another one it goes through the copies."""
+    m = mesh((4, 3, 2))
+    with Solver(L) as s:
+        assert s.set_mesh(m) == 0
+        fib, cf = np.ones(3 * len(m[1])), np.ones(len(m[1]))
+        L.fake_other_device(device)
+        rc = L.fim_set_conduction_device(s.h, ptr(fib), ptr(cf), ptr(cf))
+        L.fake_other_device(0)
+        assert rc == 0 and bool(L.fake_metric_reads(ptr(fib))) == in_place

@@ -1258,17 +1258,20 @@ extern "C" int fim_get_times(fim_solver *s, double *phi, int32_t *state)
   const uint8_t *dst = s->st_out.p ? s->st_out.p : s->st.p;
   if (phi) CUDA_TRY(s, cudaMemcpyAsync(phi, dphi, sizeof(double) * s->nV, cudaMemcpyDeviceToHost, s->stream));
   // states: above 16,384 vertices widened to 32 bits on the device, through a
-  // vertex list of the solve, which is free until the next one (with tags and
-  // vertices in no tet it may be shorter than the vertices); below, bytes
+  // vertex list of the solve, which is free until the next one; below, bytes
   // widened here, since copies of up to 64 KB to pageable memory take another,
   // slower way (times() of 9k vertices 33 us this way, 47 the other; 18k 37
-  // and 34, 87k 66 and 41, 1M 435 and 119)
+  // and 34, 87k 66 and 41, 1M 435 and 119).  With tags and vertices in no tet
+  // the list may be shorter than the vertices: then in pieces of at least
+  // 32,768 (a piece costs 10 us, as much as widening that many saves), else
+  // the bytes too (1M vertices, 120 copies: 71 ms in pieces, 0.41 as bytes;
+  // 8,463 copies: 1.45 and 0.41)
   std::vector<uint8_t> st8;
-  if (state && s->nV <= 16384) {
+  const int64_t step = s->nL & ~int64_t(3);
+  if (state && (s->nV <= 16384 || (s->nV > step && step < 32768))) {
     st8.resize(s->nV);
     CUDA_TRY(s, cudaMemcpyAsync(st8.data(), dst, s->nV, cudaMemcpyDeviceToHost, s->stream));
   } else if (state) {
-    const int64_t step = s->nL & ~int64_t(3);
     for (int64_t v = 0; v < s->nV; v += step) {
       const int64_t n = std::min(step, s->nV - v);
       CUDA_TRY(s, launch_widen(dst + v, s->list0.p, n, s->stream));

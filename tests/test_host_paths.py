@@ -209,3 +209,19 @@ def test_a_field_on_another_device_is_copied(L, device, in_place):
         rc = L.fim_set_conduction_device(s.h, ptr(fib), ptr(cf), ptr(cf))
         L.fake_other_device(0)
         assert rc == 0 and bool(L.fake_metric_reads(ptr(fib))) == in_place
+
+
+@pytest.mark.parametrize("nV", [16384, 16385, 60000, 140000])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (12, 10, 8), (30, 20, 12), (40, 30, 25)])
+def test_states_of_a_few_tagged_tets_among_many_vertices(L, cells, nV):
+    """States are read back in a few copies, however short the vertex lists
+    are that the states are widened through."""
+    xyz, tets, tags = mesh(cells, tagged=True)
+    nV = max(nV, len(xyz))
+    m = (np.concatenate([xyz, np.ones((nV - len(xyz), 3))]), tets, tags)
+    with Solver(L) as s:
+        assert s.set_mesh(m) == 0
+        s.solve(nV, len(tets))
+        L.fake_d2h()
+        s.times(nV)
+        assert L.fake_d2h() <= 5

@@ -319,3 +319,33 @@ def test_prediction_into_pinned_host_memory(F, torch_cuda):
         mlp.predict(n, dX.data_ptr(), y.data_ptr())
         mlp.predict(n, dX.data_ptr(), h.data_ptr())
         assert np.array_equal(h.numpy(), y.cpu().numpy())
+
+
+@pytest.mark.parametrize("tiles", [153, 305, 608, 609])
+def test_every_row_of_the_last_tiles(F, torch_cuda, tiles):
+    """Tiles in rounds of 304 (two groups of 152 CTAs) or, in training, 152,
+    the last one half full: every row's prediction within the bounds of the
+    others, twice the same bits, and the gradients of a loss that lies in the
+    last tile's rows."""
+    from oracle import mlp_oracle as M
+    torch = torch_cuda
+    n = 128 * tiles - 64
+    p, X, _ = _random_problem(M, n, 12)
+    _, _, _, y_o = M.forward(p, X)
+    t = (y_o + 0.01).astype(np.float32)
+    t[-64:] += np.linspace(-30.0, 30.0, 64).astype(np.float32)
+    with F.Mlp(seed=3) as mlp:
+        mlp.set_params(p)
+        dX, dt = _to_device_bf16(torch, X), torch.from_numpy(t).cuda()
+        ys = [torch.full((n + 1,), 7.0, dtype=torch.float32, device="cuda") for _ in range(2)]
+        for y in ys:
+            mlp.predict(n, dX.data_ptr(), y.data_ptr())
+        g, loss = mlp.gradients(n, dX.data_ptr(), dt.data_ptr())
+    yg = ys[0].cpu().numpy()
+    assert yg[n] == 7.0 and np.array_equal(yg, ys[1].cpu().numpy())
+    assert np.abs(yg[:n] - y_o).max() < 0.05 * np.abs(y_o).max()
+    loss_o, g_o = M.loss_and_gradients(p, X, t)
+    assert abs(loss - loss_o) <= 1e-3 * abs(loss_o)
+    for name, (a, b) in M.BLOCKS.items():
+        err = np.linalg.norm(g[a:b] - g_o[a:b]) / max(np.linalg.norm(g_o[a:b]), 1e-12)
+        assert err < 1e-2, (name, err)

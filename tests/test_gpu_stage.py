@@ -163,3 +163,16 @@ def test_states_of_vertices_in_no_tet(F, extra):
         assert np.array_equal(got[1][0][:n], got[0][0]) and np.array_equal(got[1][1][:n], got[0][1])
         assert (got[1][1][n:] == F.FAR).all() and (got[1][0][n:] > 1e300).all()
         assert len(np.unique(got[0][1])) >= 1 and got[0][1].min() >= 0
+
+
+@pytest.mark.parametrize("extra", [0, 3, 16387])
+def test_states_are_the_oracles(F, O, extra):
+    """States of a mesh with vertices in no tet, read back as bytes and widened
+    on the device: the oracle's, far for those."""
+    import fim_mesh
+    xyz, tets = fim_mesh.kuhn_box(5, 4, 3, 1.0, 0.8, 0.6, seed=3)
+    c = case_of(np.concatenate([xyz, np.full((extra, 3), 9.0)]), np.asarray(tets, dtype=np.int64))
+    with F.Solver() as s:
+        check(F, O, s, c)
+        st = s.times()[1]
+    assert set(np.unique(st[:len(xyz)])) == {F.FROZEN} and (st[len(xyz):] == F.FAR).all()

@@ -888,13 +888,16 @@ __global__ void __launch_bounds__(4 * kRedParams) mlp_reduce_kernel(int ctas, co
                                                                     const unsigned int *bad)
 {
   __shared__ float s[4][kRedParams];
+  __shared__ unsigned int s_bad;
   const int k = threadIdx.x / kRedParams, l = threadIdx.x % kRedParams;
   const int i = blockIdx.x * kRedParams + l;  // < kPartStride
   const int lo = ctas * k / 4, hi = ctas * (k + 1) / 4;
   // (launched while the training kernel still runs: it is through, with its
   // writes visible, after this wait)
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const unsigned int missing = __ldcg(bad);
+  // (one load per block: every warp's of the same word queued up in one slice
+  // of the L2, half a microsecond of a training step)
+  if (threadIdx.x == 4 * kRedParams - 1) s_bad = __ldcg(bad);
   float a = 0.f;
   if (i <= kMlpParams) {
 #pragma unroll 8
@@ -902,7 +905,7 @@ __global__ void __launch_bounds__(4 * kRedParams) mlp_reduce_kernel(int ctas, co
   }
   s[k][l] = a;
   __syncthreads();
-  if (k != 0 || i > kMlpParams || missing != 0u) return;
+  if (k != 0 || i > kMlpParams || s_bad != 0u) return;
   const float g = ((s[0][l] + s[1][l]) + s[2][l]) + s[3][l];
   if (i == kMlpParams) {
     *loss = g / (float)rows;

@@ -600,7 +600,7 @@ def run_mlp(args):
     rows; one kernel for all layers) and training steps of 4,096 rows
     (forward, backward with the weight gradients, Adam).  Features and targets are seeded synthetic values.
     Each call synchronises its stream, so the times are host wall-clock
-    around the call; the GEMM kernels' own durations come from ncu."""
+    around the call; the kernels' own durations come from ncu."""
     import torch
     import fim_api
     torch.cuda.set_device(0)

@@ -270,6 +270,7 @@ __device__ __forceinline__ CandBound tet_screen_t(const float *gv, float p1f, fl
   r.ub = ub;
   return r;
 }
+// (with branches: the self-test's second opinion; the solve runs the other)
 __device__ __forceinline__ CandBound tet_screen(const float *gv, float p1f, float p2f, float p3f, int k,
                                                 int *why = nullptr)
 {

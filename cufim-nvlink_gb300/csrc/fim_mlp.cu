@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) mlp_train_kernel(
   };
   const uint32_t tv = tmem + ((uint32_t)(q * 32) << 16);
   const int r = q * 32 + lane;  // this thread's row of the tile
-  // 64 columns of the row: from the accumulator, and where they lie in an activation block
+  // kCols columns of the row: from the accumulator, and where they lie in an activation block
   const auto load_acc = [&](uint32_t *v) { tmem_ld32(tv + kCols * h, v); };
   const auto chunk_ptr = [&](uint32_t base, int c) {  // 16-byte chunk c, at chunk c ^ (row % 8)
     return reinterpret_cast<uint4 *>(sm + (base - w1) + (uint32_t)(h >> 1) * kBlkBytes + (uint32_t)r * 128u +

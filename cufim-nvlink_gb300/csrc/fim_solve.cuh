@@ -159,7 +159,7 @@ struct BatchSh {
       alignas(16) float lbv[kCornerCap][4];  // lower bounds of the triangle pairs (1,2), (2,3), (1,3) and the tet (+inf: not valid)
       float elo[kCornerCap];        // smallest lower bound of the corner's valid edges (+inf: none)
     };
-    double dag[kDagGroups][kDagStride];  // phase D (where pf and sf are dead): scratch of the tet prefix groups
+    double dag[kDagGroups][kDagStride];  // phase D (where the arrays above are dead): scratch of the tet prefix groups
   };
   uint8_t vm[kCornerCap];           // validity bits of the three neighbours
   uint8_t cs[kCornerCap];           // slot of the corner's vertex
@@ -493,9 +493,9 @@ struct ListOut {
   bool local;         // the list is this block's own (submesh sweeps): no split over the grid
 };
 
-// One update phase over a vertex list.  Every block takes a contiguous part
-// of the list and processes it in batches of up to kSlots vertices / up to
-// kCornerCap corners, the corners of a batch spread over all threads:
+// One update phase over a vertex list.  Every block takes every gridDim.x-th
+// vertex of the list and processes them in batches of up to kSlots vertices /
+// up to kCornerCap corners, the corners of a batch spread over all threads:
 //  A -- load every corner's first-read record once (neighbour ids, float
 //       edge lengths, fp16 root-term bounds) and its neighbours' states and
 //       float times; validity of the neighbours (state >= narrow and

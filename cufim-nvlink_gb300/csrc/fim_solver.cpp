@@ -1,7 +1,7 @@
 // fim_solver.cpp -- C ABI of the GB300 FIM solver (include/fim.h): solver
-// objects, mesh staging on the host, device buffers and launches.
+// objects, mesh staging, device buffers and launches.
 //
-// Host staging replaces the reference's CudaSolverFIM constructor
+// Staging replaces the reference's CudaSolverFIM constructor
 // (src/eikonal/cuda_fim.cu:1218-1501): instead of per-submesh blobs with
 // in-blob pointers it builds flat device arrays (on the device, fim_stage.cu;
 // only the vertex copies of a mesh with submesh tags are numbered here) --

@@ -114,7 +114,7 @@ int fim_set_mesh(fim_solver *s, int64_t n_vertices, const double *xyz, int64_t n
  * succeeds. */
 int fim_set_conduction(fim_solver *s, const double *fib, const double *cf, const double *ct);
 /* Same, with device pointers (already resident in HBM on the solver's
- * device), with the same check. */
+ * device; a field elsewhere is copied first), with the same check. */
 int fim_set_conduction_device(fim_solver *s, const double *d_fib, const double *d_cf,
                               const double *d_ct);
 
@@ -303,7 +303,8 @@ int fim_mlp_gradients(fim_mlp *m, int64_t n, const void *d_features, const float
 /* One Adam step on those n rows (learning rate lr); loss before the step. */
 int fim_mlp_train_step(fim_mlp *m, int64_t n, const void *d_features, const float *d_targets, float lr,
                        float *loss);
-/* Predictions (device, FP32 [n]) for n feature rows. */
+/* Predictions (device, FP32 [n]) for n feature rows; into memory that is not
+ * on the network's device they are copied. */
 int fim_mlp_predict(fim_mlp *m, int64_t n, const void *d_features, float *d_out);
 /* Feature rows (device, BF16 [n_vertices x FIM_MLP_INPUTS]) of the solver's
  * mesh, conduction and stimuli (one submesh); *time_scale receives the

@@ -23,7 +23,7 @@ def L(tmp_path_factory):
     src = os.path.join(PKG, "csrc", "fim_solver.cpp")
     subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wall", "-Wno-subobject-linkage", "-I" + os.path.join(cuda, "include"),
                            f'-DFIM_SOLVER_CPP="{src}"', os.path.join(ROOT, "tests", "fake_cuda.cpp"), "-o", out,
-                           "-Wl,--no-undefined"])
+                           "-Wl,--no-undefined,-Bsymbolic"])  # (its own runtime, not one that torch has loaded)
     lib = C.CDLL(out)
     vp, i64, sz = C.c_void_p, C.c_int64, C.c_size_t
     lib.fim_create.argtypes = [vp, C.POINTER(vp)]
